@@ -5,7 +5,7 @@
  * throws; tlgb_last_error() gives the message of the last failing call made
  * on the calling host thread. All device pointers are raw CUDA device memory;
  * every launch goes on the given stream and no call synchronises the device,
- * except tlgb_interp_plan_build (it reads the bin histogram back once) and
+ * except tlgb_interp_plan_build (it reads the lists' lengths back once) and
  * tlgb_index_plan_build (it reads its bounds check back once).
  *
  * Reference interfaces each entry replaces (paths in the torchlinops source):
@@ -138,7 +138,8 @@ int tlgb_interp_plan_size(const tlgb_interp_desc* d, size_t* plan_bytes, size_t*
 
 /* Bin the points: sort (point, tile) pairs by output tile (stable, so points
  * keep their original order inside a tile) and cut the work into items of at
- * most `chunk` pairs. Synchronises `stream` once to size the work lists. */
+ * most `chunk` pairs. Everything is built on the device; `stream` is
+ * synchronised once, at the end, to read the lists' lengths into `info`. */
 int tlgb_interp_plan_build(const tlgb_interp_desc* d, const float* locs, void* plan, size_t plan_bytes,
                            void* tmp, size_t tmp_bytes, tlgb_interp_plan_info* info, tlgb_stream_t stream);
 

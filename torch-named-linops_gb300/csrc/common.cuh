@@ -55,10 +55,27 @@ int64_t scan_scratch_len(int64_t n);
 int exclusive_scan_u32(const uint32_t* in, uint32_t* out, int64_t n, uint32_t* total_dev, uint32_t* scratch,
                        cudaStream_t s);
 
-// Stable LSD radix sort of (key, val) pairs by the low `bits` bits of key.
-// keys/vals are sorted in place; keys_tmp/vals_tmp are ping-pong buffers of
-// the same length; counts_tmp needs radix_counts_len(n) uint32 entries.
+// Stable LSD radix sort of (key, val) pairs by the low `bits` bits of key, in
+// radix_passes(bits) passes of at most 9 bits. A job's pairs start in
+// keys[0] / vals[0] and end in keys[passes & 1] / vals[passes & 1], where
+// passes is the largest of the jobs' radix_passes; up to two jobs (two
+// independent lists) share the launches. The number of pairs is read from
+// device memory (`n`, at most n_max), so a list whose length only the device
+// knows is sorted without a copy back; n == nullptr sorts n_max pairs.
+// `counts` holds radix_counts_len(n_max) uint32.
+struct SortJob {
+  uint32_t* keys[2];
+  int32_t* vals[2];
+  uint32_t* counts;
+  const uint32_t* n;
+  int64_t n_max;
+  int bits;
+};
+int radix_passes(int bits);
 int64_t radix_counts_len(int64_t n);
+int radix_sort_jobs(const SortJob* jobs, int njobs, cudaStream_t s);
+// One list of host-known length, sorted in place (keys_tmp / vals_tmp: the
+// other halves of the ping-pong).
 int radix_sort_pairs(uint32_t* keys, int32_t* vals, uint32_t* keys_tmp, int32_t* vals_tmp,
                      uint32_t* counts_tmp, int64_t n, int bits, cudaStream_t s);
 

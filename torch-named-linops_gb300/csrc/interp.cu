@@ -55,6 +55,7 @@ struct Geo {
   int ndim;
   int N[3];   // internal dims (x, y, z); leading inactive dims have N = 1
   int T[3];   // tile edge
+  int lgT[3]; // log2 of the tile edge, -1 when it is no power of two
   int nt[3];  // tiles per dim
   int NT[3];  // taps per dim (inactive: 1)
   float r[3]; // kernel radius W/2 per dim
@@ -67,6 +68,7 @@ struct Geo {
   int wrap_safe;  // every active N >= NT: a window never overlaps itself
   long long tv_off;  // gridding: byte offset in scratch of the point-major values, -1 = none
   int skip_copy;     // test hook (tlgb_test_skip_region_copy): TMA kernels skip their region copy
+  int nrow;          // block lists: blocks a window can meet per dim (2 or 3), 0 = no block lists
 };
 
 // ---------------------------------------------------------------- kernels math
@@ -155,31 +157,11 @@ __device__ __forceinline__ float load_coord(const Geo& g, const float* locs, lon
   return __ldg(locs + p * g.ndim + (e - (3 - g.ndim)));
 }
 
-// Valid tap range [s, s+n) of one dim for one point (sequential; used by the plan).
-__device__ __forceinline__ bool axis_range(const Geo& g, const float* locs, long long p, int e, int& start, int& n) {
-  if (!g.act[e]) {
-    start = 0;
-    n = 1;
-    return true;
-  }
-  const float x = load_coord(g, locs, p, e);
-  if (!coord_ok(x)) return false;
-  const int lower = lower_of(g, e, x);
-  int s = -1;
-  n = 0;
-  for (int k = 0; k < g.NT[e]; ++k) {
-    if (tap_eval(g, e, x, lower, k).valid) {
-      if (s < 0) s = k;
-      ++n;
-    }
-  }
-  if (n == 0) return false;
-  start = lower + s;
-  if (g.pad == TLGB_PAD_CIRCULAR) start = wrapi(start, g.N[e]);
-  return true;
-}
-
 // --------------------------------------------------------------------- plan
+
+__device__ __forceinline__ int tile_of(const Geo& g, int e, int v) {
+  return g.lgT[e] >= 0 ? v >> g.lgT[e] : v / g.T[e];
+}
 
 // Distinct tiles touched along one dim by taps start .. start+n-1 (wrapped);
 // the first is the home tile. At most 3 (a window crossing a ragged last tile
@@ -189,54 +171,12 @@ __device__ __forceinline__ int axis_tiles(const Geo& g, int e, int start, int n,
   for (int k = 0; k < n; ++k) {
     int v = start + k;
     if (g.pad == TLGB_PAD_CIRCULAR) v = wrapi(v, g.N[e]);
-    const int t = v / g.T[e];
+    const int t = tile_of(g, e, v);
     bool seen = false;
     for (int i = 0; i < cnt; ++i) seen = seen || (tl[i] == t);
     if (!seen && cnt < 3) tl[cnt++] = t;
   }
   return cnt;
-}
-
-__global__ void plan_count_kernel(Geo g, const float* __restrict__ locs, uint32_t* __restrict__ cnt) {
-  const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= g.npts) return;
-  uint32_t c = 1;
-  for (int e = 0; e < 3; ++e) {
-    int st, n, tl[3];
-    if (!axis_range(g, locs, p, e, st, n)) {
-      c = 0;
-      break;
-    }
-    c *= (uint32_t)axis_tiles(g, e, st, n, tl);
-  }
-  cnt[p] = c;
-}
-
-__global__ void plan_emit_kernel(Geo g, const float* __restrict__ locs, const uint32_t* __restrict__ off,
-                                 uint32_t* __restrict__ keys, int32_t* __restrict__ vals) {
-  const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= g.npts) return;
-  int tl[3][3], nc[3];
-  for (int e = 0; e < 3; ++e) {
-    int st, n;
-    if (!axis_range(g, locs, p, e, st, n)) return;
-    nc[e] = axis_tiles(g, e, st, n, tl[e]);
-  }
-  uint32_t o = off[p];
-  for (int i = 0; i < nc[0]; ++i)
-    for (int j = 0; j < nc[1]; ++j)
-      for (int k = 0; k < nc[2]; ++k) {
-        const uint32_t tile = ((uint32_t)tl[0][i] * g.nt[1] + tl[1][j]) * g.nt[2] + tl[2][k];
-        const bool home = (i == 0 && j == 0 && k == 0);
-        keys[o] = tile * 2u + (home ? 0u : 1u);
-        vals[o] = (int32_t)p;
-        ++o;
-      }
-}
-
-__global__ void key_hist_kernel(const uint32_t* __restrict__ keys, long long n, uint32_t* __restrict__ hist) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) atomicAdd(hist + keys[i], 1u);
 }
 
 // ------------------------------------------------------------- value types
@@ -935,63 +875,18 @@ struct __align__(16) PRec {
 };
 static_assert(sizeof(PRec) == 64, "64-byte point records");
 
-__global__ void point_records_kernel(Geo g, const float* __restrict__ locs, PRec* __restrict__ out) {
-  const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= g.npts) return;
-  PRec R;
-  int cnt = 0;
-#pragma unroll
-  for (int e = 0; e < 3; ++e) {
-    float w0 = 0.f, w1 = 0.f, w2 = 0.f, w3 = 0.f;
-    int c = 0, st = 0;
-    if (!g.act[e]) {
-      // a leading dimension of a 2D geometry: one tap of weight 1 at 0
-      R.w[e] = make_float4(1.f, 0.f, 0.f, 0.f);
-      R.st[e] = 0;
-      cnt |= 1 << (4 * e);
-      continue;
-    }
-    const float x = load_coord(g, locs, p, e);
-    if (coord_ok(x)) {
-      const int lower = lower_of(g, e, x);
-      int s = -1;
-#pragma unroll
-      for (int k = 0; k < 5; ++k) {
-        const Tap t = tap_eval(g, e, x, lower, k);
-        if (t.valid) {
-          if (s < 0) s = k;
-          const float v = kern_value_approx(g.kernel, fabsf(t.d), g.beta);
-          w0 = c == 0 ? v : w0;
-          w1 = c == 1 ? v : w1;
-          w2 = c == 2 ? v : w2;
-          w3 = c == 3 ? v : w3;
-          ++c;
-        }
-      }
-      if (c > 0) {
-        st = lower + s;
-        if (g.pad == TLGB_PAD_CIRCULAR) st = wrapi(st, g.N[e]);
-      }
-    }
-    R.w[e] = make_float4(w0, w1, w2, w3);
-    R.st[e] = st;
-    cnt |= c << (4 * e);
-  }
-  R.cnt = cnt;
-  out[p] = R;
-}
-
-// ------------------------------------------------ block lists (3D gridding)
+// ------------------------------------------------ block lists (gridding)
 //
-// The 8-entry gridding works on output blocks of 4 x 4 x 4 cells in 3D and
-// 8 x 8 cells in 2D (64 cells either way). A window of 4 taps per dimension
-// meets 1.75 blocks of 4 (1.375 of 8) per dimension on average, and one warp
-// holds a whole block for 8 entries. The plan lists per block the points
-// whose window meets it, in point order.
+// The gridding of complex values works on output blocks of 4 x 4 x 4 cells
+// in 3D and 8 x 8 cells in 2D (64 cells either way). A window of 4 taps per
+// dimension meets 1.75 blocks of 4 (1.375 of 8) per dimension on average, and
+// one warp holds a whole block for 8 entries. The plan lists per block the
+// points whose window meets it, in point order. A window meets at most
+// g.nrow blocks per dim: 2, or 3 for windows of more than 5 taps over blocks
+// of 4 and for circular grids whose last block is a partial one (a window
+// can cover the end of the grid, that block and the start).
 constexpr int kBlkPart = 256;  // entries per work item: denser blocks are split into parts
-constexpr int kZeroRun = 16;   // empty blocks written by one work item
 constexpr int kCube = 4;       // blocks per edge of the cubes the gridding items visit in turn
-constexpr int kSelShift = 29;  // entry = point | (its block's index per dim, 3 bits) << 29
 
 // block edge along internal dim e: 4 in 3D; 8 along the two dims of a 2D
 // grid (1 along its inactive leading dim)
@@ -1000,93 +895,410 @@ __host__ __device__ __forceinline__ int blocks_along(int n, int edge) { return (
 __host__ __device__ __forceinline__ int blocks_along(const Geo& g, int e) {
   return blocks_along(g.N[e], block_edge(g.ndim, e));
 }
-// floats of tap rows per point: 2 rows per active dim, one weight per cell
-__host__ __device__ __forceinline__ int row_floats(int ndim) { return ndim == 3 ? 24 : 32; }
+// An entry is point | selector << shift; the selector names the block among
+// the point's blocks per dim: 3 bits i | j << 1 | k << 2 for 2 rows, 9 i +
+// 3 j + k (5 bits) for 3.
+__host__ __device__ constexpr int sel_shift(int nrow) { return nrow == 3 ? 27 : 29; }
+template <int NROW>
+__device__ __forceinline__ void sel_rows(uint32_t en, int& i, int& j, int& k) {
+  const int s = (int)(en >> sel_shift(NROW));
+  if constexpr (NROW == 2) {
+    i = s & 1, j = (s >> 1) & 1, k = s >> 2;
+  } else {
+    i = (s * 57) >> 9;  // s / 9 for s < 27
+    const int r = s - 9 * i;
+    j = (r * 11) >> 5;  // r / 3 for r < 9
+    k = r - 3 * j;
+  }
+}
+// floats of tap rows per point: nrow rows per active dim, one weight per cell
+__host__ __device__ constexpr int row_floats(int ndim, int nrow) { return nrow * (ndim == 3 ? 12 : 16); }
 
 // Distinct blocks met along one dim by the cells st .. st+c-1 of a window
-// (st in [0, N); wrapped once in circular mode, where N >= 16 > c). At most
-// 2: 5 taps over blocks of 4 or 8 cells (circular grids are multiples of the
-// block edge).
+// (st in [0, N); wrapped in circular mode). The cells are a run, so a new
+// block starts where the block index changes.
 __device__ __forceinline__ int axis_blocks(const Geo& g, int e, int st, int c, int* bl) {
-  const int edge = block_edge(g.ndim, e);
-  int cnt = 0;
+  const int lg = g.ndim == 3 ? 2 : (e == 0 ? 0 : 3);
+  int cnt = 0, prev = -1;
   for (int k = 0; k < c; ++k) {
     int v = st + k;
     if (v >= g.N[e]) v -= g.N[e];
-    const int b = v / edge;
-    bool seen = false;
-    for (int i = 0; i < cnt; ++i) seen = seen || bl[i] == b;
-    if (!seen && cnt < 3) bl[cnt++] = b;
+    const int b = v >> lg;
+    if (b != prev && cnt < 3) bl[cnt++] = b;
+    prev = b;
   }
   return cnt;
 }
 
-__global__ void blk_count_kernel(Geo g, const PRec* __restrict__ precs, uint32_t* __restrict__ cnt) {
-  const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= g.npts) return;
-  const PRec R = precs[p];
-  uint32_t c = 1;
-  for (int e = 0; e < 3; ++e) {
-    const int ce = (R.cnt >> (4 * e)) & 15;
-    int bl[3];
-    c *= ce ? (uint32_t)axis_blocks(g, e, R.st[e], ce, bl) : 0u;
+// ------------------------------------------------------------- plan kernels
+//
+// The plan is built on the device from start to end: the host reads the
+// lists' lengths back once, after the last launch. Pairs, items and splits
+// are counted per CTA, the CTAs' sums scanned, and emitted at their places,
+// so every list's order depends on the points alone. A build is 16 to 20
+// short launches: bound by them up to about 10^5 points, by the pairs' bytes
+// (sorts, rows, records) above. Measured with the Python call around it:
+// 2^21 points of a dense-centre ball in 256^3 0.85 ms (about 5.5 ms with host-built
+// item lists, read-backs between the stages and one-warp sort chunks of 2048
+// pairs), 2^18 in 160^3 0.28 ms (1.5 ms), 205,824 in 320^2 0.23 ms.
+constexpr int kPlanPts = 256;  // points (or work units) per CTA
+constexpr int kWinBits = 5;    // bits per tap count of a window
+
+// exclusive scan of a uint4 per thread over the CTA (NT threads); total to `tot`
+template <int NT>
+__device__ __forceinline__ uint4 cta_scan4(uint4 v, uint4& tot) {
+  __shared__ uint4 ws[NT / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint4 x = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t a = __shfl_up_sync(0xffffffffu, x.x, o), b = __shfl_up_sync(0xffffffffu, x.y, o),
+                   c = __shfl_up_sync(0xffffffffu, x.z, o), d = __shfl_up_sync(0xffffffffu, x.w, o);
+    if (lane >= o) x.x += a, x.y += b, x.z += c, x.w += d;
   }
-  cnt[p] = c;
+  if (lane == 31) ws[warp] = x;
+  __syncthreads();
+  uint4 base = make_uint4(0, 0, 0, 0);
+  tot = base;
+  for (int w = 0; w < NT / 32; ++w) {
+    const uint4 t = ws[w];
+    if (w < warp) base.x += t.x, base.y += t.y, base.z += t.z, base.w += t.w;
+    tot.x += t.x, tot.y += t.y, tot.z += t.z, tot.w += t.w;
+  }
+  __syncthreads();  // ws may be written again
+  return make_uint4(base.x + x.x - v.x, base.y + x.y - v.y, base.z + x.z - v.z, base.w + x.w - v.w);
 }
 
-__global__ void blk_emit_kernel(Geo g, const PRec* __restrict__ precs, const uint32_t* __restrict__ off,
-                                uint32_t* __restrict__ keys, int32_t* __restrict__ vals) {
-  const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= g.npts) return;
-  const PRec R = precs[p];
-  int bl[3][3], nc[3];
-  for (int e = 0; e < 3; ++e) {
-    const int ce = (R.cnt >> (4 * e)) & 15;
-    if (!ce) return;
-    nc[e] = axis_blocks(g, e, R.st[e], ce, bl[e]);
+// CTA j scans job j's n CTA sums in place (exclusive); totals to tot[0..3].
+struct ScanJob {
+  uint4* sums;
+  long long n;
+  uint32_t* tot;
+};
+__global__ void __launch_bounds__(1024) plan_scan_kernel(ScanJob j0, ScanJob j1) {
+  const ScanJob j = blockIdx.x ? j1 : j0;
+  const long long per = (j.n + 1023) / 1024, b = threadIdx.x * per;
+  const long long e = b + per < j.n ? b + per : j.n;
+  uint4 s = make_uint4(0, 0, 0, 0);
+  for (long long i = b; i < e; ++i) {
+    const uint4 v = j.sums[i];
+    s.x += v.x, s.y += v.y, s.z += v.z, s.w += v.w;
   }
-  const uint32_t nb1 = (uint32_t)blocks_along(g, 1), nb2 = (uint32_t)blocks_along(g, 2);
-  uint32_t o = off[p];
+  uint4 tot;
+  uint4 run = cta_scan4<1024>(s, tot);
+  for (long long i = b; i < e; ++i) {
+    const uint4 v = j.sums[i];
+    j.sums[i] = run;
+    run.x += v.x, run.y += v.y, run.z += v.z, run.w += v.w;
+  }
+  if (threadIdx.x == 0) j.tot[0] = tot.x, j.tot[1] = tot.y, j.tot[2] = tot.z, j.tot[3] = tot.w;
+}
+
+__device__ __forceinline__ int win_cnt(const int4& w, int e) { return (w.w >> (kWinBits * e)) & ((1 << kWinBits) - 1); }
+__device__ __forceinline__ int win_st(const int4& w, int e) { return e == 0 ? w.x : (e == 1 ? w.y : w.z); }
+
+// tile pairs, block pairs and whether the point has taps (a home pair)
+__device__ __forceinline__ uint4 win_pairs(const Geo& g, const int4& w) {
+  if (w.w == 0) return make_uint4(0, 0, 0, 0);
+  uint32_t t = 1, b = 1;
+  for (int e = 0; e < 3; ++e) {
+    int l[3];
+    t *= (uint32_t)axis_tiles(g, e, win_st(w, e), win_cnt(w, e), l);
+    if (g.nrow) b *= (uint32_t)axis_blocks(g, e, win_st(w, e), win_cnt(w, e), l);
+  }
+  return make_uint4(t, g.nrow ? b : 0u, 1u, 0u);
+}
+
+// Per point: its window (first valid tap per dim, wrapped into [0, N) in
+// circular mode, and the tap counts; none when a dim has no valid tap), the
+// tap record (`recs`), and the tap rows over the blocks it meets (`rows`):
+// per active dim, one weight per cell of each block in axis_blocks order; a
+// cell outside the window holds -0.0 (valid weights are >= +0), so the sign
+// bit tells the gridding which cells the window covers. Each weight is
+// evaluated once and the rows are put together in shared memory, stored as
+// one contiguous run per CTA (evaluating every cell of every row in place
+// and storing them one by one took 47 us for 2^18 points in 3D).
+// NTM: taps evaluated per dim, at least the geometry's.
+template <int NTM>
+__global__ void __launch_bounds__(kPlanPts) plan_points_kernel(Geo g, const float* __restrict__ locs,
+                                                               int4* __restrict__ win, PRec* __restrict__ recs,
+                                                               float* __restrict__ rows, uint4* __restrict__ sums) {
+  extern __shared__ __align__(16) float prow[];  // [points][row_floats], when rows are wanted
+  const long long p0 = (long long)blockIdx.x * kPlanPts, p = p0 + threadIdx.x;
+  const bool on = p < g.npts;
+  const int RF = row_floats(g.ndim, g.nrow);
+  float* mine = prow + threadIdx.x * RF;
+  if (rows) {
+    const float4 none = make_float4(-0.f, -0.f, -0.f, -0.f);
+    for (int i = 0; i < RF / 4; ++i) reinterpret_cast<float4*>(mine)[i] = none;
+  }
+  PRec R;
+  int4 w4 = make_int4(0, 0, 0, 0);
+  int cnts = 0, rcnt = 0;
+  bool ok = on;
+#pragma unroll
+  for (int e = 0; e < 3; ++e) {
+    float w[4] = {0.f, 0.f, 0.f, 0.f};
+    int c = 0, st = 0;
+    if (!g.act[e]) {
+      w[0] = 1.f;  // a leading dimension of a 1D or 2D geometry: one tap of weight 1 at 0
+      c = 1;
+    } else if (on) {
+      const float x = load_coord(g, locs, p, e);
+      if (coord_ok(x)) {
+        const int lower = lower_of(g, e, x);
+        const int lg = g.ndim == 3 ? 2 : 3;
+        float* row = mine + (e - (3 - g.ndim)) * (RF / g.ndim) - (1 << lg);
+        int prev = -1;
+#pragma unroll
+        for (int k = 0; k < NTM; ++k) {
+          if (k >= g.NT[e]) continue;
+          const Tap t = tap_eval(g, e, x, lower, k);
+          if (!t.valid) continue;
+          if (c == 0) st = g.pad == TLGB_PAD_CIRCULAR ? wrapi(lower + k, g.N[e]) : lower + k;
+          if (recs || rows) {
+            const float v = NTM == 5 ? kern_value_approx(g.kernel, fabsf(t.d), g.beta)
+                                     : kern_fast(g.kernel, fabsf(t.d), g.beta);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) w[i] = c == i ? v : w[i];
+            if (rows) {
+              int cell = st + c;
+              if (cell >= g.N[e]) cell -= g.N[e];
+              if (cell >> lg != prev) row += 1 << lg, prev = cell >> lg;
+              row[cell & ((1 << lg) - 1)] = v;
+            }
+          }
+          ++c;
+        }
+      }
+    }
+    if (c == 0) ok = false;
+    R.w[e] = make_float4(w[0], w[1], w[2], w[3]);
+    R.st[e] = st;
+    rcnt |= c << (4 * e);
+    cnts |= c << (kWinBits * e);
+    if (e == 0) w4.x = st;
+    if (e == 1) w4.y = st;
+    if (e == 2) w4.z = st;
+  }
+  w4.w = ok ? cnts : 0;
+  if (on) {
+    win[p] = w4;
+    if (recs) {
+      R.cnt = rcnt;
+      recs[p] = R;
+    }
+  }
+  uint4 tot;
+  cta_scan4<kPlanPts>(on ? win_pairs(g, w4) : make_uint4(0, 0, 0, 0), tot);  // its barriers also publish the rows
+  if (threadIdx.x == 0) sums[blockIdx.x] = tot;
+  if (rows) {
+    const long long n4 = min((long long)kPlanPts, g.npts - p0) * RF / 4;
+    float4* dst = reinterpret_cast<float4*>(rows + p0 * RF);
+    for (int i = threadIdx.x; i < n4; i += kPlanPts) dst[i] = reinterpret_cast<const float4*>(prow)[i];
+  }
+}
+
+// (key, point) pairs of both lists at their places (point order)
+__global__ void __launch_bounds__(kPlanPts) plan_emit_kernel(Geo g, const int4* __restrict__ win,
+                                                             const uint4* __restrict__ sums,
+                                                             uint32_t* __restrict__ tkeys, int32_t* __restrict__ tvals,
+                                                             uint32_t* __restrict__ bkeys,
+                                                             int32_t* __restrict__ bvals) {
+  const long long p = (long long)blockIdx.x * kPlanPts + threadIdx.x;
+  const int4 w = p < g.npts ? win[p] : make_int4(0, 0, 0, 0);
+  uint4 tot;
+  const uint4 x = cta_scan4<kPlanPts>(win_pairs(g, w), tot);
+  if (w.w == 0) return;
+  const uint4 base = sums[blockIdx.x];
+  int l[3][3], nc[3];
+  for (int e = 0; e < 3; ++e) nc[e] = axis_tiles(g, e, win_st(w, e), win_cnt(w, e), l[e]);
+  uint32_t o = base.x + x.x;
   for (int i = 0; i < nc[0]; ++i)
     for (int j = 0; j < nc[1]; ++j)
       for (int k = 0; k < nc[2]; ++k) {
-        keys[o] = ((uint32_t)bl[0][i] * nb1 + (uint32_t)bl[1][j]) * nb2 + (uint32_t)bl[2][k];
-        vals[o] = (int32_t)((uint32_t)p | (uint32_t)(i | j << 1 | k << 2) << kSelShift);
+        const uint32_t tile = ((uint32_t)l[0][i] * g.nt[1] + l[1][j]) * g.nt[2] + l[2][k];
+        tkeys[o] = tile * 2u + (i == 0 && j == 0 && k == 0 ? 0u : 1u);
+        tvals[o] = (int32_t)p;
+        ++o;
+      }
+  if (!g.nrow) return;
+  for (int e = 0; e < 3; ++e) nc[e] = axis_blocks(g, e, win_st(w, e), win_cnt(w, e), l[e]);
+  const uint32_t nb1 = (uint32_t)blocks_along(g, 1), nb2 = (uint32_t)blocks_along(g, 2);
+  o = base.y + x.y;
+  for (int i = 0; i < nc[0]; ++i)
+    for (int j = 0; j < nc[1]; ++j)
+      for (int k = 0; k < nc[2]; ++k) {
+        const uint32_t sel = g.nrow == 3 ? (uint32_t)(9 * i + 3 * j + k) : (uint32_t)(i | j << 1 | k << 2);
+        bkeys[o] = ((uint32_t)l[0][i] * nb1 + (uint32_t)l[1][j]) * nb2 + (uint32_t)l[2][k];
+        bvals[o] = (int32_t)((uint32_t)p | sel << sel_shift(g.nrow));
         ++o;
       }
 }
 
-// The tap weights of a point over each block it meets: per active dim the
-// rows of its first and second block (in axis_blocks order), one weight per
-// cell of the block (4 in 3D, 8 in 2D), from the coordinate as the tap
-// records; a cell outside the window holds -0.0 (valid weights are >= +0), so
-// the sign bit tells the gridding which cells the window covers.
-__global__ void blk_rows_kernel(Geo g, const float* __restrict__ locs, const PRec* __restrict__ precs,
-                                float* __restrict__ rows) {
-  const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= g.npts) return;
-  const PRec R = precs[p];
-  float* out = rows + p * row_floats(g.ndim);
-  for (int e = 3 - g.ndim; e < 3; ++e) {
-    const int edge = block_edge(g.ndim, e);
-    const int ce = (R.cnt >> (4 * e)) & 15;
-    int bl[3] = {0, 0, 0};
-    const int nb = ce ? axis_blocks(g, e, R.st[e], ce, bl) : 0;
-    const float x = load_coord(g, locs, p, e);
-    const int lower = coord_ok(x) ? lower_of(g, e, x) : 0;
-    for (int i = 0; i < 2; ++i) {
-      for (int q = 0; q < edge; ++q) {
-        const int v = edge * bl[i] + q;
-        int k = v - lower;
-        if (g.pad == TLGB_PAD_CIRCULAR) k = wrapi(k, g.N[e]);
-        float w = -0.0f;
-        if (i < nb && v < g.N[e] && k >= 0 && k < g.NT[e]) {
-          const Tap t = tap_eval(g, e, x, lower, k);
-          if (t.valid) w = kern_value_approx(g.kernel, fabsf(t.d), g.beta);
-        }
-        *out++ = w;
-      }
+// start[k] = first position of key k in the sorted keys, start[nkeys] = the
+// list's length: one binary search per key (a histogram of the keys by
+// atomics is slow where a dense centre puts thousands of them on one key)
+__global__ void __launch_bounds__(256) plan_starts_kernel(const uint32_t* __restrict__ tkeys,
+                                                          const uint32_t* __restrict__ bkeys,
+                                                          const uint32_t* __restrict__ cnt, long long ntk,
+                                                          long long nbk, uint32_t* __restrict__ tstart,
+                                                          uint32_t* __restrict__ bstart) {
+  long long k = (long long)blockIdx.x * 256 + threadIdx.x;
+  const bool blk = k > ntk;
+  if (blk) k -= ntk + 1;
+  if (k > (blk ? nbk : ntk)) return;
+  const uint32_t* keys = blk ? bkeys : tkeys;
+  uint32_t lo = 0, hi = blk ? cnt[1] : cnt[0];
+  while (lo < hi) {
+    const uint32_t mid = lo + (hi - lo) / 2;
+    if ((long long)keys[mid] < k)
+      lo = mid + 1;
+    else
+      hi = mid;
+  }
+  (blk ? bstart : tstart)[k] = lo;
+}
+
+// Work units the items are made from: tiles, in order, and rows of kCube
+// blocks along z, in the order of the cubes of kCube^3 blocks (kCube^2 in
+// 2D), so that the blocks a point meets are worked on close together in time
+// and find its rows and values in L2.
+struct PlanUnits {
+  long long ntiles, nrows;       // units
+  int nbx, nby, nbz;             // blocks per dim
+  int ncy, ncz;                  // cubes along y and z
+  int per;                       // rows per cube
+  int tile_ctas;
+};
+
+// the blocks [b0, b0 + n) of row unit u (n = 0: outside the grid)
+__device__ __forceinline__ int row_blocks(const PlanUnits& U, long long u, int& b0) {
+  const int in = (int)(u % U.per);
+  long long c = u / U.per;
+  const int cz = (int)(c % U.ncz);
+  c /= U.ncz;
+  const int cy = (int)(c % U.ncy), cx = (int)(c / U.ncy);
+  const int bx = cx * (U.per / kCube) + in / kCube, by = cy * kCube + in % kCube, bz = cz * kCube;
+  if (bx >= U.nbx || by >= U.nby) return 0;
+  b0 = (bx * U.nby + by) * U.nbz + bz;
+  return min(kCube, U.nbz - bz);
+}
+
+__device__ __forceinline__ int parts_of(int n, int chunk) { return (n + chunk - 1) / chunk; }
+
+// Item counts of a unit. Tile: gather items, gridding items, parts of split
+// tiles, split tiles. Block row: items, parts of split blocks, split blocks.
+// A run of empty blocks of the row is one item.
+__device__ __forceinline__ uint4 unit_items(const PlanUnits& U, bool tile, long long u, const uint32_t* tstart,
+                                            const uint32_t* bstart, int fwd_chunk, int adj_chunk) {
+  uint4 c = make_uint4(0, 0, 0, 0);
+  if (tile) {
+    const uint32_t b = tstart[2 * u], h = tstart[2 * u + 1], e = tstart[2 * u + 2];
+    const int na = (int)(e - b);
+    c.x = parts_of((int)(h - b), fwd_chunk);
+    c.y = na <= adj_chunk ? 1 : parts_of(na, adj_chunk);
+    if (na > adj_chunk) c.z = c.y, c.w = 1;
+    return c;
+  }
+  int b0 = 0;
+  const int nb = row_blocks(U, u, b0);
+  bool empty = false;
+  for (int i = 0; i < nb; ++i) {
+    const int n = (int)(bstart[b0 + i + 1] - bstart[b0 + i]);
+    if (n == 0) {
+      c.x += empty ? 0 : 1;
+    } else if (n <= kBlkPart) {
+      c.x += 1;
+    } else {
+      const int k = parts_of(n, kBlkPart);
+      c.x += k, c.y += k, c.z += 1;
     }
+    empty = n == 0;
+  }
+  return c;
+}
+
+__global__ void __launch_bounds__(kPlanPts) plan_count_items_kernel(PlanUnits U, const uint32_t* __restrict__ tstart,
+                                                                    const uint32_t* __restrict__ bstart, int fwd_chunk,
+                                                                    int adj_chunk, uint4* __restrict__ sums) {
+  const bool tile = (int)blockIdx.x < U.tile_ctas;
+  const long long u = (long long)(blockIdx.x - (tile ? 0 : U.tile_ctas)) * kPlanPts + threadIdx.x;
+  uint4 c = make_uint4(0, 0, 0, 0), tot;
+  if (u < (tile ? U.ntiles : U.nrows)) c = unit_items(U, tile, u, tstart, bstart, fwd_chunk, adj_chunk);
+  cta_scan4<kPlanPts>(c, tot);
+  if (threadIdx.x == 0) sums[blockIdx.x] = tot;
+}
+
+// The items at their places. Gather items are in tile order, so neighbouring
+// regions are read while their shared halos are in L2. The tile gridding's
+// items and the split blocks go to `adj` / `bsplit` with sort keys: they are
+// put in falling order of their length afterwards (a long item or a long sum
+// that starts last is waited for alone).
+__global__ void __launch_bounds__(kPlanPts) plan_emit_items_kernel(
+    PlanUnits U, const uint32_t* __restrict__ tstart, const uint32_t* __restrict__ bstart, int fwd_chunk, int adj_chunk,
+    const uint4* __restrict__ sums, int4* __restrict__ fwd, int4* __restrict__ adj, uint32_t* __restrict__ akey,
+    int32_t* __restrict__ aidx, int4* __restrict__ split, int4* __restrict__ bitems, int4* __restrict__ bsplit,
+    uint32_t* __restrict__ skey, int32_t* __restrict__ sidx) {
+  const bool tile = (int)blockIdx.x < U.tile_ctas;
+  const long long u = (long long)(blockIdx.x - (tile ? 0 : U.tile_ctas)) * kPlanPts + threadIdx.x;
+  const bool on = u < (tile ? U.ntiles : U.nrows);
+  uint4 c = make_uint4(0, 0, 0, 0), tot;
+  if (on) c = unit_items(U, tile, u, tstart, bstart, fwd_chunk, adj_chunk);
+  uint4 o = cta_scan4<kPlanPts>(c, tot);
+  if (!on) return;
+  const uint4 base = sums[blockIdx.x];
+  o.x += base.x, o.y += base.y, o.z += base.z, o.w += base.w;
+  if (tile) {
+    const int b = (int)tstart[2 * u], h = (int)tstart[2 * u + 1], e = (int)tstart[2 * u + 2], t = (int)u;
+    for (int k = 0; k < (int)c.x; ++k)
+      fwd[o.x + k] = make_int4(t, b + k * fwd_chunk, min(h, b + (k + 1) * fwd_chunk), -1);
+    if (c.w) split[o.w] = make_int4(t, (int)o.z, (int)c.z, 0);
+    for (int k = 0; k < (int)c.y; ++k) {
+      const int q0 = b + k * adj_chunk, q1 = min(e, q0 + adj_chunk);
+      adj[o.y + k] = make_int4(t, q0, q1, c.w ? (int)o.z + k : -1);
+      akey[o.y + k] = (uint32_t)(adj_chunk - (q1 - q0));
+      aidx[o.y + k] = (int)(o.y + k);
+    }
+    return;
+  }
+  int b0 = 0;
+  const int nb = row_blocks(U, u, b0);
+  uint32_t item = o.x, part = o.y, sp = o.z;
+  int run = 0;  // empty blocks of the run that ends here
+  for (int i = 0; i < nb; ++i) {
+    const int q0 = (int)bstart[b0 + i], q1 = (int)bstart[b0 + i + 1], n = q1 - q0;
+    if (n == 0) {
+      ++run;
+      if (run == 1) ++item;
+      bitems[item - 1] = make_int4(b0 + i + 1 - run, q0, q0, -run);
+      continue;
+    }
+    run = 0;
+    if (n <= kBlkPart) {
+      bitems[item++] = make_int4(b0 + i, q0, q1, -1);
+      continue;
+    }
+    const int k = parts_of(n, kBlkPart);
+    bsplit[sp] = make_int4(b0 + i, (int)part, k, 0);
+    skey[sp] = 65535u - (uint32_t)min(k, 65535);
+    sidx[sp] = (int)sp;
+    ++sp;
+    for (int j = 0; j < k; ++j) bitems[item++] = make_int4(b0 + i, q0 + j * kBlkPart, min(q1, q0 + (j + 1) * kBlkPart), (int)part++);
+  }
+}
+
+__global__ void __launch_bounds__(256) plan_order_kernel(const uint32_t* __restrict__ cnt, const int4* __restrict__ adj,
+                                                         const int32_t* __restrict__ aidx, int4* __restrict__ adj_out,
+                                                         const int4* __restrict__ bsplit,
+                                                         const int32_t* __restrict__ sidx,
+                                                         int4* __restrict__ bsplit_out) {
+  const uint32_t n = blockIdx.y ? cnt[10] : cnt[5];
+  for (uint32_t i = blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256) {
+    if (blockIdx.y)
+      bsplit_out[i] = bsplit[sidx[i]];
+    else
+      adj_out[i] = adj[aidx[i]];
   }
 }
 
@@ -1664,7 +1876,7 @@ __device__ __forceinline__ void frag_store(const Geo& g, float* __restrict__ gri
   }
 }
 
-template <int NDIM>
+template <int NDIM, int NROW>
 __global__ void __launch_bounds__(256, kB3Ctas) adj_b3_kernel(Geo g, const int4* __restrict__ items, int nitems,
                                                         const uint32_t* __restrict__ bentries,
                                                         const float* __restrict__ rows,
@@ -1726,16 +1938,18 @@ __global__ void __launch_bounds__(256, kB3Ctas) adj_b3_kernel(Geo g, const int4*
       else if (item < last)
         enext = lane < min(kBC, itn.z - itn.y) ? bentries[itn.y + lane] : 0u;
       if (lane < n) {
-        long long p = en & ((1u << kSelShift) - 1u);
+        long long p = en & ((1u << sel_shift(NROW)) - 1u);
         if (!TLGB_IN_RANGE(p, g.npts)) p = 0;
-        const float* rsrc = rows + p * row_floats(NDIM);
+        const float* rsrc = rows + p * row_floats(NDIM, NROW);
+        int ri, rj, rk;
+        sel_rows<NROW>(en, ri, rj, rk);
         if constexpr (NDIM == 3) {  // rows of 4 cells: x 0-3, y 4-7, z 8-11
-          cp_async16(sl + 0, rsrc + 4 * (0 + ((en >> kSelShift) & 1)));
-          cp_async16(sl + 4, rsrc + 4 * (2 + ((en >> (kSelShift + 1)) & 1)));
-          cp_async16(sl + 8, rsrc + 4 * (4 + ((en >> (kSelShift + 2)) & 1)));
+          cp_async16(sl + 0, rsrc + 4 * ri);
+          cp_async16(sl + 4, rsrc + 4 * (NROW + rj));
+          cp_async16(sl + 8, rsrc + 4 * (2 * NROW + rk));
         } else {  // rows of 8 cells: y 0-7, z 8-15
-          const float* ry = rsrc + 8 * (0 + ((en >> (kSelShift + 1)) & 1));
-          const float* rz = rsrc + 8 * (2 + ((en >> (kSelShift + 2)) & 1));
+          const float* ry = rsrc + 8 * rj;
+          const float* rz = rsrc + 8 * (NROW + rk);
           cp_async16(sl + 0, ry);
           cp_async16(sl + 4, ry + 4);
           cp_async16(sl + 8, rz);
@@ -1965,7 +2179,7 @@ __device__ __forceinline__ void bn_store(const Geo& g, float* __restrict__ gridv
   }
 }
 
-template <int E>
+template <int E, int NROW>
 __global__ void __launch_bounds__(256, kBnCtas) adj_bn_kernel(Geo g, const int4* __restrict__ items, int nitems,
                                                              const uint32_t* __restrict__ bentries,
                                                              const float* __restrict__ rows,
@@ -2018,12 +2232,14 @@ __global__ void __launch_bounds__(256, kBnCtas) adj_bn_kernel(Geo g, const int4*
       else if (item < last)
         enext = lane < min(kBC, itn.z - itn.y) ? bentries[itn.y + lane] : 0u;
       if (lane < n) {
-        long long p = en & ((1u << kSelShift) - 1u);
+        long long p = en & ((1u << sel_shift(NROW)) - 1u);
         if (!TLGB_IN_RANGE(p, g.npts)) p = 0;
-        const float* rsrc = rows + p * row_floats(3);
-        cp_async16(sl + 0, rsrc + 4 * (0 + ((en >> kSelShift) & 1)));
-        cp_async16(sl + 4, rsrc + 4 * (2 + ((en >> (kSelShift + 1)) & 1)));
-        cp_async16(sl + 8, rsrc + 4 * (4 + ((en >> (kSelShift + 2)) & 1)));
+        const float* rsrc = rows + p * row_floats(3, NROW);
+        int ri, rj, rk;
+        sel_rows<NROW>(en, ri, rj, rk);
+        cp_async16(sl + 0, rsrc + 4 * ri);
+        cp_async16(sl + 4, rsrc + 4 * (NROW + rj));
+        cp_async16(sl + 8, rsrc + 4 * (2 * NROW + rk));
 #pragma unroll
         for (int j = 0; j < E; ++j) {
           if (j < ncoil)
@@ -3296,16 +3512,42 @@ __global__ void __launch_bounds__(256, 3) grad_f2_kernel(const __grid_constant__
 struct PlanLayout {
   int64_t e_max, max_fwd, max_adj, ntiles;
   int64_t off_entries, off_fwd, off_adj, off_split, off_recs, bytes;
-  // block lists of the 3D 8-entry gridding (off_blk_entries == 0: none)
-  int64_t nblocks, eb_max, max_blk_items, off_blk_entries, off_blk_items, off_blk_split, off_blk_rows;
-  // tmp
-  int64_t t_cnt, t_keys, t_keys2, t_vals2, t_counts, t_hist, t_total, t_bytes;
+  // block lists of the gridding of complex values (off_blk_entries == 0: none)
+  int64_t nblocks, eb_max, max_blk_items, max_blk_split, off_blk_entries, off_blk_items, off_blk_split, off_blk_rows;
+  // tmp: windows, CTA sums, counters, key starts; per list the sort's two key
+  // buffers, second value buffer and counts, and the unordered items, splits
+  // and their order
+  int64_t t_win, t_sums, t_cnt, t_tstart, t_bstart;
+  int64_t t_keys[2][2], t_vals[2], t_counts[2], t_items[2], t_order[2];
+  int64_t t_bytes;
 };
 
 constexpr int64_t kFwdChunk = 512;
 constexpr int64_t kAdjChunk = 1024;
 
 std::atomic<int> g_test_skip_copy{0};  // tlgb_test_skip_region_copy
+
+// Geometries whose plan carries per-point tap records (the 3D 8-entry kernels)
+bool records_ok(const Geo& g) {
+  if (g.norm != 1) return false;
+  if (g.ndim == 3)
+    return g.T[0] == 8 && g.T[1] == 8 && g.T[2] == 8 && g.NT[0] == 5 && g.NT[1] == 5 && g.NT[2] == 5;
+  return g.ndim == 2 && g.T[1] == 16 && g.T[2] == 16 && g.NT[1] == 5 && g.NT[2] == 5;
+}
+
+// Blocks a window can meet per dim in the block lists, 0 for geometries
+// without them: those of the tap records (3D 8^3 or 2D 16 x 16 tiles, at most
+// 5 taps per dim), and in circular mode every active dim a multiple of the
+// block edge and at least 16 cells, so that a wrapped window meets at most 2
+// blocks per dim and each of them once.
+int block_rows(const Geo& g) {
+  if (g.ndim < 2 || !records_ok(g) || g.npts >= (1ll << sel_shift(2))) return 0;
+  if (g.pad == TLGB_PAD_CIRCULAR)
+    for (int e = 3 - g.ndim; e < 3; ++e)
+      if (g.N[e] < 16 || g.N[e] % block_edge(g.ndim, e) != 0) return 0;
+  const int64_t nb = (int64_t)blocks_along(g, 0) * blocks_along(g, 1) * blocks_along(g, 2);
+  return nb < (1ll << 31) ? 2 : 0;
+}
 
 int make_geo(const tlgb_interp_desc* d, Geo& g) {
   if (!d) TLGB_FAIL(TLGB_ERR_INVALID, "null interp descriptor");
@@ -3357,6 +3599,9 @@ int make_geo(const tlgb_interp_desc* d, Geo& g) {
   g.tv_off = -1;
   for (int e = 0; e < 3; ++e) {
     g.T[e] = std::min(T[e], g.N[e]);
+    g.lgT[e] = -1;
+    for (int k = 0; k < 10; ++k)
+      if (g.T[e] == 1 << k) g.lgT[e] = k;
     g.nt[e] = (int)cdiv(g.N[e], g.T[e]);
     if (g.act[e] && g.N[e] < g.NT[e]) g.wrap_safe = 0;
   }
@@ -3368,6 +3613,7 @@ int make_geo(const tlgb_interp_desc* d, Geo& g) {
   g.npts = d->npts;
   g.nbatch = d->nbatch;
   if ((int64_t)g.nt[0] * g.nt[1] * g.nt[2] >= (1ll << 30)) TLGB_FAIL(TLGB_ERR_UNSUPPORTED, "too many tiles");
+  g.nrow = block_rows(g);
   return TLGB_OK;
 }
 
@@ -3380,36 +3626,26 @@ int64_t max_tiles_per_dim(const Geo& g, int e) {
   return 2;
 }
 
-// Geometries whose plan carries per-point tap records (the 3D 8-entry kernels)
-bool records_ok(const Geo& g) {
-  if (g.norm != 1) return false;
-  if (g.ndim == 3)
-    return g.T[0] == 8 && g.T[1] == 8 && g.T[2] == 8 && g.NT[0] == 5 && g.NT[1] == 5 && g.NT[2] == 5;
-  return g.ndim == 2 && g.T[1] == 16 && g.T[2] == 16 && g.NT[1] == 5 && g.NT[2] == 5;
-}
-
-// Geometries whose plans also carry block lists (adj_b3_kernel): those of
-// the tap records (3D 8^3 or 2D 16 x 16 tiles, at most 5 taps per dim), and
-// in circular mode every active dim a multiple of the block edge and at
-// least 16 cells, so that a wrapped window meets at most 2 blocks per dim and
-// each of them once.
-bool blocks_ok(const Geo& g) {
-  if (g.ndim < 2 || !records_ok(g) || g.npts >= (1ll << kSelShift)) return false;
-  if (g.pad == TLGB_PAD_CIRCULAR)
-    for (int e = 3 - g.ndim; e < 3; ++e)
-      if (g.N[e] < 16 || g.N[e] % block_edge(g.ndim, e) != 0) return false;
-  const int64_t nb = (int64_t)blocks_along(g, 0) * blocks_along(g, 1) * blocks_along(g, 2);
-  return nb < (1ll << 31);
-}
-
-// Blocks one window can meet along a dim: 2 (at most 5 taps over 4 cells)
-int64_t max_blocks_per_dim(const Geo& g, int e) { return blocks_along(g, e) == 1 ? 1 : 2; }
+// Blocks one window can meet along a dim
+int64_t max_blocks_per_dim(const Geo& g, int e) { return std::min(blocks_along(g, e), g.nrow); }
 
 // The kernel, norm and beta a plan's records hold weights for
 int64_t kernel_key(const Geo& g) {
   uint32_t bits;
   memcpy(&bits, &g.beta, 4);
   return (int64_t)bits | ((int64_t)g.kernel << 32) | ((int64_t)g.norm << 40) | ((int64_t)1 << 48);
+}
+
+PlanUnits plan_units(const Geo& g, int64_t ntiles, bool blocks) {
+  PlanUnits U;
+  U.ntiles = ntiles;
+  U.nbx = blocks_along(g, 0), U.nby = blocks_along(g, 1), U.nbz = blocks_along(g, 2);
+  const int cx = g.ndim == 3 ? kCube : 1;
+  U.ncy = blocks_along(U.nby, kCube), U.ncz = blocks_along(U.nbz, kCube);
+  U.per = cx * kCube;
+  U.nrows = blocks ? (long long)blocks_along(U.nbx, cx) * U.ncy * U.ncz * U.per : 0;
+  U.tile_ctas = (int)cdiv(ntiles, kPlanPts);
+  return U;
 }
 
 PlanLayout layout(const Geo& g) {
@@ -3432,39 +3668,47 @@ PlanLayout layout(const Geo& g) {
     L.off_recs = o;
     o = align_up(o + (size_t)g.npts * 64, 256);
   }
-  L.nblocks = L.eb_max = L.max_blk_items = 0;
+  L.nblocks = L.eb_max = L.max_blk_items = L.max_blk_split = 0;
   L.off_blk_entries = L.off_blk_items = L.off_blk_split = L.off_blk_rows = 0;
-  if (blocks_ok(g) && g.npts > 0) {
+  if (g.nrow && g.npts > 0) {
     L.nblocks = (int64_t)blocks_along(g, 0) * blocks_along(g, 1) * blocks_along(g, 2);
     L.eb_max = g.npts * max_blocks_per_dim(g, 0) * max_blocks_per_dim(g, 1) * max_blocks_per_dim(g, 2);
     L.max_blk_items = L.nblocks + cdiv(L.eb_max, kBlkPart) + 1;
+    L.max_blk_split = std::min(L.nblocks, L.eb_max / (kBlkPart + 1)) + 1;
     L.off_blk_entries = o;
     o = align_up(o + (size_t)L.eb_max * 4, 256);
     L.off_blk_items = o;
     o = align_up(o + (size_t)L.max_blk_items * 16, 256);
     L.off_blk_split = o;
-    o = align_up(o + (size_t)(L.nblocks + 1) * 16, 256);
+    o = align_up(o + (size_t)L.max_blk_split * 16, 256);
     L.off_blk_rows = o;
-    o = align_up(o + (size_t)g.npts * row_floats(g.ndim) * 4, 256);
+    o = align_up(o + (size_t)g.npts * row_floats(g.ndim, g.nrow) * 4, 256);
   }
   L.bytes = o;
-  const int64_t pairs = std::max<int64_t>(std::max(L.e_max, L.eb_max), 1);  // sort buffers serve both lists
   size_t t = 0;
-  L.t_cnt = t;
-  t = align_up(t + (size_t)(g.npts + 1) * 4, 256);
-  L.t_keys = t;
-  t = align_up(t + (size_t)pairs * 4, 256);
-  L.t_keys2 = t;
-  t = align_up(t + (size_t)pairs * 4, 256);
-  L.t_vals2 = t;
-  t = align_up(t + (size_t)pairs * 4, 256);
-  L.t_counts = t;
-  t = align_up(t + (size_t)radix_counts_len(pairs) * 4, 256);
-  L.t_hist = t;
-  t = align_up(t + (size_t)(std::max(2 * L.ntiles, L.nblocks) + 1) * 4, 256);
-  L.t_total = t;
-  t = align_up(t + 16, 256);
-  L.t_bytes = t;
+  auto tmp = [&](int64_t bytes) {
+    const int64_t at = (int64_t)t;
+    t = align_up(t + (size_t)std::max<int64_t>(bytes, 16), 256);
+    return at;
+  };
+  const PlanUnits U = plan_units(g, L.ntiles, L.nblocks > 0);
+  L.t_win = tmp(g.npts * 16);
+  L.t_sums = tmp(std::max(cdiv(g.npts, kPlanPts), (int64_t)U.tile_ctas + cdiv(U.nrows, kPlanPts)) * 16);
+  L.t_cnt = tmp(16 * 4);
+  L.t_tstart = tmp((2 * L.ntiles + 1) * 4);
+  L.t_bstart = tmp((L.nblocks + 1) * 4);
+  for (int i = 0; i < 2; ++i) {  // the tile list and its gridding items; the block list and its splits
+    const int64_t pairs = i ? L.eb_max : L.e_max, items = i ? L.max_blk_split : L.max_adj;
+    if (i && !L.nblocks) break;
+    const int64_t n = std::max<int64_t>(std::max(pairs, items), 1);
+    L.t_keys[i][0] = tmp(n * 4);
+    L.t_keys[i][1] = tmp(n * 4);
+    L.t_vals[i] = tmp(n * 4);
+    L.t_counts[i] = tmp(radix_counts_len(n) * 4);
+    L.t_items[i] = tmp(items * 16);
+    L.t_order[i] = tmp(items * 4);
+  }
+  L.t_bytes = (int64_t)t;
   return L;
 }
 
@@ -3568,7 +3812,7 @@ int check_plan(const Geo& g, const tlgb_interp_plan_info* info, const void* plan
   for (int e = 0; e < 3; ++e)
     if (info->tile[e] != g.T[e] || info->n_tile[e] != g.nt[e])
       TLGB_FAIL(TLGB_ERR_INVALID, "plan was built for another grid");
-  if (info->off_records > 0 && records_ok(g) && info->kernel_key != kernel_key(g))
+  if (((info->off_records > 0 && records_ok(g)) || info->n_blk_items > 0) && info->kernel_key != kernel_key(g))
     TLGB_FAIL(TLGB_ERR_INVALID, "plan was built for another kernel, norm or beta (its tap weights are stored)");
   return TLGB_OK;
 }
@@ -3607,164 +3851,102 @@ extern "C" int tlgb_interp_plan_build(const tlgb_interp_desc* d, const float* lo
   cudaStream_t s = (cudaStream_t)stream;
   char* P = (char*)plan;
   char* Tm = (char*)tmp;
+  const bool blocks = L.nblocks > 0;
+  const PlanUnits U = plan_units(g, L.ntiles, blocks);
+  int4* win = (int4*)(Tm + L.t_win);
+  uint4* sums = (uint4*)(Tm + L.t_sums);
   uint32_t* cnt = (uint32_t*)(Tm + L.t_cnt);
-  uint32_t* keys = (uint32_t*)(Tm + L.t_keys);
-  uint32_t* keys2 = (uint32_t*)(Tm + L.t_keys2);
-  int32_t* vals2 = (int32_t*)(Tm + L.t_vals2);
-  uint32_t* counts = (uint32_t*)(Tm + L.t_counts);
-  uint32_t* hist = (uint32_t*)(Tm + L.t_hist);
-  uint32_t* total = (uint32_t*)(Tm + L.t_total);
-  int32_t* entries = (int32_t*)(P + L.off_entries);
-
-  uint32_t E = 0;
+  uint32_t* tstart = (uint32_t*)(Tm + L.t_tstart);
+  uint32_t* bstart = (uint32_t*)(Tm + L.t_bstart);
+  TLGB_CUDA(cudaMemsetAsync(cnt, 0, 16 * 4, s));
+  // the sort of both lists: the pairs are emitted where an even or odd number
+  // of passes leaves them in the plan
+  SortJob jobs[2];
+  const int njobs = blocks ? 2 : 1;
+  auto bits_for = [](int64_t n) {
+    int b = 1;
+    while ((1ll << b) < n) ++b;
+    return b;
+  };
+  const int tbits = bits_for(2 * L.ntiles), bbits = blocks ? bits_for(L.nblocks) : 1;
+  const int odd = std::max(radix_passes(tbits), radix_passes(bbits)) & 1;
+  for (int i = 0; i < njobs; ++i) {
+    int32_t* fin = (int32_t*)(P + (i ? L.off_blk_entries : L.off_entries));
+    int32_t* alt = (int32_t*)(Tm + L.t_vals[i]);
+    jobs[i] = {{(uint32_t*)(Tm + L.t_keys[i][0]), (uint32_t*)(Tm + L.t_keys[i][1])},
+               {odd ? alt : fin, odd ? fin : alt},
+               (uint32_t*)(Tm + L.t_counts[i]), cnt + i, i ? L.eb_max : L.e_max, i ? bbits : tbits};
+  }
   if (g.npts > 0) {
-    const unsigned nb = (unsigned)cdiv(g.npts, 256);
-    plan_count_kernel<<<nb, 256, 0, s>>>(g, locs, cnt);
-    TLGB_CHECK_LAUNCH();
-    TLGB_TRY(exclusive_scan_u32(cnt, cnt, g.npts, total, counts, s));  // counts is free until the sort
-    plan_emit_kernel<<<nb, 256, 0, s>>>(g, locs, cnt, keys, entries);
-    TLGB_CHECK_LAUNCH();
-    if (L.off_recs > 0) point_records_kernel<<<nb, 256, 0, s>>>(g, locs, (PRec*)(P + L.off_recs));
-    TLGB_CHECK_LAUNCH();
-    TLGB_CUDA(cudaMemcpyAsync(&E, total, 4, cudaMemcpyDeviceToHost, s));
-    TLGB_CUDA(cudaStreamSynchronize(s));
-  }
-  int bits = 1;
-  while ((1ll << bits) < 2 * L.ntiles) ++bits;
-  TLGB_TRY(radix_sort_pairs(keys, entries, keys2, vals2, counts, (int64_t)E, bits, s));
-  TLGB_CUDA(cudaMemsetAsync(hist, 0, (size_t)(2 * L.ntiles) * 4, s));
-  if (E > 0) {
-    key_hist_kernel<<<(unsigned)cdiv(E, 256), 256, 0, s>>>(keys, E, hist);
-    TLGB_CHECK_LAUNCH();
-  }
-  std::vector<uint32_t> h((size_t)(2 * L.ntiles));
-  TLGB_CUDA(cudaMemcpyAsync(h.data(), hist, h.size() * 4, cudaMemcpyDeviceToHost, s));
-  TLGB_CUDA(cudaStreamSynchronize(s));
-
-  // work items (host). Results do not depend on the order, because every
-  // item writes its own tile, slot or points. Gather items stay in tile
-  // order, so neighbouring regions are read while their shared halos are in
-  // L2. Gridding items go heaviest first, for load balance.
-  std::vector<int4> fwd, adj, split;
-  int64_t pos = 0, n_home = 0, n_partials = 0;
-  for (int64_t t = 0; t < L.ntiles; ++t) {
-    const int64_t nh = h[2 * t], nn = h[2 * t + 1];
-    const int64_t beg = pos, hend = pos + nh, end = pos + nh + nn;
-    n_home += nh;
-    for (int64_t b = beg; b < hend; b += kFwdChunk)
-      fwd.push_back(make_int4((int)t, (int)b, (int)std::min(hend, b + kFwdChunk), -1));
-    const int64_t na = end - beg;
-    if (na <= kAdjChunk) {
-      adj.push_back(make_int4((int)t, (int)beg, (int)end, -1));
-    } else {
-      const int64_t nch = cdiv(na, kAdjChunk);
-      split.push_back(make_int4((int)t, (int)n_partials, (int)nch, 0));
-      for (int64_t k = 0; k < nch; ++k)
-        adj.push_back(make_int4((int)t, (int)(beg + k * kAdjChunk), (int)std::min(end, beg + (k + 1) * kAdjChunk),
-                                (int)(n_partials + k)));
-      n_partials += nch;
-    }
-    pos = end;
-  }
-  auto heavier = [](const int4& a, const int4& b) { return (a.z - a.y) > (b.z - b.y); };
-  std::stable_sort(adj.begin(), adj.end(), heavier);
-  if ((int64_t)fwd.size() > L.max_fwd || (int64_t)adj.size() > L.max_adj)
-    TLGB_FAIL(TLGB_ERR_DEVICE, "work list larger than its bound");
-  if (!fwd.empty()) TLGB_CUDA(cudaMemcpyAsync(P + L.off_fwd, fwd.data(), fwd.size() * 16, cudaMemcpyHostToDevice, s));
-  if (!adj.empty()) TLGB_CUDA(cudaMemcpyAsync(P + L.off_adj, adj.data(), adj.size() * 16, cudaMemcpyHostToDevice, s));
-  if (!split.empty())
-    TLGB_CUDA(cudaMemcpyAsync(P + L.off_split, split.data(), split.size() * 16, cudaMemcpyHostToDevice, s));
-  // host vectors are freed on return: make the copies complete first
-  TLGB_CUDA(cudaStreamSynchronize(s));
-
-  // Block lists (3D 8-entry gridding): (point, block) pairs from the tap
-  // records, sorted stably by block; work items of at most kBlkPart entries
-  // (dense blocks split into parts summed in order afterwards) and runs of
-  // up to kZeroRun empty blocks. A point's blocks are neighbours, so items
-  // in spatial order read its rows and values again while they are still in
-  // L2 (in heaviest-first order nearly every read of them went to DRAM).
-  uint32_t Eb = 0;
-  std::vector<int4> bitems, bsplit;
-  int64_t n_bpartials = 0;
-  if (L.off_blk_entries > 0) {
-    const PRec* recs = (const PRec*)(P + L.off_recs);
-    int32_t* bentries = (int32_t*)(P + L.off_blk_entries);
-    const unsigned nb = (unsigned)cdiv(g.npts, 256);
-    blk_count_kernel<<<nb, 256, 0, s>>>(g, recs, cnt);
-    TLGB_CHECK_LAUNCH();
-    TLGB_TRY(exclusive_scan_u32(cnt, cnt, g.npts, total, counts, s));
-    blk_emit_kernel<<<nb, 256, 0, s>>>(g, recs, cnt, keys, bentries);
-    TLGB_CHECK_LAUNCH();
-    blk_rows_kernel<<<nb, 256, 0, s>>>(g, locs, recs, (float*)(P + L.off_blk_rows));
-    TLGB_CHECK_LAUNCH();
-    TLGB_CUDA(cudaMemcpyAsync(&Eb, total, 4, cudaMemcpyDeviceToHost, s));
-    TLGB_CUDA(cudaStreamSynchronize(s));
-    int bbits = 1;
-    while ((1ll << bbits) < L.nblocks) ++bbits;
-    TLGB_TRY(radix_sort_pairs(keys, bentries, keys2, vals2, counts, (int64_t)Eb, bbits, s));
-    TLGB_CUDA(cudaMemsetAsync(hist, 0, (size_t)L.nblocks * 4, s));
-    if (Eb > 0) {
-      key_hist_kernel<<<(unsigned)cdiv(Eb, 256), 256, 0, s>>>(keys, Eb, hist);
+    const unsigned nb = (unsigned)cdiv(g.npts, kPlanPts);
+    PRec* recs = L.off_recs > 0 ? (PRec*)(P + L.off_recs) : nullptr;
+    float* rows = blocks ? (float*)(P + L.off_blk_rows) : nullptr;
+    const size_t sm = blocks ? (size_t)kPlanPts * row_floats(g.ndim, g.nrow) * 4 : 0;
+    const int maxnt = std::max(g.NT[0], std::max(g.NT[1], g.NT[2]));
+    auto points = [&](auto* k) -> int {
+      TLGB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+      k<<<nb, kPlanPts, sm, s>>>(g, locs, win, recs, rows, sums);
       TLGB_CHECK_LAUNCH();
-    }
-    std::vector<uint32_t> hb((size_t)L.nblocks);
-    TLGB_CUDA(cudaMemcpyAsync(hb.data(), hist, hb.size() * 4, cudaMemcpyDeviceToHost, s));
-    TLGB_CUDA(cudaStreamSynchronize(s));
-    // items in cube order: cubes of kCube^3 blocks, blocks in key order
-    // inside a cube, so that the blocks a point meets are worked on close
-    // together in time and find its rows and values in L2
-    std::vector<int64_t> bstart((size_t)L.nblocks + 1, 0);
-    for (int64_t b = 0; b < L.nblocks; ++b) bstart[(size_t)b + 1] = bstart[(size_t)b] + hb[(size_t)b];
-    const int64_t nbx = blocks_along(g, 0), nby = blocks_along(g, 1), nbz = blocks_along(g, 2);
-    auto add_block = [&](int64_t b) {
-      const int64_t n = hb[(size_t)b], bpos = bstart[(size_t)b];
-      if (n == 0) {
-        int4* last = bitems.empty() ? nullptr : &bitems.back();
-        if (last && last->y == last->z && last->x - last->w == b && -last->w < kZeroRun)
-          --last->w;  // extends the run of empty blocks ending at block b - 1
-        else
-          bitems.push_back(make_int4((int)b, (int)bpos, (int)bpos, -1));
-        return;
-      }
-      if (n <= kBlkPart) {
-        bitems.push_back(make_int4((int)b, (int)bpos, (int)(bpos + n), -1));
-        return;
-      }
-      const int64_t nch = cdiv(n, kBlkPart);
-      bsplit.push_back(make_int4((int)b, (int)n_bpartials, (int)nch, 0));
-      for (int64_t k = 0; k < nch; ++k)
-        bitems.push_back(make_int4((int)b, (int)(bpos + k * kBlkPart), (int)std::min(bpos + n, bpos + (k + 1) * kBlkPart),
-                                   (int)(n_bpartials + k)));
-      n_bpartials += nch;
+      return TLGB_OK;
     };
-    for (int64_t cx = 0; cx < nbx; cx += kCube)
-      for (int64_t cy = 0; cy < nby; cy += kCube)
-        for (int64_t cz = 0; cz < nbz; cz += kCube)
-          for (int64_t bx = cx; bx < std::min(nbx, cx + kCube); ++bx)
-            for (int64_t by = cy; by < std::min(nby, cy + kCube); ++by)
-              for (int64_t bz = cz; bz < std::min(nbz, cz + kCube); ++bz) add_block((bx * nby + by) * nbz + bz);
-    if ((int64_t)bitems.size() > L.max_blk_items) TLGB_FAIL(TLGB_ERR_DEVICE, "block work list larger than its bound");
-    // split blocks with the most parts first: their sums are the longest
-    // chains of the reduction, so they start in its first wave
-    std::stable_sort(bsplit.begin(), bsplit.end(), [](const int4& a, const int4& b) { return a.z > b.z; });
-    if (!bitems.empty())
-      TLGB_CUDA(cudaMemcpyAsync(P + L.off_blk_items, bitems.data(), bitems.size() * 16, cudaMemcpyHostToDevice, s));
-    if (!bsplit.empty())
-      TLGB_CUDA(cudaMemcpyAsync(P + L.off_blk_split, bsplit.data(), bsplit.size() * 16, cudaMemcpyHostToDevice, s));
-    TLGB_CUDA(cudaStreamSynchronize(s));
+    TLGB_TRY(records_ok(g) ? points(plan_points_kernel<5>) : (maxnt <= 9 ? points(plan_points_kernel<9>) : points(plan_points_kernel<NTMAX>)));
+    plan_scan_kernel<<<1, 1024, 0, s>>>({sums, (long long)nb, cnt}, {});
+    TLGB_CHECK_LAUNCH();
+    plan_emit_kernel<<<nb, kPlanPts, 0, s>>>(g, win, sums, jobs[0].keys[0], jobs[0].vals[0],
+                                             blocks ? jobs[1].keys[0] : nullptr, blocks ? jobs[1].vals[0] : nullptr);
+    TLGB_CHECK_LAUNCH();
+    TLGB_TRY(radix_sort_jobs(jobs, njobs, s));
   }
+  const int64_t nstart = 2 * L.ntiles + 1 + (blocks ? L.nblocks + 1 : 0);
+  plan_starts_kernel<<<(unsigned)cdiv(nstart, 256), 256, 0, s>>>(jobs[0].keys[odd], blocks ? jobs[1].keys[odd] : nullptr,
+                                                                 cnt, 2 * L.ntiles, blocks ? L.nblocks : -1, tstart,
+                                                                 bstart);
+  TLGB_CHECK_LAUNCH();
+
+  // Work items. Results do not depend on their order, because every item
+  // writes its own tile, block, slot or points.
+  const unsigned row_ctas = (unsigned)cdiv(U.nrows, kPlanPts), unit_ctas = (unsigned)U.tile_ctas + row_ctas;
+  plan_count_items_kernel<<<unit_ctas, kPlanPts, 0, s>>>(U, tstart, bstart, (int)kFwdChunk, (int)kAdjChunk, sums);
+  TLGB_CHECK_LAUNCH();
+  plan_scan_kernel<<<2, 1024, 0, s>>>({sums, U.tile_ctas, cnt + 4}, {sums + U.tile_ctas, (long long)row_ctas, cnt + 8});
+  TLGB_CHECK_LAUNCH();
+  int4* adj_any = (int4*)(Tm + L.t_items[0]);
+  int4* bsplit_any = blocks ? (int4*)(Tm + L.t_items[1]) : nullptr;
+  // the keys' buffers are free again: they order the items
+  SortJob order[2];
+  for (int i = 0; i < njobs; ++i)
+    order[i] = {{jobs[i].keys[0], jobs[i].keys[1]},
+                {(int32_t*)(Tm + L.t_order[i]), (int32_t*)(Tm + L.t_vals[i])},
+                jobs[i].counts, cnt + (i ? 10 : 5), i ? L.max_blk_split : L.max_adj, i ? 16 : 11};
+  plan_emit_items_kernel<<<unit_ctas, kPlanPts, 0, s>>>(
+      U, tstart, bstart, (int)kFwdChunk, (int)kAdjChunk, sums, (int4*)(P + L.off_fwd), adj_any, order[0].keys[0],
+      order[0].vals[0], (int4*)(P + L.off_split), blocks ? (int4*)(P + L.off_blk_items) : nullptr, bsplit_any,
+      blocks ? order[1].keys[0] : nullptr, blocks ? order[1].vals[0] : nullptr);
+  TLGB_CHECK_LAUNCH();
+  TLGB_TRY(radix_sort_jobs(order, njobs, s));
+  const int ofin = std::max(radix_passes(order[0].bits), blocks ? radix_passes(order[1].bits) : 1) & 1;
+  const int64_t onmax = std::max(L.max_adj, L.max_blk_split);
+  plan_order_kernel<<<dim3((unsigned)std::min<int64_t>(cdiv(onmax, 256), 8 * sm_count()), (unsigned)njobs), 256, 0, s>>>(
+      cnt, adj_any, order[0].vals[ofin], (int4*)(P + L.off_adj), bsplit_any, blocks ? order[1].vals[ofin] : nullptr,
+      blocks ? (int4*)(P + L.off_blk_split) : nullptr);
+  TLGB_CHECK_LAUNCH();
+  uint32_t c[16];
+  TLGB_CUDA(cudaMemcpyAsync(c, cnt, sizeof(c), cudaMemcpyDeviceToHost, s));
+  TLGB_CUDA(cudaStreamSynchronize(s));
+  if ((int64_t)c[4] > L.max_fwd || (int64_t)c[5] > L.max_adj || (blocks && ((int64_t)c[8] > L.max_blk_items || (int64_t)c[10] > L.max_blk_split)))
+    TLGB_FAIL(TLGB_ERR_DEVICE, "work list larger than its bound");
 
   memset(info, 0, sizeof(*info));
-  info->n_entries = E;
+  info->n_entries = c[0];
   info->n_tiles = L.ntiles;
   for (int e = 0; e < 3; ++e) {
     info->tile[e] = g.T[e];
     info->n_tile[e] = g.nt[e];
   }
-  info->n_fwd_items = (int64_t)fwd.size();
-  info->n_adj_items = (int64_t)adj.size();
-  info->n_partials = n_partials;
-  info->n_split_tiles = (int64_t)split.size();
+  info->n_fwd_items = c[4];
+  info->n_adj_items = c[5];
+  info->n_partials = c[6];
+  info->n_split_tiles = c[7];
   info->chunk = kAdjChunk;
   info->off_entries = L.off_entries;
   info->off_fwd_items = L.off_fwd;
@@ -3772,13 +3954,13 @@ extern "C" int tlgb_interp_plan_build(const tlgb_interp_desc* d, const float* lo
   info->off_split = L.off_split;
   info->plan_bytes = L.bytes;
   info->off_records = L.off_recs;
-  info->kernel_key = L.off_recs > 0 ? kernel_key(g) : 0;
-  info->n_home = n_home;
-  if (L.off_blk_entries > 0) {
-    info->n_blk_entries = Eb;
-    info->n_blk_items = (int64_t)bitems.size();
-    info->n_blk_partials = n_bpartials;
-    info->n_blk_split = (int64_t)bsplit.size();
+  info->kernel_key = L.off_recs > 0 || blocks ? kernel_key(g) : 0;
+  info->n_home = c[2];
+  if (blocks) {
+    info->n_blk_entries = c[1];
+    info->n_blk_items = c[8];
+    info->n_blk_partials = c[9];
+    info->n_blk_split = c[10];
     info->off_blk_entries = L.off_blk_entries;
     info->off_blk_items = L.off_blk_items;
     info->off_blk_split = L.off_blk_split;
@@ -3984,11 +4166,11 @@ int launch_adj_f3(const Geo& g, const tlgb_interp_plan_info* info, const char* P
   return TLGB_OK;
 }
 
-template <int E>
+template <int E, int NROW>
 int launch_adj_bn(const Geo& g, const tlgb_interp_plan_info* info, const char* P, const void* vals, void* grid,
                   void* scratch, cudaStream_t s) {
   const size_t sm = 8 * kBC * kBSn * sizeof(float);
-  TLGB_TRY(set_smem(adj_bn_kernel<E>, sm));
+  TLGB_TRY(set_smem(adj_bn_kernel<E, NROW>, sm));
   if (((uintptr_t)P & 15) || ((uintptr_t)scratch & 15))
     TLGB_FAIL(TLGB_ERR_INVALID, "interp adjoint: plan and scratch must be 16-byte aligned");
   if ((uintptr_t)vals & 7) TLGB_FAIL(TLGB_ERR_INVALID, "interp adjoint: values must be 8-byte aligned");
@@ -3996,7 +4178,7 @@ int launch_adj_bn(const Geo& g, const tlgb_interp_plan_info* info, const char* P
   int* ctr = reinterpret_cast<int*>(static_cast<char*>(scratch) + blk_partial_bytes(info, 1, E));
   TLGB_CUDA(cudaMemsetAsync(ctr, 0, sizeof(int), s));
   const int64_t nctas = std::min<int64_t>(cdiv(info->n_blk_items, 8), (int64_t)kBnCtas * sm_count());
-  adj_bn_kernel<E><<<(unsigned)std::max<int64_t>(nctas, 1), 256, sm, s>>>(
+  adj_bn_kernel<E, NROW><<<(unsigned)std::max<int64_t>(nctas, 1), 256, sm, s>>>(
       g, (const int4*)(P + info->off_blk_items), (int)info->n_blk_items, (const uint32_t*)(P + info->off_blk_entries),
       (const float*)(P + info->off_blk_rows), (const float2*)vals, (float*)grid, (float*)scratch, ctr);
   TLGB_CHECK_LAUNCH();
@@ -4008,20 +4190,20 @@ int launch_adj_bn(const Geo& g, const tlgb_interp_plan_info* info, const char* P
   return TLGB_OK;
 }
 
-template <int NDIM>
+template <int NDIM, int NROW>
 int launch_adj_b3(const Geo& g, const tlgb_interp_plan_info* info, const char* P, const float* locs,
                   const void* vals, void* grid, void* scratch, cudaStream_t s) {
   if constexpr (NDIM == 3) {
     switch (blk_entries(g)) {
-      case 1: return launch_adj_bn<1>(g, info, P, vals, grid, scratch, s);
-      case 2: return launch_adj_bn<2>(g, info, P, vals, grid, scratch, s);
-      case 4: return launch_adj_bn<4>(g, info, P, vals, grid, scratch, s);
+      case 1: return launch_adj_bn<1, NROW>(g, info, P, vals, grid, scratch, s);
+      case 2: return launch_adj_bn<2, NROW>(g, info, P, vals, grid, scratch, s);
+      case 4: return launch_adj_bn<4, NROW>(g, info, P, vals, grid, scratch, s);
       default: break;
     }
   }
   const int64_t ncg = cdiv(g.nbatch, 8);
   const size_t sm = 8 * kBC * kBS * sizeof(float);
-  TLGB_TRY(set_smem(adj_b3_kernel<NDIM>, sm));
+  TLGB_TRY(set_smem(adj_b3_kernel<NDIM, NROW>, sm));
   // 16-byte asynchronous copies of the weight rows and transposed values
   if (((uintptr_t)P & 15) || ((uintptr_t)scratch & 15))
     TLGB_FAIL(TLGB_ERR_INVALID, "interp adjoint: plan and scratch must be 16-byte aligned");
@@ -4042,7 +4224,7 @@ int launch_adj_b3(const Geo& g, const tlgb_interp_plan_info* info, const char* P
   // number of which may be resident at once
   const int64_t nctas = std::min<int64_t>(cdiv(info->n_blk_items, 8), (int64_t)kB3Ctas * sm_count());
   dim3 grd((unsigned)std::max<int64_t>(nctas, 1), (unsigned)ncg);
-  adj_b3_kernel<NDIM><<<grd, 256, sm, s>>>(g, (const int4*)(P + info->off_blk_items), (int)info->n_blk_items,
+  adj_b3_kernel<NDIM, NROW><<<grd, 256, sm, s>>>(g, (const int4*)(P + info->off_blk_items), (int)info->n_blk_items,
                                           (const uint32_t*)(P + info->off_blk_entries),
                                           (const float*)(P + info->off_blk_rows), (const float2*)vals, tv,
                                           (float*)grid, (float*)scratch, ctr);
@@ -4101,11 +4283,11 @@ int launch_adj_t(const Geo& g, int cg, const tlgb_interp_plan_info* info, const 
                  const void* vals, void* grid, void* scratch, cudaStream_t s) {
   if constexpr (N == 4 && NDIM == 3 && NTB == 5)
     if (fast3(g, cg) && info->off_records > 0 && info->n_blk_items > 0)
-      return launch_adj_b3<3>(g, info, P, locs, vals, grid, scratch, s);
+      return launch_adj_b3<3, 2>(g, info, P, locs, vals, grid, scratch, s);
     if (fast3(g, cg) && info->off_records > 0) return launch_adj_f3(g, info, P, locs, vals, grid, scratch, s);
   if constexpr (NDIM == 2 && NTB == 5)
     if (fast2(g, cg) && info->off_records > 0 && info->n_blk_items > 0)
-      return launch_adj_b3<2>(g, info, P, locs, vals, grid, scratch, s);
+      return launch_adj_b3<2, 2>(g, info, P, locs, vals, grid, scratch, s);
     if (fast2(g, cg) && info->off_records > 0) return launch_adj_f2(g, info, P, locs, vals, grid, scratch, s);
   return launch_adj_t2<N, NDIM, NTB, false>(g, cg, info, P, locs, vals, grid, scratch, s);
 }
