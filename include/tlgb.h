@@ -89,7 +89,7 @@ typedef struct tlgb_interp_desc {
   int32_t norm;         /* 1: product of 1D weights; 2: radial weight */
   int32_t pad_mode;     /* TLGB_PAD_* */
   int32_t is_complex;
-  int32_t reserved;
+  int32_t reserved;     /* 0, or the float32 bits of beta's own rounding remainder */
   int64_t grid_size[3];
   float width[3];       /* kernel width per dimension, grid units */
   float beta;           /* Kaiser-Bessel shape parameter */

@@ -21,7 +21,7 @@ CASES = [
     ((40, 36, 48), 4096, "circular"),
     ((64, 48), 4097, "circular"),
     ((700,), 4095, "circular"),
-    ((9, 12, 13), 3000, "circular"),  # tile lists only: too small for block lists
+    ((7, 12, 13), 3000, "circular"),  # tile lists only: a window could meet a block twice
     ((520, 520, 520), 3000, "zero"),  # three sort passes
 ]
 

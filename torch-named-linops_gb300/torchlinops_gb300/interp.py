@@ -20,6 +20,7 @@ from __future__ import annotations
 
 import ctypes
 import math
+import struct
 import weakref
 from collections import OrderedDict
 from math import prod
@@ -41,6 +42,8 @@ __all__ = [
     "clear_plan_cache",
     "kaiser_bessel_beta",
 ]
+
+_F32, _F32_BITS = struct.Struct("f"), struct.Struct("i")
 
 # Maximum kernel width per dimension handled by the CUDA kernels
 MAX_WIDTH_1D_2D = 15.0
@@ -92,7 +95,8 @@ def _desc(ndim, grid_size, width, kernel, norm, pad_mode, beta, is_complex, nbat
     for i in range(ndim):
         d.grid_size[i] = int(grid_size[i])
         d.width[i] = float(width[i])
-    d.beta = float(beta)
+    d.beta = beta  # the struct holds it in float32, and what that rounding leaves beside it
+    d.reserved = _F32_BITS.unpack(_F32.pack(beta - d.beta))[0]
     d.nbatch = int(nbatch)
     d.npts = int(npts)
     return d
