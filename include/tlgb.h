@@ -116,7 +116,8 @@ typedef struct tlgb_interp_plan_info {
   int64_t plan_bytes;
   int64_t n_home;         /* points with at least one valid tap (home pairs) */
   int64_t off_records;    /* byte offset of the per-point tap records, 0 = none */
-  int64_t kernel_key;     /* kernel, norm and beta the records were built for */
+  int64_t kernel_key;     /* kernel, norm and beta the records and rows were built for;
+                           * bit 52: the points are in no spatial order */
   /* Block lists of the 2D/3D gridding of complex batches (0 when the plan has
    * none): the (point, block) pairs of 4x4x4-cell (3D) or 8x8-cell (2D) output
    * blocks, sorted stably by block, and their work items (dense blocks are
@@ -156,6 +157,16 @@ int tlgb_interp_adjoint_scratch_size(const tlgb_interp_desc* d, const tlgb_inter
 /* out[b, p] = sum over taps of w(p, tap) * grid[b, tap]         (ungrid) */
 int tlgb_interp_forward(const tlgb_interp_desc* d, const tlgb_interp_plan_info* info, const void* plan,
                         const float* locs, const void* grid, void* out, tlgb_stream_t stream);
+
+/* The same with scratch (16-byte aligned, no initial contents needed), which
+ * tlgb_interp_forward_scratch_size sizes: 0 where it would not help, else room
+ * for the results in the order of the work items. For points in random order
+ * with a large output it is faster; with less scratch than that size, or none,
+ * the call does what tlgb_interp_forward does. */
+int tlgb_interp_forward_scratch_size(const tlgb_interp_desc* d, const tlgb_interp_plan_info* info, size_t* bytes);
+int tlgb_interp_forward_scratch(const tlgb_interp_desc* d, const tlgb_interp_plan_info* info, const void* plan,
+                                const float* locs, const void* grid, void* out, void* scratch,
+                                size_t scratch_bytes, tlgb_stream_t stream);
 
 /* grid[b, v] = sum over points p with v in their window of w(p, v) * vals[b, p]
  * (gridding). Every element of `grid` is written (no accumulation into the

@@ -461,7 +461,7 @@ __device__ __forceinline__ void for_lane_taps(const Geo& g, const Rec<NTB>& R, c
 
 // CTA = NW warps sharing one staged region (tile + halo, [x][y][z][batch]);
 // each warp interpolates 32 home points per batch.
-template <int N, int NDIM, int NTB, int NW, bool F3>
+template <int N, int NDIM, int NTB, int NW>
 __global__ void __launch_bounds__(NW * 32, 1) interp_fwd_kernel(Geo g, const int4* __restrict__ items,
                                                                 const int32_t* __restrict__ entries,
                                                                 const float* __restrict__ locs,
@@ -576,41 +576,7 @@ __global__ void __launch_bounds__(NW * 32, 1) interp_fwd_kernel(Geo g, const int
       VecF<N> acc;
 #pragma unroll
       for (int i = 0; i < N; ++i) acc.v[i] = 0.f;
-      bool done = false;
-      if constexpr (F3) {
-        // 3D, 8^3 tile + 4-wide halo (12^3 region), 8 complex batch entries
-        // (16 floats per voxel), <= 4 taps per dim: unrolled, immediate offsets
-        if (R.fast) {
-          constexpr int SZ = 16, SY = 12 * 16, SX = 12 * 12 * 16;
-          const bool zin = L.uz < R.m[2];
-          const float wz = zin ? R.wv[2][L.uz] : 0.f;
-          float wy[4];
-#pragma unroll
-          for (int ky = 0; ky < 4; ++ky) wy[ky] = ky < R.m[1] ? R.wv[1][ky] : 0.f;
-          const float* base = reg + (R.lc[0][0] * SX + R.lc[1][0] * SY + (R.lc[2][0] + L.uz) * SZ) + L.cu * 4;
-#pragma unroll
-          for (int i = 0; i < 2; ++i) {
-            const int kx = L.ux + 2 * i;
-            if (zin && kx < R.m[0]) {
-              const float wxz = R.wv[0][kx] * wz;
-              const float* bx = base + kx * SX;
-#pragma unroll
-              for (int ky = 0; ky < 4; ++ky) {
-                if (ky < R.m[1]) {
-                  const float w = wxz * wy[ky];
-                  const float4 v = *reinterpret_cast<const float4*>(bx + ky * SY);
-                  acc.v[0] = fmaf(w, v.x, acc.v[0]);
-                  acc.v[1] = fmaf(w, v.y, acc.v[1]);
-                  acc.v[2] = fmaf(w, v.z, acc.v[2]);
-                  acc.v[3] = fmaf(w, v.w, acc.v[3]);
-                }
-              }
-            }
-          }
-          done = true;
-        }
-      }
-      if (!done && L.cu < nunits) {
+      if (L.cu < nunits) {
         const float* base = reg + L.cu * N;
         for_lane_taps<NDIM, NTB>(g, R, L, [&](int lx, int ly, int lz, float w) {
           const VecF<N> v = ldv<N>(base + ((size_t)(lx * S[1] + ly) * S[2] + lz) * vstride);
@@ -802,12 +768,12 @@ __global__ void __launch_bounds__(32) interp_adj_kernel(Geo g, const int4* __res
 // rows' bytes.
 __device__ __forceinline__ float kern_precise(int kernel, float diff, float r, float d, float beta,
                                               float beta_lo) {
-  const float x = fabsf(d), xe = __fdiv_rn(fmaf(-x, r, fabsf(diff)), r);  // d = x + xe
+  const float x = fabsf(d), xe = __fdividef(fmaf(-x, r, fabsf(diff)), r);  // d = x + xe
   if (kernel != TLGB_KERNEL_KAISER_BESSEL) return fmaxf(1.0f - x - xe, 0.0f);
   const float p = x * x, pe = fmaf(x, x, -p) + 2.0f * x * xe;
   const float s = 1.0f - p, se = (1.0f - s) - p - pe;
   if (!(s > 0.f)) return 1.0f;  // I0(0)
-  const float q = __fsqrt_rn(s), qe = __fdiv_rn(fmaf(-q, q, s) + se, 2.0f * q);
+  const float q = __fsqrt_rn(s), qe = (fmaf(-q, q, s) + se) * 0.5f * rsqrtf(s);
   const float z = beta * q, ze = fmaf(beta, q, -z) + fmaf(beta_lo, q, beta * qe);
   if (z < 3.75f) {
     const float u = (z * (1.0f / 3.75f)) * (z * (1.0f / 3.75f));
@@ -817,35 +783,12 @@ __device__ __forceinline__ float kern_precise(int kernel, float diff, float r, f
                      u * (5.f * 0.0360768f + u * (6.f * 0.0045813f)))));
     return fmaf(dv * (2.0f / (3.75f * 3.75f)) * z, ze, v);
   }
-  const float v = __fdiv_rn(3.75f, z);
+  const float v = __fdividef(3.75f, z);
   const float h = 0.39894228f + v * (0.01328592f + v * (0.00225319f + v * (-0.00157565f + v * (0.00916281f +
                   v * (-0.02057706f + v * (0.02635537f + v * (-0.01647633f + v * 0.00392377f)))))));
-  const float f = __fdiv_rn(expf(z), __fsqrt_rn(z)) * h;
+  const float f = expf(z) * rsqrtf(z) * h;
   return fmaf(f, ze, f);
 }
-
-// A staged entry of the 3D 8-entry kernels in shared memory: the point's
-// weights, its view word (region_view) and the point index.
-struct __align__(16) R3 {
-  float4 w[3];
-  unsigned view;
-  int pad0, pad1;
-  int p;  // point index
-};
-
-// Per-point tap record, built with the plan for 3D geometries with 8^3 tiles
-// and at most 5 taps per dimension: the kernel weights of the first 4 valid
-// taps of each dimension (zero beyond), the position of the first valid tap
-// (wrapped into [0, N) in circular mode) and the number of valid taps per
-// dimension (cnt_x | cnt_y << 4 | cnt_z << 8; a zero count marks a point
-// without taps). Valid taps form one run of tap indices: |x - g| <= W/2 is
-// an interval, and so is [0, N) for zero padding.
-struct __align__(16) PRec {
-  float4 w[3];
-  int st[3];
-  int cnt;
-};
-static_assert(sizeof(PRec) == 64, "64-byte point records");
 
 // ------------------------------------------------ block lists (gridding)
 //
@@ -947,8 +890,8 @@ struct ScanJob {
   long long n;
   uint32_t* tot;
 };
-__global__ void __launch_bounds__(1024) plan_scan_kernel(ScanJob j0, ScanJob j1) {
-  const ScanJob j = blockIdx.x ? j1 : j0;
+__global__ void __launch_bounds__(1024) plan_scan_kernel(ScanJob j0, ScanJob j1, ScanJob j2) {
+  const ScanJob j = blockIdx.x == 2 ? j2 : (blockIdx.x ? j1 : j0);
   const long long per = (j.n + 1023) / 1024, b = threadIdx.x * per;
   const long long e = b + per < j.n ? b + per : j.n;
   uint4 s = make_uint4(0, 0, 0, 0);
@@ -982,8 +925,8 @@ __device__ __forceinline__ uint4 win_pairs(const Geo& g, const int4& w) {
 }
 
 // Per point: its window (first valid tap per dim, wrapped into [0, N) in
-// circular mode, and the tap counts; none when a dim has no valid tap), the
-// tap record (`recs`), and the tap rows over the blocks it meets (`rows`):
+// circular mode, and the tap counts; none when a dim has no valid tap) and the
+// tap rows over the blocks it meets (`rows`):
 // per active dim, one weight per cell of each block in axis_blocks order; a
 // cell outside the window holds -0.0 (valid weights are >= +0), so the sign
 // bit tells the gridding which cells the window covers. Each weight is
@@ -993,8 +936,8 @@ __device__ __forceinline__ uint4 win_pairs(const Geo& g, const int4& w) {
 // NTM: taps evaluated per dim, at least the geometry's.
 template <int NTM>
 __global__ void __launch_bounds__(kPlanPts) plan_points_kernel(Geo g, const float* __restrict__ locs,
-                                                               int4* __restrict__ win, PRec* __restrict__ recs,
-                                                               float* __restrict__ rows, uint4* __restrict__ sums) {
+                                                               int4* __restrict__ win, float* __restrict__ rows,
+                                                               uint4* __restrict__ sums) {
   extern __shared__ __align__(16) float prow[];  // [points][row_floats], when rows are wanted
   const long long p0 = (long long)blockIdx.x * kPlanPts, p = p0 + threadIdx.x;
   const bool on = p < g.npts;
@@ -1004,17 +947,14 @@ __global__ void __launch_bounds__(kPlanPts) plan_points_kernel(Geo g, const floa
     const float4 none = make_float4(-0.f, -0.f, -0.f, -0.f);
     for (int i = 0; i < RF / 4; ++i) reinterpret_cast<float4*>(mine)[i] = none;
   }
-  PRec R;
   int4 w4 = make_int4(0, 0, 0, 0);
-  int cnts = 0, rcnt = 0;
+  int cnts = 0;
   bool ok = on;
 #pragma unroll
   for (int e = 0; e < 3; ++e) {
-    float w[4] = {0.f, 0.f, 0.f, 0.f};
     int c = 0, st = 0;
     if (!g.act[e]) {
-      w[0] = 1.f;  // a leading dimension of a 1D or 2D geometry: one tap of weight 1 at 0
-      c = 1;
+      c = 1;  // a leading dimension of a 1D or 2D geometry: one tap at 0
     } else if (on) {
       const float x = load_coord(g, locs, p, e);
       if (coord_ok(x)) {
@@ -1028,38 +968,25 @@ __global__ void __launch_bounds__(kPlanPts) plan_points_kernel(Geo g, const floa
           const Tap t = tap_eval(g, e, x, lower, k);
           if (!t.valid) continue;
           if (c == 0) st = g.pad == TLGB_PAD_CIRCULAR ? wrapi(lower + k, g.N[e]) : lower + k;
-          if (recs || rows) {
+          if (rows) {
             const float v = kern_precise(g.kernel, __fsub_rn(x, (float)(lower + k)), g.r[e], t.d, g.beta, g.beta_lo);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) w[i] = c == i ? v : w[i];
-            if (rows) {
-              int cell = st + c;
-              if (cell >= g.N[e]) cell -= g.N[e];
-              if (cell >> lg != prev) row += 1 << lg, prev = cell >> lg;
-              row[cell & ((1 << lg) - 1)] = v;
-            }
+            int cell = st + c;
+            if (cell >= g.N[e]) cell -= g.N[e];
+            if (cell >> lg != prev) row += 1 << lg, prev = cell >> lg;
+            row[cell & ((1 << lg) - 1)] = v;
           }
           ++c;
         }
       }
     }
     if (c == 0) ok = false;
-    R.w[e] = make_float4(w[0], w[1], w[2], w[3]);
-    R.st[e] = st;
-    rcnt |= c << (4 * e);
     cnts |= c << (kWinBits * e);
     if (e == 0) w4.x = st;
     if (e == 1) w4.y = st;
     if (e == 2) w4.z = st;
   }
   w4.w = ok ? cnts : 0;
-  if (on) {
-    win[p] = w4;
-    if (recs) {
-      R.cnt = rcnt;
-      recs[p] = R;
-    }
-  }
+  if (on) win[p] = w4;
   uint4 tot;
   cta_scan4<kPlanPts>(on ? win_pairs(g, w4) : make_uint4(0, 0, 0, 0), tot);  // its barriers also publish the rows
   if (threadIdx.x == 0) sums[blockIdx.x] = tot;
@@ -1131,17 +1058,37 @@ __global__ void __launch_bounds__(256) plan_starts_kernel(const uint32_t* __rest
   (blk ? bstart : tstart)[k] = lo;
 }
 
-// Work units the items are made from: tiles, in order, and rows of kCube
-// blocks along z, in the order of the cubes of kCube^3 blocks (kCube^2 in
-// 2D), so that the blocks a point meets are worked on close together in time
-// and find its rows and values in L2.
+// Work units the items are made from: tiles, in the order of cubes of
+// kTileCube^3 tiles (squares in 2D), and rows of kCube blocks along z, in the
+// order of the cubes of kCube^3 blocks (kCube^2 in 2D). Neighbouring regions
+// are so gathered close together in time and find their shared halos in L2,
+// and the blocks a point meets its rows and values. Gathering 8 x 256^3 at
+// 2^21 points of a ball in random order: 735 us in plain tile order, 587 in
+// cubes of 2, 592 of 4, 590 of 8; 8 x 160^3 at 2^18 even points: 176, 153, 186,
+// 198 us.
+constexpr int kTileCube = 2;
 struct PlanUnits {
-  long long ntiles, nrows;       // units
+  long long ntiles, ntu, nrows;  // tiles; units: of tiles (some outside the grid), of block rows
+  int ntx, nty, ntz;             // tiles per dim
   int nbx, nby, nbz;             // blocks per dim
   int ncy, ncz;                  // cubes along y and z
   int per;                       // rows per cube
   int tile_ctas;
 };
+
+// the tile of unit u, -1 outside the grid
+__device__ __forceinline__ long long unit_tile(const PlanUnits& U, long long u) {
+  constexpr int C = kTileCube;
+  if (u >= U.ntu) return -1;
+  const int cx = U.ntx == 1 ? 1 : C, in = (int)(u % (cx * C * C));
+  long long q = u / (cx * C * C);
+  const int cy = (U.nty + C - 1) / C, cz = (U.ntz + C - 1) / C;
+  const int z = (int)(q % cz) * C + in % C;
+  q /= cz;
+  const int y = (int)(q % cy) * C + in / C % C, x = (int)(q / cy) * cx + in / (C * C);
+  if (x >= U.ntx || y >= U.nty || z >= U.ntz) return -1;
+  return ((long long)x * U.nty + y) * U.ntz + z;
+}
 
 // the blocks [b0, b0 + n) of row unit u (n = 0: outside the grid)
 __device__ __forceinline__ int row_blocks(const PlanUnits& U, long long u, int& b0) {
@@ -1158,7 +1105,7 @@ __device__ __forceinline__ int row_blocks(const PlanUnits& U, long long u, int& 
 
 __device__ __forceinline__ int parts_of(int n, int chunk) { return (n + chunk - 1) / chunk; }
 
-// Item counts of a unit. Tile: gather items, gridding items, parts of split
+// Item counts of a unit (`u`: a tile or a block row). Tile: gather items, gridding items, parts of split
 // tiles, split tiles. Block row: items, parts of split blocks, split blocks.
 // A run of empty blocks of the row is one item.
 __device__ __forceinline__ uint4 unit_items(const PlanUnits& U, bool tile, long long u, const uint32_t* tstart,
@@ -1192,38 +1139,51 @@ __device__ __forceinline__ uint4 unit_items(const PlanUnits& U, bool tile, long 
 
 __global__ void __launch_bounds__(kPlanPts) plan_count_items_kernel(PlanUnits U, const uint32_t* __restrict__ tstart,
                                                                     const uint32_t* __restrict__ bstart, int fwd_chunk,
-                                                                    int adj_chunk, uint4* __restrict__ sums) {
+                                                                    int adj_chunk, uint4* __restrict__ sums,
+                                                                    uint4* __restrict__ homes) {
   const bool tile = (int)blockIdx.x < U.tile_ctas;
   const long long u = (long long)(blockIdx.x - (tile ? 0 : U.tile_ctas)) * kPlanPts + threadIdx.x;
   uint4 c = make_uint4(0, 0, 0, 0), tot;
-  if (u < (tile ? U.ntiles : U.nrows)) c = unit_items(U, tile, u, tstart, bstart, fwd_chunk, adj_chunk);
+  const long long t = tile ? unit_tile(U, u) : (u < U.nrows ? u : -1);
+  if (t >= 0) c = unit_items(U, tile, t, tstart, bstart, fwd_chunk, adj_chunk);
   cta_scan4<kPlanPts>(c, tot);
   if (threadIdx.x == 0) sums[blockIdx.x] = tot;
+  if (!tile) return;
+  c = make_uint4(0, 0, 0, 0);
+  if (t >= 0) c.x = tstart[2 * t + 1] - tstart[2 * t];
+  cta_scan4<kPlanPts>(c, tot);
+  if (threadIdx.x == 0) homes[blockIdx.x] = tot;
 }
 
-// The items at their places. Gather items are in tile order, so neighbouring
-// regions are read while their shared halos are in L2. The tile gridding's
+// The items at their places. A gather item is (tile, its entries [begin,
+// end), index of its first point among the home points in item order). The tile gridding's
 // items and the split blocks go to `adj` / `bsplit` with sort keys: they are
 // put in falling order of their length afterwards (a long item or a long sum
 // that starts last is waited for alone).
 __global__ void __launch_bounds__(kPlanPts) plan_emit_items_kernel(
     PlanUnits U, const uint32_t* __restrict__ tstart, const uint32_t* __restrict__ bstart, int fwd_chunk, int adj_chunk,
-    const uint4* __restrict__ sums, int4* __restrict__ fwd, int4* __restrict__ adj, uint32_t* __restrict__ akey,
+    const uint4* __restrict__ sums, const uint4* __restrict__ homes, int4* __restrict__ fwd, int4* __restrict__ adj, uint32_t* __restrict__ akey,
     int32_t* __restrict__ aidx, int4* __restrict__ split, int4* __restrict__ bitems, int4* __restrict__ bsplit,
     uint32_t* __restrict__ skey, int32_t* __restrict__ sidx) {
   const bool tile = (int)blockIdx.x < U.tile_ctas;
   const long long u = (long long)(blockIdx.x - (tile ? 0 : U.tile_ctas)) * kPlanPts + threadIdx.x;
-  const bool on = u < (tile ? U.ntiles : U.nrows);
+  const long long ut = tile ? unit_tile(U, u) : (u < U.nrows ? u : -1);
+  const bool on = ut >= 0;
   uint4 c = make_uint4(0, 0, 0, 0), tot;
-  if (on) c = unit_items(U, tile, u, tstart, bstart, fwd_chunk, adj_chunk);
-  uint4 o = cta_scan4<kPlanPts>(c, tot);
+  if (on) c = unit_items(U, tile, ut, tstart, bstart, fwd_chunk, adj_chunk);
+  uint4 o = cta_scan4<kPlanPts>(c, tot), ho = make_uint4(0, 0, 0, 0);
+  if (tile) {
+    if (on) ho.x = tstart[2 * ut + 1] - tstart[2 * ut];
+    ho = cta_scan4<kPlanPts>(ho, tot);
+  }
   if (!on) return;
   const uint4 base = sums[blockIdx.x];
   o.x += base.x, o.y += base.y, o.z += base.z, o.w += base.w;
   if (tile) {
-    const int b = (int)tstart[2 * u], h = (int)tstart[2 * u + 1], e = (int)tstart[2 * u + 2], t = (int)u;
+    const int b = (int)tstart[2 * ut], h = (int)tstart[2 * ut + 1], e = (int)tstart[2 * ut + 2], t = (int)ut;
+    const int h0 = (int)(homes[blockIdx.x].x + ho.x);
     for (int k = 0; k < (int)c.x; ++k)
-      fwd[o.x + k] = make_int4(t, b + k * fwd_chunk, min(h, b + (k + 1) * fwd_chunk), -1);
+      fwd[o.x + k] = make_int4(t, b + k * fwd_chunk, min(h, b + (k + 1) * fwd_chunk), h0 + k * fwd_chunk);
     if (c.w) split[o.w] = make_int4(t, (int)o.z, (int)c.z, 0);
     for (int k = 0; k < (int)c.y; ++k) {
       const int q0 = b + k * adj_chunk, q1 = min(e, q0 + adj_chunk);
@@ -1271,41 +1231,6 @@ __global__ void __launch_bounds__(256) plan_order_kernel(const uint32_t* __restr
     else
       adj_out[i] = adj[aidx[i]];
   }
-}
-
-// The gather view of a home record in the 12^3 region at o: region base
-// (11 bits) | mx << 11 | my << 14 | mz << 17 | fast << 20 | ok << 21. The
-// region is staged with wrap, so the window is always one run there.
-__device__ __forceinline__ unsigned region_view(const Geo& g, const PRec& R, const int (&o)[3]) {
-  const int c = R.cnt;
-  const int cx = c & 15, cy = (c >> 4) & 15, cz = (c >> 8) & 15;
-  const bool ok = cx && cy && cz;
-  int f[3];
-#pragma unroll
-  for (int e = 0; e < 3; ++e) {
-    int d = R.st[e] - o[e];
-    if (g.pad == TLGB_PAD_CIRCULAR && d < 0) d += g.N[e];
-    f[e] = d;
-  }
-  const bool fast = ok && cx <= 4 && cy <= 4 && cz <= 4 && f[0] >= 0 && f[0] < 8 && f[1] >= 0 && f[1] < 8 &&
-                    f[2] >= 0 && f[2] < 8;
-  const unsigned base = fast ? (unsigned)((f[0] * 12 + f[1]) * 12 + f[2]) : 0u;
-  return base | (min(cx, 7) << 11) | (min(cy, 7) << 14) | (min(cz, 7) << 17) | ((fast ? 1u : 0u) << 20) |
-         ((ok ? 1u : 0u) << 21);
-}
-
-__device__ __forceinline__ PRec load_prec(const PRec* __restrict__ recs, long long p) {
-  const float4* q = reinterpret_cast<const float4*>(recs + p);
-  PRec R;
-  R.w[0] = __ldg(q);
-  R.w[1] = __ldg(q + 1);
-  R.w[2] = __ldg(q + 2);
-  const int4 t = __ldg(reinterpret_cast<const int4*>(q + 3));
-  R.st[0] = t.x;
-  R.st[1] = t.y;
-  R.st[2] = t.z;
-  R.cnt = t.w;
-  return R;
 }
 
 // Compensated summation (Neumaier's variant of Kahan's method): s + c
@@ -2035,449 +1960,472 @@ __global__ void __launch_bounds__(256) adj_reduce_bn_kernel(Geo g, const int4* _
       make_float2(sum.x + comp.x, sum.y + comp.y);
 }
 
-// Gather: CTA = 8 warps sharing one 12^3 x CG-entry region ([entry][x][y][z],
-// loaded by one TMA bulk tensor copy when the region needs no wrap). Each warp
-// takes every 8th point of the item, building the records of its next 8
-// points itself (kGB = 8 warps x 8 slots). Lanes = (point, entry, z-tap): a
-// lane sums its entry's 4 y-taps x 4 x-taps, then the 4 z-tap lanes add up.
-// CG = 8 (two CTAs per SM): one point per step across the lanes, two steps
-// interleaved. CG = 1, 2 or 4 (batches of at most 4 entries, 4 CTAs per SM):
-// 8 / CG points per step, so a one-entry batch stages and reads an eighth
-// of the region.
-constexpr int kGB = 64;
+// ------------------------------------------------------------------ gather
+//
+// Ungridding of complex values in 2D and 3D from the plan's gather records.
+// A persistent CTA works through units: one item (at most kGatherPts home
+// points of one tile) and a run of groups of CG batch entries. The tile's
+// region (12^3 cells in 3D; 20^2, or 24^2 for kernels of more than 5 taps, in
+// 2D) of a group is one stage of a ring of NST buffers in shared memory, the
+// item's records one of two record buffers, each with a full and an empty
+// mbarrier. Five producer warps fill them ahead of the NW consumer warps: the
+// region by one TMA tensor copy when it needs no wrap and its rows are 16-byte
+// multiples, else by 8-byte asynchronous copies; the records, which lie in
+// the items' order, by one bulk copy. So a copy's latency is paid once per
+// CTA, not once per item (with one CTA per item, a tile of 33 points cost
+// 8.6 us of latency and its 110 KB of copies 1.3).
+// A consumer warp takes PPW points per step: lane = (point h, entry c, z tap
+// kz); a lane sums its entry's y (and x) taps for EPL entries, the 4 z-tap
+// lanes add up. The regions of the entries are a multiple of 128 bytes
+// apart (the same banks), so lane group l reads its y taps from row l & 3 on:
+// one load of a half-warp then spans all banks.
+// Every wait is bounded: on a timeout the warp sets the device status and a
+// CTA flag and returns, the producer waits (bounded) for its copies in flight.
+constexpr int kGatherPts = 256;
+constexpr int kGatherProd = 160;  // producer threads (a 12 x 12 plane of a 3D region takes 144)
 
-template <int CG>
-__global__ void __launch_bounds__(256, CG == 8 ? 2 : 4) fwd_f3_kernel(const __grid_constant__ CUtensorMap tmap,
-                                                                      int use_tma, Geo g,
-                                                                      const int4* __restrict__ items,
-                                                                      const int32_t* __restrict__ entries,
-                                                                      const PRec* __restrict__ precs,
-                                                                      const float* __restrict__ locs,
-                                                                      const float* __restrict__ gridv,
-                                                                      float* __restrict__ out) {
-  constexpr int S = 12, PLANE = S * S, VOL = S * S * S, NW = 8;
-  constexpr int PPW = 8 / CG;  // points per warp step
-  constexpr uint32_t RBYTES = VOL * CG * 8;
-  extern __shared__ __align__(128) unsigned char smem[];
-  float2* reg = reinterpret_cast<float2*>(smem);               // [8][12][12][12]
-  R3* rec = reinterpret_cast<R3*>(smem + RBYTES);              // [kGB]
-  Rec<5>* slow = reinterpret_cast<Rec<5>*>(rec + kGB);         // [NW]
-  static_assert((kGB * sizeof(R3) + NW * sizeof(Rec<5>)) % 8 == 0, "mbarrier alignment");
-  uint64_t* bar = reinterpret_cast<uint64_t*>(slow + NW);
+template <int NDIM, int KT>
+struct __align__(16) GatherRec {
+  float w[NDIM][KT];  // weights of the first KT valid taps per dim, zero beyond
+  unsigned view;      // region cell of the first tap | fast << 20 | ok << 21
+  int p;              // point index
+  int pad[2];
+};
+static_assert(sizeof(GatherRec<3, 4>) == 64 && sizeof(GatherRec<2, 4>) == 48 && sizeof(GatherRec<2, 8>) == 80, "records");
+
+// region edge along an active dim: the tile and one cell more than KT - 1,
+// for windows of KT + 1 taps (exact-integer coordinates)
+template <int NDIM, int KT>
+constexpr int region_edge() { return (NDIM == 3 ? 8 : 16) + KT; }
+template <int NDIM, int KT>
+constexpr int region_cells() {
+  return (NDIM == 3 ? region_edge<NDIM, KT>() : 1) * region_edge<NDIM, KT>() * region_edge<NDIM, KT>();
+}
+
+template <int NDIM, int KT>
+struct SlowTaps {  // a window of more than KT taps, one per consumer warp
+  float w[NDIM][KT + 1];
+  int n[NDIM], f[NDIM];
+};
+
+template <int NDIM, int KT, int CG, int NW, int NST>
+constexpr size_t gather_smem() {
+  return (size_t)NST * region_cells<NDIM, KT>() * CG * 8 + 2 * kGatherPts * sizeof(GatherRec<NDIM, KT>) +
+         NW * sizeof(SlowTaps<NDIM, KT>) + 8 * (2 * NST + 4) + 16;
+}
+
+__device__ __forceinline__ void item_origin(const Geo& g, int tile, int (&o)[3]) {
+  int t = tile;
+  o[2] = (t % g.nt[2]) * g.T[2];
+  t /= g.nt[2];
+  o[1] = (t % g.nt[1]) * g.T[1];
+  o[0] = (t / g.nt[1]) * g.T[0];
+}
+
+// One record per home point, in the order of the gather items' points
+// (item.w is the first one's index), so an item's records are one run. For 3D
+// plans also each point's place in that order (`rank`), and of every 16th
+// item's points (jumps[-1]) how many lie in another 32-byte sector of an output
+// row than the point before (jumps[0]: nearly all for points in random order,
+// a quarter in runs).
+template <int NDIM, int KT, bool FROM_ROWS>
+__global__ void __launch_bounds__(128) plan_records_kernel(Geo g, const uint32_t* __restrict__ cnt,
+                                                           const int4* __restrict__ win,
+                                                           const float* __restrict__ rows,
+                                                           const int4* __restrict__ items,
+                                                           const int32_t* __restrict__ entries,
+                                                           const float* __restrict__ locs,
+                                                           GatherRec<NDIM, KT>* __restrict__ recs,
+                                                           int32_t* __restrict__ rank, uint32_t* __restrict__ jumps) {
+  constexpr int S = region_edge<NDIM, KT>();
+  if (blockIdx.x >= cnt[4]) return;
   const int4 it = items[blockIdx.x];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int c0 = blockIdx.y * CG;
   int o[3];
-  {
-    int t = it.x;
-    o[2] = (t % g.nt[2]) * 8;
-    t /= g.nt[2];
-    o[1] = (t % g.nt[1]) * 8;
-    o[0] = (t / g.nt[1]) * 8;
-  }
-  // the region needs wrap in circular mode when it crosses the upper edge
-  const bool wraps = g.pad == TLGB_PAD_CIRCULAR && (o[0] + S > g.N[0] || o[1] + S > g.N[1] || o[2] + S > g.N[2]);
-  const bool tma = use_tma && !wraps;
-  if (tma) {
-    if (tid == 0) {
-      mbar_init(bar, 1);
-      fence_mbar_init();
-    }
-    __syncthreads();
-    if (tid == 0) {
-      if (!g.skip_copy) {  // test hook: nothing in flight, so the bounded wait runs out
-        mbar_arrive_expect_tx(bar, RBYTES);
-        tma_load_4d(reg, &tmap, bar, o[2], o[1], o[0], c0);
-      }
-    }
-  } else {
-    // plain loads with wrap / zero fill: rows (entry, x, y) of 12 z
-    const int ncoil = (int)min((long long)CG, g.nbatch - c0);
-    const long long gvol = (long long)g.N[0] * g.N[1] * g.N[2];
-    for (int idx = tid; idx < CG * VOL; idx += NW * 32) {
-      const int z = idx % S;
-      const int r = idx / S;
-      const int y = r % S, x = (r / S) % S, c = r / PLANE;
-      int gx = o[0] + x, gy = o[1] + y, gz = o[2] + z;
-      bool in = c < ncoil;
-      if (g.pad == TLGB_PAD_CIRCULAR) {
-        gx = wrapi(gx, g.N[0]);
-        gy = wrapi(gy, g.N[1]);
-        gz = wrapi(gz, g.N[2]);
+  item_origin(g, it.x, o);
+  for (int j = it.y + threadIdx.x; j < it.z; j += 128) {
+    const int p = entries[j];
+    GatherRec<NDIM, KT> R;
+    unsigned base = 0;
+    bool fast = true;
+    int4 w4;
+    if constexpr (FROM_ROWS) w4 = win[p];
+#pragma unroll
+    for (int d = 0; d < NDIM; ++d) {
+      const int e = d + 3 - NDIM;
+      int c = 0, st = 0;
+      float w[KT + 1];
+#pragma unroll
+      for (int k = 0; k <= KT; ++k) w[k] = 0.f;
+      if constexpr (FROM_ROWS) {
+        // the window's weights are the row's cells with a clear sign, in order
+        st = win_st(w4, e), c = win_cnt(w4, e);
+        constexpr int EDGE = NDIM == 3 ? 4 : 8;
+        const float4* row = reinterpret_cast<const float4*>(rows + (long long)p * row_floats(NDIM, g.nrow) + d * g.nrow * EDGE);
+        int i0 = 0;
+        for (int q = 0; q < g.nrow * EDGE / 4; ++q) {
+          const float4 v4 = __ldg(row + q);
+          const float v[4] = {v4.x, v4.y, v4.z, v4.w};
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            if (signbit(v[k])) continue;
+#pragma unroll
+            for (int i = 0; i < KT; ++i) w[i] = i0 == i ? v[k] : w[i];
+            ++i0;
+          }
+        }
       } else {
-        in = in && gx < g.N[0] && gy < g.N[1] && gz < g.N[2];
+        const float x = load_coord(g, locs, p, e);
+        const int lower = lower_of(g, e, x);
+#pragma unroll
+        for (int k = 0; k <= KT; ++k) {
+          if (k >= g.NT[e]) continue;
+          const Tap t = tap_eval(g, e, x, lower, k);
+          if (!t.valid) continue;
+          if (c == 0) st = g.pad == TLGB_PAD_CIRCULAR ? wrapi(lower + k, g.N[e]) : lower + k;
+          const float v = kern_precise(g.kernel, __fsub_rn(x, (float)(lower + k)), g.r[e], t.d, g.beta, g.beta_lo);
+#pragma unroll
+          for (int i = 0; i < KT; ++i) w[i] = c == i ? v : w[i];
+          ++c;
+        }
       }
-      reg[idx] = in ? __ldg(reinterpret_cast<const float2*>(gridv) + (long long)(c0 + c) * gvol +
-                           ((long long)gx * g.N[1] + gy) * g.N[2] + gz)
-                    : make_float2(0.f, 0.f);
+#pragma unroll
+      for (int k = 0; k < KT; ++k) R.w[d][k] = w[k];
+      // a home point's first tap lies in the tile
+      base = base * S + (unsigned)(st - o[e]);
+      fast = fast && c <= KT;
+    }
+    R.view = (fast ? base : 0u) | ((fast ? 1u : 0u) << 20) | (1u << 21);
+    R.p = p;
+    R.pad[0] = R.pad[1] = 0;
+    const float4* src = reinterpret_cast<const float4*>(&R);
+    float4* dst = reinterpret_cast<float4*>(recs + it.w + (j - it.y));
+#pragma unroll
+    for (int q = 0; q < (int)(sizeof(R) / 16); ++q) dst[q] = src[q];
+    if (rank) {
+      rank[p] = it.w + (j - it.y);
+      if (blockIdx.x % 16 == 0) {
+        const unsigned on = __activemask();
+        const unsigned m = __ballot_sync(on, j == it.y || entries[j - 1] >> 2 != p >> 2);
+        if ((threadIdx.x & 31) == 0) {
+          atomicAdd(jumps, (uint32_t)__popc(m));
+          atomicAdd(jumps - 1, (uint32_t)__popc(on));
+        }
+      }
     }
   }
-  // lane = (point q, entry c, z tap kz). Iteration t reads y tap (t + lane /
-  // 4) & 3: the 8 entries' regions are 13,824 B apart (the same banks), so
-  // rotating the y taps by lane group spreads one load instruction over 4
-  // bank windows.
-  const int q = lane / (4 * CG), c = (lane >> 2) % CG, kz = lane & 3;
+}
+
+template <int NDIM, int KT, int CG, int NW, int NST, int CTAS>
+__global__ void __launch_bounds__(NW * 32 + kGatherProd, CTAS)
+    gather_kernel(const __grid_constant__ CUtensorMap tmap, int use_tma, Geo g, const int4* __restrict__ items, int nruns,
+                  int run, int nunits, const GatherRec<NDIM, KT>* __restrict__ recs, const float* __restrict__ locs,
+                  const float* __restrict__ gridv, float* __restrict__ out, float* __restrict__ sorted) {
+  constexpr int S = region_edge<NDIM, KT>(), VOL = region_cells<NDIM, KT>(), PLANE = S * S;
+  constexpr int CL = CG < 4 ? CG : 4, EPL = CG / CL, PPW = 8 / CL;
+  constexpr uint32_t RBYTES = VOL * CG * 8;
+  using Rec = GatherRec<NDIM, KT>;
+  extern __shared__ __align__(128) unsigned char smem[];
+  Rec* recbuf = reinterpret_cast<Rec*>(smem + NST * RBYTES);
+  SlowTaps<NDIM, KT>* slow = reinterpret_cast<SlowTaps<NDIM, KT>*>(recbuf + 2 * kGatherPts);
+  uint64_t* full = reinterpret_cast<uint64_t*>((reinterpret_cast<uintptr_t>(slow + NW) + 7) & ~(uintptr_t)7);
+  uint64_t* empty = full + NST;
+  uint64_t* rfull = empty + NST;
+  uint64_t* rempty = rfull + 2;
+  __shared__ int failed;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (tid == 0) {
+    for (int i = 0; i < NST; ++i) {
+      mbar_init(&full[i], kGatherProd);
+      mbar_init(&empty[i], NW);
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&rfull[i], 1);
+      mbar_init(&rempty[i], NW);
+    }
+    fence_mbar_init();
+    failed = 0;
+  }
+  __syncthreads();
+  const uint32_t limit = g.skip_copy ? 1u : 1u << 22;  // test hook: nothing is copied, so the waits run out
+  const int ncg = (int)((g.nbatch + CG - 1) / CG);
+  volatile int* vfailed = &failed;
+  if (warp >= NW) {
+    // ---- producers
+    if (g.skip_copy) return;
+    const int pt = tid - NW * 32;
+    uint32_t k = 0, u_done = 0;
+    bool ok = true;
+    int4 next = blockIdx.x < nunits ? items[blockIdx.x / nruns] : make_int4(0, 0, 0, 0);
+    for (int u = blockIdx.x; u < nunits && ok; u += gridDim.x, ++u_done) {
+      const int4 it = next;
+      if (u + (int)gridDim.x < nunits) next = items[(u + gridDim.x) / nruns];
+      const int g0 = (u % nruns) * run, g1 = min(ncg, g0 + run);
+      int o[3];
+      item_origin(g, it.x, o);
+      bool wraps = false;
+      for (int e = 3 - NDIM; e < 3; ++e) wraps = wraps || (g.pad == TLGB_PAD_CIRCULAR && o[e] + S > g.N[e]);
+      const bool tma = use_tma && !wraps;
+      if (pt == 0) {
+        const uint32_t b = u_done & 1;
+        ok = mbar_wait_bounded(&rempty[b], ((u_done >> 1) & 1) ^ 1, limit);
+        if (ok) {
+          const uint32_t bytes = (uint32_t)(it.z - it.y) * (uint32_t)sizeof(Rec);
+          mbar_arrive_expect_tx(&rfull[b], bytes);
+          sm100::bulk_load(recbuf + b * kGatherPts, recs + it.w, bytes, &rfull[b]);
+        }
+      }
+      for (int cg = g0; cg < g1 && ok; ++cg, ++k) {
+        const uint32_t s = k % NST;
+        ok = mbar_wait_bounded(&empty[s], ((k / NST) & 1) ^ 1, limit) && !*vfailed;
+        if (!ok) break;
+        float2* reg = reinterpret_cast<float2*>(smem + s * RBYTES);
+        if (tma) {
+          if (pt == 0) {
+            sm100::fence_proxy_async_smem();  // the buffer may last have been filled by plain copies
+            mbar_arrive_expect_tx(&full[s], RBYTES);
+            tma_load_4d(reg, &tmap, &full[s], o[2], o[1], o[0], cg * CG);
+          } else {
+            sm100::mbar_arrive(&full[s]);
+          }
+          continue;
+        }
+        // a thread copies its (y, z) cells of every (entry, x) plane
+        constexpr int Q = (PLANE + kGatherProd - 1) / kGatherProd;
+        const long long gpl = (long long)g.N[1] * g.N[2], gvol = gpl * g.N[0];
+#pragma unroll
+        for (int q = 0; q < Q; ++q) {
+          const int cell = pt + q * kGatherProd;
+          if (cell >= PLANE) break;
+          const int y = cell / S, z = cell - y * S;
+          int gy = o[1] + y, gz = o[2] + z;
+          bool in = gy < g.N[1] && gz < g.N[2];
+          if (g.pad == TLGB_PAD_CIRCULAR) gy = wrapi(gy, g.N[1]), gz = wrapi(gz, g.N[2]), in = true;
+          const float2* src = reinterpret_cast<const float2*>(gridv) + (long long)(cg * CG) * gvol +
+                              (in ? (long long)gy * g.N[2] + gz : 0);
+          float2* dst = reg + cell;
+          for (int c = 0; c < CG; ++c, src += gvol) {
+            const bool cin = in && cg * CG + c < g.nbatch;
+            if constexpr (NDIM == 3) {
+              int gx = o[0];
+              const float2* sx = src + (long long)gx * gpl;
+              for (int x = 0; x < S; ++x, dst += PLANE, sx += gpl) {
+                bool xin = cin;
+                if (gx >= g.N[0]) {  // past the upper edge
+                  if (g.pad == TLGB_PAD_CIRCULAR)
+                    gx -= g.N[0], sx -= gvol;
+                  else
+                    xin = false;
+                }
+                sm100::cp_async8_zfill(dst, xin ? sx : reinterpret_cast<const float2*>(gridv), xin);
+                ++gx;
+              }
+            } else {
+              sm100::cp_async8_zfill(dst, cin ? src : reinterpret_cast<const float2*>(gridv), cin);
+              dst += PLANE;
+            }
+          }
+        }
+        sm100::cp_async_mbar_arrive(&full[s]);
+      }
+      ok = ok && !*vfailed;
+    }
+    if (!ok) {  // every copy lands before the CTA ends
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      if (pt == 0) {
+        *vfailed = 1;
+        atomicExch(&g_tlgb_status, 1);
+        for (uint32_t i = k > NST ? k - NST : 0; i < k; ++i) mbar_wait_bounded(&full[i % NST], (i / NST) & 1, limit);
+        for (uint32_t i = u_done > 1 ? u_done - 1 : 0; i <= u_done; ++i) mbar_wait_bounded(&rfull[i & 1], (i >> 1) & 1, 1u << 12);
+      }
+    }
+    return;
+  }
+  // ---- consumers
+  const int kz = lane & 3, c = (lane >> 2) % CL, h = lane / (4 * CL);
   int kyo[4], rowoff[4];
 #pragma unroll
   for (int t = 0; t < 4; ++t) {
     kyo[t] = (t + (lane >> 2)) & 3;
     rowoff[t] = kyo[t] * S;
   }
-  // Each warp takes the item's points warp, warp + 8, ... in mini-batches of
-  // 8 and keeps its own 8 record slots. Lanes 0-7 run two mini-batches
-  // ahead: the point indices of mini-batch m + 2 and the point records of
-  // m + 1 are in flight in registers while the warp gathers mini-batch m.
-  R3* wrec = rec + warp * 8;
-  const int npt = it.z - it.y;
-  auto point_at = [&](int base) -> int {
-    const int j = base + 8 * lane;
-    return (lane < 8 && j < npt) ? entries[it.y + j] : -1;
-  };
-  auto fetch = [&](int p) {
-    PRec R;
-    if (p >= 0) R = load_prec(precs, p);
-    return R;
-  };
-  auto publish = [&](int p, const PRec& R) {
-    if (p >= 0) {
-      R3& S = wrec[lane];
-      S.w[0] = R.w[0];
-      S.w[1] = R.w[1];
-      S.w[2] = R.w[2];
-      S.view = region_view(g, R, o);
-      S.p = p;
-    }
-    __syncwarp();
-  };
-  int pc = point_at(warp);           // mini-batch 0: indices
-  int pn = point_at(warp + 8 * NW);  // mini-batch 1: indices
-  PRec Rc = fetch(pc);               // mini-batch 0: records
-  auto build_records = [&](int base) {
-    publish(pc, Rc);  // the mini-batch at base
-    Rc = fetch(pn);   // the next one's records (its indices are in)
-    pc = pn;
-    pn = point_at(base + 16 * NW);  // the one after's indices
-  };
-  build_records(warp);  // while the region copy is in flight
-  {
-    // the copy must have landed: one thread polls (bounded), the others
-    // wait at the barrier without taking issue slots; then a CTA-wide vote
-    bool ok = true;
-    if (tma && tid == 0) ok = mbar_wait_bounded(bar, 0, g.skip_copy ? 1u : 1u << 22);
-    if (__syncthreads_or(!ok)) {
-      if (tid == 0) atomicExch(&g_tlgb_status, 1);
-      return;
-    }
-  }
-  {
-    // points of the plain-run view, two per step: sum over y taps of
-    // wy wz (sum over x taps of wx v). A record's weights are zero past its
-    // tap count, so taps outside the window contribute 0; every tap of the
-    // 4^3 box lies inside the staged region.
-    auto gather_box = [&](const R3& R) {
-      const float4 wx = R.w[0];
-      const float wz = (&R.w[2].x)[kz];
-      const float* wy = &R.w[1].x;
-      const float2* a = reg + c * VOL + (R.view & 2047) + kz;
-      // the box's farthest cell: 3 x, 3 y and the last z lane from the base
-      if (!TLGB_IN_RANGE((R.view & 2047) + kz + 3 * PLANE + 3 * S, VOL)) return make_float2(0.f, 0.f);
-      float2 acc = make_float2(0.f, 0.f);
-#pragma unroll
-      for (int t = 0; t < 4; ++t) {
-        const float wyz = wy[kyo[t]] * wz;
-        const float2* ar = a + rowoff[t];
-        float2 sx = mul2_bcast(wx.x, ar[0]);
-        fma2_bcast(sx, wx.y, ar[PLANE]);
-        fma2_bcast(sx, wx.z, ar[2 * PLANE]);
-        fma2_bcast(sx, wx.w, ar[3 * PLANE]);
-        acc.x = fmaf(wyz, sx.x, acc.x);
-        acc.y = fmaf(wyz, sx.y, acc.y);
-      }
-      return acc;
-    };
-    // the generic record path (exact-integer coordinates); with CG < 8 only
-    // the lanes of point group 0 sum (warp-uniform call)
-    auto gather_rec = [&](const R3& R) {
-      if (lane == 0) {
-        float x3[3];
-        for (int e = 0; e < 3; ++e) x3[e] = load_coord(g, locs, R.p, e);
-        lane_rec<5>(g, x3, o, true, slow[warp]);
-      }
-      __syncwarp();
-      const Rec<5>& Sr = slow[warp];
-      float2 acc = make_float2(0.f, 0.f);
-      if (q == 0)
-      for (int kzz = kz; kzz < Sr.m[2]; kzz += 4)
-        for (int kyy = 0; kyy < Sr.m[1]; ++kyy)
-          for (int kx = 0; kx < Sr.m[0]; ++kx) {
-            const float w = g.norm == 1 ? Sr.wv[0][kx] * Sr.wv[1][kyy] * Sr.wv[2][kzz]
-                                        : radial_w(g, Sr.wv[0][kx], Sr.wv[1][kyy], Sr.wv[2][kzz]);
-            const int ri = c * VOL + (Sr.lc[0][kx] * S + Sr.lc[1][kyy]) * S + Sr.lc[2][kzz];
-            if (TLGB_IN_RANGE(ri, CG * VOL)) fma2_bcast(acc, w, reg[ri]);
-          }
-      __syncwarp();
-      return acc;
-    };
-    // sum over the 4 z-tap lanes of each entry, then lane kz = 0 stores
-    auto finish = [&](float2 acc, int p, bool store) {
-      acc.x += __shfl_xor_sync(0xffffffffu, acc.x, 1);
-      acc.y += __shfl_xor_sync(0xffffffffu, acc.y, 1);
-      acc.x += __shfl_xor_sync(0xffffffffu, acc.x, 2);
-      acc.y += __shfl_xor_sync(0xffffffffu, acc.y, 2);
-      if (store && kz == 0 && c0 + c < g.nbatch && TLGB_IN_RANGE(p, g.npts))
-        *reinterpret_cast<float2*>(out + ((long long)(c0 + c) * g.npts + p) * 2) = acc;
-    };
-    auto one = [&](const R3& R) {
-      const unsigned view = R.view;
-      if (!((view >> 21) & 1)) return;  // no valid tap (warp-uniform)
-      const bool box = (view >> 20) & 1;
-      finish(box ? gather_box(R) : gather_rec(R), R.p, box || q == 0);
-    };
-    for (int base = warp; base < npt; base += 8 * NW) {
-      if (base != warp) {
-        __syncwarp();  // the previous mini-batch has been read
-        build_records(base);
-      }
-      const int nb = min(8, (npt - base + NW - 1) / NW);
-      if constexpr (CG == 8) {
-        int i = 0;
-        for (; i + 1 < nb; i += 2) {
-          const R3& R0 = wrec[i];
-          const R3& R1 = wrec[i + 1];
-          if ((R0.view & R1.view) >> 20 & 1) {
-            // both on the plain-run path (which implies a valid tap): interleaved
-            const float2 a0 = gather_box(R0), a1 = gather_box(R1);
-            finish(a0, R0.p, true);
-            finish(a1, R1.p, true);
-          } else {
-            one(R0);
-            one(R1);
-          }
-        }
-        if (i < nb) one(wrec[i]);
-      } else {
-        for (int i0 = 0; i0 < nb; i0 += PPW) {
-          // the plain-run points of this step, one per lane group
-          const int i = i0 + q;
-          const R3& R = wrec[i < nb ? i : i0];
-          const bool box = i < nb && ((R.view >> 20) & 1);
-          finish(box ? gather_box(R) : make_float2(0.f, 0.f), R.p, box);
-          // then the step's points with a valid tap off that path, one at a
-          // time by the whole warp
-#pragma unroll 1
-          for (int k = 0; k < PPW && i0 + k < nb; ++k) {
-            const unsigned v = wrec[i0 + k].view;
-            if (((v >> 21) & 1) && !((v >> 20) & 1)) finish(gather_rec(wrec[i0 + k]), wrec[i0 + k].p, q == 0);
-          }
-        }
-      }
-    }
-  }
-}
-
-// The gather view of a home record in the 20 x 20 region of a 2D tile at o:
-// region base (y * 20 + z, 9 bits) | my << 11 | mz << 14 | fast << 20 |
-// ok << 21 (the bit positions of region_view).
-__device__ __forceinline__ unsigned region_view2(const Geo& g, const PRec& R, const int (&o)[3]) {
-  const int c = R.cnt;
-  const int cy = (c >> 4) & 15, cz = (c >> 8) & 15;
-  const bool ok = (c & 15) && cy && cz;
-  int f[3];
-#pragma unroll
-  for (int e = 1; e < 3; ++e) {
-    int d = R.st[e] - o[e];
-    if (g.pad == TLGB_PAD_CIRCULAR && d < 0) d += g.N[e];
-    f[e] = d;
-  }
-  const bool fast = ok && cy <= 4 && cz <= 4 && f[1] >= 0 && f[1] < 16 && f[2] >= 0 && f[2] < 16;
-  const unsigned base = fast ? (unsigned)(f[1] * 20 + f[2]) : 0u;
-  return base | (min(cy, 7) << 11) | (min(cz, 7) << 14) | ((fast ? 1u : 0u) << 20) | ((ok ? 1u : 0u) << 21);
-}
-
-// 2D gather: CTA = 8 warps sharing the 20 x 20 x 8-entry region
-// ([entry][y][z]) of one 16 x 16 tile, loaded by one TMA bulk tensor copy
-// when the region needs no wrap. Each warp takes every 8th point of the
-// item, building the records of its next 8 points itself, two mini-batches
-// ahead. Lanes = (entry, z-tap): a lane sums its entry's 4 y-taps, two points
-// at a time, then the 4 z-tap lanes of each entry add up; the y taps of entry
-// c start at row (c & 3), so one load instruction spans 4 bank windows.
-__global__ void __launch_bounds__(256, 3) fwd_f2_kernel(const __grid_constant__ CUtensorMap tmap, int use_tma, Geo g,
-                                                        const int4* __restrict__ items,
-                                                        const int32_t* __restrict__ entries,
-                                                        const PRec* __restrict__ precs,
-                                                        const float* __restrict__ locs,
-                                                        const float* __restrict__ gridv, float* __restrict__ out) {
-  constexpr int CG = 8, S = 20, VOL = S * S, NW = 8;
-  constexpr uint32_t RBYTES = VOL * CG * 8;
-  extern __shared__ __align__(128) unsigned char smem[];
-  float2* reg = reinterpret_cast<float2*>(smem);               // [8][20][20]
-  R3* rec = reinterpret_cast<R3*>(smem + RBYTES);              // [8 warps][8]
-  Rec<5>* slow = reinterpret_cast<Rec<5>*>(rec + 64);          // [NW]
-  static_assert((64 * sizeof(R3) + NW * sizeof(Rec<5>)) % 8 == 0, "mbarrier alignment");
-  uint64_t* bar = reinterpret_cast<uint64_t*>(slow + NW);
-  const int4 it = items[blockIdx.x];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int c0 = blockIdx.y * CG;
-  int o[3];
-  {
-    int t = it.x;
-    o[2] = (t % g.nt[2]) * g.T[2];
-    t /= g.nt[2];
-    o[1] = (t % g.nt[1]) * g.T[1];
-    o[0] = 0;
-  }
-  const bool wraps = g.pad == TLGB_PAD_CIRCULAR && (o[1] + S > g.N[1] || o[2] + S > g.N[2]);
-  const bool tma = use_tma && !wraps;
-  if (tma) {
-    if (tid == 0) {
-      mbar_init(bar, 1);
-      fence_mbar_init();
-    }
-    __syncthreads();
-    if (tid == 0) {
-      if (!g.skip_copy) {  // test hook: nothing in flight, so the bounded wait runs out
-        mbar_arrive_expect_tx(bar, RBYTES);
-        tma_load_4d(reg, &tmap, bar, o[2], o[1], 0, c0);
-      }
-    }
-  } else {
-    // plain loads with wrap / zero fill: rows (entry, y) of 20 z
-    const int ncoil = (int)min((long long)CG, g.nbatch - c0);
-    const long long gvol = (long long)g.N[1] * g.N[2];
-    for (int idx = tid; idx < CG * VOL; idx += NW * 32) {
-      const int z = idx % S;
-      const int r = idx / S;
-      const int y = r % S, c = r / S;
-      int gy = o[1] + y, gz = o[2] + z;
-      bool in = c < ncoil;
-      if (g.pad == TLGB_PAD_CIRCULAR) {
-        gy = wrapi(gy, g.N[1]);
-        gz = wrapi(gz, g.N[2]);
-      } else {
-        in = in && gy < g.N[1] && gz < g.N[2];
-      }
-      reg[idx] = in ? __ldg(reinterpret_cast<const float2*>(gridv) + (long long)(c0 + c) * gvol +
-                           (long long)gy * g.N[2] + gz)
-                    : make_float2(0.f, 0.f);
-    }
-  }
-  const int c = lane >> 2, kz = lane & 3;
-  int kyo[4], rowoff[4];
-#pragma unroll
-  for (int t = 0; t < 4; ++t) {
-    kyo[t] = (t + c) & 3;
-    rowoff[t] = kyo[t] * S;
-  }
-  R3* wrec = rec + warp * 8;
-  const int npt = it.z - it.y;
-  auto point_at = [&](int base) -> int {
-    const int j = base + 8 * lane;
-    return (lane < 8 && j < npt) ? entries[it.y + j] : -1;
-  };
-  auto fetch = [&](int p) {
-    PRec R;
-    if (p >= 0) R = load_prec(precs, p);
-    return R;
-  };
-  auto publish = [&](int p, const PRec& R) {
-    if (p >= 0) {
-      R3& Sr = wrec[lane];
-      Sr.w[0] = R.w[0];
-      Sr.w[1] = R.w[1];
-      Sr.w[2] = R.w[2];
-      Sr.view = region_view2(g, R, o);
-      Sr.p = p;
-    }
-    __syncwarp();
-  };
-  int pc = point_at(warp);
-  int pn = point_at(warp + 8 * NW);
-  PRec Rc = fetch(pc);
-  auto build_records = [&](int base) {
-    publish(pc, Rc);
-    Rc = fetch(pn);
-    pc = pn;
-    pn = point_at(base + 16 * NW);
-  };
-  build_records(warp);  // while the region copy is in flight
-  {
-    bool ok = true;
-    if (tma && tid == 0) ok = mbar_wait_bounded(bar, 0, g.skip_copy ? 1u : 1u << 22);
-    if (__syncthreads_or(!ok)) {
-      if (tid == 0) atomicExch(&g_tlgb_status, 1);
-      return;
-    }
-  }
-  // sum over y taps of wy wz v; weights are zero past a record's tap count
-  // and every tap of the 4 x 4 box lies inside the region
-  auto gather_box = [&](const R3& R) {
-    const float wz = (&R.w[2].x)[kz];
-    const float* wy = &R.w[1].x;
-    const float2* a = reg + c * VOL + (R.view & 2047) + kz;
-    float2 acc = make_float2(0.f, 0.f);
-#pragma unroll
-    for (int t = 0; t < 4; ++t) {
-      const float w = wy[kyo[t]] * wz;
-      const float2 v = a[rowoff[t]];
-      acc.x = fmaf(w, v.x, acc.x);
-      acc.y = fmaf(w, v.y, acc.y);
-    }
-    return acc;
-  };
-  auto gather_rec = [&](const R3& R) {
+  auto give_up = [&]() {
     if (lane == 0) {
-      float x3[3] = {0.f, 0.f, 0.f};
-      for (int e = 1; e < 3; ++e) x3[e] = load_coord(g, locs, R.p, e);
-      lane_rec<5>(g, x3, o, true, slow[warp]);
+      *vfailed = 1;
+      atomicExch(&g_tlgb_status, 1);
     }
-    __syncwarp();
-    const Rec<5>& Sr = slow[warp];
-    float2 acc = make_float2(0.f, 0.f);
-    if (Sr.m[0] > 0)
-      for (int kzz = kz; kzz < Sr.m[2]; kzz += 4)
-        for (int kyy = 0; kyy < Sr.m[1]; ++kyy) {
-          const float w = Sr.wv[1][kyy] * Sr.wv[2][kzz];
-          const int ri = c * VOL + Sr.lc[1][kyy] * S + Sr.lc[2][kzz];
-          const float2 v = TLGB_IN_RANGE(ri, CG * VOL) ? reg[ri] : make_float2(0.f, 0.f);
-          acc.x = fmaf(w, v.x, acc.x);
-          acc.y = fmaf(w, v.y, acc.y);
+  };
+  uint32_t k = 0, ui = 0;
+  int4 next = blockIdx.x < nunits ? items[blockIdx.x / nruns] : make_int4(0, 0, 0, 0);
+  for (int u = blockIdx.x; u < nunits; u += gridDim.x, ++ui) {
+    const int4 it = next;
+    if (u + (int)gridDim.x < nunits) next = items[(u + gridDim.x) / nruns];
+    const int g0 = (u % nruns) * run, g1 = min(ncg, g0 + run), npt = it.z - it.y;
+    const Rec* rec = recbuf + (ui & 1) * kGatherPts;
+    if (!mbar_wait_bounded(&rfull[ui & 1], (ui >> 1) & 1, limit)) return give_up();
+    for (int cg = g0; cg < g1; ++cg, ++k) {
+      const uint32_t s = k % NST;
+      if (!mbar_wait_bounded(&full[s], (k / NST) & 1, limit)) return give_up();
+      const float2* reg = reinterpret_cast<const float2*>(smem + s * RBYTES);
+      const int c0 = cg * CG;
+      for (int base = warp * PPW; base < npt; base += NW * PPW) {
+        const bool on = base + h < npt;
+        const Rec& R = rec[on ? base + h : base];
+        const unsigned view = R.view;
+        const int p = R.p;
+        const float2* a = reg + c * VOL + (view & 0xfffff) + kz;
+        float2 acc[EPL];
+#pragma unroll
+        for (int q = 0; q < EPL; ++q) acc[q] = make_float2(0.f, 0.f);
+        // the box's farthest cell from its first one, for the last entry
+        if (TLGB_IN_RANGE((view & 0xfffff) + ((NDIM == 3 ? 3 * PLANE : 0) + (KT - 1) * S + KT - 1), VOL)) {
+          if constexpr (NDIM == 3) {
+            const float4 wx = *reinterpret_cast<const float4*>(R.w[0]);
+            const float wz = R.w[2][kz];
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+              const float wyz = R.w[1][kyo[t]] * wz;
+#pragma unroll
+              for (int q = 0; q < EPL; ++q) {
+                const float2* ar = a + q * CL * VOL + rowoff[t];
+                float2 sx = mul2_bcast(wx.x, ar[0]);
+                fma2_bcast(sx, wx.y, ar[PLANE]);
+                fma2_bcast(sx, wx.z, ar[2 * PLANE]);
+                fma2_bcast(sx, wx.w, ar[3 * PLANE]);
+                acc[q].x = fmaf(wyz, sx.x, acc[q].x);
+                acc[q].y = fmaf(wyz, sx.y, acc[q].y);
+              }
+            }
+          } else {
+#pragma unroll
+            for (int zb = 0; zb < KT; zb += 4) {
+              const float wz = R.w[1][zb + kz];
+#pragma unroll
+              for (int yb = 0; yb < KT; yb += 4) {
+#pragma unroll
+                for (int t = 0; t < 4; ++t) {
+                  const float w = R.w[0][yb + kyo[t]] * wz;
+#pragma unroll
+                  for (int q = 0; q < EPL; ++q) {
+                    const float2 v = a[q * CL * VOL + yb * S + rowoff[t] + zb];
+                    acc[q].x = fmaf(w, v.x, acc[q].x);
+                    acc[q].y = fmaf(w, v.y, acc[q].y);
+                  }
+                }
+              }
+            }
+          }
         }
-    __syncwarp();
-    return acc;
-  };
-  auto finish = [&](float2 acc, int p) {
-    acc.x += __shfl_xor_sync(0xffffffffu, acc.x, 1);
-    acc.y += __shfl_xor_sync(0xffffffffu, acc.y, 1);
-    acc.x += __shfl_xor_sync(0xffffffffu, acc.x, 2);
-    acc.y += __shfl_xor_sync(0xffffffffu, acc.y, 2);
-    if (kz == 0 && c0 + c < g.nbatch)
-      *reinterpret_cast<float2*>(out + ((long long)(c0 + c) * g.npts + p) * 2) = acc;
-  };
-  auto one = [&](const R3& R) {
-    const unsigned view = R.view;
-    if (!((view >> 21) & 1)) return;  // no valid tap (warp-uniform)
-    finish((view >> 20) & 1 ? gather_box(R) : gather_rec(R), R.p);
-  };
-  for (int base = warp; base < npt; base += 8 * NW) {
-    if (base != warp) {
-      __syncwarp();  // the previous mini-batch has been read
-      build_records(base);
-    }
-    const int nb = min(8, (npt - base + NW - 1) / NW);
-    int i = 0;
-    for (; i + 1 < nb; i += 2) {
-      const R3& R0 = wrec[i];
-      const R3& R1 = wrec[i + 1];
-      if ((R0.view & R1.view) >> 20 & 1) {
-        const float2 a0 = gather_box(R0), a1 = gather_box(R1);
-        finish(a0, R0.p);
-        finish(a1, R1.p);
-      } else {
-        one(R0);
-        one(R1);
+        // the 4 z-tap lanes add up, each ending with one component
+        float sum;
+        int ent, comp;
+        if constexpr (EPL == 2) {
+          const bool hi = kz & 2;
+          float2 keep = hi ? acc[1] : acc[0];
+          const float2 send = hi ? acc[0] : acc[1];
+          keep.x += __shfl_xor_sync(0xffffffffu, send.x, 2);
+          keep.y += __shfl_xor_sync(0xffffffffu, send.y, 2);
+          sum = kz & 1 ? keep.y : keep.x;
+          sum += __shfl_xor_sync(0xffffffffu, kz & 1 ? keep.x : keep.y, 1);
+          ent = c + (hi ? CL : 0), comp = kz & 1;
+        } else {
+          sum = kz & 1 ? acc[0].y : acc[0].x;
+          sum += __shfl_xor_sync(0xffffffffu, kz & 1 ? acc[0].x : acc[0].y, 1);
+          sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+          ent = c, comp = kz & 1;
+        }
+        const bool fast = (view >> 20) & 1;
+        if (on && fast && (EPL == 2 || kz < 2) && c0 + ent < g.nbatch && TLGB_IN_RANGE(p, g.npts)) {
+          if (sorted)
+            sorted[(((long long)cg * g.npts + it.w + base + h) * CG + ent) * 2 + comp] = sum;
+          else
+            out[((long long)(c0 + ent) * g.npts + p) * 2 + comp] = sum;
+        }
+        // the step's points with more than KT taps in a dim, one at a time by the whole warp
+        unsigned rest = __ballot_sync(0xffffffffu, on && !fast);
+        while (rest) {
+          const int hh = (__ffs(rest) - 1) / (4 * CL);
+          rest &= ~(((1u << (4 * CL)) - 1u) << (4 * CL * hh));
+          const Rec& Q = rec[base + hh];
+          SlowTaps<NDIM, KT>& T = slow[warp];
+          {
+            constexpr int NTM = KT + 1;
+            const int d = lane / NTM, kk = lane % NTM, e = d + 3 - NDIM;
+            Tap t;
+            t.valid = false;
+            float x = 0.f;
+            int lower = 0;
+            if (d < NDIM) {
+              x = load_coord(g, locs, Q.p, e);
+              lower = lower_of(g, e, x);
+              if (kk < g.NT[e]) t = tap_eval(g, e, x, lower, kk);
+            }
+            const unsigned m = (__ballot_sync(0xffffffffu, t.valid) >> (d < NDIM ? d * NTM : 0)) & ((1u << NTM) - 1);
+            if (t.valid)
+              T.w[d][kk - (__ffs(m) - 1)] = kern_precise(g.kernel, __fsub_rn(x, (float)(lower + kk)), g.r[e], t.d, g.beta, g.beta_lo);
+            if (d < NDIM && kk == 0) {
+              int st = lower + __ffs(m) - 1;
+              if (g.pad == TLGB_PAD_CIRCULAR) st = wrapi(st, g.N[e]);
+              T.n[d] = __popc(m);
+              int o[3];
+              item_origin(g, it.x, o);
+              T.f[d] = st - (e == 2 ? o[2] : (e == 1 ? o[1] : o[0]));
+            }
+          }
+          __syncwarp();
+          const int e8 = lane % CG, n2 = T.n[NDIM - 1], n1 = T.n[NDIM - 2], tot = n1 * n2 * (NDIM == 3 ? T.n[0] : 1);
+          float2 v2 = make_float2(0.f, 0.f);
+          for (int t = lane / CG; t < tot; t += 32 / CG) {
+            const int z = t % n2, yx = t / n2, y = yx % n1, x = yx / n1;
+            float w = T.w[NDIM - 2][y] * T.w[NDIM - 1][z];
+            int cell = (T.f[NDIM - 2] + y) * S + T.f[NDIM - 1] + z;
+            if (NDIM == 3) {
+              w *= T.w[0][x];
+              cell += (T.f[0] + x) * PLANE;
+            }
+            if (TLGB_IN_RANGE(cell, VOL)) fma2_bcast(v2, w, reg[e8 * VOL + cell]);
+          }
+          for (int m = CG; m < 32; m <<= 1) {
+            v2.x += __shfl_xor_sync(0xffffffffu, v2.x, m);
+            v2.y += __shfl_xor_sync(0xffffffffu, v2.y, m);
+          }
+          if (lane < CG && c0 + lane < g.nbatch && TLGB_IN_RANGE(Q.p, g.npts))
+            *reinterpret_cast<float2*>(sorted ? sorted + (((long long)cg * g.npts + it.w + base + hh) * CG + lane) * 2
+                                              : out + ((long long)(c0 + lane) * g.npts + Q.p) * 2) = v2;
+          __syncwarp();
+        }
       }
+      __syncwarp();
+      if (lane == 0) sm100::mbar_arrive(&empty[s]);
     }
-    if (i < nb) one(wrec[i]);
+    if (lane == 0) sm100::mbar_arrive(&rempty[ui & 1]);
+  }
+}
+
+// [group][place][4] -> [entry][point]: the gather's results out of the items'
+// order (zero for points without taps). CTA = 128 points of one group; a
+// thread reads 16 of a point's 32 bytes, a warp writes 32 points of an entry.
+// HBM-bound: 64 MB out of 64 MB take 23 us.
+__global__ void __launch_bounds__(256) unsort_kernel(const float4* __restrict__ sorted, const int32_t* __restrict__ rank,
+                                                     long long npts, long long nbatch, float2* __restrict__ out) {
+  __shared__ float2 sm[4][128 + 4];
+  const int t = threadIdx.x, grp = blockIdx.y;
+  const long long p0 = (long long)blockIdx.x * 128;
+  {
+    const int i = t >> 1, q = t & 1;
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (p0 + i < npts) {
+      const int r = rank[p0 + i];
+      if (r >= 0) v = __ldg(sorted + ((long long)grp * npts + r) * 2 + q);
+    }
+    sm[2 * q][i] = make_float2(v.x, v.y);
+    sm[2 * q + 1][i] = make_float2(v.z, v.w);
+  }
+  __syncthreads();
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int c = (t >> 7) + 2 * h, i = t & 127;
+    const long long cc = (long long)grp * 4 + c;
+    if (p0 + i < npts && cc < nbatch) out[cc * npts + p0 + i] = sm[c][i];
   }
 }
 
@@ -2904,7 +2852,7 @@ struct PlanLayout {
   // tmp: windows, CTA sums, counters, key starts; per list the sort's two key
   // buffers, second value buffer and counts, and the unordered items, splits
   // and their order
-  int64_t t_win, t_sums, t_cnt, t_tstart, t_bstart;
+  int64_t t_win, t_sums, t_homes, t_cnt, t_tstart, t_bstart;
   int64_t t_keys[2][2], t_vals[2], t_counts[2], t_items[2], t_order[2];
   int64_t t_bytes;
 };
@@ -2914,13 +2862,22 @@ constexpr int64_t kAdjChunk = 1024;
 
 std::atomic<int> g_test_skip_copy{0};  // tlgb_test_skip_region_copy
 
-// Geometries whose plan carries per-point tap records (the 3D 8-entry kernels)
-bool records_ok(const Geo& g) {
-  if (g.norm != 1) return false;
-  if (g.ndim == 3)
-    return g.T[0] == 8 && g.T[1] == 8 && g.T[2] == 8 && g.NT[0] == 5 && g.NT[1] == 5 && g.NT[2] == 5;
-  return g.ndim == 2 && g.T[1] == 16 && g.T[2] == 16 && g.NT[1] == 5 && g.NT[2] == 5;
+// Taps per dim of the gather records, 0 for geometries without them: 3D grids
+// of at least 8 cells per dim with at most 5 taps per dim (4 in a record; the
+// fifth only at exact-integer coordinates), 2D grids of at least 16 with at
+// most 9 (4 or 8 in a record), separable weights.
+int rec_taps(const Geo& g) {
+  if (g.norm != 1) return 0;
+  const int nt = std::max(g.NT[0], std::max(g.NT[1], g.NT[2]));
+  if (g.ndim == 3) return g.T[0] == 8 && g.T[1] == 8 && g.T[2] == 8 && nt <= 5 ? 4 : 0;
+  return g.ndim == 2 && g.T[1] == 16 && g.T[2] == 16 && nt <= 9 ? (nt <= 5 ? 4 : 8) : 0;
 }
+bool records_ok(const Geo& g) { return rec_taps(g) > 0; }
+size_t rec_bytes(const Geo& g) { return g.ndim == 3 ? 64 : (rec_taps(g) == 4 ? 48 : 80); }
+// 3D plans: the points' places among the records follow the records
+size_t rank_offset(const Geo& g, size_t off_records) { return align_up(off_records + (size_t)g.npts * rec_bytes(g), 256); }
+// points of a gather item: what the record buffers of gather_kernel hold
+int fwd_chunk(const Geo& g) { return records_ok(g) ? kGatherPts : (int)kFwdChunk; }
 
 // The most blocks a window of NT cells meets along a dim (4 = too many for
 // the block lists): the windows inside the grid at every offset in a block,
@@ -3052,6 +3009,9 @@ int64_t max_tiles_per_dim(const Geo& g, int e) {
   return 2;
 }
 
+// in kernel_key: most points' outputs lie in another sector than the point's before
+constexpr int64_t kScattered = (int64_t)1 << 52;
+
 // The kernel, norm and beta a plan's records hold weights for
 int64_t kernel_key(const Geo& g) {
   uint32_t bits;
@@ -3067,7 +3027,11 @@ PlanUnits plan_units(const Geo& g, int64_t ntiles, bool blocks) {
   U.ncy = blocks_along(U.nby, kCube), U.ncz = blocks_along(U.nbz, kCube);
   U.per = cx * kCube;
   U.nrows = blocks ? (long long)blocks_along(U.nbx, cx) * U.ncy * U.ncz * U.per : 0;
-  U.tile_ctas = (int)cdiv(ntiles, kPlanPts);
+  U.ntx = g.nt[0], U.nty = g.nt[1], U.ntz = g.nt[2];
+  const int tx = g.nt[0] == 1 ? 1 : kTileCube;
+  U.ntu = (long long)blocks_along(g.nt[0], tx) * blocks_along(g.nt[1], kTileCube) * blocks_along(g.nt[2], kTileCube) * tx *
+          kTileCube * kTileCube;
+  U.tile_ctas = (int)cdiv(U.ntu, kPlanPts);
   return U;
 }
 
@@ -3075,7 +3039,7 @@ PlanLayout layout(const Geo& g) {
   PlanLayout L;
   L.e_max = g.npts * max_tiles_per_dim(g, 0) * max_tiles_per_dim(g, 1) * max_tiles_per_dim(g, 2);
   L.ntiles = (int64_t)g.nt[0] * g.nt[1] * g.nt[2];
-  L.max_fwd = L.ntiles + cdiv(g.npts, kFwdChunk) + 1;
+  L.max_fwd = L.ntiles + cdiv(g.npts, fwd_chunk(g)) + 1;
   L.max_adj = L.ntiles + cdiv(L.e_max, kAdjChunk) + 1;
   size_t o = 0;
   L.off_entries = o;
@@ -3089,7 +3053,8 @@ PlanLayout layout(const Geo& g) {
   L.off_recs = 0;
   if (records_ok(g) && g.npts > 0) {
     L.off_recs = o;
-    o = align_up(o + (size_t)g.npts * 64, 256);
+    o = rank_offset(g, o);
+    if (g.ndim == 3) o = align_up(o + (size_t)g.npts * 4, 256);
   }
   L.nblocks = L.eb_max = L.max_blk_items = L.max_blk_split = 0;
   L.off_blk_entries = L.off_blk_items = L.off_blk_split = L.off_blk_rows = 0;
@@ -3117,6 +3082,7 @@ PlanLayout layout(const Geo& g) {
   const PlanUnits U = plan_units(g, L.ntiles, L.nblocks > 0);
   L.t_win = tmp(g.npts * 16);
   L.t_sums = tmp(std::max(cdiv(g.npts, kPlanPts), (int64_t)U.tile_ctas + cdiv(U.nrows, kPlanPts)) * 16);
+  L.t_homes = tmp((int64_t)U.tile_ctas * 16);
   L.t_cnt = tmp(16 * 4);
   L.t_tstart = tmp((2 * L.ntiles + 1) * 4);
   L.t_bstart = tmp((L.nblocks + 1) * 4);
@@ -3154,18 +3120,7 @@ int64_t region_vol(const Geo& g) {
 }
 
 // batch entries staged per forward CTA
-bool fast3(const Geo& g, int cg);
-bool fast2(const Geo& g, int cg);
-
-// A batch of fewer than 8 entries on a geometry of the dedicated 8-entry
-// kernels (3D 8^3 or 2D 16 x 16 tiles, width in (3, 4], norm 1, complex) runs
-// on them as one group: the missing entries are staged as zeros and never
-// written. Those kernels stage each point once for all entries, so even one
-// entry runs faster there than on the generic kernels.
-bool small_batch_on_fast_kernels(const Geo& g) { return g.nbatch < 8 && (fast3(g, 8) || fast2(g, 8)); }
-
 int fwd_cg(const Geo& g) {
-  if (small_batch_on_fast_kernels(g)) return 8;
   int cg = (int)std::min<long long>(std::max<long long>(g.nbatch, 1), CGMAX);
   const int64_t cap = 220 * 1024 - NWF * 32 * (int64_t)pt_bytes(ntb_for(g));
   while (cg > 1 && region_vol(g) * cg * value_size(g) > cap) --cg;
@@ -3240,16 +3195,59 @@ int check_plan(const Geo& g, const tlgb_interp_plan_info* info, const void* plan
   for (int e = 0; e < 3; ++e)
     if (info->tile[e] != g.T[e] || info->n_tile[e] != g.nt[e])
       TLGB_FAIL(TLGB_ERR_INVALID, "plan was built for another grid");
-  if (((info->off_records > 0 && records_ok(g)) || info->n_blk_items > 0) && info->kernel_key != kernel_key(g))
+  if (((info->off_records > 0 && records_ok(g)) || info->n_blk_items > 0) && (info->kernel_key & ~kScattered) != kernel_key(g))
     TLGB_FAIL(TLGB_ERR_INVALID, "plan was built for another kernel, norm or beta (its tap weights are stored)");
   return TLGB_OK;
 }
 
-template <typename F>
-int set_smem(F* kernel, size_t bytes) {
+using CtxGetCurrentFn = CUresult (*)(CUcontext*);
+
+CtxGetCurrentFn ctx_get_current() {
+  static CtxGetCurrentFn fn = nullptr;
+  static std::once_flag once;
+  std::call_once(once, [] {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPointByVersion("cuCtxGetCurrent", &p, 12000, cudaEnableDefault, &q) == cudaSuccess &&
+        q == cudaDriverEntryPointSuccess)
+      fn = reinterpret_cast<CtxGetCurrentFn>(p);
+  });
+  return fn;
+}
+
+// A kernel's shared-memory limit and carveout, set once per CUDA context (the
+// attributes belong to the context's module; two calls of about 2 us each on
+// every launch otherwise) and again when a launch needs more.
+int set_smem(const void* kernel, size_t bytes) {
+  struct Entry {
+    CUcontext ctx;
+    const void* kernel;
+    size_t bytes;
+  };
+  static std::mutex mu;
+  static std::vector<Entry> known;
+  CUcontext ctx = nullptr;
+  CtxGetCurrentFn get = ctx_get_current();
+  const bool keyed = get && get(&ctx) == CUDA_SUCCESS && ctx;
+  std::lock_guard<std::mutex> lock(mu);
+  if (keyed)
+    for (const Entry& e : known)
+      if (e.kernel == kernel && e.ctx == ctx && e.bytes >= bytes) return TLGB_OK;
   TLGB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
   TLGB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
+  if (!keyed) return TLGB_OK;
+  for (Entry& e : known)
+    if (e.kernel == kernel && e.ctx == ctx) {
+      e.bytes = bytes;
+      return TLGB_OK;
+    }
+  if (known.size() >= 1024) known.clear();  // contexts come and go in a long-lived host
+  known.push_back({ctx, kernel, bytes});
   return TLGB_OK;
+}
+template <typename F>
+int set_smem(F* kernel, size_t bytes) {
+  return set_smem(reinterpret_cast<const void*>(kernel), bytes);
 }
 
 }  // namespace
@@ -3283,6 +3281,7 @@ extern "C" int tlgb_interp_plan_build(const tlgb_interp_desc* d, const float* lo
   const PlanUnits U = plan_units(g, L.ntiles, blocks);
   int4* win = (int4*)(Tm + L.t_win);
   uint4* sums = (uint4*)(Tm + L.t_sums);
+  uint4* homes = (uint4*)(Tm + L.t_homes);
   uint32_t* cnt = (uint32_t*)(Tm + L.t_cnt);
   uint32_t* tstart = (uint32_t*)(Tm + L.t_tstart);
   uint32_t* bstart = (uint32_t*)(Tm + L.t_bstart);
@@ -3307,18 +3306,17 @@ extern "C" int tlgb_interp_plan_build(const tlgb_interp_desc* d, const float* lo
   }
   if (g.npts > 0) {
     const unsigned nb = (unsigned)cdiv(g.npts, kPlanPts);
-    PRec* recs = L.off_recs > 0 ? (PRec*)(P + L.off_recs) : nullptr;
     float* rows = blocks ? (float*)(P + L.off_blk_rows) : nullptr;
     const size_t sm = blocks ? (size_t)kPlanPts * row_floats(g.ndim, g.nrow) * 4 : 0;
     const int maxnt = std::max(g.NT[0], std::max(g.NT[1], g.NT[2]));
     auto points = [&](auto* k) -> int {
-      TLGB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-      k<<<nb, kPlanPts, sm, s>>>(g, locs, win, recs, rows, sums);
+      TLGB_TRY(set_smem(k, sm));
+      k<<<nb, kPlanPts, sm, s>>>(g, locs, win, rows, sums);
       TLGB_CHECK_LAUNCH();
       return TLGB_OK;
     };
-    TLGB_TRY(records_ok(g) ? points(plan_points_kernel<5>) : (maxnt <= 9 ? points(plan_points_kernel<9>) : points(plan_points_kernel<NTMAX>)));
-    plan_scan_kernel<<<1, 1024, 0, s>>>({sums, (long long)nb, cnt}, {});
+    TLGB_TRY(maxnt <= 5 ? points(plan_points_kernel<5>) : (maxnt <= 9 ? points(plan_points_kernel<9>) : points(plan_points_kernel<NTMAX>)));
+    plan_scan_kernel<<<1, 1024, 0, s>>>({sums, (long long)nb, cnt}, {}, {});
     TLGB_CHECK_LAUNCH();
     plan_emit_kernel<<<nb, kPlanPts, 0, s>>>(g, win, sums, jobs[0].keys[0], jobs[0].vals[0],
                                              blocks ? jobs[1].keys[0] : nullptr, blocks ? jobs[1].vals[0] : nullptr);
@@ -3334,9 +3332,10 @@ extern "C" int tlgb_interp_plan_build(const tlgb_interp_desc* d, const float* lo
   // Work items. Results do not depend on their order, because every item
   // writes its own tile, block, slot or points.
   const unsigned row_ctas = (unsigned)cdiv(U.nrows, kPlanPts), unit_ctas = (unsigned)U.tile_ctas + row_ctas;
-  plan_count_items_kernel<<<unit_ctas, kPlanPts, 0, s>>>(U, tstart, bstart, (int)kFwdChunk, (int)kAdjChunk, sums);
+  plan_count_items_kernel<<<unit_ctas, kPlanPts, 0, s>>>(U, tstart, bstart, fwd_chunk(g), (int)kAdjChunk, sums, homes);
   TLGB_CHECK_LAUNCH();
-  plan_scan_kernel<<<2, 1024, 0, s>>>({sums, U.tile_ctas, cnt + 4}, {sums + U.tile_ctas, (long long)row_ctas, cnt + 8});
+  plan_scan_kernel<<<3, 1024, 0, s>>>({sums, U.tile_ctas, cnt + 4}, {sums + U.tile_ctas, (long long)row_ctas, cnt + 8},
+                                      {homes, U.tile_ctas, cnt + 12});
   TLGB_CHECK_LAUNCH();
   int4* adj_any = (int4*)(Tm + L.t_items[0]);
   int4* bsplit_any = blocks ? (int4*)(Tm + L.t_items[1]) : nullptr;
@@ -3347,10 +3346,29 @@ extern "C" int tlgb_interp_plan_build(const tlgb_interp_desc* d, const float* lo
                 {(int32_t*)(Tm + L.t_order[i]), (int32_t*)(Tm + L.t_vals[i])},
                 jobs[i].counts, cnt + (i ? 10 : 5), i ? L.max_blk_split : L.max_adj, i ? 16 : 11};
   plan_emit_items_kernel<<<unit_ctas, kPlanPts, 0, s>>>(
-      U, tstart, bstart, (int)kFwdChunk, (int)kAdjChunk, sums, (int4*)(P + L.off_fwd), adj_any, order[0].keys[0],
+      U, tstart, bstart, fwd_chunk(g), (int)kAdjChunk, sums, homes, (int4*)(P + L.off_fwd), adj_any, order[0].keys[0],
       order[0].vals[0], (int4*)(P + L.off_split), blocks ? (int4*)(P + L.off_blk_items) : nullptr, bsplit_any,
       blocks ? order[1].keys[0] : nullptr, blocks ? order[1].vals[0] : nullptr);
   TLGB_CHECK_LAUNCH();
+  if (L.off_recs > 0) {
+    const int4* fwd = (const int4*)(P + L.off_fwd);
+    const int32_t* entries = (const int32_t*)(P + L.off_entries);
+    char* R = P + L.off_recs;
+    const unsigned n = (unsigned)L.max_fwd;
+    int32_t* rank = g.ndim == 3 ? (int32_t*)(P + rank_offset(g, L.off_recs)) : nullptr;
+    if (rank) TLGB_CUDA(cudaMemsetAsync(rank, 0xff, (size_t)g.npts * 4, s));  // -1: no taps
+    const float* rows = blocks ? (const float*)(P + L.off_blk_rows) : nullptr;
+    auto records = [&](auto* from_rows, auto* from_locs, auto* out) {
+      (blocks ? from_rows : from_locs)<<<n, 128, 0, s>>>(g, cnt, win, rows, fwd, entries, locs, out, rank, cnt + 15);
+    };
+    if (g.ndim == 3)
+      records(plan_records_kernel<3, 4, true>, plan_records_kernel<3, 4, false>, (GatherRec<3, 4>*)R);
+    else if (rec_taps(g) == 4)
+      records(plan_records_kernel<2, 4, true>, plan_records_kernel<2, 4, false>, (GatherRec<2, 4>*)R);
+    else
+      records(plan_records_kernel<2, 8, true>, plan_records_kernel<2, 8, false>, (GatherRec<2, 8>*)R);
+    TLGB_CHECK_LAUNCH();
+  }
   TLGB_TRY(radix_sort_jobs(order, njobs, s));
   const int ofin = std::max(radix_passes(order[0].bits), blocks ? radix_passes(order[1].bits) : 1) & 1;
   const int64_t onmax = std::max(L.max_adj, L.max_blk_split);
@@ -3383,6 +3401,7 @@ extern "C" int tlgb_interp_plan_build(const tlgb_interp_desc* d, const float* lo
   info->plan_bytes = L.bytes;
   info->off_records = L.off_recs;
   info->kernel_key = L.off_recs > 0 || blocks ? kernel_key(g) : 0;
+  if (2ll * c[15] > (int64_t)c[14]) info->kernel_key |= kScattered;
   info->n_home = c[2];
   if (blocks) {
     info->n_blk_entries = c[1];
@@ -3399,7 +3418,6 @@ extern "C" int tlgb_interp_plan_build(const tlgb_interp_desc* d, const float* lo
 
 namespace tlgb {
 namespace {
-bool fast3(const Geo& g, int cg);
 bool fast2(const Geo& g, int cg);
 
 // Batch entries per group of the block gridding: 1, 2 or 4 for 3D batches of
@@ -3448,18 +3466,12 @@ extern "C" int tlgb_interp_adjoint_scratch_size(const tlgb_interp_desc* d, const
 namespace tlgb {
 namespace {
 
-// the unrolled paths: 3D, 8^3 tiles, 5 taps per dim (width in (3, 4]), 8 complex batch entries
-bool fast3(const Geo& g, int cg) {
-  return g.ndim == 3 && g.cplx && cg == 8 && g.norm == 1 && g.T[0] == 8 && g.T[1] == 8 && g.T[2] == 8 && g.NT[0] == 5 &&
-         g.NT[1] == 5 && g.NT[2] == 5;
-}
-
-template <int N, int NDIM, int NTB, bool F3>
+template <int N, int NDIM, int NTB>
 int launch_fwd_t2(const Geo& g, int cg, const tlgb_interp_plan_info* info, const char* P, const float* locs,
                   const void* grid, void* out, cudaStream_t s) {
   const int64_t ncg = cdiv(g.nbatch, cg);
   const size_t sm = fwd_smem(g, cg);
-  auto* k = interp_fwd_kernel<N, NDIM, NTB, NWF, F3>;
+  auto* k = interp_fwd_kernel<N, NDIM, NTB, NWF>;
   TLGB_TRY(set_smem(k, sm));
   dim3 grd((unsigned)info->n_fwd_items, (unsigned)ncg);
   k<<<grd, NWF * 32, sm, s>>>(g, (const int4*)(P + info->off_fwd_items), (const int32_t*)(P + info->off_entries),
@@ -3490,60 +3502,16 @@ int launch_adj_t2(const Geo& g, int cg, const tlgb_interp_plan_info* info, const
 
 using sm100::tensor_map_encoder;
 
-template <int CG>
-int launch_fwd_f3_t(const Geo& g, const tlgb_interp_plan_info* info, const char* P, const float* locs,
-                    const void* grid, void* out, cudaStream_t s) {
-  const int64_t ncg = cdiv(g.nbatch, CG);
-  const size_t sm = 12 * 12 * 12 * CG * 8 + kGB * sizeof(R3) + 8 * sizeof(Rec<5>) + 8;
-  // 4D tensor map over [batch][X][Y][Z] complex64 (8-byte elements), box 12^3 x CG
-  CUtensorMap tmap;
-  memset(&tmap, 0, sizeof(tmap));
-  int use_tma = 0;
-  auto enc = tensor_map_encoder();
-  const uint64_t zb = (uint64_t)g.N[2] * 8;
-  if (enc && (zb % 16) == 0 && ((uintptr_t)grid % 16) == 0) {
-    const cuuint64_t dims[4] = {(cuuint64_t)g.N[2], (cuuint64_t)g.N[1], (cuuint64_t)g.N[0], (cuuint64_t)g.nbatch};
-    const cuuint64_t strides[3] = {zb, zb * g.N[1], zb * g.N[1] * g.N[0]};
-    const cuuint32_t box[4] = {12, 12, 12, (cuuint32_t)CG};
-    const cuuint32_t estr[4] = {1, 1, 1, 1};
-    const CUresult r = enc(&tmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4, const_cast<void*>(grid), dims, strides, box, estr,
-                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                           CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    use_tma = (r == CUDA_SUCCESS) ? 1 : 0;
-  }
-  TLGB_TRY(set_smem(fwd_f3_kernel<CG>, sm));
-  dim3 grd((unsigned)info->n_fwd_items, (unsigned)ncg);
-  fwd_f3_kernel<CG><<<grd, 256, sm, s>>>(tmap, use_tma, g, (const int4*)(P + info->off_fwd_items),
-                                         (const int32_t*)(P + info->off_entries), (const PRec*)(P + info->off_records),
-                                         locs, (const float*)grid, (float*)out);
-  TLGB_CHECK_LAUNCH();
-  return TLGB_OK;
-}
-
-// batches of at most 4 entries stage only their own entries' regions
-int launch_fwd_f3(const Geo& g, const tlgb_interp_plan_info* info, const char* P, const float* locs,
-                  const void* grid, void* out, cudaStream_t s) {
-  if (g.nbatch <= 1) return launch_fwd_f3_t<1>(g, info, P, locs, grid, out, s);
-  if (g.nbatch <= 2) return launch_fwd_f3_t<2>(g, info, P, locs, grid, out, s);
-  if (g.nbatch <= 4) return launch_fwd_f3_t<4>(g, info, P, locs, grid, out, s);
-  return launch_fwd_f3_t<8>(g, info, P, locs, grid, out, s);
-}
-
-bool fast2(const Geo& g, int cg) {
-  return g.ndim == 2 && g.cplx && cg == 8 && g.norm == 1 && g.T[1] == 16 && g.T[2] == 16 && g.NT[1] == 5 &&
-         g.NT[2] == 5;
-}
-
-// [batch][Y][Z] complex64 as a 4D map {Z, Y, 1, batch}, box 20 x 20 x 1 x 8
-// (the staged region of a 16 x 16 tile); 0 when TMA cannot be used
-int region_map2(const Geo& g, const void* grid, CUtensorMap& tmap) {
+// [batch][X][Y][Z] complex64 as a 4D map of 8-byte elements, box edge^2
+// (edge^3 in 3D) x cg entries; 0 when TMA cannot be used
+int region_map(const Geo& g, const void* grid, int edge, int cg, CUtensorMap& tmap) {
   memset(&tmap, 0, sizeof(tmap));
   auto enc = tensor_map_encoder();
   const uint64_t zb = (uint64_t)g.N[2] * 8;
   if (!enc || (zb % 16) != 0 || ((uintptr_t)grid % 16) != 0) return 0;
-  const cuuint64_t dims[4] = {(cuuint64_t)g.N[2], (cuuint64_t)g.N[1], 1, (cuuint64_t)g.nbatch};
-  const cuuint64_t strides[3] = {zb, zb * g.N[1], zb * g.N[1]};
-  const cuuint32_t box[4] = {20, 20, 1, 8};
+  const cuuint64_t dims[4] = {(cuuint64_t)g.N[2], (cuuint64_t)g.N[1], (cuuint64_t)g.N[0], (cuuint64_t)g.nbatch};
+  const cuuint64_t strides[3] = {zb, zb * g.N[1], zb * g.N[1] * g.N[0]};
+  const cuuint32_t e = (cuuint32_t)edge, box[4] = {e, e, g.ndim == 3 ? e : 1, (cuuint32_t)cg};
   const cuuint32_t estr[4] = {1, 1, 1, 1};
   const CUresult r = enc(&tmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4, const_cast<void*>(grid), dims, strides, box, estr,
                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -3551,19 +3519,75 @@ int region_map2(const Geo& g, const void* grid, CUtensorMap& tmap) {
   return r == CUDA_SUCCESS ? 1 : 0;
 }
 
-int launch_fwd_f2(const Geo& g, const tlgb_interp_plan_info* info, const char* P, const float* locs,
-                  const void* grid, void* out, cudaStream_t s) {
-  const int64_t ncg = cdiv(g.nbatch, 8);
-  const size_t sm = 20 * 20 * 8 * 8 + 64 * sizeof(R3) + 8 * sizeof(Rec<5>) + 8;
+// A unit is an item and `run` groups: all of them (an item's records are
+// fetched once) unless that leaves fewer than 6 units per CTA.
+template <int NDIM, int KT, int CG, int NW, int NST, int CTAS>
+int launch_gather(const Geo& g, const tlgb_interp_plan_info* info, const char* P, const float* locs, const void* grid,
+                  void* out, cudaStream_t s, float* sorted = nullptr) {
+  if ((uintptr_t)P & 15) TLGB_FAIL(TLGB_ERR_INVALID, "interp forward: the plan must be 16-byte aligned");
   CUtensorMap tmap;
-  const int use_tma = region_map2(g, grid, tmap);
-  TLGB_TRY(set_smem(fwd_f2_kernel, sm));
-  dim3 grd((unsigned)info->n_fwd_items, (unsigned)ncg);
-  fwd_f2_kernel<<<grd, 256, sm, s>>>(tmap, use_tma, g, (const int4*)(P + info->off_fwd_items),
-                                     (const int32_t*)(P + info->off_entries), (const PRec*)(P + info->off_records), locs,
-                                     (const float*)grid, (float*)out);
+  const int use_tma = region_map(g, grid, region_edge<NDIM, KT>(), CG, tmap);
+  constexpr size_t sm = gather_smem<NDIM, KT, CG, NW, NST>();
+  auto* k = gather_kernel<NDIM, KT, CG, NW, NST, CTAS>;
+  TLGB_TRY(set_smem(k, sm));
+  const int64_t ncg = cdiv(g.nbatch, CG), items = info->n_fwd_items, ctas = (int64_t)CTAS * sm_count();
+  int64_t run = ncg;
+  while (run > 1 && items * cdiv(ncg, run) < 6 * ctas) run = cdiv(run, 2);
+  const int64_t nruns = cdiv(ncg, run), nunits = items * nruns;
+  if (nunits >= (1ll << 31) - ctas) TLGB_FAIL(TLGB_ERR_UNSUPPORTED, "interp forward: too many points and batch entries in one call");
+  k<<<(unsigned)std::min(nunits, ctas), NW * 32 + kGatherProd, sm, s>>>(
+      tmap, use_tma, g, (const int4*)(P + info->off_fwd_items), (int)nruns, (int)run, (int)nunits,
+      (const GatherRec<NDIM, KT>*)(P + info->off_records), locs, (const float*)grid, (float*)out, sorted);
   TLGB_CHECK_LAUNCH();
   return TLGB_OK;
+}
+
+// Points in random order: their 8-byte results are scattered over an output
+// that L2 cannot hold, and every 32-byte sector is written back in pieces. With
+// scratch the results go in the items' order (32 contiguous bytes per point
+// and group) and a second pass brings them to the points' order. It pays where
+// the output is a large part of L2: 8 x 2^21 points (134 MB) 720 -> 590 us.
+size_t forward_scratch_bytes(const Geo& g, const tlgb_interp_plan_info* info) {
+  if (g.ndim != 3 || !g.cplx || g.nbatch < 3 || !records_ok(g) || info->off_records == 0 || !(info->kernel_key & kScattered))
+    return 0;
+  if (g.nbatch * g.npts * 8 < (48ll << 20) || cdiv(g.nbatch, 4) > 65535) return 0;
+  return (size_t)cdiv(g.nbatch, 4) * g.npts * 32;
+}
+
+// Ring shapes: what fits 227 KB with two record buffers beside it, for the
+// fewest groups. 3D stages are 13.8 KB per entry: 4 entries per group in a ring
+// of 3 feed 16 consumer warps; small batches run two CTAs per SM.
+int launch_gather_any(const Geo& g, const tlgb_interp_plan_info* info, const char* P, const float* locs,
+                      const void* grid, void* out, cudaStream_t s, void* scratch = nullptr, size_t scratch_bytes = 0) {
+  const long long n = g.nbatch;
+  if (g.ndim == 3) {
+    const size_t need = forward_scratch_bytes(g, info);
+    if (need > 0 && scratch && scratch_bytes >= need && ((uintptr_t)scratch & 15) == 0) {
+      TLGB_TRY((launch_gather<3, 4, 4, 16, 3, 1>(g, info, P, locs, grid, out, s, (float*)scratch)));
+      const dim3 grd((unsigned)cdiv(g.npts, 128), (unsigned)cdiv(n, 4));
+      unsort_kernel<<<grd, 256, 0, s>>>((const float4*)scratch, (const int32_t*)(P + rank_offset(g, info->off_records)),
+                                        g.npts, n, (float2*)out);
+      TLGB_CHECK_LAUNCH();
+      return TLGB_OK;
+    }
+    if (n == 1) return launch_gather<3, 4, 1, 8, 5, 2>(g, info, P, locs, grid, out, s);
+    if (n == 2) return launch_gather<3, 4, 2, 16, 5, 1>(g, info, P, locs, grid, out, s);
+    return launch_gather<3, 4, 4, 16, 3, 1>(g, info, P, locs, grid, out, s);
+  }
+  if (rec_taps(g) == 4) {
+    if (n == 1) return launch_gather<2, 4, 1, 8, 6, 2>(g, info, P, locs, grid, out, s);
+    if (n == 2) return launch_gather<2, 4, 2, 8, 6, 2>(g, info, P, locs, grid, out, s);
+    if (n <= 4) return launch_gather<2, 4, 4, 8, 5, 2>(g, info, P, locs, grid, out, s);
+    return launch_gather<2, 4, 8, 8, 3, 2>(g, info, P, locs, grid, out, s);
+  }
+  if (n <= 2) return launch_gather<2, 8, 2, 8, 4, 2>(g, info, P, locs, grid, out, s);
+  if (n <= 4) return launch_gather<2, 8, 4, 8, 3, 2>(g, info, P, locs, grid, out, s);
+  return launch_gather<2, 8, 8, 16, 4, 1>(g, info, P, locs, grid, out, s);
+}
+
+bool fast2(const Geo& g, int cg) {
+  return g.ndim == 2 && g.cplx && cg == 8 && g.norm == 1 && g.T[1] == 16 && g.T[2] == 16 && g.NT[1] == 5 &&
+         g.NT[2] == 5;
 }
 
 template <int E, int NROW>
@@ -3638,16 +3662,6 @@ int launch_adj_b3(const Geo& g, const tlgb_interp_plan_info* info, const char* P
   return TLGB_OK;
 }
 
-template <int N, int NDIM, int NTB>
-int launch_fwd_t(const Geo& g, int cg, const tlgb_interp_plan_info* info, const char* P, const float* locs,
-                 const void* grid, void* out, cudaStream_t s) {
-  if constexpr (N == 4 && NDIM == 3 && NTB == 5)
-    if (fast3(g, cg) && info->off_records > 0) return launch_fwd_f3(g, info, P, locs, grid, out, s);
-  if constexpr (NDIM == 2 && NTB == 5)
-    if (fast2(g, cg) && info->off_records > 0) return launch_fwd_f2(g, info, P, locs, grid, out, s);
-  return launch_fwd_t2<N, NDIM, NTB, false>(g, cg, info, P, locs, grid, out, s);
-}
-
 // floats per coil unit: 2 batch entries per unit when the group size is even
 inline int unit_floats(const Geo& g, int cg) { return (g.cplx ? 2 : 1) * ((cg % 2 == 0) ? 2 : 1); }
 
@@ -3655,9 +3669,9 @@ template <int NDIM, int NTB>
 int dispatch_fwd_n(const Geo& g, int cg, const tlgb_interp_plan_info* info, const char* P, const float* locs,
                    const void* grid, void* out, cudaStream_t s) {
   switch (unit_floats(g, cg)) {
-    case 4: return launch_fwd_t<4, NDIM, NTB>(g, cg, info, P, locs, grid, out, s);
-    case 2: return launch_fwd_t<2, NDIM, NTB>(g, cg, info, P, locs, grid, out, s);
-    default: return launch_fwd_t<1, NDIM, NTB>(g, cg, info, P, locs, grid, out, s);
+    case 4: return launch_fwd_t2<4, NDIM, NTB>(g, cg, info, P, locs, grid, out, s);
+    case 2: return launch_fwd_t2<2, NDIM, NTB>(g, cg, info, P, locs, grid, out, s);
+    default: return launch_fwd_t2<1, NDIM, NTB>(g, cg, info, P, locs, grid, out, s);
   }
 }
 
@@ -3685,7 +3699,8 @@ int launch_fwd_rows(const Geo& g, const tlgb_interp_plan_info* info, const char*
 // memory), so a batch below TLGB_INTERP_MAX_BATCH can still need more rows:
 // batch entries are independent, so such a batch is launched in parts.
 int launch_fwd(const Geo& g, const tlgb_interp_plan_info* info, const char* P, const float* locs, const void* grid,
-               void* out, cudaStream_t s) {
+               void* out, void* scratch, size_t scratch_bytes, cudaStream_t s) {
+  if (g.cplx && records_ok(g) && info->off_records > 0) return launch_gather_any(g, info, P, locs, grid, out, s, scratch, scratch_bytes);
   const int64_t per = (int64_t)65535 * fwd_cg(g);
   if (g.nbatch <= per) return launch_fwd_rows(g, info, P, locs, grid, out, s);
   const int64_t vs = value_size(g), vol = (int64_t)g.N[0] * g.N[1] * g.N[2];
@@ -3727,7 +3742,7 @@ int launch_grad_f2(const Geo& g, const tlgb_interp_plan_info* info, const char* 
   if (ncg > 1 && info->n_home < g.npts)  // points without taps get no partial writes
     TLGB_CUDA(cudaMemsetAsync(partial, 0, (size_t)ncg * n * sizeof(float), s));
   CUtensorMap tmap;
-  const int use_tma = region_map2(g, grid, tmap);
+  const int use_tma = region_map(g, grid, 20, 8, tmap);
   const size_t sm = 20 * 20 * 8 * 8 + 64 * sizeof(GRec2) + 8 * sizeof(PTaps<true>) + 8;
   TLGB_TRY(set_smem(grad_f2_kernel, sm));
   dim3 grd((unsigned)info->n_fwd_items, (unsigned)ncg);
@@ -3774,8 +3789,18 @@ int launch_grad(const Geo& g, const tlgb_interp_plan_info* info, const char* P, 
 }  // namespace
 }  // namespace tlgb
 
-extern "C" int tlgb_interp_forward(const tlgb_interp_desc* d, const tlgb_interp_plan_info* info, const void* plan,
-                                   const float* locs, const void* grid, void* out, tlgb_stream_t stream) {
+extern "C" int tlgb_interp_forward_scratch_size(const tlgb_interp_desc* d, const tlgb_interp_plan_info* info,
+                                                size_t* bytes) {
+  Geo g;
+  TLGB_TRY(make_geo(d, g));
+  if (!info || !bytes) TLGB_FAIL(TLGB_ERR_INVALID, "null pointer");
+  *bytes = forward_scratch_bytes(g, info);
+  return TLGB_OK;
+}
+
+extern "C" int tlgb_interp_forward_scratch(const tlgb_interp_desc* d, const tlgb_interp_plan_info* info,
+                                           const void* plan, const float* locs, const void* grid, void* out,
+                                           void* scratch, size_t scratch_bytes, tlgb_stream_t stream) {
   Geo g;
   TLGB_TRY(make_geo(d, g));
   TLGB_TRY(check_plan(g, info, plan));
@@ -3786,7 +3811,12 @@ extern "C" int tlgb_interp_forward(const tlgb_interp_desc* d, const tlgb_interp_
     TLGB_CUDA(cudaMemsetAsync(out, 0, (size_t)g.nbatch * g.npts * value_size(g), s));
   if (info->n_fwd_items == 0) return TLGB_OK;
   const char* P = (const char*)plan;
-  return launch_fwd(g, info, P, locs, grid, out, s);
+  return launch_fwd(g, info, P, locs, grid, out, scratch, scratch_bytes, s);
+}
+
+extern "C" int tlgb_interp_forward(const tlgb_interp_desc* d, const tlgb_interp_plan_info* info, const void* plan,
+                                   const float* locs, const void* grid, void* out, tlgb_stream_t stream) {
+  return tlgb_interp_forward_scratch(d, info, plan, locs, grid, out, nullptr, 0, stream);
 }
 
 extern "C" int tlgb_interp_adjoint(const tlgb_interp_desc* d, const tlgb_interp_plan_info* info, const void* plan,
@@ -3865,21 +3895,6 @@ namespace {
 // module there, which is when the buffer is allocated on that GPU.
 std::mutex g_fixed_mu;
 std::vector<std::pair<CUcontext, void*>> g_fixed_addr;
-
-using CtxGetCurrentFn = CUresult (*)(CUcontext*);
-
-CtxGetCurrentFn ctx_get_current() {
-  static CtxGetCurrentFn fn = nullptr;
-  static std::once_flag once;
-  std::call_once(once, [] {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPointByVersion("cuCtxGetCurrent", &p, 12000, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<CtxGetCurrentFn>(p);
-  });
-  return fn;
-}
 
 // Device address of the fixed buffer in the current context.
 int fixed_scratch_address(void** out) {

@@ -139,6 +139,8 @@ class InterpolatePlan:
             self.ready = torch.cuda.Event()
             self.ready.record(self.stream)
         del tmp
+        # the points are in no spatial order (bit 52 of the plan's key)
+        self.scattered = bool((int(self.info.kernel_key) >> 52) & 1)
 
     def use_on_current_stream(self) -> None:
         """Plans are cached across streams: another stream waits for the
@@ -267,13 +269,22 @@ def ungrid(
     if nbatch > MAX_BATCH:
         v = v.reshape(nbatch, -1)
     lc = _locs_f32(locs)
+    L = _ext.lib()
+    scratch = None
+    if plan.scattered and is_complex:
+        sb = ctypes.c_size_t(0)
+        d.nbatch = min(nbatch, MAX_BATCH)
+        _ext.check(L.tlgb_interp_forward_scratch_size(ctypes.byref(d), ctypes.byref(plan.info), ctypes.byref(sb)), "ungrid")
+        if sb.value:
+            scratch = torch.empty(sb.value, dtype=torch.uint8, device=dev)
     with torch.cuda.device(dev):
         for b0, b1 in _batch_chunks(nbatch):
             d.nbatch = b1 - b0
             _ext.check(
-                _ext.lib().tlgb_interp_forward(
+                L.tlgb_interp_forward_scratch(
                     ctypes.byref(d), ctypes.byref(plan.info), _ext.ptr(plan.buffer), _ext.ptr(lc),
-                    _ext.ptr(v[b0:b1] if nbatch > MAX_BATCH else v), _ext.ptr(out[b0:b1]), _ext.stream_ptr(dev),
+                    _ext.ptr(v[b0:b1] if nbatch > MAX_BATCH else v), _ext.ptr(out[b0:b1]), _ext.ptr(scratch),
+                    scratch.numel() if scratch is not None else 0, _ext.stream_ptr(dev),
                 ),
                 "ungrid",
             )
