@@ -228,10 +228,14 @@ class BlocksToArrayFn(Function):
 
 
 def array_to_blocks(input, block_shape, stride=None, mask=None, out=None):
+    if out is None and _ext.plain_call(input):
+        return unfold(input, block_shape, stride, mask)
     return ArrayToBlocksFn.apply(input, block_shape, stride, mask, out)
 
 
 def blocks_to_array(input, im_size, block_shape, stride=None, mask=None, out=None):
+    if out is None and _ext.plain_call(input):
+        return fold(input, im_size, block_shape, stride, mask)
     return BlocksToArrayFn.apply(input, im_size, block_shape, stride, mask, out)
 
 

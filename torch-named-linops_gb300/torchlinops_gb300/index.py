@@ -239,6 +239,8 @@ def index(vals: Tensor, idx: tuple, deterministic_backward: bool = False) -> Ten
         return IndexFn.apply(v, flat, (prod(grid_size),), plan, shape)
     idx = tuple(i.to(vals.device) for i in idx)
     plan, shape = get_index_plan(idx, grid_size, broadcast=True)
+    if _ext.plain_call(vals):
+        return _forward(vals, idx, grid_size, plan, shape)
     return IndexFn.apply(vals, idx, grid_size, plan, shape)
 
 
@@ -251,4 +253,6 @@ def index_adjoint(vals: Tensor, idx: tuple, grid_size: tuple[int, ...]) -> Tenso
     if len(idx) != len(grid_size):
         raise ValueError(f"final_size should be of dimension {len(idx)} but got {grid_size}")
     plan, shape = get_index_plan(idx, grid_size, broadcast=False)
+    if _ext.plain_call(vals):
+        return _adjoint(vals, plan, shape, grid_size)
     return IndexAdjointFn.apply(vals, plan, shape, grid_size)

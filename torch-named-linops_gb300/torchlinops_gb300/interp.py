@@ -136,11 +136,33 @@ class InterpolatePlan:
             )
             # the build's last kernels are still in flight on this stream
             self.stream = torch.cuda.current_stream(dev)
+            self._raw_stream = self.stream.cuda_stream
             self.ready = torch.cuda.Event()
             self.ready.record(self.stream)
         del tmp
         # the points are in no spatial order (bit 52 of the plan's key)
         self.scattered = bool((int(self.info.kernel_key) >> 52) & 1)
+        self._calls: dict = {}
+
+    def call(self, is_complex: bool, nbatch: int) -> tuple:
+        """(descriptor, ungrid scratch bytes, grid scratch bytes) for a call on
+        ``nbatch`` entries: functions of the plan and the batch alone, so kept
+        with the plan for the last few batch sizes. Not to be written to."""
+        key = (is_complex, nbatch)
+        hit = self._calls.get(key)
+        if hit is None:
+            d = _desc(self.ndim, self.grid_size, self.width, self.kernel, self.norm, self.pad_mode, self.beta, is_complex,
+                      nbatch, self.npts)
+            L = _ext.lib()
+            fb, ab = ctypes.c_size_t(0), ctypes.c_size_t(0)
+            info = ctypes.byref(self.info)
+            _ext.check(L.tlgb_interp_forward_scratch_size(ctypes.byref(d), info, ctypes.byref(fb)), "ungrid")
+            _ext.check(L.tlgb_interp_adjoint_scratch_size(ctypes.byref(d), info, ctypes.byref(ab)), "grid")
+            hit = (d, fb.value, ab.value)
+            if len(self._calls) >= 16:
+                self._calls = {}
+            self._calls[key] = hit
+        return hit
 
     def use_on_current_stream(self) -> None:
         """Plans are cached across streams: another stream waits for the
@@ -148,6 +170,9 @@ class InterpolatePlan:
         being reused while its own work may still read it. Under stream
         capture nothing is added (plans are built before capture: a build
         synchronises its stream)."""
+        raw = getattr(self, "_raw_stream", None)
+        if raw is not None and raw == _ext.raw_stream(self.device):
+            return
         cur = torch.cuda.current_stream(self.device)
         if cur.cuda_stream != self.stream.cuda_stream and not torch.cuda.is_current_stream_capturing():
             cur.wait_event(self.ready)
@@ -235,7 +260,16 @@ def _as_f32_view(t: Tensor, is_complex: bool) -> Tensor:
     return torch.view_as_real(t) if is_complex else t
 
 
+def _dense(t: Tensor) -> Tensor:
+    """``t`` itself when its memory is the values in order, else such a copy."""
+    if t.is_conj() or t.is_neg():
+        t = t.resolve_conj().resolve_neg()
+    return t if t.is_contiguous() else t.contiguous()
+
+
 def _locs_f32(locs: Tensor) -> Tensor:
+    if locs.dtype == torch.float32 and locs.is_contiguous():
+        return locs
     return locs.detach().to(torch.float32).contiguous()
 
 
@@ -263,32 +297,27 @@ def ungrid(
     is_complex = _check_values(vals)
     beta = kernel_params["beta"] if kernel == "kaiser_bessel" else 1.0
     plan = get_plan(locs, grid_size, width, kernel, pad_mode, beta, norm)
-    out = torch.empty(nbatch, npts, dtype=vals.dtype, device=dev)
-    d = _desc(ndim, grid_size, width, kernel, norm, pad_mode, beta, is_complex, nbatch, npts)
-    v = _as_f32_view(vals, is_complex)
-    if nbatch > MAX_BATCH:
-        v = v.reshape(nbatch, -1)
-    lc = _locs_f32(locs)
+    out = torch.empty((*batch_shape, *locs_batch_shape), dtype=vals.dtype, device=dev)
+    v, lc = _dense(vals), _locs_f32(locs)
+    step = (8 if is_complex else 4)  # bytes of a value
+    vol = prod(grid_size)
     L = _ext.lib()
     scratch = None
-    if plan.scattered and is_complex:
-        sb = ctypes.c_size_t(0)
-        d.nbatch = min(nbatch, MAX_BATCH)
-        _ext.check(L.tlgb_interp_forward_scratch_size(ctypes.byref(d), ctypes.byref(plan.info), ctypes.byref(sb)), "ungrid")
-        if sb.value:
-            scratch = torch.empty(sb.value, dtype=torch.uint8, device=dev)
-    with torch.cuda.device(dev):
+    with _ext.on_device(dev):
+        stream = _ext.raw_stream(dev)
         for b0, b1 in _batch_chunks(nbatch):
-            d.nbatch = b1 - b0
+            d, need, _ = plan.call(is_complex, b1 - b0)
+            if need and (scratch is None or scratch.numel() < need):
+                scratch = torch.empty(need, dtype=torch.uint8, device=dev)
             _ext.check(
                 L.tlgb_interp_forward_scratch(
-                    ctypes.byref(d), ctypes.byref(plan.info), _ext.ptr(plan.buffer), _ext.ptr(lc),
-                    _ext.ptr(v[b0:b1] if nbatch > MAX_BATCH else v), _ext.ptr(out[b0:b1]), _ext.ptr(scratch),
-                    scratch.numel() if scratch is not None else 0, _ext.stream_ptr(dev),
+                    ctypes.byref(d), ctypes.byref(plan.info), plan.buffer.data_ptr(), lc.data_ptr(),
+                    v.data_ptr() + b0 * vol * step, out.data_ptr() + b0 * npts * step,
+                    scratch.data_ptr() if need else 0, need, stream,
                 ),
                 "ungrid",
             )
-    return out.reshape(*batch_shape, *locs_batch_shape)
+    return out
 
 
 def grid(
@@ -327,29 +356,26 @@ def grid(
     is_complex = _check_values(vals)
     beta = kernel_params["beta"] if kernel == "kaiser_bessel" else 1.0
     plan = get_plan(locs, grid_size, width, kernel, pad_mode, beta, norm)
-    # the first batch range is the largest: its scratch serves every range
-    d = _desc(ndim, grid_size, width, kernel, norm, pad_mode, beta, is_complex, min(nbatch, MAX_BATCH), npts)
     L = _ext.lib()
-    sb = ctypes.c_size_t(0)
-    _ext.check(L.tlgb_interp_adjoint_scratch_size(ctypes.byref(d), ctypes.byref(plan.info), ctypes.byref(sb)), "grid")
-    out = torch.empty(nbatch, *grid_size, dtype=vals.dtype, device=dev)
-    scratch = torch.empty(max(sb.value, 1), dtype=torch.uint8, device=dev)
-    v = _as_f32_view(vals, is_complex)
-    if nbatch > MAX_BATCH:
-        v = v.reshape(nbatch, -1)
-    lc = _locs_f32(locs)
-    with torch.cuda.device(dev):
+    out = torch.empty((*batch_shape, *grid_size), dtype=vals.dtype, device=dev)
+    v, lc = _dense(vals), _locs_f32(locs)
+    step = (8 if is_complex else 4)  # bytes of a value
+    vol = prod(grid_size)
+    scratch = None
+    with _ext.on_device(dev):
+        stream = _ext.raw_stream(dev)
         for b0, b1 in _batch_chunks(nbatch):
-            d.nbatch = b1 - b0
+            d, _, need = plan.call(is_complex, b1 - b0)
+            if scratch is None or scratch.numel() < need:
+                scratch = torch.empty(max(need, 1), dtype=torch.uint8, device=dev)
             _ext.check(
                 L.tlgb_interp_adjoint(
-                    ctypes.byref(d), ctypes.byref(plan.info), _ext.ptr(plan.buffer), _ext.ptr(lc),
-                    _ext.ptr(v[b0:b1] if nbatch > MAX_BATCH else v), _ext.ptr(out[b0:b1]), _ext.ptr(scratch),
-                    sb.value, _ext.stream_ptr(dev),
+                    ctypes.byref(d), ctypes.byref(plan.info), plan.buffer.data_ptr(), lc.data_ptr(),
+                    v.data_ptr() + b0 * npts * step, out.data_ptr() + b0 * vol * step, scratch.data_ptr(), need, stream,
                 ),
                 "grid",
             )
-    return out.reshape(*batch_shape, *grid_size)
+    return out
 
 
 def _grad_locs(gridvals: Tensor, a: Tensor, locs: Tensor, width, kernel, norm, pad_mode, kernel_params) -> Tensor:
@@ -465,6 +491,8 @@ def interpolate(
     kernel_params: dict = None,
 ) -> Tensor:
     """Interpolate from a regular grid to scattered locations (reference interp.py:73)."""
+    if _ext.plain_call(vals, locs):
+        return ungrid(vals, locs, width, kernel, norm, pad_mode, kernel_params)
     return InterpolateFn.apply(vals, locs, width, kernel, norm, pad_mode, kernel_params)
 
 
@@ -479,4 +507,6 @@ def interpolate_adjoint(
     kernel_params: dict = None,
 ) -> Tensor:
     """Adjoint of interpolation (gridding) (reference interp.py:184)."""
+    if _ext.plain_call(vals, locs):
+        return grid(vals, locs, grid_size, width, kernel, norm, pad_mode, kernel_params)
     return InterpolateAdjointFn.apply(vals, locs, grid_size, width, kernel, norm, pad_mode, kernel_params)
