@@ -19,8 +19,7 @@ namespace tlgb {
 namespace {
 
 constexpr int kTileW = 64;               // output voxels along W per CTA (4 warps x 16)
-constexpr int kHaloW = kTileW + 2;       // input voxels along W per (kd, kh) row
-constexpr int kHaloRows = 9;             // (kd, kh) rows
+constexpr int kHaloW = kTileW + 2;       // input voxels along W per staged row
 constexpr int kVoxBytes = 32;            // 16 bf16 channels
 constexpr int kTaps = 27;
 
@@ -44,22 +43,6 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1
 }
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-// The 9 (kd, kh) input rows of kHaloW voxels around output row (d, h, w0..):
-// zero outside the volume. Row r = kd*3 + kh, voxel j = input w0 - 1 + j.
-__device__ __forceinline__ void load_halo(unsigned char* halo, const uint4* __restrict__ x, int D, int H, int W, int d,
-                                          int h, int w0) {
-  for (int i = threadIdx.x; i < kHaloRows * kHaloW * 2; i += blockDim.x) {
-    const int c = i & 1;
-    const int j = (i >> 1) % kHaloW;
-    const int r = (i >> 1) / kHaloW;
-    const int di = d + r / 3 - 1, hi = h + r % 3 - 1, wi = w0 - 1 + j;
-    uint4 v = make_uint4(0u, 0u, 0u, 0u);
-    if (di >= 0 && di < D && hi >= 0 && hi < H && wi >= 0 && wi < W)
-      v = __ldg(x + ((((long long)di * H + hi) * W + wi) * 2 + c));
-    *reinterpret_cast<uint4*>(halo + r * kHaloW * kVoxBytes + swz(j, c)) = v;
-  }
-}
 
 // ---- the tcgen05 path of the forward / data gradient
 //
@@ -226,17 +209,32 @@ __global__ void __launch_bounds__(128) conv3d_tc_kernel(const __grid_constant__ 
 }
 
 // Weight gradient: dW[t][co][ci] = sum over output voxels v of gy[v][co] *
-// x[v + offset(t)][ci]. CTA b takes output rows b, b + grid, ... (fixed), warp
-// w the taps w, w + 4, ...; partial sums per CTA are reduced in CTA order.
+// x[v + offset(t)][ci]. A work unit is a column segment of up to kWgRows output
+// rows (fixed d, consecutive h) of 64 voxels along W; CTA b takes units b, b +
+// grid, ... (fixed), warp w the taps w, w + 4, ...; partial sums per CTA are
+// reduced in CTA order. The input rows (d + kd - 1, h') sit in a ring of 4
+// slots per kd: a new output row needs 3 new input rows and its gy row, copied
+// asynchronously while the row before is multiplied (loading all 9 rows for
+// every output row, with nothing in flight meanwhile, took 290 us at 128^3). What
+// bounds it now are the ldmatrix reads: 512 shared-memory wavefronts per row
+// of 64 voxels against 448 cycles of mma.sync.
 constexpr int kWgTapsPerWarp = 7;
+constexpr int kWgRows = 16;                                // output rows per unit
+constexpr int kWgRowBytes = kHaloW * kVoxBytes;            // one staged input row
+constexpr int kWgCopies = (3 * kHaloW * 2 + 127) / 128;    // 16-byte copies per thread for the 3 kd rows
 
-__global__ void __launch_bounds__(128) conv3d_wgrad_kernel(int D, int H, int W, const uint4* __restrict__ x,
-                                                           const uint4* __restrict__ gy, float* __restrict__ partial) {
-  __shared__ __align__(128) unsigned char halo[kHaloRows * kHaloW * kVoxBytes];
-  __shared__ __align__(128) unsigned char gsm[kTileW * kVoxBytes];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int ntw = (W + kTileW - 1) / kTileW;
-  const long long nrows = (long long)D * H * ntw;
+__device__ __forceinline__ void cp_async16_zfill(uint32_t dst, const void* src, bool on) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(on ? 16 : 0) : "memory");
+}
+
+__global__ void __launch_bounds__(128, 4) conv3d_wgrad_kernel(int D, int H, int W, const uint4* __restrict__ x,
+                                                              const uint4* __restrict__ gy,
+                                                              float* __restrict__ partial) {
+  __shared__ __align__(128) unsigned char halo[3 * 4 * kWgRowBytes];  // [kd][slot][voxel][32 B]
+  __shared__ __align__(128) unsigned char gsm[2 * kTileW * kVoxBytes];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int ntw = (W + kTileW - 1) / kTileW, nseg = (H + kWgRows - 1) / kWgRows;
+  const long long nunits = (long long)D * ntw * nseg;
   float acc[kWgTapsPerWarp][2][4];
 #pragma unroll
   for (int i = 0; i < kWgTapsPerWarp; ++i)
@@ -251,40 +249,71 @@ __global__ void __launch_bounds__(128) conv3d_wgrad_kernel(int D, int H, int W, 
   // voxels 8*(q & 1).., channels 8*(q >> 1)..
   const int xb_row = (lane & 7) + 8 * ((lane >> 3) & 1), xb_chunk = lane >> 4;
   const uint32_t hbase = smem_addr(halo), gbase = smem_addr(gsm);
-  for (long long row = blockIdx.x; row < nrows; row += gridDim.x) {
-    const int wt = (int)(row % ntw);
-    const long long dh = row / ntw;
-    const int h = (int)(dh % H), d = (int)(dh / H);
-    const int w0 = wt * kTileW;
-    __syncthreads();  // the previous row's tiles have been read
-    load_halo(halo, x, D, H, W, d, h, w0);
-    for (int i = threadIdx.x; i < kTileW * 2; i += blockDim.x) {
-      const int c = i & 1, j = i >> 1;
-      const int w = w0 + j;
-      uint4 v = make_uint4(0u, 0u, 0u, 0u);
-      if (w < W) v = __ldg(gy + ((((long long)d * H + h) * W + w) * 2 + c));
-      *reinterpret_cast<uint4*>(gsm + swz(j, c)) = v;
-    }
-    __syncthreads();
-#pragma unroll 1
-    for (int ks = 0; ks < kTileW / 16; ++ks) {
-      uint32_t a0, a1, a2, a3;
-      ldsm_x4_t(gbase + swz(ks * 16 + ga_row, ga_chunk), a0, a1, a2, a3);
-      // A fragment order: (co 0-7, v 0-7), (co 8-15, v 0-7), (co 0-7, v 8-15), (co 8-15, v 8-15)
-      // = stored blocks (v lo, c lo), (v lo, c hi), (v hi, c lo), (v hi, c hi): a0, a1, a2, a3
+  for (long long u = blockIdx.x; u < nunits; u += gridDim.x) {
+    const int hs = (int)(u % nseg);
+    const long long dw = u / nseg;
+    const int wt = (int)(dw % ntw), d = (int)(dw / ntw);
+    const int w0 = wt * kTileW, h0 = hs * kWgRows, h1 = min(H, h0 + kWgRows);
+    // this thread's copies of an input row set: source (without the row) and slot offset
+    long long xoff[kWgCopies];
+    int soff[kWgCopies];
 #pragma unroll
-      for (int i = 0; i < kWgTapsPerWarp; ++i) {
-        const int t = warp + 4 * i;
-        if (t < kTaps) {
-          const int r = t / 3, kw = t % 3;
-          uint32_t b0, b1, b2, b3;
-          ldsm_x4_t(hbase + r * kHaloW * kVoxBytes + swz(ks * 16 + kw + xb_row, xb_chunk), b0, b1, b2, b3);
-          // b0: (v lo, ci lo), b1: (v hi, ci lo), b2: (v lo, ci hi), b3: (v hi, ci hi)
-          mma_bf16(acc[i][0], a0, a1, a2, a3, b0, b1);
-          mma_bf16(acc[i][1], a0, a1, a2, a3, b2, b3);
+    for (int i = 0; i < kWgCopies; ++i) {
+      const int q = tid + 128 * i, kd = q / (kHaloW * 2), j = (q >> 1) % kHaloW, c = q & 1;
+      const int di = d + kd - 1, wi = w0 - 1 + j;
+      soff[i] = q < 3 * kHaloW * 2 ? kd * 4 * kWgRowBytes + (int)swz(j, c) : -1;
+      xoff[i] = di >= 0 && di < D && wi >= 0 && wi < W ? ((long long)di * H * W + wi) * 2 + c : -1;
+    }
+    auto load_x = [&](int hr) {  // the 3 kd rows (d + kd - 1, hr) into slot hr mod 4, zero outside the volume
+      const bool hin = hr >= 0 && hr < H;
+#pragma unroll
+      for (int i = 0; i < kWgCopies; ++i)
+        if (soff[i] >= 0) {
+          const bool in = hin && xoff[i] >= 0;
+          cp_async16_zfill(hbase + (hr & 3) * kWgRowBytes + soff[i], in ? x + xoff[i] + (long long)hr * W * 2 : x, in);
+        }
+    };
+    auto load_g = [&](int h) {
+      const int c = tid & 1, j = tid >> 1, w = w0 + j;
+      const bool in = w < W;
+      cp_async16_zfill(gbase + (h & 1) * kTileW * kVoxBytes + swz(j, c), in ? gy + (((long long)d * H + h) * W + w) * 2 + c : gy, in);
+    };
+    load_x(h0 - 1);
+    load_x(h0);
+    load_x(h0 + 1);
+    load_g(h0);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    for (int h = h0; h < h1; ++h) {
+      if (h + 1 < h1) {
+        load_x(h + 2);
+        load_g(h + 1);
+      }
+      asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 1;" ::: "memory");
+      __syncthreads();
+      const uint32_t gb = gbase + (h & 1) * kTileW * kVoxBytes;
+#pragma unroll
+      for (int ks = 0; ks < kTileW / 16; ++ks) {
+        uint32_t a0, a1, a2, a3;
+        ldsm_x4_t(gb + swz(ks * 16 + ga_row, ga_chunk), a0, a1, a2, a3);
+        // A fragment order: (co 0-7, v 0-7), (co 8-15, v 0-7), (co 0-7, v 8-15), (co 8-15, v 8-15)
+        // = stored blocks (v lo, c lo), (v lo, c hi), (v hi, c lo), (v hi, c hi): a0, a1, a2, a3
+#pragma unroll
+        for (int i = 0; i < kWgTapsPerWarp; ++i) {
+          const int t = warp + 4 * i;
+          if (t < kTaps) {
+            const int kd = t / 9, kh = t / 3 % 3, kw = t % 3;
+            uint32_t b0, b1, b2, b3;
+            ldsm_x4_t(hbase + (kd * 4 + ((h + kh - 1) & 3)) * kWgRowBytes + swz(ks * 16 + kw + xb_row, xb_chunk), b0, b1, b2,
+                      b3);
+            // b0: (v lo, ci lo), b1: (v hi, ci lo), b2: (v lo, ci hi), b3: (v hi, ci hi)
+            mma_bf16(acc[i][0], a0, a1, a2, a3, b0, b1);
+            mma_bf16(acc[i][1], a0, a1, a2, a3, b2, b3);
+          }
         }
       }
+      __syncthreads();  // the row's slots have been read before the copies of the next step
     }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
   }
   const int gid = lane >> 2, tig = lane & 3;
   float* dst = partial + (long long)blockIdx.x * kTaps * 256;
@@ -302,12 +331,24 @@ __global__ void __launch_bounds__(128) conv3d_wgrad_kernel(int D, int H, int W, 
   }
 }
 
-__global__ void wgrad_reduce_kernel(const float* __restrict__ partial, int nparts, float* __restrict__ dw) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= kTaps * 256) return;
+// Sum of the CTAs' parts in order: thread (range r of 8, value) sums its
+// range's parts, then the ranges are added in order. One chain of all parts
+// per value took 28 us for 608 parts.
+__global__ void __launch_bounds__(256) wgrad_reduce_kernel(const float* __restrict__ partial, int nparts,
+                                                           float* __restrict__ dw) {
+  __shared__ float rs[8][32];
+  const int v = threadIdx.x & 31, r = threadIdx.x >> 5, i = blockIdx.x * 32 + v;
+  const int b0 = (int)((long long)nparts * r / 8), b1 = (int)((long long)nparts * (r + 1) / 8);
   float s = 0.f;
-  for (int b = 0; b < nparts; ++b) s += partial[(long long)b * kTaps * 256 + i];
-  dw[i] = s;
+#pragma unroll 8
+  for (int b = b0; b < b1; ++b) s += partial[(long long)b * kTaps * 256 + i];
+  rs[r][v] = s;
+  __syncthreads();
+  if (r == 0) {
+#pragma unroll
+    for (int k = 1; k < 8; ++k) s += rs[k][v];
+    dw[i] = s;
+  }
 }
 
 // complex64 [V] * scale -> bf16 [V][16]: channels 0, 1 = re, im rounded to
@@ -382,8 +423,8 @@ int launch_conv_tc(const tlgb_conv3d_desc* d, const CUtensorMap& map, const void
 }
 
 int wgrad_parts(const tlgb_conv3d_desc* d) {
-  const long long rows = (long long)d->D * d->H * ((d->W + kTileW - 1) / kTileW);
-  return (int)std::min<long long>(rows, 4 * 152);
+  const long long units = (long long)d->D * ((d->H + kWgRows - 1) / kWgRows) * ((d->W + kTileW - 1) / kTileW);
+  return (int)std::min<long long>(units, 4 * 152);  // 4 CTAs per SM
 }
 
 }  // namespace
@@ -433,7 +474,8 @@ extern "C" int tlgb_conv3d_wgrad(const tlgb_conv3d_desc* d, const void* x, const
   const int parts = wgrad_parts(d);
   conv3d_wgrad_kernel<<<parts, 128, 0, s>>>(d->D, d->H, d->W, (const uint4*)x, (const uint4*)gy, (float*)scratch);
   TLGB_CHECK_LAUNCH();
-  wgrad_reduce_kernel<<<(kTaps * 256 + 255) / 256, 256, 0, s>>>((const float*)scratch, parts, dw);
+  static_assert(kTaps * 256 % 32 == 0, "32 values per CTA");
+  wgrad_reduce_kernel<<<kTaps * 256 / 32, 256, 0, s>>>((const float*)scratch, parts, dw);
   TLGB_CHECK_LAUNCH();
   return TLGB_OK;
 }
