@@ -10,7 +10,7 @@
 
 #include <cuda_bf16.h>
 
-#include <cstring>
+#include <algorithm>
 
 #include "common.cuh"
 #include "sm100.cuh"
@@ -44,47 +44,68 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
+__device__ __forceinline__ void cp_async16_zfill(uint32_t dst, const void* src, bool on) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(on ? 16 : 0) : "memory");
+}
+
 // ---- the tcgen05 path of the forward / data gradient
 //
-// Persistent CTAs of 4 warps. A work unit is a column segment of up to kTcRows
-// output rows (fixed d, consecutive h) of 128 voxels along W (MMA M = 128)
-// x 16 output channels (N = 16). Input rows (d + kd - 1, h') sit in a ring of
-// 4 slots per kd; output row h reads rows h - 1, h, h + 1 of each kd, so
-// after the first row each output row needs 3 new rows (6 TMA copies of 8
-// channels x 130 voxels, zero fill outside the volume) instead of 9. Layout:
-// the canonical no-swizzle K-major one, 16-byte rows, the two 8-channel
-// halves of a row 2176 bytes apart; tap (kd, kh, kw) is the A operand kw rows
-// into slot (h + kh - 1) mod 4 of kd, and the 27 taps are 27 MMAs of K = 16
-// into one 128 x 16 FP32 TMEM accumulator. Two accumulators alternate, so
-// the MMAs of row r overlap the epilogue of row r - 1. Weights stay in
-// shared memory ([tap][k half][n group][8][16 B]) for the CTA's lifetime.
-// Thread 0 issues copies and MMAs; every wait is bounded, and a timeout sets
-// the status word and ends the CTA's work after freeing its TMEM.
+// Persistent CTAs, two per SM: 4 epilogue warps, 4 loader warps and one warp
+// that issues the MMAs. A work unit is a column segment of up to kTcRows output
+// rows (fixed d, consecutive h) of 128 voxels along W (MMA M = 128). The input
+// rows (d + kd - 1, h'), kd = 0..2, contribute through their taps to the output
+// rows h' - 1, h', h' + 1: one MMA of N = 48 per (kd, kw), whose B operand holds
+// the weights of kh = 2, 1, 0 side by side, into the 128 x 48 FP32 accumulator
+// of h'. An output row is the sum of one 16-column block of three neighbouring
+// accumulators, added in the epilogue. So an output row costs 9 MMAs that read
+// their A operand from shared memory, not 27 of N = 16 (those read 4 KB for 8
+// cycles of products). The loaders copy the 3 kd rows of an h' as one ring slot,
+// 16 bytes at a time into the canonical no-swizzle K-major layout (16-byte
+// rows, the two 8-channel halves of a row 2176 bytes apart; a TMA box of this
+// layout is 16 bytes wide, 780 such rows per h'); tap kw is the A operand kw
+// rows into the slot. Accumulators sit in a ring of 5, so the epilogue of one
+// row overlaps the MMAs of the next. Weights stay in shared memory for the
+// CTA's lifetime. 128^3: 79 us (99 with 27 MMAs per row fed by TMA; 110 with one
+// CTA per SM, whose waits nothing covers; 54 without the copies, 33 with one
+// MMA per row and no copies or stores; HBM floor 20 us).
+// Every wait is bounded; a timeout sets the status word and a CTA flag, every
+// role stops, and the MMAs and copies in flight are waited for before TMEM is
+// freed.
 constexpr int kTcM = 128;
 constexpr int kTcHalo = kTcM + 2;
 constexpr int kTcRows = 16;                               // output rows per work unit
-constexpr int kTcHalfBytes = 2176;                       // >= 130 * 16, a multiple of 128
-constexpr int kTcSlotBytes = 2 * kTcHalfBytes;
-constexpr uint32_t kTcABytes = 3 * 4 * kTcSlotBytes;     // 3 kd x 4 ring slots
-constexpr uint32_t kTcBBytes = kTaps * 512;              // 13824
-constexpr uint32_t kTcCopyBytes = kTcHalo * 16;          // one 8-channel row copy
-constexpr uint32_t kTcSmem = kTcABytes + kTcBBytes + 64;
-constexpr uint32_t kTcCols = 32;                         // two 16-column accumulators
+constexpr int kTcHalfBytes = 2176;                        // >= 130 * 16, a multiple of 128
+constexpr int kTcRowBytes = 2 * kTcHalfBytes;
+constexpr int kTcSlotBytes = 3 * kTcRowBytes;             // the 3 kd rows of one h'
+constexpr int kTcSlots = 5;
+constexpr int kTcAhead = 3;                               // slots being copied at once
+constexpr uint32_t kTcBTap = 1536;                        // B of one (kd, kw): [k half][6 n groups][8][16 B]
+constexpr uint32_t kTcBBytes = 9 * kTcBTap;
+constexpr int kTcAcc = 5;                                 // accumulators of 48 columns
+constexpr int kTcBars = 2 * kTcSlots + 2 * kTcAcc + 1;    // slots full, empty; accumulators done, free; drain
+constexpr uint32_t kTcSmem = kTcSlots * kTcSlotBytes + kTcBBytes + 8 * kTcBars + 16;
+constexpr uint32_t kTcCols = 256;                         // TMEM columns, 240 used
+constexpr int kTcCtas = 2;                                // CTAs per SM
+constexpr int kTcThreads = 288;
 constexpr uint32_t kTcWait = 1u << 22;
 
 __device__ int g_conv_status;
 
 template <int MODE, bool OUTF32>
-__global__ void __launch_bounds__(128) conv3d_tc_kernel(const __grid_constant__ CUtensorMap xmap, int D, int H, int W,
-                                                        const uint4* __restrict__ wts,
-                                                        const __nv_bfloat16* __restrict__ aux,
-                                                        void* __restrict__ y) {
+__global__ void __launch_bounds__(kTcThreads, kTcCtas) conv3d_tc_kernel(int D, int H, int W, const uint4* __restrict__ x,
+                                                                  const uint4* __restrict__ wts,
+                                                                  const __nv_bfloat16* __restrict__ aux,
+                                                                  void* __restrict__ y) {
   using namespace sm100;
   extern __shared__ __align__(1024) unsigned char smem[];
-  unsigned char* sa = smem;
-  unsigned char* sb = smem + kTcABytes;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sb + kTcBBytes);  // [0,1] copies, [2,3] MMAs
-  uint32_t* slot = reinterpret_cast<uint32_t*>(bars + 4);        // [0] TMEM address, [1] failure flag
+  unsigned char* sb = smem + kTcSlots * kTcSlotBytes;
+  uint64_t* full = reinterpret_cast<uint64_t*>(sb + kTcBBytes);
+  uint64_t* empty = full + kTcSlots;
+  uint64_t* done = empty + kTcSlots;
+  uint64_t* freed = done + kTcAcc;
+  uint64_t* drain = freed + kTcAcc;
+  uint32_t* slot = reinterpret_cast<uint32_t*>(drain + 1);  // [0] TMEM address, [1] failure flag
+  volatile uint32_t* failed = slot + 1;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int ntw = (W + kTcM - 1) / kTcM, nseg = (H + kTcRows - 1) / kTcRows;
   const long long nunits = (long long)D * ntw * nseg;
@@ -93,117 +114,171 @@ __global__ void __launch_bounds__(128) conv3d_tc_kernel(const __grid_constant__ 
     tmem_relinquish();
   }
   if (tid == 0) {
-    for (int i = 0; i < 4; ++i) mbar_init(&bars[i], 1);
+    for (int i = 0; i < kTcSlots; ++i) {
+      mbar_init(&full[i], 128);
+      mbar_init(&empty[i], 1);
+    }
+    for (int i = 0; i < kTcAcc; ++i) {
+      mbar_init(&done[i], 1);
+      mbar_init(&freed[i], 128);
+    }
+    mbar_init(drain, 1);
     fence_mbar_init();
     slot[1] = 0;
   }
-  for (int i = tid; i < kTaps * 16 * 2; i += 128) {
-    const int kh2 = i & 1, co = (i >> 1) & 15, t = i >> 5;
-    *reinterpret_cast<uint4*>(sb + t * 512 + kh2 * 256 + (co >> 3) * 128 + (co & 7) * 16) = __ldg(wts + i);
+  for (int i = tid; i < kTaps * 16 * 2; i += kTcThreads) {
+    const int half = i & 1, co = (i >> 1) & 15, t = i >> 5, kd = t / 9, kh = t / 3 % 3, kw = t % 3;
+    const int n = (2 - kh) * 16 + co;
+    *reinterpret_cast<uint4*>(sb + (kd * 3 + kw) * kTcBTap + half * 768 + (n >> 3) * 128 + (n & 7) * 16) = __ldg(wts + i);
   }
   fence_proxy_async_smem();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = slot[0];
-  const uint32_t a0 = smem_u32(sa), b0 = smem_u32(sb);
-  constexpr uint32_t idesc = idesc_bf16_f32(kTcM, 16);
-  uint32_t lg = 0;     // copy groups issued (thread 0): group k arms bars[k & 1]
-  uint32_t lw = 0;     // copy groups waited on (thread 0)
-  uint32_t og = 0;     // output rows issued in this CTA: row k uses accumulator k & 1 and bars[2 + (k & 1)]
-  bool fail = false;
-
-  auto load_row = [&](int d, int hr, int w0) {  // the 3 kd rows (d + kd - 1, hr) into slot hr mod 4
-    for (int kd = 0; kd < 3; ++kd)
-      for (int hf = 0; hf < 2; ++hf)
-        tma_load_4d(sa + (kd * 4 + (hr & 3)) * kTcSlotBytes + hf * kTcHalfBytes, &xmap, &bars[lg & 1], hf * 8, w0 - 1,
-                    hr, d + kd - 1);
+  auto give_up = [&]() {
+    *failed = 1;
+    atomicExch(&g_conv_status, 2);
   };
-
-  for (long long u = blockIdx.x; u < nunits && !fail; u += gridDim.x) {
+  auto unit = [&](long long u, int& d, int& w0, int& h0, int& R) {
     const int hs = (int)(u % nseg);
     const long long dw = u / nseg;
-    const int wt = (int)(dw % ntw), d = (int)(dw / ntw);
-    const int w0 = wt * kTcM, h0 = hs * kTcRows;
-    const int R = min(kTcRows, H - h0);
-    if (tid == 0) {
-      mbar_arrive_expect_tx(&bars[lg & 1], 9 * 2 * kTcCopyBytes);
-      for (int hr = h0 - 1; hr <= h0 + 1; ++hr) load_row(d, hr, w0);
-      ++lg;
-    }
-    for (int r = 0; r <= R; ++r) {
-      const int h = h0 + r;
-      if (tid == 0 && r < R && !fail) {
-        if (r + 1 < R) {
-          // row h + 2 (for output h + 1) replaces row h - 2, last read by output h - 1
-          if (r >= 1 && !mbar_wait_bounded(&bars[2 + ((og - 1) & 1)], ((og - 1) >> 1) & 1, kTcWait)) fail = true;
-          mbar_arrive_expect_tx(&bars[lg & 1], 3 * 2 * kTcCopyBytes);
-          load_row(d, h + 2, w0);
-          ++lg;
-        }
-        if (!mbar_wait_bounded(&bars[lw & 1], (lw >> 1) & 1, kTcWait)) fail = true;
-        ++lw;
-        if (!fail) {
-          tc_fence_after();
-          const uint32_t acc = tmem + (og & 1) * 16;
-          for (int t = 0; t < kTaps; ++t) {
-            const int kd = t / 9, kh = (t / 3) % 3, kw = t % 3;
-            const uint32_t aa = a0 + (kd * 4 + ((h + kh - 1) & 3)) * kTcSlotBytes + kw * 16;
-            umma_bf16(acc, smem_desc(aa, kTcHalfBytes, 128), smem_desc(b0 + t * 512, 256, 128), idesc,
-                      t > 0 ? 1u : 0u);
-          }
-          umma_commit(&bars[2 + (og & 1)]);
-        }
-        if (fail) slot[1] = 1;
+    w0 = (int)(dw % ntw) * kTcM, d = (int)(dw / ntw), h0 = hs * kTcRows, R = min(kTcRows, H - h0);
+  };
+
+  if (warp >= 4 && warp < 8) {
+    // ---- loaders
+    const int lt = tid - 128;
+    const uint32_t s0 = smem_u32(smem);
+    constexpr int NC = (3 * kTcHalo * 2 + 127) / 128;
+    uint32_t k = 0, sent = 0;  // slots begun, slots handed over
+    bool ok = true;
+    auto hand_over = [&]() {   // this thread's copies of slot `sent` have landed
+      fence_proxy_async_smem();
+      mbar_arrive(&full[sent % kTcSlots]);
+      ++sent;
+    };
+    for (long long u = blockIdx.x; u < nunits && ok; u += gridDim.x) {
+      int d, w0, h0, R;
+      unit(u, d, w0, h0, R);
+      long long xoff[NC];
+      uint32_t soff[NC];
+#pragma unroll
+      for (int i = 0; i < NC; ++i) {
+        const int q = lt + 128 * i, kd = q / (kTcHalo * 2), j = (q >> 1) % kTcHalo, c = q & 1;
+        const int di = d + kd - 1, wi = w0 - 1 + j;
+        soff[i] = (uint32_t)(kd * kTcRowBytes + c * kTcHalfBytes + j * 16);
+        xoff[i] = di >= 0 && di < D && wi >= 0 && wi < W ? ((long long)di * H * W + wi) * 2 + c : -1;
       }
-      if (r < R) ++og;
-      if (r >= 1) {
-        // epilogue of output h - 1 (accumulator (og - 2) & 1 after this row's increment)
-        const uint32_t k = r < R ? og - 2 : og - 1;
-        const bool done = mbar_wait_bounded(&bars[2 + (k & 1)], (k >> 1) & 1, kTcWait);
-        if (!done) slot[1] = 1;
-        if (__syncthreads_and(done)) {
-          tc_fence_after();
-          float v[16];
-          tmem_ld16(tmem + (k & 1) * 16 + ((uint32_t)(warp * 32) << 16), v);
-          const int w = w0 + warp * 32 + lane;
-          if (w < W) {
-            const long long vox = ((long long)d * H + (h - 1)) * W + w;
-            if (MODE == 1) {
+      for (int hr = h0 - 1; hr <= h0 + R; ++hr, ++k) {
+        const uint32_t s = k % kTcSlots;
+        ok = mbar_wait_bounded(&empty[s], ((k / kTcSlots) & 1) ^ 1, kTcWait) && !*failed;
+        if (!ok) break;
+        const bool hin = hr >= 0 && hr < H;
 #pragma unroll
-              for (int i = 0; i < 16; ++i) v[i] = fmaxf(v[i], 0.f);
-            } else if (MODE == 2) {
-              const uint4* m4 = reinterpret_cast<const uint4*>(aux + vox * 16);
-              uint4 mm[2] = {__ldg(m4), __ldg(m4 + 1)};
-              const __nv_bfloat16* mb = reinterpret_cast<const __nv_bfloat16*>(mm);
-#pragma unroll
-              for (int i = 0; i < 16; ++i) v[i] = __bfloat162float(mb[i]) > 0.f ? v[i] : 0.f;
-            }
-            if (OUTF32) {
-              float4* o = reinterpret_cast<float4*>(reinterpret_cast<float*>(y) + vox * 16);
-#pragma unroll
-              for (int q = 0; q < 4; ++q) o[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-            } else {
-              uint4 pk[2];
-              __nv_bfloat162* pb = reinterpret_cast<__nv_bfloat162*>(pk);
-#pragma unroll
-              for (int i = 0; i < 8; ++i) pb[i] = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
-              uint4* o = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(y) + vox * 16);
-              o[0] = pk[0];
-              o[1] = pk[1];
-            }
+        for (int i = 0; i < NC; ++i)
+          if (lt + 128 * i < 3 * kTcHalo * 2) {
+            const bool in = hin && xoff[i] >= 0;
+            cp_async16_zfill(s0 + s * kTcSlotBytes + soff[i], in ? x + xoff[i] + (long long)hr * W * 2 : x, in);
           }
-        }
-      }
-      tc_fence_before();
-      __syncthreads();
-      if (slot[1]) {
-        fail = true;
-        break;
+        asm volatile("cp.async.commit_group;\n\tcp.async.wait_group %0;" ::"n"(kTcAhead - 1) : "memory");
+        if (k >= kTcAhead - 1) hand_over();
       }
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    if (ok)
+      while (sent < k) hand_over();
+    else
+      give_up();
+  } else if (warp == 8) {
+    // ---- MMA issue, one thread
+    if (lane == 0) {
+      const uint32_t a0 = smem_u32(smem), b0 = smem_u32(sb);
+      constexpr uint32_t idesc = idesc_bf16_f32(kTcM, 48);
+      uint32_t k = 0;
+      bool ok = true;
+      for (long long u = blockIdx.x; u < nunits && ok; u += gridDim.x) {
+        int d, w0, h0, R;
+        unit(u, d, w0, h0, R);
+        for (int i = 0; i < R + 2; ++i, ++k) {  // input row h0 - 1 + i
+          const uint32_t s = k % kTcSlots, q = k % kTcAcc;
+          ok = mbar_wait_bounded(&freed[q], ((k / kTcAcc) & 1) ^ 1, kTcWait) &&
+               mbar_wait_bounded(&full[s], (k / kTcSlots) & 1, kTcWait) && !*failed;
+          if (!ok) break;
+          tc_fence_after();
+          for (int t = 0; t < 9; ++t)
+            umma_bf16(tmem + q * 48,
+                      smem_desc(a0 + s * kTcSlotBytes + (t / 3) * kTcRowBytes + (t % 3) * 16, kTcHalfBytes, 128),
+                      smem_desc(b0 + t * kTcBTap, 768, 128), idesc, t > 0 ? 1u : 0u);
+          umma_commit(&empty[s]);
+          umma_commit(&done[q]);
+        }
+      }
+      if (!ok) give_up();
+      umma_commit(drain);  // nothing in flight when TMEM is freed
+      if (!mbar_wait_bounded(drain, 0, kTcWait)) atomicExch(&g_conv_status, 2);
+    }
+    __syncwarp();
+  } else {
+    // ---- epilogue: warp = TMEM lanes 32 warp .., thread = voxel
+    uint32_t k = 0;  // input row of the unit's first
+    bool ok = true;
+    for (long long u = blockIdx.x; u < nunits && ok; u += gridDim.x) {
+      int d, w0, h0, R;
+      unit(u, d, w0, h0, R);
+      const int w = w0 + tid;
+      const uint32_t lanes = (uint32_t)(warp * 32) << 16;
+      for (int r = 0; r < R; ++r) {
+        // output row r: kh 0 of input row r, kh 1 of r + 1, kh 2 of r + 2 (whose MMAs follow the others')
+        const uint32_t k2 = k + r + 2;
+        ok = mbar_wait_bounded(&done[k2 % kTcAcc], (k2 / kTcAcc) & 1, kTcWait);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        tc_fence_after();
+        float v[16], v1[16], v2[16];
+        tmem_ld16(tmem + (k + r) % kTcAcc * 48 + 32 + lanes, v);
+        tmem_ld16(tmem + (k + r + 1) % kTcAcc * 48 + 16 + lanes, v1);
+        tmem_ld16(tmem + k2 % kTcAcc * 48 + lanes, v2);
+        tc_fence_before();
+        mbar_arrive(&freed[(k + r) % kTcAcc]);
+        if (r == R - 1) {  // the unit's last two input rows have no further output row
+          mbar_arrive(&freed[(k + r + 1) % kTcAcc]);
+          mbar_arrive(&freed[k2 % kTcAcc]);
+        }
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] = v[i] + v1[i] + v2[i];
+        if (w < W) {
+          const long long vox = ((long long)d * H + (h0 + r)) * W + w;
+          if (MODE == 1) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) v[i] = fmaxf(v[i], 0.f);
+          } else if (MODE == 2) {
+            const uint4* m4 = reinterpret_cast<const uint4*>(aux + vox * 16);
+            uint4 mm[2] = {__ldg(m4), __ldg(m4 + 1)};
+            const __nv_bfloat16* mb = reinterpret_cast<const __nv_bfloat16*>(mm);
+#pragma unroll
+            for (int i = 0; i < 16; ++i) v[i] = __bfloat162float(mb[i]) > 0.f ? v[i] : 0.f;
+          }
+          if (OUTF32) {
+            float4* o = reinterpret_cast<float4*>(reinterpret_cast<float*>(y) + vox * 16);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) o[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+          } else {
+            uint4 pk[2];
+            __nv_bfloat162* pb = reinterpret_cast<__nv_bfloat162*>(pk);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) pb[i] = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+            uint4* o = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(y) + vox * 16);
+            o[0] = pk[0];
+            o[1] = pk[1];
+          }
+        }
+      }
+      k += R + 2;
+    }
+    if (!ok && lane == 0) give_up();
   }
-  if (fail && tid == 0) atomicExch(&g_conv_status, 2);
+  tc_fence_before();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tmem, kTcCols);
 }
@@ -222,10 +297,6 @@ constexpr int kWgTapsPerWarp = 7;
 constexpr int kWgRows = 16;                                // output rows per unit
 constexpr int kWgRowBytes = kHaloW * kVoxBytes;            // one staged input row
 constexpr int kWgCopies = (3 * kHaloW * 2 + 127) / 128;    // 16-byte copies per thread for the 3 kd rows
-
-__device__ __forceinline__ void cp_async16_zfill(uint32_t dst, const void* src, bool on) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(on ? 16 : 0) : "memory");
-}
 
 __global__ void __launch_bounds__(128, 4) conv3d_wgrad_kernel(int D, int H, int W, const uint4* __restrict__ x,
                                                               const uint4* __restrict__ gy,
@@ -396,28 +467,13 @@ int check_conv(const tlgb_conv3d_desc* d) {
   return TLGB_OK;
 }
 
-// 4D tensor map over an activation [D][H][W][16] bf16 for 8-channel x 130-voxel boxes
-bool conv_tensor_map(const tlgb_conv3d_desc* d, const void* x, CUtensorMap* map) {
-  auto enc = sm100::tensor_map_encoder();
-  if (!enc || ((uintptr_t)x & 15)) return false;
-  memset(map, 0, sizeof(*map));
-  const cuuint64_t dims[4] = {16, (cuuint64_t)d->W, (cuuint64_t)d->H, (cuuint64_t)d->D};
-  const cuuint64_t strides[3] = {32, (cuuint64_t)d->W * 32, (cuuint64_t)d->W * d->H * 32};
-  const cuuint32_t box[4] = {8, (cuuint32_t)kTcHalo, 1, 1};
-  const cuuint32_t estr[4] = {1, 1, 1, 1};
-  return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(x), dims, strides, box, estr,
-             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
 template <int MODE, bool OUTF32>
-int launch_conv_tc(const tlgb_conv3d_desc* d, const CUtensorMap& map, const void* w, const void* aux, void* y,
-                   cudaStream_t s) {
+int launch_conv_tc(const tlgb_conv3d_desc* d, const void* x, const void* w, const void* aux, void* y, cudaStream_t s) {
   auto* k = conv3d_tc_kernel<MODE, OUTF32>;
   TLGB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem));
   const long long units = (long long)d->D * ((d->W + kTcM - 1) / kTcM) * ((d->H + kTcRows - 1) / kTcRows);
-  const unsigned grid = (unsigned)std::min<long long>(units, 3ll * sm_count());  // 3 CTAs of 66 KB per SM
-  k<<<grid, 128, kTcSmem, s>>>(map, d->D, d->H, d->W, (const uint4*)w, (const __nv_bfloat16*)aux, y);
+  const unsigned grid = (unsigned)std::min<long long>(units, (long long)kTcCtas * sm_count());
+  k<<<grid, kTcThreads, kTcSmem, s>>>(d->D, d->H, d->W, (const uint4*)x, (const uint4*)w, (const __nv_bfloat16*)aux, y);
   TLGB_CHECK_LAUNCH();
   return TLGB_OK;
 }
@@ -439,19 +495,14 @@ extern "C" int tlgb_conv3d_fwd(const tlgb_conv3d_desc* d, const void* x, const v
   if (((uintptr_t)x | (uintptr_t)w | (uintptr_t)y | (uintptr_t)aux) & 15)
     TLGB_FAIL(TLGB_ERR_INVALID, "conv3d: buffers must be 16-byte aligned");
   cudaStream_t s = (cudaStream_t)stream;
-  CUtensorMap map;
-  if (conv_tensor_map(d, x, &map)) {
-    if (d->out_f32) {
-      if (d->mode == 0) return launch_conv_tc<0, true>(d, map, w, aux, y, s);
-      if (d->mode == 1) return launch_conv_tc<1, true>(d, map, w, aux, y, s);
-      return launch_conv_tc<2, true>(d, map, w, aux, y, s);
-    }
-    if (d->mode == 0) return launch_conv_tc<0, false>(d, map, w, aux, y, s);
-    if (d->mode == 1) return launch_conv_tc<1, false>(d, map, w, aux, y, s);
-    return launch_conv_tc<2, false>(d, map, w, aux, y, s);
+  if (d->out_f32) {
+    if (d->mode == 0) return launch_conv_tc<0, true>(d, x, w, aux, y, s);
+    if (d->mode == 1) return launch_conv_tc<1, true>(d, x, w, aux, y, s);
+    return launch_conv_tc<2, true>(d, x, w, aux, y, s);
   }
-  TLGB_FAIL(TLGB_ERR_UNSUPPORTED,
-            "conv3d: the driver offers no tensor-map encoder, which the TMA-fed tcgen05 kernel needs");
+  if (d->mode == 0) return launch_conv_tc<0, false>(d, x, w, aux, y, s);
+  if (d->mode == 1) return launch_conv_tc<1, false>(d, x, w, aux, y, s);
+  return launch_conv_tc<2, false>(d, x, w, aux, y, s);
 }
 
 extern "C" int tlgb_conv3d_wgrad_scratch_size(const tlgb_conv3d_desc* d, size_t* bytes) {
