@@ -2115,6 +2115,49 @@ __global__ void __launch_bounds__(128) plan_records_kernel(Geo g, const uint32_t
   }
 }
 
+// A region by asynchronous 8-byte copies of the producer threads, wrapped or
+// zero-filled: a thread copies its (y, z) cells of every (entry, x) plane.
+template <int NDIM, int KT, int CG>
+__device__ __forceinline__ void copy_region(const Geo& g, const float* __restrict__ gridv, float2* reg, const int (&o)[3],
+                                            int cg, int pt) {
+  constexpr int S = region_edge<NDIM, KT>(), PLANE = S * S;
+  constexpr int Q = (PLANE + kGatherProd - 1) / kGatherProd;
+  const long long gpl = (long long)g.N[1] * g.N[2], gvol = gpl * g.N[0];
+#pragma unroll
+  for (int q = 0; q < Q; ++q) {
+    const int cell = pt + q * kGatherProd;
+    if (cell >= PLANE) break;
+    const int y = cell / S, z = cell - y * S;
+    int gy = o[1] + y, gz = o[2] + z;
+    bool in = gy < g.N[1] && gz < g.N[2];
+    if (g.pad == TLGB_PAD_CIRCULAR) gy = wrapi(gy, g.N[1]), gz = wrapi(gz, g.N[2]), in = true;
+    const float2* src = reinterpret_cast<const float2*>(gridv) + (long long)(cg * CG) * gvol +
+                        (in ? (long long)gy * g.N[2] + gz : 0);
+    float2* dst = reg + cell;
+    for (int c = 0; c < CG; ++c, src += gvol) {
+      const bool cin = in && cg * CG + c < g.nbatch;
+      if constexpr (NDIM == 3) {
+        int gx = o[0];
+        const float2* sx = src + (long long)gx * gpl;
+        for (int x = 0; x < S; ++x, dst += PLANE, sx += gpl) {
+          bool xin = cin;
+          if (gx >= g.N[0]) {  // past the upper edge
+            if (g.pad == TLGB_PAD_CIRCULAR)
+              gx -= g.N[0], sx -= gvol;
+            else
+              xin = false;
+          }
+          sm100::cp_async8_zfill(dst, xin ? sx : reinterpret_cast<const float2*>(gridv), xin);
+          ++gx;
+        }
+      } else {
+        sm100::cp_async8_zfill(dst, cin ? src : reinterpret_cast<const float2*>(gridv), cin);
+        dst += PLANE;
+      }
+    }
+  }
+}
+
 template <int NDIM, int KT, int CG, int NW, int NST, int CTAS>
 __global__ void __launch_bounds__(NW * 32 + kGatherProd, CTAS)
     gather_kernel(const __grid_constant__ CUtensorMap tmap, int use_tma, Geo g, const int4* __restrict__ items, int nruns,
@@ -2189,42 +2232,7 @@ __global__ void __launch_bounds__(NW * 32 + kGatherProd, CTAS)
           }
           continue;
         }
-        // a thread copies its (y, z) cells of every (entry, x) plane
-        constexpr int Q = (PLANE + kGatherProd - 1) / kGatherProd;
-        const long long gpl = (long long)g.N[1] * g.N[2], gvol = gpl * g.N[0];
-#pragma unroll
-        for (int q = 0; q < Q; ++q) {
-          const int cell = pt + q * kGatherProd;
-          if (cell >= PLANE) break;
-          const int y = cell / S, z = cell - y * S;
-          int gy = o[1] + y, gz = o[2] + z;
-          bool in = gy < g.N[1] && gz < g.N[2];
-          if (g.pad == TLGB_PAD_CIRCULAR) gy = wrapi(gy, g.N[1]), gz = wrapi(gz, g.N[2]), in = true;
-          const float2* src = reinterpret_cast<const float2*>(gridv) + (long long)(cg * CG) * gvol +
-                              (in ? (long long)gy * g.N[2] + gz : 0);
-          float2* dst = reg + cell;
-          for (int c = 0; c < CG; ++c, src += gvol) {
-            const bool cin = in && cg * CG + c < g.nbatch;
-            if constexpr (NDIM == 3) {
-              int gx = o[0];
-              const float2* sx = src + (long long)gx * gpl;
-              for (int x = 0; x < S; ++x, dst += PLANE, sx += gpl) {
-                bool xin = cin;
-                if (gx >= g.N[0]) {  // past the upper edge
-                  if (g.pad == TLGB_PAD_CIRCULAR)
-                    gx -= g.N[0], sx -= gvol;
-                  else
-                    xin = false;
-                }
-                sm100::cp_async8_zfill(dst, xin ? sx : reinterpret_cast<const float2*>(gridv), xin);
-                ++gx;
-              }
-            } else {
-              sm100::cp_async8_zfill(dst, cin ? src : reinterpret_cast<const float2*>(gridv), cin);
-              dst += PLANE;
-            }
-          }
-        }
+        copy_region<NDIM, KT, CG>(g, gridv, reg, o, cg, pt);
         sm100::cp_async_mbar_arrive(&full[s]);
       }
       ok = ok && !*vfailed;
@@ -2611,234 +2619,288 @@ __global__ void __launch_bounds__(256) grad_reduce_kernel(const float* __restric
 
 // ------------------------------------------------ 2D trajectory gradient
 //
-// Per-point gradient records for 2D geometries (built per call, since the
-// trajectory may change between calls): the weights and derivative weights
-// of the first 4 valid taps in y and z (zero beyond), the first valid tap's
-// position (wrapped in circular mode) and the tap counts (cy | cz << 4; a
-// zero count marks a point without taps). The taps follow tap_eval; weights
-// and derivatives are kern_value and kern_deriv / r, as in warp_point_taps.
-struct __align__(16) GRec2 {
-  float4 w[2], dw[2];
-  int st[2];
-  int cnt;
-  int pad;
-};
-static_assert(sizeof(GRec2) == 80, "80-byte gradient records");
+// d/d(y, z) of sum_b Re(conj(a[b, p]) ungrid(grid)[b, p]) for 2D geometries of at
+// most 5 taps per dim, on the gather's ring (gather_kernel): a stage is the
+// region of a group of 8 entries and the item's 8 x 256 values of a, gathered by
+// the producers in the records' order, so runs of points are read in whole
+// lines. The sum over the entries comes first: a tap's weight and derivative are
+// the same for every entry, so a lane adds Re(conj(a) v) per tap over all groups
+// of the unit in registers (4 y taps x 8 steps of 2 points) and the weights are
+// applied once per point at the end, the derivatives evaluated there by 16
+// lanes. (Weighting every product, adding the 32 lanes up for each group and the
+// groups' partial results in a further pass took 1243 us for 205,824 points x
+// 256 entries on 320^2; this takes 607 us.)
+constexpr int kGradWarps = 16;
+constexpr int kGradStages = 4;
+constexpr int kGradSteps = kGatherPts / (2 * kGradWarps);
+constexpr uint32_t kGradRegion = 20 * 20 * 8 * 8;
+constexpr uint32_t kGradStage = kGradRegion + 8 * kGatherPts * 8;
 
-__global__ void __launch_bounds__(256) grad_records2_kernel(Geo g, const float* __restrict__ locs,
-                                                            GRec2* __restrict__ out) {
-  const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= g.npts) return;
-  GRec2 R;
-  int cnt = 0;
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    const int e = 1 + i;
-    float w[4] = {0.f, 0.f, 0.f, 0.f}, dw[4] = {0.f, 0.f, 0.f, 0.f};
-    int c = 0, st = 0;
-    const float x = load_coord(g, locs, p, e);
-    if (coord_ok(x)) {
-      const int lower = lower_of(g, e, x);
-      int s = -1;
-#pragma unroll
-      for (int k = 0; k < 5; ++k) {
-        const Tap t = tap_eval(g, e, x, lower, k);
-        if (!t.valid) continue;
-        if (s < 0) s = k;
-        if (c < 4) {
-          w[c] = kern_value(g.kernel, fabsf(t.d), g.beta);
-          dw[c] = kern_deriv(g.kernel, t.d, g.beta) / g.r[e];
-        }
-        ++c;
-      }
-      if (c > 0) {
-        st = lower + s;
-        if (g.pad == TLGB_PAD_CIRCULAR) st = wrapi(st, g.N[e]);
-      }
-    }
-    R.w[i] = make_float4(w[0], w[1], w[2], w[3]);
-    R.dw[i] = make_float4(dw[0], dw[1], dw[2], dw[3]);
-    R.st[i] = st;
-    cnt |= c << (4 * i);
-  }
-  R.cnt = cnt;
-  R.pad = 0;
-  out[p] = R;
+struct GradTaps {  // a window of 5 taps, one per consumer warp
+  float w[2][5], dw[2][5];
+  int n[2], f[2];
+};
+
+constexpr size_t grad2_smem() {
+  return (size_t)kGradStages * kGradStage + 2 * kGatherPts * sizeof(GatherRec<2, 4>) + kGatherPts * sizeof(float2) +
+         kGradWarps * (sizeof(GradTaps) + 16 * sizeof(float)) + 8 * (2 * kGradStages + 4) + 16;
 }
 
-// d/d(y, z) of sum_b Re(conj(a[b, p]) ungrid(grid)[b, p]) for one coil group
-// (blockIdx.y) of a 2D geometry with 8 complex entries per group: CTA = 8
-// warps sharing the 20 x 20 x 8-entry region of one 16 x 16 tile, as
-// fwd_f2_kernel. Lanes = (entry, z-tap): a lane sums its entry's 4 y-taps
-// for both derivatives, then all 32 lanes add up. With several coil groups
-// the group's sums go to its partial slot (added in order afterwards).
-__global__ void __launch_bounds__(256, 3) grad_f2_kernel(const __grid_constant__ CUtensorMap tmap, int use_tma, Geo g,
-                                                         const int4* __restrict__ items,
-                                                         const int32_t* __restrict__ entries,
-                                                         const GRec2* __restrict__ grecs,
-                                                         const float* __restrict__ locs,
-                                                         const float* __restrict__ gridv, const float2* __restrict__ a,
-                                                         float* __restrict__ grad, float* __restrict__ partial) {
-  constexpr int CG = 8, S = 20, VOL = S * S, NW = 8;
-  constexpr uint32_t RBYTES = VOL * CG * 8;
+__global__ void __launch_bounds__(kGradWarps * 32 + kGatherProd, 1)
+    grad2_kernel(const __grid_constant__ CUtensorMap tmap, int use_tma, Geo g, const int4* __restrict__ items, int nruns,
+                 int run, int nunits, const GatherRec<2, 4>* __restrict__ recs, const float* __restrict__ locs,
+                 const float* __restrict__ gridv, const float2* __restrict__ a, float* __restrict__ grad,
+                 float* __restrict__ partial) {
+  constexpr int S = 20, VOL = S * S, NW = kGradWarps, NST = kGradStages;
+  using Rec = GatherRec<2, 4>;
   extern __shared__ __align__(128) unsigned char smem[];
-  float2* reg = reinterpret_cast<float2*>(smem);                  // [8][20][20]
-  GRec2* rec = reinterpret_cast<GRec2*>(smem + RBYTES);           // [8 warps][8]
-  PTaps<true>* slow = reinterpret_cast<PTaps<true>*>(rec + 64);   // [NW]
-  uint64_t* bar = reinterpret_cast<uint64_t*>(slow + NW);
-  const int4 it = items[blockIdx.x];
+  Rec* recbuf = reinterpret_cast<Rec*>(smem + NST * kGradStage);
+  float2* far = reinterpret_cast<float2*>(recbuf + 2 * kGatherPts);  // sums of the unit's 5-tap windows
+  GradTaps* slow = reinterpret_cast<GradTaps*>(far + kGatherPts);
+  float* dwb = reinterpret_cast<float*>(slow + NW);                  // [warp][point][dim][4]
+  uint64_t* full = reinterpret_cast<uint64_t*>((reinterpret_cast<uintptr_t>(dwb + NW * 16) + 7) & ~(uintptr_t)7);
+  uint64_t* empty = full + NST;
+  uint64_t* rfull = empty + NST;
+  uint64_t* rempty = rfull + 2;
+  __shared__ int failed;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int cg = blockIdx.y;
-  const int c0 = cg * CG;
-  float* dst = gridDim.y == 1 ? grad : partial + (long long)cg * g.npts * 2;
-  int o[3];
-  {
-    int t = it.x;
-    o[2] = (t % g.nt[2]) * g.T[2];
-    t /= g.nt[2];
-    o[1] = (t % g.nt[1]) * g.T[1];
-    o[0] = 0;
-  }
-  const bool wraps = g.pad == TLGB_PAD_CIRCULAR && (o[1] + S > g.N[1] || o[2] + S > g.N[2]);
-  const bool tma = use_tma && !wraps;
-  if (tma) {
-    if (tid == 0) {
-      mbar_init(bar, 1);
-      fence_mbar_init();
+  if (tid == 0) {
+    for (int i = 0; i < NST; ++i) {
+      mbar_init(&full[i], kGatherProd);
+      mbar_init(&empty[i], NW);
     }
-    __syncthreads();
-    if (tid == 0) {
-      if (!g.skip_copy) {  // test hook: nothing in flight, so the bounded wait runs out
-        mbar_arrive_expect_tx(bar, RBYTES);
-        tma_load_4d(reg, &tmap, bar, o[2], o[1], 0, c0);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&rfull[i], 1);
+      mbar_init(&rempty[i], NW);
+    }
+    fence_mbar_init();
+    failed = 0;
+  }
+  __syncthreads();
+  const uint32_t limit = g.skip_copy ? 1u : 1u << 22;  // test hook: nothing is copied, so the waits run out
+  const int ncg = (int)((g.nbatch + 7) / 8);
+  volatile int* vfailed = &failed;
+  if (warp >= NW) {
+    // ---- producers
+    if (g.skip_copy) return;
+    const int pt = tid - NW * 32;
+    uint32_t k = 0, ui = 0;
+    bool ok = true;
+    int4 next = items[blockIdx.x / nruns];
+    for (int u = blockIdx.x; u < nunits && ok; u += gridDim.x, ++ui) {
+      const int4 it = next;
+      if (u + (int)gridDim.x < nunits) next = items[(u + gridDim.x) / nruns];
+      const int g0 = (u % nruns) * run, g1 = min(ncg, g0 + run), npt = it.z - it.y;
+      int o[3];
+      item_origin(g, it.x, o);
+      const bool wraps = g.pad == TLGB_PAD_CIRCULAR && (o[1] + S > g.N[1] || o[2] + S > g.N[2]);
+      const bool tma = use_tma && !wraps;
+      const Rec* rec = recbuf + (ui & 1) * kGatherPts;
+      if (pt == 0) {
+        ok = mbar_wait_bounded(&rempty[ui & 1], ((ui >> 1) & 1) ^ 1, limit);
+        if (ok) {
+          const uint32_t bytes = (uint32_t)npt * (uint32_t)sizeof(Rec);
+          mbar_arrive_expect_tx(&rfull[ui & 1], bytes);
+          sm100::bulk_load(recbuf + (ui & 1) * kGatherPts, recs + it.w, bytes, &rfull[ui & 1]);
+        }
+      }
+      ok = ok && mbar_wait_bounded(&rfull[ui & 1], (ui >> 1) & 1, limit);
+      for (int cg = g0; cg < g1 && ok; ++cg, ++k) {
+        const uint32_t s = k % NST;
+        ok = mbar_wait_bounded(&empty[s], ((k / NST) & 1) ^ 1, limit) && !*vfailed;
+        if (!ok) break;
+        float2* reg = reinterpret_cast<float2*>(smem + s * kGradStage);
+        float2* av = reinterpret_cast<float2*>(smem + s * kGradStage + kGradRegion);
+        if (tma) {
+          if (pt == 0) {
+            sm100::fence_proxy_async_smem();  // the buffer may last have been filled by plain copies
+            sm100::mbar_expect_tx(&full[s], kGradRegion);
+            tma_load_4d(reg, &tmap, &full[s], o[2], o[1], 0, cg * 8);
+          }
+        } else {
+          copy_region<2, 4, 8>(g, gridv, reg, o, cg, pt);
+        }
+        for (int i = pt; i < npt; i += kGatherProd) {
+          const int p = rec[i].p;
+#pragma unroll
+          for (int c = 0; c < 8; ++c) {
+            const bool in = cg * 8 + c < g.nbatch && TLGB_IN_RANGE(p, g.npts);
+            sm100::cp_async8_zfill(av + c * kGatherPts + i, in ? a + (long long)(cg * 8 + c) * g.npts + p : a, in);
+          }
+        }
+        sm100::cp_async_mbar_arrive(&full[s]);
+      }
+      ok = ok && !*vfailed;
+    }
+    if (!ok) {  // every copy lands before the CTA ends
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      if (pt == 0) {
+        *vfailed = 1;
+        atomicExch(&g_tlgb_status, 1);
+        for (uint32_t i = k > NST ? k - NST : 0; i < k; ++i) mbar_wait_bounded(&full[i % NST], (i / NST) & 1, limit);
+        for (uint32_t i = ui > 1 ? ui - 1 : 0; i <= ui; ++i) mbar_wait_bounded(&rfull[i & 1], (i >> 1) & 1, 1u << 12);
       }
     }
-  } else {
-    const int ncoil = (int)min((long long)CG, g.nbatch - c0);
-    const long long gvol = (long long)g.N[1] * g.N[2];
-    for (int idx = tid; idx < CG * VOL; idx += NW * 32) {
-      const int z = idx % S;
-      const int r = idx / S;
-      const int y = r % S, c = r / S;
-      int gy = o[1] + y, gz = o[2] + z;
-      bool in = c < ncoil;
-      if (g.pad == TLGB_PAD_CIRCULAR) {
-        gy = wrapi(gy, g.N[1]);
-        gz = wrapi(gz, g.N[2]);
-      } else {
-        in = in && gy < g.N[1] && gz < g.N[2];
-      }
-      reg[idx] = in ? __ldg(reinterpret_cast<const float2*>(gridv) + (long long)(c0 + c) * gvol +
-                           (long long)gy * g.N[2] + gz)
-                    : make_float2(0.f, 0.f);
-    }
+    return;
   }
-  const int c = lane >> 2, kz = lane & 3;
+  // ---- consumers: lane = (point h of a step, entry c and c + 4, z tap kz)
+  const int kz = lane & 3, c = (lane >> 2) & 3, h = lane >> 4;
   int kyo[4], rowoff[4];
 #pragma unroll
   for (int t = 0; t < 4; ++t) {
     kyo[t] = (t + c) & 3;
     rowoff[t] = kyo[t] * S;
   }
-  GRec2* wrec = rec + warp * 8;
-  const int npt = it.z - it.y;
-  // records of the warp's next 8 points: lanes 0-7 copy them into the
-  // warp's slots; pad = region base | fast << 20 | ok << 21, cnt unchanged
-  auto build_records = [&](int base) {
-    const int j = base + 8 * lane;
-    if (lane < 8 && j < npt) {
-      const int p = entries[it.y + j];
-      GRec2 R = grecs[p];
-      const int cy = R.cnt & 15, cz = (R.cnt >> 4) & 15;
-      const bool ok = cy && cz;
-      int f[2];
+  auto give_up = [&]() {
+    if (lane == 0) {
+      *vfailed = 1;
+      atomicExch(&g_tlgb_status, 1);
+    }
+  };
+  uint32_t k = 0, ui = 0;
+  int4 next = items[blockIdx.x / nruns];
+  for (int u = blockIdx.x; u < nunits; u += gridDim.x, ++ui) {
+    const int4 it = next;
+    if (u + (int)gridDim.x < nunits) next = items[(u + gridDim.x) / nruns];
+    const int g0 = (u % nruns) * run, g1 = min(ncg, g0 + run), npt = it.z - it.y;
+    const Rec* rec = recbuf + (ui & 1) * kGatherPts;
+    if (!mbar_wait_bounded(&rfull[ui & 1], (ui >> 1) & 1, limit)) return give_up();
+    float sum[kGradSteps][4];
 #pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        int d = R.st[i] - o[1 + i];
-        if (g.pad == TLGB_PAD_CIRCULAR && d < 0) d += g.N[1 + i];
-        f[i] = d;
-      }
-      const bool fast = ok && cy <= 4 && cz <= 4 && f[0] >= 0 && f[0] < 16 && f[1] >= 0 && f[1] < 16;
-      R.pad = (fast ? (f[0] * S + f[1]) : 0) | ((fast ? 1 : 0) << 20) | ((ok ? 1 : 0) << 21);
-      R.st[0] = p;  // the point index replaces the start (no longer needed)
-      wrec[lane] = R;
+    for (int st = 0; st < kGradSteps; ++st) {
+#pragma unroll
+      for (int t = 0; t < 4; ++t) sum[st][t] = 0.f;
+      const int i = (st * NW + warp) * 2 + h;
+      if ((lane & 15) == 0 && i < npt) far[i] = make_float2(0.f, 0.f);
     }
     __syncwarp();
-  };
-  build_records(warp);  // while the region copy is in flight
-  {
-    bool ok = true;
-    if (tma && tid == 0) ok = mbar_wait_bounded(bar, 0, g.skip_copy ? 1u : 1u << 22);
-    if (__syncthreads_or(!ok)) {
-      if (tid == 0) atomicExch(&g_tlgb_status, 1);
-      return;
-    }
-  }
-  auto finish = [&](float ry, float rz, int p) {
+    for (int cg = g0; cg < g1; ++cg, ++k) {
+      const uint32_t s = k % NST;
+      if (!mbar_wait_bounded(&full[s], (k / NST) & 1, limit)) return give_up();
+      const float2* reg = reinterpret_cast<const float2*>(smem + s * kGradStage);
+      const float2* av = reinterpret_cast<const float2*>(smem + s * kGradStage + kGradRegion);
 #pragma unroll
-    for (int m = 1; m < 32; m <<= 1) {
-      ry += __shfl_xor_sync(0xffffffffu, ry, m);
-      rz += __shfl_xor_sync(0xffffffffu, rz, m);
-    }
-    if (lane == 0) *reinterpret_cast<float2*>(dst + (long long)p * 2) = make_float2(ry, rz);
-  };
-  for (int base = warp; base < npt; base += 8 * NW) {
-    if (base != warp) {
-      __syncwarp();  // the previous mini-batch has been read
-      build_records(base);
-    }
-    const int nb = min(8, (npt - base + NW - 1) / NW);
-    for (int i = 0; i < nb; ++i) {
-      const GRec2& R = wrec[i];
-      const int p = R.st[0];
-      const int info = R.pad;
-      if (!((info >> 21) & 1)) {
-        if (lane == 0) *reinterpret_cast<float2*>(dst + (long long)p * 2) = make_float2(0.f, 0.f);
-        continue;
-      }
-      const float2 av = c0 + c < g.nbatch ? __ldg(a + (long long)(c0 + c) * g.npts + p) : make_float2(0.f, 0.f);
-      float2 gy = make_float2(0.f, 0.f), gz = make_float2(0.f, 0.f);
-      if ((info >> 20) & 1) {
-        const float wz = (&R.w[1].x)[kz], dwz = (&R.dw[1].x)[kz];
-        const float* wy = &R.w[0].x;
-        const float* dwy = &R.dw[0].x;
-        const float2* ab = reg + c * VOL + (info & 1023) + kz;
+      for (int st = 0; st < kGradSteps; ++st) {
+        const int base = (st * NW + warp) * 2;
+        if (base >= npt) break;
+        const bool on = base + h < npt;
+        const int i = on ? base + h : base;
+        const unsigned view = rec[i].view;
+        const float2* v = reg + c * VOL + (view & 0xfffff) + kz;
+        const float2 a0 = av[c * kGatherPts + i], a1 = av[(c + 4) * kGatherPts + i];
+        if (TLGB_IN_RANGE((view & 0xfffff) + 3 * S + 3, VOL)) {
 #pragma unroll
-        for (int t = 0; t < 4; ++t) {
-          const float2 v = ab[rowoff[t]];
-          const float a1 = dwy[kyo[t]] * wz, a2 = wy[kyo[t]] * dwz;
-          gy.x = fmaf(a1, v.x, gy.x);
-          gy.y = fmaf(a1, v.y, gy.y);
-          gz.x = fmaf(a2, v.x, gz.x);
-          gz.y = fmaf(a2, v.y, gz.y);
-        }
-      } else {
-        // 5-tap windows: the warp evaluates the taps, as interp_grad_kernel
-        PTaps<true>& pt = slow[warp];
-        if (warp_point_taps<1, true>(g, locs, p, pt, lane)) {
-          const int l1 = pt.start[1] - o[1], l2 = pt.start[2] - o[2];
-          for (int kb = 0; kb < pt.n[1]; ++kb) {
-            int yy = l1 + kb;
-            if (g.pad == TLGB_PAD_CIRCULAR && yy < 0) yy += g.N[1];
-            for (int kc = kz; kc < pt.n[2]; kc += 4) {
-              int zz = l2 + kc;
-              if (g.pad == TLGB_PAD_CIRCULAR && zz < 0) zz += g.N[2];
-              if (yy < 0 || yy >= S || zz < 0 || zz >= S) continue;
-              const int ri = c * VOL + yy * S + zz;
-              const float2 v = TLGB_IN_RANGE(ri, 8 * VOL) ? reg[ri] : make_float2(0.f, 0.f);
-              const float a1 = pt.dw[1][kb] * pt.w[2][kc], a2 = pt.w[1][kb] * pt.dw[2][kc];
-              gy.x = fmaf(a1, v.x, gy.x);
-              gy.y = fmaf(a1, v.y, gy.y);
-              gz.x = fmaf(a2, v.x, gz.x);
-              gz.y = fmaf(a2, v.y, gz.y);
-            }
+          for (int t = 0; t < 4; ++t) {
+            const float2 v0 = v[rowoff[t]], v1 = v[4 * VOL + rowoff[t]];
+            sum[st][t] = fmaf(a0.x, v0.x, sum[st][t]);
+            sum[st][t] = fmaf(a0.y, v0.y, sum[st][t]);
+            sum[st][t] = fmaf(a1.x, v1.x, sum[st][t]);
+            sum[st][t] = fmaf(a1.y, v1.y, sum[st][t]);
           }
         }
-        __syncwarp();
+        // windows of 5 taps, one at a time by the whole warp
+        unsigned rest = __ballot_sync(0xffffffffu, on && !((view >> 20) & 1));
+        while (rest) {
+          const int hh = (__ffs(rest) - 1) >> 4;
+          rest &= ~(0xffffu << (16 * hh));
+          const int p = rec[base + hh].p;
+          GradTaps& T = slow[warp];
+          {
+            const int d = lane / 5, kk = lane % 5, e = 1 + d;
+            Tap t;
+            t.valid = false;
+            t.d = 0.f;
+            float x = 0.f;
+            int lower = 0;
+            if (d < 2) {
+              x = load_coord(g, locs, p, e);
+              lower = lower_of(g, e, x);
+              if (kk < g.NT[e]) t = tap_eval(g, e, x, lower, kk);
+            }
+            const unsigned m = (__ballot_sync(0xffffffffu, t.valid) >> (d < 2 ? 5 * d : 0)) & 31u;
+            if (t.valid) {
+              const int q = kk - (__ffs(m) - 1);
+              T.w[d][q] = kern_value(g.kernel, fabsf(t.d), g.beta);
+              T.dw[d][q] = kern_deriv(g.kernel, t.d, g.beta) / g.r[e];
+            }
+            if (d < 2 && kk == 0) {
+              int stt = lower + __ffs(m) - 1, o[3];
+              if (g.pad == TLGB_PAD_CIRCULAR) stt = wrapi(stt, g.N[e]);
+              item_origin(g, it.x, o);
+              T.n[d] = __popc(m);
+              T.f[d] = stt - (e == 1 ? o[1] : o[2]);
+            }
+          }
+          __syncwarp();
+          const int c8 = lane & 7, n2 = T.n[1], tot = T.n[0] * n2;
+          const float2 ac = av[c8 * kGatherPts + base + hh];
+          float ry = 0.f, rz = 0.f;
+          for (int t = lane >> 3; t < tot; t += 4) {
+            const int z = t % n2, y = t / n2, cell = (T.f[0] + y) * S + T.f[1] + z;
+            if (!TLGB_IN_RANGE(cell, VOL)) continue;
+            const float2 vv = reg[c8 * VOL + cell];
+            const float dot = fmaf(ac.x, vv.x, ac.y * vv.y);
+            ry = fmaf(T.dw[0][y] * T.w[1][z], dot, ry);
+            rz = fmaf(T.w[0][y] * T.dw[1][z], dot, rz);
+          }
+#pragma unroll
+          for (int m = 1; m < 32; m <<= 1) {
+            ry += __shfl_xor_sync(0xffffffffu, ry, m);
+            rz += __shfl_xor_sync(0xffffffffu, rz, m);
+          }
+          if (lane == 0) {
+            far[base + hh].x += ry;
+            far[base + hh].y += rz;
+          }
+          __syncwarp();
+        }
       }
-      // Re(conj(a) g)
-      finish(av.x * gy.x + av.y * gy.y, av.x * gz.x + av.y * gz.y, p);
+      __syncwarp();
+      if (lane == 0) sm100::mbar_arrive(&empty[s]);
     }
+    // the weights, once per point
+    float* dst = nruns == 1 ? grad : partial + (long long)(u % nruns) * g.npts * 2;
+    float* dw = dwb + warp * 16 + h * 8;
+#pragma unroll
+    for (int st = 0; st < kGradSteps; ++st) {
+      const int base = (st * NW + warp) * 2;
+      if (base >= npt) break;
+      const bool on = base + h < npt;
+      const int i = on ? base + h : base;
+      const Rec& R = rec[i];
+      const int d = (lane >> 3) & 1, kk = lane & 7, e = 1 + d;
+      if (kk < 4) dw[4 * d + kk] = 0.f;
+      __syncwarp();
+      {
+        Tap t;
+        t.valid = false;
+        t.d = 0.f;
+        const float x = load_coord(g, locs, R.p, e);
+        const int lower = lower_of(g, e, x);
+        if (kk < 5 && kk < g.NT[e]) t = tap_eval(g, e, x, lower, kk);
+        const unsigned m = (__ballot_sync(0xffffffffu, t.valid) >> (lane & 24)) & 255u;
+        const int q = kk - (__ffs(m) - 1);
+        if (t.valid && q < 4) dw[4 * d + q] = kern_deriv(g.kernel, t.d, g.beta) / g.r[e];
+      }
+      __syncwarp();
+      float ry = 0.f, rz = 0.f;
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        ry = fmaf(dw[kyo[t]], sum[st][t], ry);
+        rz = fmaf(R.w[0][kyo[t]], sum[st][t], rz);
+      }
+      ry *= R.w[1][kz];
+      rz *= dw[4 + kz];
+#pragma unroll
+      for (int m = 1; m < 16; m <<= 1) {
+        ry += __shfl_xor_sync(0xffffffffu, ry, m);
+        rz += __shfl_xor_sync(0xffffffffu, rz, m);
+      }
+      if (on && (lane & 15) == 0 && TLGB_IN_RANGE(R.p, g.npts))
+        *reinterpret_cast<float2*>(dst + (long long)R.p * 2) = (R.view >> 20) & 1 ? make_float2(ry, rz) : far[i];
+      __syncwarp();
+    }
+    if (lane == 0) sm100::mbar_arrive(&rempty[ui & 1]);
   }
 }
 
@@ -3176,18 +3238,21 @@ size_t grad_scratch_bytes(const Geo& g, int nsplit) {
   return nsplit > 1 ? (size_t)nsplit * g.npts * g.ndim * sizeof(float) : 0;
 }
 
-bool fast2(const Geo& g, int cg);
-
-// The 2D 8-entry gradient (grad_f2_kernel): complex values, norm 1, 8
-// entries per coil group. Its scratch holds the per-point gradient records
-// and, with more than one coil group, one partial slot per group.
-bool grad_fast2(const Geo& g) { return g.cplx && g.norm == 1 && g.nbatch >= 8 && fast2(g, 8); }
-
-size_t grad2_records_bytes(const Geo& g) { return align_up((size_t)g.npts * sizeof(GRec2), 256); }
-
-size_t grad2_scratch_bytes(const Geo& g) {
-  const long long ncg = cdiv(g.nbatch, 8);
-  return grad2_records_bytes(g) + (ncg > 1 ? (size_t)ncg * g.npts * 2 * sizeof(float) : 0);
+// The 2D gradient on the gather's ring (grad2_kernel). A unit is an item and a
+// run of groups of 8 entries; with several runs each adds its own partial slot.
+// One run (no partial results) unless that leaves fewer than 4 units per SM.
+bool grad_on_ring(const Geo& g, const tlgb_interp_plan_info* info) {
+  return g.cplx && g.ndim == 2 && rec_taps(g) == 4 && info->off_records > 0;
+}
+int64_t grad2_runs(const Geo& g, const tlgb_interp_plan_info* info) {
+  const int64_t ncg = cdiv(std::max<long long>(g.nbatch, 1), 8), items = std::max<int64_t>(info->n_fwd_items, 1);
+  int64_t run = ncg;
+  while (run > 1 && items * cdiv(ncg, run) < 4 * sm_count()) run = cdiv(run, 2);
+  return cdiv(ncg, run);
+}
+size_t grad2_scratch_bytes(const Geo& g, const tlgb_interp_plan_info* info) {
+  const int64_t n = grad2_runs(g, info);
+  return n > 1 ? (size_t)n * g.npts * 2 * sizeof(float) : 0;
 }
 
 int check_plan(const Geo& g, const tlgb_interp_plan_info* info, const void* plan) {
@@ -3418,7 +3483,6 @@ extern "C" int tlgb_interp_plan_build(const tlgb_interp_desc* d, const float* lo
 
 namespace tlgb {
 namespace {
-bool fast2(const Geo& g, int cg);
 
 // Batch entries per group of the block gridding: 1, 2 or 4 for 3D batches of
 // at most 4 entries (adj_bn_kernel), else 8 (adj_b3_kernel).
@@ -3585,11 +3649,6 @@ int launch_gather_any(const Geo& g, const tlgb_interp_plan_info* info, const cha
   return launch_gather<2, 8, 8, 16, 4, 1>(g, info, P, locs, grid, out, s);
 }
 
-bool fast2(const Geo& g, int cg) {
-  return g.ndim == 2 && g.cplx && cg == 8 && g.norm == 1 && g.T[1] == 16 && g.T[2] == 16 && g.NT[1] == 5 &&
-         g.NT[2] == 5;
-}
-
 template <int E, int NROW>
 int launch_adj_bn(const Geo& g, const tlgb_interp_plan_info* info, const char* P, const void* vals, void* grid,
                   void* scratch, cudaStream_t s) {
@@ -3731,27 +3790,27 @@ int launch_adj(const Geo& g, const tlgb_interp_plan_info* info, const char* P, c
   return small ? dispatch_adj_n<1, 5>(g, cg, info, P, locs, vals, grid, scratch, s) : dispatch_adj_n<1, 16>(g, cg, info, P, locs, vals, grid, scratch, s);
 }
 
-int launch_grad_f2(const Geo& g, const tlgb_interp_plan_info* info, const char* P, const float* locs,
-                   const void* grid, const void* a, float* grad, void* scratch, cudaStream_t s) {
-  const long long ncg = cdiv(g.nbatch, 8);
-  GRec2* recs = static_cast<GRec2*>(scratch);
-  float* partial = reinterpret_cast<float*>(static_cast<char*>(scratch) + grad2_records_bytes(g));
-  grad_records2_kernel<<<(unsigned)cdiv(g.npts, 256), 256, 0, s>>>(g, locs, recs);
-  TLGB_CHECK_LAUNCH();
+int launch_grad2(const Geo& g, const tlgb_interp_plan_info* info, const char* P, const float* locs, const void* grid,
+                 const void* a, float* grad, void* scratch, size_t scratch_bytes, cudaStream_t s) {
+  if ((uintptr_t)P & 15) TLGB_FAIL(TLGB_ERR_INVALID, "trajectory gradient: the plan must be 16-byte aligned");
+  const int64_t ncg = cdiv(g.nbatch, 8);
+  int64_t nruns = grad2_runs(g, info);
+  if (nruns > 1 && (!scratch || scratch_bytes < grad2_scratch_bytes(g, info) || ((uintptr_t)scratch & 7))) nruns = 1;
+  const int64_t run = cdiv(ncg, nruns), nunits = info->n_fwd_items * nruns;
+  if (nunits >= (1ll << 31) - sm_count()) TLGB_FAIL(TLGB_ERR_UNSUPPORTED, "trajectory gradient: too many points and batch entries in one call");
   const long long n = (long long)g.npts * 2;
-  if (ncg > 1 && info->n_home < g.npts)  // points without taps get no partial writes
-    TLGB_CUDA(cudaMemsetAsync(partial, 0, (size_t)ncg * n * sizeof(float), s));
+  float* partial = static_cast<float*>(scratch);
+  if (nruns > 1 && info->n_home < g.npts)  // points without taps get no partial writes
+    TLGB_CUDA(cudaMemsetAsync(partial, 0, (size_t)nruns * n * sizeof(float), s));
   CUtensorMap tmap;
   const int use_tma = region_map(g, grid, 20, 8, tmap);
-  const size_t sm = 20 * 20 * 8 * 8 + 64 * sizeof(GRec2) + 8 * sizeof(PTaps<true>) + 8;
-  TLGB_TRY(set_smem(grad_f2_kernel, sm));
-  dim3 grd((unsigned)info->n_fwd_items, (unsigned)ncg);
-  grad_f2_kernel<<<grd, 256, sm, s>>>(tmap, use_tma, g, (const int4*)(P + info->off_fwd_items),
-                                      (const int32_t*)(P + info->off_entries), recs, locs, (const float*)grid,
-                                      (const float2*)a, grad, partial);
+  TLGB_TRY(set_smem(grad2_kernel, grad2_smem()));
+  grad2_kernel<<<(unsigned)std::min<int64_t>(nunits, sm_count()), kGradWarps * 32 + kGatherProd, grad2_smem(), s>>>(
+      tmap, use_tma, g, (const int4*)(P + info->off_fwd_items), (int)nruns, (int)run, (int)nunits,
+      (const GatherRec<2, 4>*)(P + info->off_records), locs, (const float*)grid, (const float2*)a, grad, partial);
   TLGB_CHECK_LAUNCH();
-  if (ncg > 1) {
-    grad_reduce_kernel<<<(unsigned)cdiv(n, 256), 256, 0, s>>>(partial, (int)ncg, n, grad);
+  if (nruns > 1) {
+    grad_reduce_kernel<<<(unsigned)cdiv(n, 256), 256, 0, s>>>(partial, (int)nruns, n, grad);
     TLGB_CHECK_LAUNCH();
   }
   return TLGB_OK;
@@ -3761,9 +3820,7 @@ template <typename V, int NORM>
 int launch_grad(const Geo& g, const tlgb_interp_plan_info* info, const char* P, const float* locs, const void* grid,
                 const void* a, float* grad, void* scratch, size_t scratch_bytes, cudaStream_t s) {
   if constexpr (std::is_same<V, float2>::value && NORM == 1)
-    if (grad_fast2(g) && info->off_records > 0 && scratch && scratch_bytes >= grad2_scratch_bytes(g) &&
-        ((uintptr_t)scratch & 15) == 0)
-      return launch_grad_f2(g, info, P, locs, grid, a, grad, scratch, s);
+    if (grad_on_ring(g, info)) return launch_grad2(g, info, P, locs, grid, a, grad, scratch, scratch_bytes, s);
   const int cg = grad_cg(g, sizeof(PTaps<true>));
   const size_t sm = grad_smem(g, cg, sizeof(PTaps<true>)) + kFwdChunk * 3 * sizeof(float);
   auto* k = interp_grad_kernel<V, NORM>;
@@ -3841,7 +3898,7 @@ extern "C" int tlgb_interp_grad_scratch_size(const tlgb_interp_desc* d, const tl
   Geo g;
   TLGB_TRY(make_geo(d, g));
   if (!info || !bytes) TLGB_FAIL(TLGB_ERR_INVALID, "null pointer");
-  *bytes = grad_fast2(g) && info->off_records > 0 ? grad2_scratch_bytes(g) : grad_scratch_bytes(g, grad_splits(g, info));
+  *bytes = grad_on_ring(g, info) ? grad2_scratch_bytes(g, info) : grad_scratch_bytes(g, grad_splits(g, info));
   return TLGB_OK;
 }
 
