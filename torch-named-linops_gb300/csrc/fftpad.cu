@@ -17,6 +17,8 @@
 // is one gather (tlgb_crop_shift), which can also apply the conjugate coil
 // maps, the coil sum and an axpy.
 
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace tlgb {
@@ -53,88 +55,142 @@ __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
   return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
 
-__device__ __forceinline__ int wrapm(int v, int m) {
-  v %= m;
-  return v < 0 ? v + m : v;
+// row and column indices of voxel v of a volume with last extents n1, n2
+__device__ __forceinline__ void split_index(long long v, long long vol, int n1, int n2, int& i0, int& i1, int& i2) {
+  if (vol <= 0xffffffffll) {  // 32-bit divisions wherever the volume allows them
+    const unsigned u = (unsigned)v, r = u / (unsigned)n2;
+    i2 = (int)(u - r * (unsigned)n2);
+    i0 = (int)(r / (unsigned)n1);
+    i1 = (int)(r - (unsigned)i0 * (unsigned)n1);
+  } else {
+    const long long r = v / n2;
+    i2 = (int)(v - r * n2);
+    i0 = (int)(r / n1);
+    i1 = (int)(r - (long long)i0 * n1);
+  }
 }
 
-// out[(b*C + c)][j] = maps[c][i] * apod[i] * x[b][i] for the source i of j, else 0
-__global__ void pad_shift_kernel(PadGeo G, const float2* __restrict__ x, long long nbatch, const float* __restrict__ apod,
-                                 const float2* __restrict__ maps, int nmaps, float2* __restrict__ out) {
+// Both kernels move a voxel of many batch entries per thread and are bound by
+// memory. One thread per voxel that walks the whole batch leaves one load in
+// flight per thread and too few CTAs for a 2D grid (256 entries of 256^2 in
+// 320^2: 400 CTAs, 165 us to pad and 137 us to crop, 2.1 and 2.5 TB/s), so the
+// batch is cut into blockIdx.y runs (batch_runs) and kBatchAhead loads are
+// issued before the first store: 56 and 42 us, 6.1 and 8 TB/s (part of it from L2).
+constexpr int kBatchAhead = 8;
+
+// out[e][j] = maps[e % C][i] * apod[i] * x[e / C][i] for the source i of j, else 0
+template <bool MAPS>
+__global__ void __launch_bounds__(256) pad_shift_kernel(PadGeo G, const float2* __restrict__ x, long long nent, long long run,
+                                                        const float* __restrict__ apod, const float2* __restrict__ maps,
+                                                        int nmaps, float2* __restrict__ out) {
   const long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= G.npvol) return;
-  const int j2 = (int)(j % G.np[2]);
-  const long long r = j / G.np[2];
-  const int j1 = (int)(r % G.np[1]), j0 = (int)(r / G.np[1]);
-  const int i0 = wrapm(j0 + G.sh[0], G.np[0]) - G.off[0];
-  const int i1 = wrapm(j1 + G.sh[1], G.np[1]) - G.off[1];
-  const int i2 = wrapm(j2 + G.sh[2], G.np[2]) - G.off[2];
+  int j0, j1, j2;
+  split_index(j, G.npvol, G.np[1], G.np[2], j0, j1, j2);
+  int i0 = j0 + G.sh[0], i1 = j1 + G.sh[1], i2 = j2 + G.sh[2];  // shifts are below the extents
+  i0 -= (i0 >= G.np[0] ? G.np[0] : 0) + G.off[0];
+  i1 -= (i1 >= G.np[1] ? G.np[1] : 0) + G.off[1];
+  i2 -= (i2 >= G.np[2] ? G.np[2] : 0) + G.off[2];
   const bool in = i0 >= 0 && i0 < G.n[0] && i1 >= 0 && i1 < G.n[1] && i2 >= 0 && i2 < G.n[2];
   const long long i = in ? ((long long)i0 * G.n[1] + i1) * G.n[2] + i2 : 0;
   const float a = (in && apod) ? apod[i] : 1.f;
-  const int C = maps ? nmaps : 1;
-  const float2 md = G.modulate ? modulation(G, j0, j1, j2) : make_float2(1.f, 0.f);
-  for (long long b = 0; b < nbatch; ++b) {
-    float2 v = make_float2(0.f, 0.f);
-    if (in) {
-      v = x[b * G.nvol + i];
-      v.x *= a;
-      v.y *= a;
-    }
-    for (int c = 0; c < C; ++c) {
-      float2 o = v;
-      if (maps && in) {
-        const float2 m = maps[(long long)c * G.nvol + i];
-        o = make_float2(m.x * v.x - m.y * v.y, m.x * v.y + m.y * v.x);
+  const float2 md = (in && G.modulate) ? modulation(G, j0, j1, j2) : make_float2(1.f, 0.f);
+  const long long e0 = blockIdx.y * run, e1 = min(nent, e0 + run);
+  long long b = MAPS ? e0 / nmaps : e0;
+  int c = MAPS ? (int)(e0 - b * nmaps) : 0;
+  for (long long e = e0; e < e1; e += kBatchAhead) {
+    float2 v[kBatchAhead];
+#pragma unroll
+    for (int u = 0; u < kBatchAhead; ++u) {
+      v[u] = make_float2(0.f, 0.f);
+      if (!in || e + u >= e1) continue;
+      const float2 q = x[b * G.nvol + i];
+      v[u] = make_float2(q.x * a, q.y * a);
+      if (MAPS) v[u] = cmul(maps[c * G.nvol + i], v[u]);
+      if (!MAPS || ++c == nmaps) {
+        c = 0;
+        ++b;
       }
-      if (G.modulate) o = cmul(o, md);
-      out[(b * C + c) * G.npvol + j] = o;
+    }
+#pragma unroll
+    for (int u = 0; u < kBatchAhead; ++u) {
+      if (e + u >= e1) break;
+      out[(e + u) * G.npvol + j] = in && G.modulate ? cmul(v[u], md) : v[u];
     }
   }
 }
 
 // out[b][i] = alpha * apod[i] * sum_c conj(maps[c][i]) z[(b*C + c)][src(i)] + beta * add[b][i]
-__global__ void crop_shift_kernel(PadGeo G, const float2* __restrict__ z, long long nbatch, const float* __restrict__ apod,
-                                  const float2* __restrict__ maps, int nmaps, float alpha, const float2* __restrict__ add,
-                                  float beta, float2* __restrict__ out) {
+template <bool MAPS>
+__global__ void __launch_bounds__(256) crop_shift_kernel(PadGeo G, const float2* __restrict__ z, long long nbatch,
+                                                         long long run, const float* __restrict__ apod,
+                                                         const float2* __restrict__ maps, int nmaps, float alpha,
+                                                         const float2* __restrict__ add, float beta,
+                                                         float2* __restrict__ out) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= G.nvol) return;
-  const int i2 = (int)(i % G.n[2]);
-  const long long r = i / G.n[2];
-  const int i1 = (int)(r % G.n[1]), i0 = (int)(r / G.n[1]);
-  const int j0 = wrapm(i0 + G.off[0] - G.sh[0], G.np[0]);
-  const int j1 = wrapm(i1 + G.off[1] - G.sh[1], G.np[1]);
-  const int j2 = wrapm(i2 + G.off[2] - G.sh[2], G.np[2]);
+  int i0, i1, i2;
+  split_index(i, G.nvol, G.n[1], G.n[2], i0, i1, i2);
+  int j0 = i0 + G.off[0] - G.sh[0], j1 = i1 + G.off[1] - G.sh[1], j2 = i2 + G.off[2] - G.sh[2];
+  j0 += j0 < 0 ? G.np[0] : 0;  // off + n fits in Np, so one extent is enough
+  j1 += j1 < 0 ? G.np[1] : 0;
+  j2 += j2 < 0 ? G.np[2] : 0;
   const long long j = ((long long)j0 * G.np[1] + j1) * G.np[2] + j2;
   const float a = (apod ? apod[i] : 1.f) * alpha;
-  const int C = maps ? nmaps : 1;
   float2 md = make_float2(1.f, 0.f);
   if (G.modulate) {
     md = modulation(G, j0, j1, j2);
     md.y = -md.y;  // conj(m[j])
   }
-  for (long long b = 0; b < nbatch; ++b) {
-    float sx = 0.f, sy = 0.f;
-    for (int c = 0; c < C; ++c) {
-      float2 v = z[(b * C + c) * G.npvol + j];
-      if (G.modulate) v = cmul(v, md);
-      if (maps) {
-        const float2 m = maps[(long long)c * G.nvol + i];
-        sx += m.x * v.x + m.y * v.y;  // conj(m) * v
-        sy += m.x * v.y - m.y * v.x;
-      } else {
-        sx += v.x;
-        sy += v.y;
+  const long long b0 = blockIdx.y * run, b1 = min(nbatch, b0 + run);
+  constexpr int UB = MAPS ? 1 : kBatchAhead, UC = MAPS ? kBatchAhead : 1;  // coils ahead, or entries ahead
+  const int C = MAPS ? nmaps : 1;
+  for (long long b = b0; b < b1; b += UB) {
+    float2 s[UB];
+#pragma unroll
+    for (int u = 0; u < UB; ++u) s[u] = make_float2(0.f, 0.f);
+    for (int c = 0; c < C; c += UC) {
+      float2 v[UB * UC], m[UC];
+#pragma unroll
+      for (int u = 0; u < UB * UC; ++u) {
+        const bool live = MAPS ? c + u < C : b + u < b1;
+        v[u] = live ? z[(MAPS ? b * C + c + u : b + u) * G.npvol + j] : make_float2(0.f, 0.f);
+        if (MAPS) m[u] = live ? maps[(long long)(c + u) * G.nvol + i] : make_float2(0.f, 0.f);
+      }
+#pragma unroll
+      for (int u = 0; u < UB * UC; ++u) {
+        if (MAPS && c + u >= C) break;
+        if (G.modulate) v[u] = cmul(v[u], md);
+        if (MAPS) {  // conj(m) * v
+          s[0].x += m[u].x * v[u].x + m[u].y * v[u].y;
+          s[0].y += m[u].x * v[u].y - m[u].y * v[u].x;
+        } else {
+          s[u] = v[u];
+        }
       }
     }
-    float2 o = make_float2(a * sx, a * sy);
-    if (add) {
-      const float2 q = add[b * G.nvol + i];
-      o.x = fmaf(beta, q.x, o.x);
-      o.y = fmaf(beta, q.y, o.y);
+#pragma unroll
+    for (int u = 0; u < UB; ++u) {
+      if (b + u >= b1) break;
+      float2 o = make_float2(a * s[u].x, a * s[u].y);
+      if (add) {
+        const float2 q = add[(b + u) * G.nvol + i];
+        o.x = fmaf(beta, q.x, o.x);
+        o.y = fmaf(beta, q.y, o.y);
+      }
+      out[(b + u) * G.nvol + i] = o;
     }
-    out[b * G.nvol + i] = o;
   }
+}
+
+// Entries per blockIdx.y: whole groups of `ahead`, in as many runs as it
+// takes for 16 CTAs per SM (8 fit at a time) where the volume alone has fewer.
+long long batch_runs(long long ctas, long long nent, int ahead, unsigned& gy) {
+  const long long groups = cdiv(nent, ahead);
+  const long long want = std::min<long long>(std::max<long long>(cdiv(16ll * sm_count(), ctas), 1), std::min<long long>(groups, 65535));
+  const long long run = cdiv(groups, want) * ahead;
+  gy = (unsigned)cdiv(nent, run);
+  return run;
 }
 
 int make_pad_geo(int32_t ndim, const int64_t* n, const int64_t* np, const int64_t* off, const int64_t* shift,
@@ -173,8 +229,11 @@ extern "C" int tlgb_pad_shift_c64(const void* x, int64_t nbatch, int32_t ndim, c
   if (nbatch < 0 || (maps && nmaps < 1)) TLGB_FAIL(TLGB_ERR_INVALID, "pad_shift: bad batch or map count");
   if (nbatch == 0) return TLGB_OK;
   if (!x || !out) TLGB_FAIL(TLGB_ERR_INVALID, "null pointer");
-  pad_shift_kernel<<<(unsigned)cdiv(G.npvol, 256), 256, 0, (cudaStream_t)stream>>>(
-      G, (const float2*)x, nbatch, apod, (const float2*)maps, nmaps, (float2*)out);
+  const long long nent = (long long)nbatch * (maps ? nmaps : 1), ctas = cdiv(G.npvol, 256);
+  dim3 grid((unsigned)ctas);
+  const long long run = batch_runs(ctas, nent, kBatchAhead, grid.y);
+  (maps ? pad_shift_kernel<true> : pad_shift_kernel<false>)<<<grid, 256, 0, (cudaStream_t)stream>>>(
+      G, (const float2*)x, nent, run, apod, (const float2*)maps, nmaps, (float2*)out);
   TLGB_CHECK_LAUNCH();
   return TLGB_OK;
 }
@@ -188,8 +247,11 @@ extern "C" int tlgb_crop_shift_c64(const void* z, int64_t nbatch, int32_t ndim, 
   if (nbatch < 0 || (maps && nmaps < 1)) TLGB_FAIL(TLGB_ERR_INVALID, "crop_shift: bad batch or map count");
   if (nbatch == 0) return TLGB_OK;
   if (!z || !out) TLGB_FAIL(TLGB_ERR_INVALID, "null pointer");
-  crop_shift_kernel<<<(unsigned)cdiv(G.nvol, 256), 256, 0, (cudaStream_t)stream>>>(
-      G, (const float2*)z, nbatch, apod, (const float2*)maps, nmaps, alpha, (const float2*)add, beta, (float2*)out);
+  const long long ctas = cdiv(G.nvol, 256);
+  dim3 grid((unsigned)ctas);
+  const long long run = batch_runs(ctas, nbatch, maps ? 1 : kBatchAhead, grid.y);
+  (maps ? crop_shift_kernel<true> : crop_shift_kernel<false>)<<<grid, 256, 0, (cudaStream_t)stream>>>(
+      G, (const float2*)z, nbatch, run, apod, (const float2*)maps, nmaps, alpha, (const float2*)add, beta, (float2*)out);
   TLGB_CHECK_LAUNCH();
   return TLGB_OK;
 }

@@ -898,13 +898,19 @@ _APOD: "OrderedDict[tuple, Tensor]" = OrderedDict()
 
 
 def _apod_on(device, grid_size, padded, oversamp: float, width: float, beta: float) -> Tensor:
-    """The apodization weights on ``device``, computed once per sizes and
-    kernel (the functional transforms would otherwise rebuild them on the
-    host and copy them over on every call)."""
+    """The weights of the functional transforms on ``device``: apodization,
+    the transform's 1 / width^ndim sqrt(prod(grid) / prod(padded)) and the
+    1 / sqrt(prod(padded)) of an ortho-normalised FFT in one factor per voxel,
+    so that the FFT runs without normalisation and neither scale is a pass of
+    its own (256 entries of 256^2 with 205,824 points: 55 us for the FFT's and
+    115 us for the division). Computed once per sizes and kernel (the
+    transforms would otherwise rebuild them on the host and copy them over on
+    every call)."""
     key = (str(device), tuple(grid_size), tuple(padded), float(oversamp), float(width), float(beta))
     w = _APOD.get(key)
     if w is None:
-        w = apodize_weights(grid_size, padded, oversamp, width, beta).to(device)
+        scale = width ** len(grid_size) * prod(grid_size) ** 0.5
+        w = (apodize_weights(grid_size, padded, oversamp, width, beta).double() / scale).float().to(device)
         _APOD[key] = w
         while len(_APOD) > 16:
             _APOD.popitem(last=False)
@@ -945,10 +951,9 @@ def nufft(x: Tensor, locs: Tensor, oversamp: float = 1.25, width: float = 4.0) -
     padded = tuple(int(s * oversamp) for s in grid_size)
     beta = nufft_beta(width, oversamp)
     x = pad_shift(x, grid_size, padded, apod=_apod_on(x.device, grid_size, padded, oversamp, width, beta), modulate=True)
-    x = torch.fft.fftn(x, dim=tuple(range(-ndim, 0)), norm="ortho")
-    x = I.interpolate(x, _prepared_locs(locs, grid_size, padded), width, kernel="kaiser_bessel",
-                      kernel_params=dict(beta=beta))
-    return x / (width**ndim * (prod(grid_size) / prod(padded)) ** 0.5)
+    x = torch.fft.fftn(x, dim=tuple(range(-ndim, 0)), norm="backward")  # unscaled; see _apod_on
+    return I.interpolate(x, _prepared_locs(locs, grid_size, padded), width, kernel="kaiser_bessel",
+                         kernel_params=dict(beta=beta))
 
 
 def nufft_adjoint(x: Tensor, locs: Tensor, grid_size, oversamp: float = 1.25, width: float = 4.0) -> Tensor:
@@ -958,9 +963,10 @@ def nufft_adjoint(x: Tensor, locs: Tensor, grid_size, oversamp: float = 1.25, wi
     ndim = locs.shape[-1]
     padded = tuple(int(s * oversamp) for s in grid_size)
     beta = nufft_beta(width, oversamp)
-    x = x / (width**ndim * (prod(grid_size) / prod(padded)) ** 0.5)
+    if not (x.is_floating_point() or x.is_complex()):
+        x = x.to(torch.get_default_dtype())
     x = I.interpolate_adjoint(x, _prepared_locs(locs, grid_size, padded), padded, width, kernel="kaiser_bessel",
                               kernel_params=dict(beta=beta))
-    x = torch.fft.ifftn(x, dim=tuple(range(-ndim, 0)), norm="ortho")
+    x = torch.fft.ifftn(x, dim=tuple(range(-ndim, 0)), norm="forward")  # unscaled; see _apod_on
     return crop_shift(x, grid_size, padded, apod=_apod_on(x.device, grid_size, padded, oversamp, width, beta),
                       modulate=True)
