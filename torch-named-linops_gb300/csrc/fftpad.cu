@@ -75,7 +75,7 @@ __device__ __forceinline__ void split_index(long long v, long long vol, int n1, 
 // flight per thread and too few CTAs for a 2D grid (256 entries of 256^2 in
 // 320^2: 400 CTAs, 165 us to pad and 137 us to crop, 2.1 and 2.5 TB/s), so the
 // batch is cut into blockIdx.y runs (batch_runs) and kBatchAhead loads are
-// issued before the first store: 56 and 42 us, 6.1 and 8 TB/s (part of it from L2).
+// issued before the first store: 56 and 42 us, 6.1 and 6.4 TB/s.
 constexpr int kBatchAhead = 8;
 
 // out[e][j] = maps[e % C][i] * apod[i] * x[e / C][i] for the source i of j, else 0

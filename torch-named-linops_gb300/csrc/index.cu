@@ -61,14 +61,40 @@ __global__ void index_ravel_kernel(IdxGeo g, const int64_t* __restrict__ idx, in
   }
 }
 
-// out[b][m] = vals[b][flat[m]]: a copy of E-sized elements
-template <typename E>
-__global__ void index_fwd_kernel(const E* __restrict__ vals, const int32_t* __restrict__ flat, E* __restrict__ out,
-                                 int64_t npts, int64_t ncells, int64_t nbatch) {
-  for (int64_t m = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; m < npts; m += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t c = flat[m];
-    for (int64_t b = 0; b < nbatch; ++b) out[b * npts + m] = vals[b * ncells + c];
+// out[b][m] = vals[b][flat[m]]: a copy of E-sized elements. Bound by the
+// scattered reads, of which each moves a 32-byte sector: the entries go one
+// after the other over blockIdx.y, so that one entry's grid is read at a time
+// and stays in L2 (33 MB of 160^3 complex64; all 8 entries at once are 262 MB),
+// and a thread has S reads in flight. The output is stored to leave L2 early. 8 entries of 160^3 at 2^20 samples:
+// 79 us with one read in flight and the entries in the inner loop, 48 us now.
+template <typename E, int S>
+__global__ void __launch_bounds__(256) index_fwd_kernel(const E* __restrict__ vals, const int32_t* __restrict__ flat,
+                                                        E* __restrict__ out, int64_t npts, int64_t ncells, int64_t nbatch) {
+  const int64_t m0 = (int64_t)blockIdx.x * (256 * S) + threadIdx.x;
+  int32_t c[S];
+#pragma unroll
+  for (int i = 0; i < S; ++i) c[i] = m0 + i * 256 < npts ? flat[m0 + i * 256] : 0;  // cell 0 is always there
+  for (int64_t b = blockIdx.y; b < nbatch; b += gridDim.y) {
+    E v[S];
+#pragma unroll
+    for (int i = 0; i < S; ++i) v[i] = vals[b * ncells + c[i]];
+#pragma unroll
+    for (int i = 0; i < S; ++i)
+      if (m0 + i * 256 < npts) __stcs(&out[b * npts + m0 + i * 256], v[i]);
   }
+}
+
+template <typename E>
+void launch_index_fwd(const IdxGeo& g, const void* vals, const int32_t* flat, void* out, cudaStream_t s) {
+  constexpr int S = 8;
+  const unsigned gy = (unsigned)std::min<int64_t>(g.nbatch, 65535);
+  // eight reads in flight where that leaves four CTAs per SM, one (and eight times the CTAs) below
+  if (cdiv(g.npts, 256 * S) * g.nbatch >= 4ll * sm_count())
+    index_fwd_kernel<E, S><<<dim3((unsigned)cdiv(g.npts, 256 * S), gy), 256, 0, s>>>((const E*)vals, flat, (E*)out, g.npts,
+                                                                                   g.ncells, g.nbatch);
+  else
+    index_fwd_kernel<E, 1><<<dim3((unsigned)cdiv(g.npts, 256), gy), 256, 0, s>>>((const E*)vals, flat, (E*)out, g.npts,
+                                                                                g.ncells, g.nbatch);
 }
 
 template <typename T>
@@ -97,20 +123,116 @@ struct Acc<double2> {
 };
 
 // out[b][c] = sum over the samples of cell c, in ascending sample order,
-// starting from zero; every cell is written
-template <typename T>
-__global__ void index_adj_kernel(const T* __restrict__ vals, const int32_t* __restrict__ perm,
-                                 const uint32_t* __restrict__ off, T* __restrict__ out, int64_t npts, int64_t ncells,
-                                 int64_t nbatch) {
-  for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < ncells; c += (int64_t)gridDim.x * blockDim.x) {
-    const uint32_t k0 = off[c], k1 = off[c + 1];
-    for (int64_t b = 0; b < nbatch; ++b) {
-      Acc<T> a;
-      const T* vb = vals + b * npts;
-      for (uint32_t k = k0; k < k1; ++k) a.add(vb[perm[k]]);
-      out[b * ncells + c] = a.v;
-    }
+// starting from zero; every cell is written. A thread that follows its cells'
+// bounds, sample numbers and values itself is bound by that chain of three
+// loads, most of them by lanes whose neighbours have nothing to do (a cell
+// holds a quarter sample on average in the case below). The samples of a run of cells are a
+// run of perm, though, so a CTA fetches the values of its 256 C cells in sorted
+// order into shared memory with all lanes, U entries at a time, and each thread
+// then adds its own cells' values from there, in the same order as before.
+// Results are stored to leave L2 early: the values, which are read in random
+// order, stay there. 8 entries of 160^3 at 2^20 samples: 156 us as a chain of
+// single loads, 143 with eight entries per chain, 104 us now.
+constexpr int kAdjChunk = 256;  // samples in shared memory
+// Resident CTAs, by registers: 104 us with 4, 124 and 143 with 5 and 6, which spill
+constexpr int adj_ctas(size_t bytes, int entries) { return (entries == 1 ? 8 : 4) / (bytes > 8 ? 2 : 1); }
+
+template <typename T, int U, int C>
+__global__ void __launch_bounds__(256, adj_ctas(sizeof(T), U)) index_adj_kernel(const T* __restrict__ vals, const int32_t* __restrict__ perm,
+                                                        const uint32_t* __restrict__ off, T* __restrict__ out, int64_t npts,
+                                                        int64_t ncells, int64_t nbatch) {
+  __shared__ T sm[U][kAdjChunk];
+  const int64_t first = (int64_t)blockIdx.x * (256 * C), c0 = first + threadIdx.x;
+  const uint32_t ka = off[first], kb = off[min(first + 256 * C, ncells)];
+  uint32_t k0[C], k1[C];
+#pragma unroll
+  for (int j = 0; j < C; ++j) {
+    const int64_t c = min(c0 + j * 256, ncells - 1);
+    k0[j] = off[c];
+    k1[j] = off[c + 1];
   }
+  for (int64_t b = (int64_t)blockIdx.y * U; b < nbatch; b += (int64_t)gridDim.y * U) {
+    Acc<T> a[U][C];
+    for (uint32_t s0 = ka; s0 < kb; s0 += kAdjChunk) {
+      const uint32_t n = min(kb - s0, (uint32_t)kAdjChunk);
+      __syncthreads();  // the chunk before has been added
+      if (threadIdx.x < n) {
+        const int64_t m = perm[s0 + threadIdx.x];
+        T v[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          if (b + u < nbatch) v[u] = vals[(b + u) * npts + m];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          if (b + u < nbatch) sm[u][threadIdx.x] = v[u];
+      }
+      __syncthreads();
+#pragma unroll
+      for (int j = 0; j < C; ++j) {
+        const uint32_t hi = min(k1[j], s0 + n);
+        for (uint32_t k = max(k0[j], s0); k < hi; ++k)
+#pragma unroll
+          for (int u = 0; u < U; ++u) a[u][j].add(sm[u][k - s0]);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int j = 0; j < C; ++j)
+        if (b + u < nbatch && c0 + j * 256 < ncells) __stcs(&out[(b + u) * ncells + c0 + j * 256], a[u][j].v);
+  }
+}
+
+// The same on grids whose cells hold several samples: a cell's samples are
+// contiguous in perm, and K of its values are read ahead of adding them. 8
+// entries of 64^2 at 2^20 samples: 2150 us one value at a time, 292 and 254 us
+// with K = 4 and 8, 807 us through shared memory, where a chunk holds one cell
+// and its CTA waits for that one lane; 12 entries of 320^2 (10 samples per
+// cell): 187, 79 and 78, 129 us; at a quarter sample per cell 160^3 prefers
+// shared memory, 104 against 160 us. The line is at two samples per cell.
+template <typename T, int K>
+__global__ void __launch_bounds__(256) index_adj_dense_kernel(const T* __restrict__ vals, const int32_t* __restrict__ perm,
+                                                              const uint32_t* __restrict__ off, T* __restrict__ out,
+                                                              int64_t npts, int64_t ncells, int64_t nbatch) {
+  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= ncells) return;
+  const uint32_t k0 = off[c], k1 = off[c + 1];
+  for (int64_t b = blockIdx.y; b < nbatch; b += gridDim.y) {
+    const T* vb = vals + b * npts;
+    Acc<T> a;
+    for (uint32_t k = k0; k < k1; k += K) {
+      T v[K];
+#pragma unroll
+      for (int i = 0; i < K; ++i)
+        if (k + i < k1) v[i] = vb[perm[k + i]];
+#pragma unroll
+      for (int i = 0; i < K; ++i)
+        if (k + i < k1) a.add(v[i]);
+    }
+    out[b * ncells + c] = a.v;
+  }
+}
+
+template <typename T, int U, int C>
+void launch_index_adj_at(const IdxGeo& g, const void* vals, const int32_t* perm, const uint32_t* off, void* out,
+                         cudaStream_t s) {
+  const dim3 grd((unsigned)cdiv(g.ncells, 256 * C), (unsigned)std::min<int64_t>(cdiv(g.nbatch, U), 65535));
+  index_adj_kernel<T, U, C><<<grd, 256, 0, s>>>((const T*)vals, perm, off, (T*)out, g.npts, g.ncells, g.nbatch);
+}
+// As many cells and entries per CTA as leave four CTAs per SM; small grids
+// take one cell per thread, and one entry where that is still too few.
+template <typename T>
+void launch_index_adj(const IdxGeo& g, const void* vals, const int32_t* perm, const uint32_t* off, void* out, cudaStream_t s) {
+  if (g.npts >= 2 * g.ncells) {
+    const dim3 grd((unsigned)cdiv(g.ncells, 128), (unsigned)std::min<int64_t>(g.nbatch, 65535));
+    index_adj_dense_kernel<T, 8><<<grd, 128, 0, s>>>((const T*)vals, perm, off, (T*)out, g.npts, g.ncells, g.nbatch);
+    return;
+  }
+  const int64_t want = 4ll * sm_count(), groups = cdiv(g.nbatch, 4);
+  if (g.nbatch > 1 && cdiv(g.ncells, 1024) * groups >= want) launch_index_adj_at<T, 4, 4>(g, vals, perm, off, out, s);
+  else if (g.nbatch == 1 && cdiv(g.ncells, 1024) >= want) launch_index_adj_at<T, 1, 4>(g, vals, perm, off, out, s);
+  else if (g.nbatch > 1 && cdiv(g.ncells, 256) * groups >= want) launch_index_adj_at<T, 4, 1>(g, vals, perm, off, out, s);
+  else launch_index_adj_at<T, 1, 1>(g, vals, perm, off, out, s);
 }
 
 int make_idx_geo(const tlgb_index_desc* d, IdxGeo& g) {
@@ -260,13 +382,12 @@ extern "C" int tlgb_index_forward(const tlgb_index_desc* d, const tlgb_index_pla
   if (!vals || !out) TLGB_FAIL(TLGB_ERR_INVALID, "null pointer");
   cudaStream_t s = (cudaStream_t)stream;
   const int32_t* flat = reinterpret_cast<const int32_t*>(static_cast<const char*>(plan) + info->off_flat);
-  const unsigned grd = grid_for(g.npts);
   switch (elem_bytes(d->dtype)) {
-    case 1: index_fwd_kernel<uint8_t><<<grd, 256, 0, s>>>((const uint8_t*)vals, flat, (uint8_t*)out, g.npts, g.ncells, g.nbatch); break;
-    case 2: index_fwd_kernel<uint16_t><<<grd, 256, 0, s>>>((const uint16_t*)vals, flat, (uint16_t*)out, g.npts, g.ncells, g.nbatch); break;
-    case 4: index_fwd_kernel<uint32_t><<<grd, 256, 0, s>>>((const uint32_t*)vals, flat, (uint32_t*)out, g.npts, g.ncells, g.nbatch); break;
-    case 8: index_fwd_kernel<uint2><<<grd, 256, 0, s>>>((const uint2*)vals, flat, (uint2*)out, g.npts, g.ncells, g.nbatch); break;
-    case 16: index_fwd_kernel<uint4><<<grd, 256, 0, s>>>((const uint4*)vals, flat, (uint4*)out, g.npts, g.ncells, g.nbatch); break;
+    case 1: launch_index_fwd<uint8_t>(g, vals, flat, out, s); break;
+    case 2: launch_index_fwd<uint16_t>(g, vals, flat, out, s); break;
+    case 4: launch_index_fwd<uint32_t>(g, vals, flat, out, s); break;
+    case 8: launch_index_fwd<uint2>(g, vals, flat, out, s); break;
+    case 16: launch_index_fwd<uint4>(g, vals, flat, out, s); break;
     default: TLGB_FAIL(TLGB_ERR_UNSUPPORTED, "index: unsupported element type");
   }
   TLGB_CHECK_LAUNCH();
@@ -284,14 +405,13 @@ extern "C" int tlgb_index_adjoint(const tlgb_index_desc* d, const tlgb_index_pla
   const char* P = static_cast<const char*>(plan);
   const int32_t* perm = reinterpret_cast<const int32_t*>(P + info->off_perm);
   const uint32_t* off = reinterpret_cast<const uint32_t*>(P + info->off_cells);
-  const unsigned grd = grid_for(g.ncells);
   switch (d->dtype) {
-    case TLGB_F32: index_adj_kernel<float><<<grd, 256, 0, s>>>((const float*)vals, perm, off, (float*)out, g.npts, g.ncells, g.nbatch); break;
-    case TLGB_F64: index_adj_kernel<double><<<grd, 256, 0, s>>>((const double*)vals, perm, off, (double*)out, g.npts, g.ncells, g.nbatch); break;
-    case TLGB_C64: index_adj_kernel<float2><<<grd, 256, 0, s>>>((const float2*)vals, perm, off, (float2*)out, g.npts, g.ncells, g.nbatch); break;
-    case TLGB_C128: index_adj_kernel<double2><<<grd, 256, 0, s>>>((const double2*)vals, perm, off, (double2*)out, g.npts, g.ncells, g.nbatch); break;
-    case TLGB_I32: index_adj_kernel<int32_t><<<grd, 256, 0, s>>>((const int32_t*)vals, perm, off, (int32_t*)out, g.npts, g.ncells, g.nbatch); break;
-    case TLGB_I64: index_adj_kernel<long long><<<grd, 256, 0, s>>>((const long long*)vals, perm, off, (long long*)out, g.npts, g.ncells, g.nbatch); break;
+    case TLGB_F32: launch_index_adj<float>(g, vals, perm, off, out, s); break;
+    case TLGB_F64: launch_index_adj<double>(g, vals, perm, off, out, s); break;
+    case TLGB_C64: launch_index_adj<float2>(g, vals, perm, off, out, s); break;
+    case TLGB_C128: launch_index_adj<double2>(g, vals, perm, off, out, s); break;
+    case TLGB_I32: launch_index_adj<int32_t>(g, vals, perm, off, out, s); break;
+    case TLGB_I64: launch_index_adj<long long>(g, vals, perm, off, out, s); break;
     default: TLGB_FAIL(TLGB_ERR_UNSUPPORTED, "index adjoint: unsupported element type");
   }
   TLGB_CHECK_LAUNCH();
