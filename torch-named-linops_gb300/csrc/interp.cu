@@ -1314,6 +1314,11 @@ __device__ __forceinline__ void fma2_bcast(float2& acc, float w, float2 v) {
   asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(a) : "l"(f2_bits(make_float2(w, w))), "l"(f2_bits(v)));
   acc = bits_f2(a);
 }
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  unsigned long long r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(f2_bits(a)), "l"(f2_bits(b)));
+  return bits_f2(r);
+}
 // (s, s) * v
 __device__ __forceinline__ float2 mul2_bcast(float s, float2 v) {
   unsigned long long r;
@@ -1332,19 +1337,36 @@ __device__ __forceinline__ float2 mul2_bcast(float s, float2 v) {
 // products (mma.sync m16n8k8, tf32 inputs, fp32 accumulation): the block's
 // 64 cells are the 4 row tiles (one per x, rows (y, z)), the 8 entries'
 // real and imaginary parts the 2 column tiles. The warp walks the block's
-// list in chunks of 32 entries: each lane copies one entry's values and the
-// point's three rows of tap weights over this block (from the plan) into the
-// warp's staging slots (cp.async). Then each group of 8 entries is one rank-8
+// list in chunks of 16 entries: two lanes copy one entry's values and the
+// point's three rows of tap weights over this block (from the plan) into a
+// buffer of the warp (cp.async). Then each group of 8 entries is one rank-8
 // update of the block: weights (x row * y row * z row, built in registers)
 // times values. fp32 accuracy from tf32 inputs: each operand is split into a
 // high and a low tf32 part and the update is hi*hi + hi*lo + lo*hi (the
 // lo*lo term is below 2^-22 of the product). The result depends only on the
-// plan's order: bit-identical run to run. A chunk with a non-finite value is
-// applied entry by entry on the CUDA cores instead, each such entry to the
+// plan's order: bit-identical run to run. An item whose sums are not all
+// finite is summed again entry by entry on the CUDA cores, each entry over the
 // cells of its window only (a zero weight would carry its NaN or Inf to the
 // whole block); the rows mark the cells outside the window with -0.0.
-constexpr int kBC = 32;       // entries per chunk (one per lane while staging)
-constexpr int kB3Ctas = 3;    // resident CTAs per SM of the persistent grid
+//
+// Bound by issue and by the latency of dependent instructions at four warps
+// per scheduler: with the same points for every block (all reads from L2) and
+// without the stores it still takes 535 of 610 us at 2^21 points in 256^3 x 8.
+// With one buffer of 32 entries per warp a chunk's copies were waited for in
+// full (684 us, 830 us for 256 entries of 320^2 at 205,824 points with its
+// transposition and reduction, whose groups were rows of the launch grid with
+// a warp per item); now the next chunk is copied during a chunk's products,
+// across items and groups, the splits and sums are packed two to an
+// instruction, whole blocks are stored without a check per cell, and values
+// are checked once per item: 610 and 671 us. Not faster: four lanes per entry
+// (fewer lines per copy, 755 against 726 us at that stage), three or four
+// buffers, two or four row tiles' products interleaved.
+constexpr int kBC = 16;       // entries per chunk, two lanes per entry while staging
+constexpr int kBWarps = 4;    // per CTA
+constexpr int kBStages = 2;   // chunks of a warp in shared memory: one worked on, the other in flight
+// Resident CTAs per SM of the persistent grid: with 128 registers nothing
+// spills (256^3 below: 706 us with 4 CTAs, 735 and 860 with 5 and 6)
+constexpr int kB3Ctas = 4;
 constexpr int kBS = 40;       // floats per staged entry: x row 0-3 | y row 4-7 | z row 8-11 | values 16-31
                               // (40: the tensor-core operand loads of a group of 8 entries are free of
                               // bank conflicts)
@@ -1355,9 +1377,66 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
 __device__ __forceinline__ void cp_async8(void* dst, const void* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
 }
-__device__ __forceinline__ void cp_async_wait_all() {
-  asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
-}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+// all copies of this thread but those of the last N committed groups
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// The chunks of the items that one warp takes, ahead of the warp's work on
+// them. A unit is (group of 8 entries, item), group after group; a warp's first
+// unit is its number in the grid, the others come from the counter. Lane
+// k & 7 keeps the descriptor and the group of the warp's k-th unit, requested
+// when the cursor reaches unit k - 1, and the counter is asked one request
+// ahead, so nothing waits for an atomic or a descriptor just issued.
+struct ChunkStream {
+  int4 desc;   // of unit k in lane k & 7; y < 0: past the end
+  int group;
+  int ticket;  // lane 0
+  int k, y, z, cg;  // cursor: unit, next chunk's first entry, end of the unit, its group
+
+  __device__ __forceinline__ void ask(int* ctr, int lane) {
+    if (lane == 0) ticket = atomicAdd(ctr, 1) + (int)gridDim.x * kBWarps;
+  }
+  __device__ __forceinline__ void read(int slot, int unit, int nunits, int nitems, const int4* __restrict__ items, int lane) {
+    if (lane != slot) return;
+    group = unit / nitems;
+    desc = unit < nunits ? items[unit - group * nitems] : make_int4(0, -1, -1, 0);
+  }
+  __device__ __forceinline__ void request(int slot, int nunits, int nitems, const int4* __restrict__ items, int* ctr, int lane) {
+    const int unit = __shfl_sync(0xffffffffu, ticket, 0);
+    read(slot, unit, nunits, nitems, items, lane);
+    if (unit < nunits) ask(ctr, lane);
+  }
+  __device__ __forceinline__ void move_to(int unit) {
+    k = unit;
+    y = __shfl_sync(0xffffffffu, desc.y, k & 7);
+    z = __shfl_sync(0xffffffffu, desc.z, k & 7);
+    cg = __shfl_sync(0xffffffffu, group, k & 7);
+  }
+  __device__ __forceinline__ void start(int nunits, int nitems, const int4* __restrict__ items, int* ctr, int lane, int warp) {
+    desc = make_int4(0, -1, -1, 0);
+    group = 0;
+    ticket = 0;
+    ask(ctr, lane);
+    read(0, (int)blockIdx.x * kBWarps + warp, nunits, nitems, items, lane);
+    if ((int)blockIdx.x * kBWarps + warp < nunits) request(1, nunits, nitems, items, ctr, lane);
+    move_to(0);
+  }
+  // this lane's entry of the next chunk, its group and size: -1 past the end, 0 for a run of empty blocks
+  __device__ __forceinline__ int next(uint32_t& entry, int& ecg, int nunits, int nitems, const int4* __restrict__ items,
+                                      const uint32_t* __restrict__ bentries, int* ctr, int lane) {
+    if (y < 0) return -1;
+    const int n = min(kBC, z - y), j = lane & (kBC - 1);
+    entry = j < n ? bentries[y + j] : 0u;
+    ecg = cg;
+    y += kBC;
+    if (y >= z) {
+      move_to(k + 1);
+      if (y >= 0) request((k + 1) & 7, nunits, nitems, items, ctr, lane);
+    }
+    return n;
+  }
+};
 
 // x = hi + lo: hi the nearest tf32 value, lo the rest (exact; the tensor
 // cores read its upper 11 bits). With cvt.rna (ties away) and a rounded lo the
@@ -1372,6 +1451,16 @@ __device__ __forceinline__ void split_tf32(float x, unsigned& hi, unsigned& lo) 
 __device__ __forceinline__ void split_tf32_mul(float x, float y, unsigned& hi, unsigned& lo) {
   asm("cvt.rn.tf32.f32 %0, %1;" : "=r"(hi) : "f"(x * y));
   lo = __float_as_uint(fmaf(x, y, -__uint_as_float(hi)));
+}
+
+// the same of two products x * y.x and x * y.y, two at a time
+__device__ __forceinline__ void split_tf32_mul2(float x, float2 y, unsigned* hi, unsigned* lo) {
+  const float2 p = mul2_bcast(x, y);
+  asm("cvt.rn.tf32.f32 %0, %1;" : "=r"(hi[0]) : "f"(p.x));
+  asm("cvt.rn.tf32.f32 %0, %1;" : "=r"(hi[1]) : "f"(p.y));
+  float2 l = mul2_bcast(-1.f, make_float2(__uint_as_float(hi[0]), __uint_as_float(hi[1])));
+  fma2_bcast(l, x, y);
+  lo[0] = __float_as_uint(l.x), lo[1] = __float_as_uint(l.y);
 }
 
 // d = a * b + c, m16n8k8, tf32 inputs, fp32 accumulators
@@ -1395,7 +1484,10 @@ __device__ __forceinline__ void mma_split(float (&d)[4], const unsigned (&ah)[4]
   mma_tf32(t, al, bh[0], bh[1], t);
   mma_tf32(t, ah, bh[0], bh[1], t);
 #pragma unroll
-  for (int i = 0; i < 4; ++i) d[i] += t[i];
+  for (int i = 0; i < 4; i += 2) {
+    const float2 r = add2(make_float2(d[i], d[i + 1]), make_float2(t[i], t[i + 1]));
+    d[i] = r.x, d[i + 1] = r.y;
+  }
 }
 
 __device__ __forceinline__ void block_origin(const Geo& g, int key, int& bx, int& by, int& bz) {
@@ -1431,6 +1523,19 @@ __device__ __forceinline__ void frag_store(const Geo& g, float* __restrict__ gri
   block_origin(g, blk, bx, by, bz);
   const int B0 = bx * block_edge(NDIM, 0), B1 = by * block_edge(NDIM, 1), B2 = bz * block_edge(NDIM, 2);
   const long long gvol = (long long)g.N[0] * g.N[1] * g.N[2];
+  if (ncoil == 8 && B0 + block_edge(NDIM, 0) <= g.N[0] && B1 + block_edge(NDIM, 1) <= g.N[1] && B2 + block_edge(NDIM, 2) <= g.N[2]) {
+    int lx, ly, lz;
+    frag_cell<NDIM>(0, 0, g8, lx, ly, lz);
+    const long long s1 = g.N[2], sm = NDIM == 3 ? (long long)g.N[1] * s1 : 2 * s1, sh = NDIM == 3 ? 2 * s1 : s1;
+    float2* q = reinterpret_cast<float2*>(gridv) + (c0 + t4) * gvol + ((long long)(B0 + lx) * g.N[1] + B1 + ly) * s1 + B2 + lz;
+#pragma unroll
+    for (int nt = 0; nt < 2; ++nt, q += 4 * gvol)
+#pragma unroll
+      for (int m = 0; m < 4; ++m)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) q[m * sm + h * sh] = make_float2(D[m][nt][2 * h], D[m][nt][2 * h + 1]);
+    return;
+  }
 #pragma unroll
   for (int m = 0; m < 4; ++m) {
 #pragma unroll
@@ -1451,8 +1556,51 @@ __device__ __forceinline__ void frag_store(const Geo& g, float* __restrict__ gri
   }
 }
 
+// Sums of one item again, entry by entry on the CUDA cores, where the tensor
+// cores gave a non-finite one: a NaN or Inf among the values only reaches the
+// cells of its point's window (the rows hold -0.0 outside it).
 template <int NDIM, int NROW>
-__global__ void __launch_bounds__(256, kB3Ctas) adj_b3_kernel(Geo g, const int4* __restrict__ items, int nitems,
+__device__ __noinline__ void block_by_entry(const Geo& g, const uint32_t* __restrict__ bentries, const float* __restrict__ rows,
+                                            const float2* __restrict__ vals, const float4* __restrict__ tv, int cg, int ncoil,
+                                            int from, int to, int g8, int t4, float (&D)[4][2][4]) {
+  for (int m = 0; m < 4; ++m)
+    for (int nt = 0; nt < 2; ++nt)
+      for (int i = 0; i < 4; ++i) D[m][nt][i] = 0.f;
+  for (int q = from; q < to; ++q) {
+    const uint32_t en = bentries[q];
+    long long p = en & ((1u << sel_shift(NROW)) - 1u);
+    if (!TLGB_IN_RANGE(p, g.npts)) p = 0;
+    int ri, rj, rk;
+    sel_rows<NROW>(en, ri, rj, rk);
+    const float* r = rows + p * row_floats(NDIM, NROW);
+    const float* rx = r + 4 * ri;
+    const float* ry = NDIM == 3 ? r + 4 * (NROW + rj) : r + 8 * rj;
+    const float* rz = NDIM == 3 ? r + 4 * (2 * NROW + rk) : r + 8 * (NROW + rk);
+    float2 v[2];
+    for (int nt = 0; nt < 2; ++nt) {
+      const int e = 4 * nt + t4;
+      v[nt] = make_float2(0.f, 0.f);
+      if (e < ncoil)
+        v[nt] = tv ? reinterpret_cast<const float2*>(tv + ((long long)cg * g.npts + p) * 4)[e]
+                   : vals[((long long)cg * 8 + e) * g.npts + p];
+    }
+    for (int m = 0; m < 4; ++m)
+      for (int h = 0; h < 2; ++h) {
+        int lx, ly, lz;
+        frag_cell<NDIM>(m, h, g8, lx, ly, lz);
+        const float wx = NDIM == 3 ? rx[lx] : 1.f, y = ry[ly], z = rz[lz], w = wx * (y * z);
+        if (signbit(wx) || signbit(y) || signbit(z)) continue;
+        for (int nt = 0; nt < 2; ++nt) {
+          D[m][nt][2 * h] = fmaf(w, v[nt].x, D[m][nt][2 * h]);
+          D[m][nt][2 * h + 1] = fmaf(w, v[nt].y, D[m][nt][2 * h + 1]);
+        }
+      }
+  }
+}
+
+template <int NDIM, int NROW>
+__global__ void __launch_bounds__(kBWarps * 32, kB3Ctas) adj_b3_kernel(Geo g, const int4* __restrict__ items, int nitems,
+                                                        int nunits, int cg0, int ncg,
                                                         const uint32_t* __restrict__ bentries,
                                                         const float* __restrict__ rows,
                                                         const float2* __restrict__ vals,
@@ -1460,204 +1608,173 @@ __global__ void __launch_bounds__(256, kB3Ctas) adj_b3_kernel(Geo g, const int4*
                                                         float* __restrict__ partial, int* __restrict__ ctr) {
   extern __shared__ __align__(16) float bsm[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  float* S = bsm + warp * (kBC * kBS);
-  const int cg = blockIdx.y, c0 = cg * 8;
-  const int ncoil = (int)min(8ll, g.nbatch - c0);
-  const int g8 = lane >> 2, t4 = lane & 3;
-  const int last = nitems;
-  // the warps of all CTAs take the items in list order from the group's
-  // counter (zeroed before the launch), so the items worked on at one time
-  // are neighbours in the list; the warps never wait for one another
-  auto grab = [&]() {
-    int i = 0;
-    if (lane == 0) i = atomicAdd(ctr + cg, 1);
-    return __shfl_sync(0xffffffffu, i, 0);
-  };
-  // one item and the next chunk's point indices ahead: a chunk's copies wait
-  // only for their own data, not for the descriptor and index loads before it
-  int item = grab();
-  if (item >= last) return;
-  int4 itn = items[item];
-  int inext = grab();
-  int4 itnn = inext < last ? items[inext] : make_int4(0, 0, 0, 0);
-  uint32_t enext = lane < min(kBC, itn.z - itn.y) ? bentries[itn.y + lane] : 0u;
-  for (;;) {
-    if (item >= last) return;
-    const int4 it = itn;
-    itn = itnn;
-    item = inext;
-    if (item < last) {
-      inext = grab();
-      itnn = inext < last ? items[inext] : make_int4(0, 0, 0, 0);
-    }
-    float D[4][2][4];
-#pragma unroll
-    for (int m = 0; m < 4; ++m)
-#pragma unroll
-      for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) D[m][nt][i] = 0.f;
-    if (it.y == it.z) {  // a run of -it.w empty blocks
-      for (int b = 0; b < -it.w; ++b) frag_store<NDIM>(g, gridv, c0, ncoil, it.x + b, g8, t4, D);
-      if (item < last) enext = lane < min(kBC, itn.z - itn.y) ? bentries[itn.y + lane] : 0u;
-      continue;
-    }
-    for (int c = it.y; c < it.z; c += kBC) {
-      const int n = min(kBC, it.z - c);
-      const int n8 = (n + 7) & ~7;  // the tensor-core steps read whole groups of 8 entries
-      float* sl = S + lane * kBS;
-      const uint32_t en = enext;
-      // the point indices of the next chunk: this item's, or the next item's first
-      if (c + kBC < it.z)
-        enext = lane < min(kBC, it.z - c - kBC) ? bentries[c + kBC + lane] : 0u;
-      else if (item < last)
-        enext = lane < min(kBC, itn.z - itn.y) ? bentries[itn.y + lane] : 0u;
-      if (lane < n) {
-        long long p = en & ((1u << sel_shift(NROW)) - 1u);
-        if (!TLGB_IN_RANGE(p, g.npts)) p = 0;
-        const float* rsrc = rows + p * row_floats(NDIM, NROW);
-        int ri, rj, rk;
-        sel_rows<NROW>(en, ri, rj, rk);
-        if constexpr (NDIM == 3) {  // rows of 4 cells: x 0-3, y 4-7, z 8-11
+  float* S = bsm + warp * (kBStages * kBC * kBS);
+  const int g8 = lane >> 2, t4 = lane & 3, half = lane / kBC;
+  float* const mine = S + (lane & (kBC - 1)) * kBS;  // this lane's entry of a chunk; it copies half of it
+  ChunkStream cs;
+  cs.start(nunits, nitems, items, ctr, lane, warp);
+  auto stage = [&](float* sl, int n, uint32_t en, int cg) {
+    const int j = lane & (kBC - 1);
+    if (j < n) {
+      long long p = en & ((1u << sel_shift(NROW)) - 1u);
+      if (!TLGB_IN_RANGE(p, g.npts)) p = 0;
+      const float* rsrc = rows + p * row_floats(NDIM, NROW);
+      int ri, rj, rk;
+      sel_rows<NROW>(en, ri, rj, rk);
+      if constexpr (NDIM == 3) {  // rows of 4 cells: x 0-3, y 4-7, z 8-11
+        if (half == 0) {
           cp_async16(sl + 0, rsrc + 4 * ri);
           cp_async16(sl + 4, rsrc + 4 * (NROW + rj));
-          cp_async16(sl + 8, rsrc + 4 * (2 * NROW + rk));
-        } else {  // rows of 8 cells: y 0-7, z 8-15
-          const float* ry = rsrc + 8 * rj;
-          const float* rz = rsrc + 8 * (NROW + rk);
-          cp_async16(sl + 0, ry);
-          cp_async16(sl + 4, ry + 4);
-          cp_async16(sl + 8, rz);
-          cp_async16(sl + 12, rz + 4);
-        }
-        if (tv) {
-          const float4* vsrc = tv + ((long long)cg * g.npts + p) * 4;
-#pragma unroll
-          for (int q = 0; q < 4; ++q) cp_async16(sl + 16 + 4 * q, vsrc + q);
         } else {
-#pragma unroll
-          for (int k = 0; k < 8; ++k) {
-            if (k < ncoil)
-              cp_async8(sl + 16 + 2 * k, vals + (long long)(c0 + k) * g.npts + p);
-            else
-              *reinterpret_cast<float2*>(sl + 16 + 2 * k) = make_float2(0.f, 0.f);
-          }
+          cp_async16(sl + 8, rsrc + 4 * (2 * NROW + rk));
         }
-      } else if (lane < n8) {  // padding entries of the last group: zero weights and values
-        const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
-        float4* q4 = reinterpret_cast<float4*>(sl);
-        q4[0] = q4[1] = q4[2] = q4[3] = z4;
-        q4[4] = q4[5] = q4[6] = q4[7] = z4;
+      } else {  // rows of 8 cells: y 0-7, z 8-15
+        const float* r = rsrc + 8 * (half ? NROW + rk : rj);
+        cp_async16(sl + 8 * half, r);
+        cp_async16(sl + 8 * half + 4, r + 4);
       }
-      cp_async_wait_all();
-      bool nonfinite = false;
-      if (lane < n) {  // a non-finite value turns the zero product into NaN
-        float chk = 0.f;
-        const float4* vq = reinterpret_cast<const float4*>(sl + 16);
+      if (tv) {
+        const float4* vsrc = tv + ((long long)(cg0 + cg) * g.npts + p) * 4 + 2 * half;
+        cp_async16(sl + 16 + 8 * half, vsrc);
+        cp_async16(sl + 20 + 8 * half, vsrc + 1);
+      } else {
+        const long long c0 = (long long)(cg0 + cg) * 8 + 4 * half;
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-          const float4 v = vq[q];
-          chk = fmaf(v.x, 0.f, chk);
-          chk = fmaf(v.y, 0.f, chk);
-          chk = fmaf(v.z, 0.f, chk);
-          chk = fmaf(v.w, 0.f, chk);
-        }
-        nonfinite = !(chk == 0.f);
-      }
-      const unsigned guarded = __ballot_sync(0xffffffffu, nonfinite);
-      __syncwarp();
-      if (!guarded) {
-        for (int kk = 0; kk < n8; kk += 8) {  // entries kk + t4 and kk + t4 + 4 of this lane's fragments
-          const float* e0 = S + (kk + t4) * kBS;
-          const float* e1 = e0 + 4 * kBS;
-          unsigned bh[2][2], bl[2][2];
-#pragma unroll
-          for (int nt = 0; nt < 2; ++nt) {
-            split_tf32(e0[16 + 8 * nt + g8], bh[nt][0], bl[nt][0]);
-            split_tf32(e1[16 + 8 * nt + g8], bh[nt][1], bl[nt][1]);
-          }
-          // A fragments of row tile m: the weights of rows g8 and g8 + 8 for entries e0 and e1
-          float u0[4], u1[4], va, vb, vc, vd;
-          if constexpr (NDIM == 3) {  // x m * (y (g8 >> 2) + 2h * z g8 & 3)
-            const float z0 = e0[8 + (g8 & 3)], z1 = e1[8 + (g8 & 3)];
-            const float4 x0 = *reinterpret_cast<const float4*>(e0), x1 = *reinterpret_cast<const float4*>(e1);
-            u0[0] = x0.x, u0[1] = x0.y, u0[2] = x0.z, u0[3] = x0.w;
-            u1[0] = x1.x, u1[1] = x1.y, u1[2] = x1.z, u1[3] = x1.w;
-            va = e0[4 + (g8 >> 2)] * z0, vb = e0[6 + (g8 >> 2)] * z0;
-            vc = e1[4 + (g8 >> 2)] * z1, vd = e1[6 + (g8 >> 2)] * z1;
-          } else {  // y 2m + h * z g8
-            va = vb = e0[8 + g8], vc = vd = e1[8 + g8];
-          }
-#pragma unroll
-          for (int m = 0; m < 4; ++m) {
-            unsigned ah[4], al[4];
-            if constexpr (NDIM == 3) {
-              split_tf32_mul(u0[m], va, ah[0], al[0]);
-              split_tf32_mul(u0[m], vb, ah[1], al[1]);
-              split_tf32_mul(u1[m], vc, ah[2], al[2]);
-              split_tf32_mul(u1[m], vd, ah[3], al[3]);
-            } else {
-              const float2 y0 = *reinterpret_cast<const float2*>(e0 + 2 * m);
-              const float2 y1 = *reinterpret_cast<const float2*>(e1 + 2 * m);
-              split_tf32_mul(y0.x, va, ah[0], al[0]);
-              split_tf32_mul(y0.y, vb, ah[1], al[1]);
-              split_tf32_mul(y1.x, vc, ah[2], al[2]);
-              split_tf32_mul(y1.y, vd, ah[3], al[3]);
-            }
-#pragma unroll
-            for (int nt = 0; nt < 2; ++nt) {
-              mma_split(D[m][nt], ah, al, bh[nt], bl[nt]);
-            }
-          }
-        }
-      } else {
-        // entry by entry on the CUDA cores, in order; a non-finite entry only
-        // reaches the cells of its window (weights with a clear sign bit)
-        for (int j = 0; j < n; ++j) {
-          const float* e = S + j * kBS;
-          const bool nf = (guarded >> j) & 1u;
-#pragma unroll
-          for (int m = 0; m < 4; ++m) {
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              int lx, ly, lz;
-              frag_cell<NDIM>(m, h, g8, lx, ly, lz);
-              // weights of the cell along each dim: 3D rows x 0-3, y 4-7, z 8-11; 2D y 0-7, z 8-15
-              const float wx = NDIM == 3 ? e[lx] : 1.f;
-              const float y = NDIM == 3 ? e[4 + ly] : e[ly], z = e[8 + lz];
-              const float w = wx * (y * z);
-              const bool ok = !nf || (!signbit(wx) && !signbit(y) && !signbit(z));
-#pragma unroll
-              for (int nt = 0; nt < 2; ++nt) {
-                const float2 v = *reinterpret_cast<const float2*>(e + 16 + 2 * (4 * nt + t4));
-                if (ok) {
-                  D[m][nt][2 * h] = fmaf(w, v.x, D[m][nt][2 * h]);
-                  D[m][nt][2 * h + 1] = fmaf(w, v.y, D[m][nt][2 * h + 1]);
-                }
-              }
-            }
-          }
+          if (c0 + q < g.nbatch)
+            cp_async8(sl + 16 + 8 * half + 2 * q, vals + (c0 + q) * g.npts + p);
+          else
+            *reinterpret_cast<float2*>(sl + 16 + 8 * half + 2 * q) = make_float2(0.f, 0.f);
         }
       }
-      __syncwarp();  // the chunk has been read before the next one is staged
+    } else if (j < ((n + 7) & ~7)) {  // padding entries of the last group: zero weights and values
+      const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
+      float4* q4 = reinterpret_cast<float4*>(sl) + 2 * half;
+      q4[0] = q4[1] = q4[4] = q4[5] = z4;
     }
-    if (it.w >= 0) {  // a part of a split block: its slot of the partial blocks, [cell][entry] complex
-      float* dst = partial + ((long long)it.w * gridDim.y + cg) * 64 * 16;
+  };
+  // the copies of kBStages - 1 chunks and the entry numbers of the one after
+  // them are in flight during the work on a chunk, across items
+  uint32_t en = 0;
+  int ecg = 0;
+  unsigned sizes = 0;  // byte i: 1 + size of the i-th chunk from here, 0 past the end
+  int n = cs.next(en, ecg, nunits, nitems, items, bentries, ctr, lane);
+  if (n < 0) return;
+#pragma unroll
+  for (int i = 0; i < kBStages - 1; ++i) {
+    if (n >= 0) stage(mine + i * (kBC * kBS), n, en, ecg);
+    cp_async_commit();
+    sizes |= (unsigned)(n + 1) << (8 * i);
+    n = cs.next(en, ecg, nunits, nitems, items, bentries, ctr, lane);
+  }
+  float D[4][2][4];
+#pragma unroll
+  for (int m = 0; m < 4; ++m)
+#pragma unroll
+    for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) D[m][nt][i] = 0.f;
+  int unit = 0;  // of this warp
+  int c = __shfl_sync(0xffffffffu, cs.desc.y, 0), cend = __shfl_sync(0xffffffffu, cs.desc.z, 0);
+  for (int buf = 0;; buf = buf + 1 == kBStages ? 0 : buf + 1) {
+    if (n >= 0) stage(mine + (buf == 0 ? kBStages - 1 : buf - 1) * (kBC * kBS), n, en, ecg);
+    cp_async_commit();
+    sizes |= (unsigned)(n + 1) << (8 * (kBStages - 1));
+    n = cs.next(en, ecg, nunits, nitems, items, bentries, ctr, lane);
+    cp_async_wait<kBStages - 1>();
+    const int now = (int)(sizes & 255u) - 1;  // entries of this chunk
+    sizes >>= 8;
+    const float* B = S + buf * (kBC * kBS);
+    const int n8 = (now + 7) & ~7;  // the tensor-core steps read whole groups of 8 entries
+    __syncwarp();  // the lanes' copies are in
+    for (int kk = 0; kk < n8; kk += 8) {  // entries kk + t4 and kk + t4 + 4 of this lane's fragments
+      const float* e0 = B + (kk + t4) * kBS;
+      const float* e1 = e0 + 4 * kBS;
+      unsigned bh[2][2], bl[2][2];
+#pragma unroll
+      for (int nt = 0; nt < 2; ++nt) {
+        split_tf32(e0[16 + 8 * nt + g8], bh[nt][0], bl[nt][0]);
+        split_tf32(e1[16 + 8 * nt + g8], bh[nt][1], bl[nt][1]);
+      }
+      // A fragments of row tile m: the weights of rows g8 and g8 + 8 for entries e0 and e1
+      float u0[4], u1[4], va, vb, vc, vd;
+      if constexpr (NDIM == 3) {  // x m * (y (g8 >> 2) + 2h * z g8 & 3)
+        const float z0 = e0[8 + (g8 & 3)], z1 = e1[8 + (g8 & 3)];
+        const float4 x0 = *reinterpret_cast<const float4*>(e0), x1 = *reinterpret_cast<const float4*>(e1);
+        u0[0] = x0.x, u0[1] = x0.y, u0[2] = x0.z, u0[3] = x0.w;
+        u1[0] = x1.x, u1[1] = x1.y, u1[2] = x1.z, u1[3] = x1.w;
+        va = e0[4 + (g8 >> 2)] * z0, vb = e0[6 + (g8 >> 2)] * z0;
+        vc = e1[4 + (g8 >> 2)] * z1, vd = e1[6 + (g8 >> 2)] * z1;
+      } else {  // y 2m + h * z g8
+        va = vb = e0[8 + g8], vc = vd = e1[8 + g8];
+      }
+#pragma unroll
+      for (int m = 0; m < 4; ++m) {
+        unsigned ah[4], al[4];
+        if constexpr (NDIM == 3) {
+          split_tf32_mul2(u0[m], make_float2(va, vb), ah, al);
+          split_tf32_mul2(u1[m], make_float2(vc, vd), ah + 2, al + 2);
+        } else {
+          split_tf32_mul2(va, *reinterpret_cast<const float2*>(e0 + 2 * m), ah, al);
+          split_tf32_mul2(vc, *reinterpret_cast<const float2*>(e1 + 2 * m), ah + 2, al + 2);
+        }
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt) {
+          mma_split(D[m][nt], ah, al, bh[nt], bl[nt]);
+        }
+      }
+    }
+    c += kBC;
+    if (c >= cend) {  // the item's last chunk
+      const int ix = __shfl_sync(0xffffffffu, cs.desc.x, unit & 7), iw = __shfl_sync(0xffffffffu, cs.desc.w, unit & 7);
+      const int cg = cg0 + __shfl_sync(0xffffffffu, cs.group, unit & 7), c0 = cg * 8;
+      const int ncoil = (int)min(8ll, g.nbatch - c0);
+      float bad = 0.f;  // NaN if any sum is not finite
 #pragma unroll
       for (int m = 0; m < 4; ++m)
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          int lx, ly, lz;
-          frag_cell<NDIM>(m, h, g8, lx, ly, lz);
-          const int cell = cell_index<NDIM>(lx, ly, lz);
+        for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) bad = fmaf(D[m][nt][i], 0.f, bad);
+      if (__any_sync(0xffffffffu, !(bad == 0.f))) {
+        float again[4][2][4];
+        block_by_entry<NDIM, NROW>(g, bentries, rows, vals, tv, cg, ncoil, __shfl_sync(0xffffffffu, cs.desc.y, unit & 7), cend,
+                                   g8, t4, again);
+#pragma unroll
+        for (int m = 0; m < 4; ++m)
 #pragma unroll
           for (int nt = 0; nt < 2; ++nt)
-            *reinterpret_cast<float2*>(dst + cell * 16 + 2 * (4 * nt + t4)) =
-                make_float2(D[m][nt][2 * h], D[m][nt][2 * h + 1]);
-        }
-    } else {
-      frag_store<NDIM>(g, gridv, c0, ncoil, it.x, g8, t4, D);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) D[m][nt][i] = again[m][nt][i];
+      }
+      if (iw >= 0) {  // a part of a split block: its slot of the partial blocks, [cell][entry] complex
+        float* dst = partial + ((long long)iw * ncg + cg) * 64 * 16;
+#pragma unroll
+        for (int m = 0; m < 4; ++m)
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            int lx, ly, lz;
+            frag_cell<NDIM>(m, h, g8, lx, ly, lz);
+            const int cell = cell_index<NDIM>(lx, ly, lz);
+#pragma unroll
+            for (int nt = 0; nt < 2; ++nt)
+              *reinterpret_cast<float2*>(dst + cell * 16 + 2 * (4 * nt + t4)) =
+                  make_float2(D[m][nt][2 * h], D[m][nt][2 * h + 1]);
+          }
+      } else {  // one block, or a run of -iw empty ones
+        for (int b = 0; b < -iw; ++b) frag_store<NDIM>(g, gridv, c0, ncoil, ix + b, g8, t4, D);
+      }
+      if ((sizes & 255u) == 0) return;
+#pragma unroll
+      for (int m = 0; m < 4; ++m)
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) D[m][nt][i] = 0.f;
+      ++unit;
+      c = __shfl_sync(0xffffffffu, cs.desc.y, unit & 7), cend = __shfl_sync(0xffffffffu, cs.desc.z, unit & 7);
     }
+    __syncwarp();  // the chunk has been read before its buffer is staged again
   }
 }
 
@@ -1733,7 +1850,7 @@ __global__ void __launch_bounds__(256) adj_reduce_b3_kernel(Geo g, const int4* _
 // z g8 & 3) (d0, d1) and (x t4, y (g8 >> 2) + 2, z g8 & 3) (d2, d3).
 constexpr int kBSn = 20;  // floats per staged entry: x row 0-3 | y row 4-7 | z row 8-11 | E values 12-19
                           // (20: the operand loads of a group of 8 entries are free of bank conflicts)
-constexpr int kBnCtas = 4;  // resident CTAs per SM of the persistent grid
+constexpr int kBnCtas = 6;  // resident CTAs per SM of the persistent grid
 
 template <int E>
 __device__ __forceinline__ void bn_store(const Geo& g, float* __restrict__ gridv, int ncoil, int blk, int g8, int t4,
@@ -1755,8 +1872,35 @@ __device__ __forceinline__ void bn_store(const Geo& g, float* __restrict__ gridv
   }
 }
 
+// Sums of one item again where one is not finite (see block_by_entry).
 template <int E, int NROW>
-__global__ void __launch_bounds__(256, kBnCtas) adj_bn_kernel(Geo g, const int4* __restrict__ items, int nitems,
+__device__ __noinline__ void block_by_entry_n(const Geo& g, const uint32_t* __restrict__ bentries, const float* __restrict__ rows,
+                                              const float2* __restrict__ vals, int ncoil, int from, int to, int g8, int t4,
+                                              float (&D)[E][4]) {
+  for (int j = 0; j < E; ++j)
+    for (int i = 0; i < 4; ++i) D[j][i] = 0.f;
+  for (int q = from; q < to; ++q) {
+    const uint32_t en = bentries[q];
+    long long p = en & ((1u << sel_shift(NROW)) - 1u);
+    if (!TLGB_IN_RANGE(p, g.npts)) p = 0;
+    int ri, rj, rk;
+    sel_rows<NROW>(en, ri, rj, rk);
+    const float* r = rows + p * row_floats(3, NROW);
+    const float wx = r[4 * ri + t4], z = r[4 * (2 * NROW + rk) + (g8 & 3)];
+    for (int h = 0; h < 2; ++h) {
+      const float y = r[4 * (NROW + rj) + (g8 >> 2) + 2 * h], w = wx * (y * z);
+      if (signbit(wx) || signbit(y) || signbit(z)) continue;
+      for (int j = 0; j < ncoil; ++j) {
+        const float2 v = vals[(long long)j * g.npts + p];
+        D[j][2 * h] = fmaf(w, v.x, D[j][2 * h]);
+        D[j][2 * h + 1] = fmaf(w, v.y, D[j][2 * h + 1]);
+      }
+    }
+  }
+}
+
+template <int E, int NROW>
+__global__ void __launch_bounds__(kBWarps * 32, kBnCtas) adj_bn_kernel(Geo g, const int4* __restrict__ items, int nitems,
                                                              const uint32_t* __restrict__ bentries,
                                                              const float* __restrict__ rows,
                                                              const float2* __restrict__ vals,
@@ -1764,140 +1908,128 @@ __global__ void __launch_bounds__(256, kBnCtas) adj_bn_kernel(Geo g, const int4*
                                                              int* __restrict__ ctr) {
   extern __shared__ __align__(16) float bsm[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  float* S = bsm + warp * (kBC * kBSn);
+  float* S = bsm + warp * (kBStages * kBC * kBSn);
   const int ncoil = (int)min((long long)E, g.nbatch);
-  const int g8 = lane >> 2, t4 = lane & 3;
-  const int last = nitems;
-  auto grab = [&]() {
-    int i = 0;
-    if (lane == 0) i = atomicAdd(ctr, 1);
-    return __shfl_sync(0xffffffffu, i, 0);
-  };
-  int item = grab();
-  if (item >= last) return;
-  int4 itn = items[item];
-  int inext = grab();
-  int4 itnn = inext < last ? items[inext] : make_int4(0, 0, 0, 0);
-  uint32_t enext = lane < min(kBC, itn.z - itn.y) ? bentries[itn.y + lane] : 0u;
-  for (;;) {
-    if (item >= last) return;
-    const int4 it = itn;
-    itn = itnn;
-    item = inext;
-    if (item < last) {
-      inext = grab();
-      itnn = inext < last ? items[inext] : make_int4(0, 0, 0, 0);
-    }
-    float D[E][4];
-#pragma unroll
-    for (int j = 0; j < E; ++j)
-#pragma unroll
-      for (int i = 0; i < 4; ++i) D[j][i] = 0.f;
-    if (it.y == it.z) {  // a run of -it.w empty blocks
-      for (int b = 0; b < -it.w; ++b) bn_store<E>(g, gridv, ncoil, it.x + b, g8, t4, D);
-      if (item < last) enext = lane < min(kBC, itn.z - itn.y) ? bentries[itn.y + lane] : 0u;
-      continue;
-    }
-    for (int c = it.y; c < it.z; c += kBC) {
-      const int n = min(kBC, it.z - c);
-      const int n8 = (n + 7) & ~7;
-      float* sl = S + lane * kBSn;
-      const uint32_t en = enext;
-      if (c + kBC < it.z)
-        enext = lane < min(kBC, it.z - c - kBC) ? bentries[c + kBC + lane] : 0u;
-      else if (item < last)
-        enext = lane < min(kBC, itn.z - itn.y) ? bentries[itn.y + lane] : 0u;
-      if (lane < n) {
-        long long p = en & ((1u << sel_shift(NROW)) - 1u);
-        if (!TLGB_IN_RANGE(p, g.npts)) p = 0;
-        const float* rsrc = rows + p * row_floats(3, NROW);
-        int ri, rj, rk;
-        sel_rows<NROW>(en, ri, rj, rk);
+  const int g8 = lane >> 2, t4 = lane & 3, half = lane / kBC;
+  float* const mine = S + (lane & (kBC - 1)) * kBSn;
+  ChunkStream cs;
+  cs.start(nitems, nitems, items, ctr, lane, warp);
+  auto stage = [&](float* sl, int n, uint32_t en) {
+    const int q = lane & (kBC - 1);
+    if (q < n) {
+      long long p = en & ((1u << sel_shift(NROW)) - 1u);
+      if (!TLGB_IN_RANGE(p, g.npts)) p = 0;
+      const float* rsrc = rows + p * row_floats(3, NROW);
+      int ri, rj, rk;
+      sel_rows<NROW>(en, ri, rj, rk);
+      if (half == 0) {
         cp_async16(sl + 0, rsrc + 4 * ri);
         cp_async16(sl + 4, rsrc + 4 * (NROW + rj));
-        cp_async16(sl + 8, rsrc + 4 * (2 * NROW + rk));
-#pragma unroll
-        for (int j = 0; j < E; ++j) {
-          if (j < ncoil)
-            cp_async8(sl + 12 + 2 * j, vals + (long long)j * g.npts + p);
-          else
-            *reinterpret_cast<float2*>(sl + 12 + 2 * j) = make_float2(0.f, 0.f);
-        }
-      } else if (lane < n8) {  // padding entries of the last group: zero weights and values
-        const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
-        float4* q4 = reinterpret_cast<float4*>(sl);
-        q4[0] = q4[1] = q4[2] = z4;
-#pragma unroll
-        for (int j = 0; j < E; ++j) *reinterpret_cast<float2*>(sl + 12 + 2 * j) = make_float2(0.f, 0.f);
-      }
-      cp_async_wait_all();
-      bool nonfinite = false;
-      if (lane < n) {  // a non-finite value turns the zero product into NaN
-        float chk = 0.f;
-#pragma unroll
-        for (int j = 0; j < 2 * E; ++j) chk = fmaf(sl[12 + j], 0.f, chk);
-        nonfinite = !(chk == 0.f);
-      }
-      const unsigned guarded = __ballot_sync(0xffffffffu, nonfinite);
-      __syncwarp();
-      if (!guarded) {
-        for (int kk = 0; kk < n8; kk += 8) {  // entries kk + t4 and kk + t4 + 4 of this lane's fragments
-          const float* e0 = S + (kk + t4) * kBSn;
-          const float* e1 = e0 + 4 * kBSn;
-          // A: rows g8 and g8 + 8 = (y (g8 >> 2) + 2h, z g8 & 3)
-          const float z0 = e0[8 + (g8 & 3)], z1 = e1[8 + (g8 & 3)];
-          unsigned ah[4], al[4];
-          split_tf32_mul(e0[4 + (g8 >> 2)], z0, ah[0], al[0]);
-          split_tf32_mul(e0[6 + (g8 >> 2)], z0, ah[1], al[1]);
-          split_tf32_mul(e1[4 + (g8 >> 2)], z1, ah[2], al[2]);
-          split_tf32_mul(e1[6 + (g8 >> 2)], z1, ah[3], al[3]);
-          // B: column g8 = (x g8 >> 1, c g8 & 1) of entry j
-          const float x0 = e0[g8 >> 1], x1 = e1[g8 >> 1];
-#pragma unroll
-          for (int j = 0; j < E; ++j) {
-            unsigned bh[2], bl[2];
-            split_tf32_mul(e0[12 + 2 * j + (g8 & 1)], x0, bh[0], bl[0]);
-            split_tf32_mul(e1[12 + 2 * j + (g8 & 1)], x1, bh[1], bl[1]);
-            mma_split(D[j], ah, al, bh, bl);
-          }
-        }
       } else {
-        // entry by entry on the CUDA cores, in order; a non-finite entry only
-        // reaches the cells of its window (weights with a clear sign bit)
-        for (int q = 0; q < n; ++q) {
-          const float* e = S + q * kBSn;
-          const bool nf = (guarded >> q) & 1u;
-          const float wx = e[t4], z = e[8 + (g8 & 3)];
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const float y = e[4 + (g8 >> 2) + 2 * h];
-            const float w = wx * (y * z);
-            const bool ok = !nf || (!signbit(wx) && !signbit(y) && !signbit(z));
-#pragma unroll
-            for (int j = 0; j < E; ++j) {
-              const float2 v = *reinterpret_cast<const float2*>(e + 12 + 2 * j);
-              if (ok) {
-                D[j][2 * h] = fmaf(w, v.x, D[j][2 * h]);
-                D[j][2 * h + 1] = fmaf(w, v.y, D[j][2 * h + 1]);
-              }
-            }
-          }
-        }
+        cp_async16(sl + 8, rsrc + 4 * (2 * NROW + rk));
       }
-      __syncwarp();  // the chunk has been read before the next one is staged
-    }
-    if (it.w >= 0) {  // a part of a split block: its slot of the partial blocks, [cell][entry] complex
-      float* dst = partial + (long long)it.w * 64 * 2 * E;
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int cell = cell_index<3>(t4, (g8 >> 2) + 2 * h, g8 & 3);
+      for (int j = 0; j < E; ++j) {
+        if ((j & 1) == half) continue;  // the lane with one row takes entries 0 and 2
+        if (j < ncoil)
+          cp_async8(sl + 12 + 2 * j, vals + (long long)j * g.npts + p);
+        else
+          *reinterpret_cast<float2*>(sl + 12 + 2 * j) = make_float2(0.f, 0.f);
+      }
+    } else if (q < ((n + 7) & ~7) && half == 0) {  // padding entries of the last group: zero weights and values
+      const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
+      float4* q4 = reinterpret_cast<float4*>(sl);
+      q4[0] = q4[1] = q4[2] = z4;
+#pragma unroll
+      for (int j = 0; j < E; ++j) *reinterpret_cast<float2*>(sl + 12 + 2 * j) = make_float2(0.f, 0.f);
+    }
+  };
+  uint32_t en = 0;
+  int ecg = 0;
+  unsigned sizes = 0;  // byte i: 1 + size of the i-th chunk from here, 0 past the end
+  int n = cs.next(en, ecg, nitems, nitems, items, bentries, ctr, lane);
+  if (n < 0) return;
+#pragma unroll
+  for (int i = 0; i < kBStages - 1; ++i) {
+    if (n >= 0) stage(mine + i * (kBC * kBSn), n, en);
+    cp_async_commit();
+    sizes |= (unsigned)(n + 1) << (8 * i);
+    n = cs.next(en, ecg, nitems, nitems, items, bentries, ctr, lane);
+  }
+  float D[E][4];
+#pragma unroll
+  for (int j = 0; j < E; ++j)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) D[j][i] = 0.f;
+  int unit = 0;
+  int c = __shfl_sync(0xffffffffu, cs.desc.y, 0), cend = __shfl_sync(0xffffffffu, cs.desc.z, 0);
+  for (int buf = 0;; buf = buf + 1 == kBStages ? 0 : buf + 1) {
+    if (n >= 0) stage(mine + (buf == 0 ? kBStages - 1 : buf - 1) * (kBC * kBSn), n, en);
+    cp_async_commit();
+    sizes |= (unsigned)(n + 1) << (8 * (kBStages - 1));
+    n = cs.next(en, ecg, nitems, nitems, items, bentries, ctr, lane);
+    cp_async_wait<kBStages - 1>();
+    const int now = (int)(sizes & 255u) - 1;  // entries of this chunk
+    sizes >>= 8;
+    const float* B = S + buf * (kBC * kBSn);
+    const int n8 = (now + 7) & ~7;
+    __syncwarp();  // the lanes' copies are in
+    for (int kk = 0; kk < n8; kk += 8) {  // entries kk + t4 and kk + t4 + 4 of this lane's fragments
+      const float* e0 = B + (kk + t4) * kBSn;
+      const float* e1 = e0 + 4 * kBSn;
+      // A: rows g8 and g8 + 8 = (y (g8 >> 2) + 2h, z g8 & 3)
+      const float z0 = e0[8 + (g8 & 3)], z1 = e1[8 + (g8 & 3)];
+      unsigned ah[4], al[4];
+      split_tf32_mul2(z0, make_float2(e0[4 + (g8 >> 2)], e0[6 + (g8 >> 2)]), ah, al);
+      split_tf32_mul2(z1, make_float2(e1[4 + (g8 >> 2)], e1[6 + (g8 >> 2)]), ah + 2, al + 2);
+      // B: column g8 = (x g8 >> 1, c g8 & 1) of entry j
+      const float x0 = e0[g8 >> 1], x1 = e1[g8 >> 1];
+#pragma unroll
+      for (int j = 0; j < E; ++j) {
+        unsigned bh[2], bl[2];
+        split_tf32_mul(e0[12 + 2 * j + (g8 & 1)], x0, bh[0], bl[0]);
+        split_tf32_mul(e1[12 + 2 * j + (g8 & 1)], x1, bh[1], bl[1]);
+        mma_split(D[j], ah, al, bh, bl);
+      }
+    }
+    c += kBC;
+    if (c >= cend) {  // the item's last chunk
+      const int ix = __shfl_sync(0xffffffffu, cs.desc.x, unit & 7), iw = __shfl_sync(0xffffffffu, cs.desc.w, unit & 7);
+      float bad = 0.f;  // NaN if any sum is not finite
+#pragma unroll
+      for (int j = 0; j < E; ++j)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) bad = fmaf(D[j][i], 0.f, bad);
+      if (__any_sync(0xffffffffu, !(bad == 0.f))) {
+        float again[E][4];
+        block_by_entry_n<E, NROW>(g, bentries, rows, vals, ncoil, __shfl_sync(0xffffffffu, cs.desc.y, unit & 7), cend, g8, t4,
+                                  again);
 #pragma unroll
         for (int j = 0; j < E; ++j)
-          *reinterpret_cast<float2*>(dst + (cell * E + j) * 2) = make_float2(D[j][2 * h], D[j][2 * h + 1]);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) D[j][i] = again[j][i];
       }
-    } else {
-      bn_store<E>(g, gridv, ncoil, it.x, g8, t4, D);
+      if (iw >= 0) {  // a part of a split block: its slot of the partial blocks, [cell][entry] complex
+        float* dst = partial + (long long)iw * 64 * 2 * E;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int cell = cell_index<3>(t4, (g8 >> 2) + 2 * h, g8 & 3);
+#pragma unroll
+          for (int j = 0; j < E; ++j)
+            *reinterpret_cast<float2*>(dst + (cell * E + j) * 2) = make_float2(D[j][2 * h], D[j][2 * h + 1]);
+        }
+      } else {  // one block, or a run of -iw empty ones
+        for (int b = 0; b < -iw; ++b) bn_store<E>(g, gridv, ncoil, ix + b, g8, t4, D);
+      }
+      if ((sizes & 255u) == 0) return;
+#pragma unroll
+      for (int j = 0; j < E; ++j)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) D[j][i] = 0.f;
+      ++unit;
+      c = __shfl_sync(0xffffffffu, cs.desc.y, unit & 7), cend = __shfl_sync(0xffffffffu, cs.desc.z, unit & 7);
     }
+    __syncwarp();  // the chunk has been read before its buffer is staged again
   }
 }
 
@@ -3652,7 +3784,7 @@ int launch_gather_any(const Geo& g, const tlgb_interp_plan_info* info, const cha
 template <int E, int NROW>
 int launch_adj_bn(const Geo& g, const tlgb_interp_plan_info* info, const char* P, const void* vals, void* grid,
                   void* scratch, cudaStream_t s) {
-  const size_t sm = 8 * kBC * kBSn * sizeof(float);
+  const size_t sm = kBWarps * kBStages * kBC * kBSn * sizeof(float);
   TLGB_TRY(set_smem(adj_bn_kernel<E, NROW>, sm));
   if (((uintptr_t)P & 15) || ((uintptr_t)scratch & 15))
     TLGB_FAIL(TLGB_ERR_INVALID, "interp adjoint: plan and scratch must be 16-byte aligned");
@@ -3660,8 +3792,8 @@ int launch_adj_bn(const Geo& g, const tlgb_interp_plan_info* info, const char* P
   // the work counter follows the partial blocks
   int* ctr = reinterpret_cast<int*>(static_cast<char*>(scratch) + blk_partial_bytes(info, 1, E));
   TLGB_CUDA(cudaMemsetAsync(ctr, 0, sizeof(int), s));
-  const int64_t nctas = std::min<int64_t>(cdiv(info->n_blk_items, 8), (int64_t)kBnCtas * sm_count());
-  adj_bn_kernel<E, NROW><<<(unsigned)std::max<int64_t>(nctas, 1), 256, sm, s>>>(
+  const int64_t nctas = std::min<int64_t>(cdiv(info->n_blk_items, kBWarps), (int64_t)kBnCtas * sm_count());
+  adj_bn_kernel<E, NROW><<<(unsigned)std::max<int64_t>(nctas, 1), kBWarps * 32, sm, s>>>(
       g, (const int4*)(P + info->off_blk_items), (int)info->n_blk_items, (const uint32_t*)(P + info->off_blk_entries),
       (const float*)(P + info->off_blk_rows), (const float2*)vals, (float*)grid, (float*)scratch, ctr);
   TLGB_CHECK_LAUNCH();
@@ -3685,7 +3817,7 @@ int launch_adj_b3(const Geo& g, const tlgb_interp_plan_info* info, const char* P
     }
   }
   const int64_t ncg = cdiv(g.nbatch, 8);
-  const size_t sm = 8 * kBC * kBS * sizeof(float);
+  const size_t sm = kBWarps * kBStages * kBC * kBS * sizeof(float);
   TLGB_TRY(set_smem(adj_b3_kernel<NDIM, NROW>, sm));
   // 16-byte asynchronous copies of the weight rows and transposed values
   if (((uintptr_t)P & 15) || ((uintptr_t)scratch & 15))
@@ -3703,15 +3835,20 @@ int launch_adj_b3(const Geo& g, const tlgb_interp_plan_info* info, const char* P
   } else {
     TLGB_CUDA(cudaMemsetAsync(ctr, 0, (size_t)ncg * sizeof(int), s));
   }
-  // persistent: kB3Ctas CTAs per SM (fewer when there are few items), any
-  // number of which may be resident at once
-  const int64_t nctas = std::min<int64_t>(cdiv(info->n_blk_items, 8), (int64_t)kB3Ctas * sm_count());
-  dim3 grd((unsigned)std::max<int64_t>(nctas, 1), (unsigned)ncg);
-  adj_b3_kernel<NDIM, NROW><<<grd, 256, sm, s>>>(g, (const int4*)(P + info->off_blk_items), (int)info->n_blk_items,
-                                          (const uint32_t*)(P + info->off_blk_entries),
-                                          (const float*)(P + info->off_blk_rows), (const float2*)vals, tv,
-                                          (float*)grid, (float*)scratch, ctr);
-  TLGB_CHECK_LAUNCH();
+  // persistent: kB3Ctas CTAs per SM (fewer when there are few units), any
+  // number of which may be resident at once; (group, item) units are counted
+  // in 32 bits, the tickets of all warps above their number included
+  const int64_t nitems = info->n_blk_items, max_ctas = (int64_t)kB3Ctas * sm_count();
+  const int64_t per = std::max<int64_t>(1, (((int64_t)1 << 31) - 1 - 16 * max_ctas) / std::max<int64_t>(nitems, 1));
+  for (int64_t cg0 = 0; cg0 < ncg; cg0 += per) {
+    const int64_t nunits = nitems * std::min(per, ncg - cg0);
+    const int64_t nctas = std::max<int64_t>(1, std::min(cdiv(nunits, kBWarps), max_ctas));
+    adj_b3_kernel<NDIM, NROW><<<(unsigned)nctas, kBWarps * 32, sm, s>>>(
+        g, (const int4*)(P + info->off_blk_items), (int)nitems, (int)nunits, (int)cg0, (int)ncg,
+        (const uint32_t*)(P + info->off_blk_entries), (const float*)(P + info->off_blk_rows), (const float2*)vals, tv,
+        (float*)grid, (float*)scratch, ctr + cg0);
+    TLGB_CHECK_LAUNCH();
+  }
   if (info->n_blk_split > 0) {
     dim3 g2((unsigned)info->n_blk_split, (unsigned)ncg);
     adj_reduce_b3_kernel<NDIM><<<g2, 256, 0, s>>>(g, (const int4*)(P + info->off_blk_split),
