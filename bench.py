@@ -348,11 +348,12 @@ def run_gpu(args, world, rank, local):
     plan = get_plan(locs, (N_GRID,) * 3, WIDTH, "kaiser_bessel", "circular", beta)
     torch.cuda.synchronize()
     plan_ms = (time.perf_counter() - t0) * 1e3
-    # per step: the gather, the point-major value transpose, the gridding and
-    # (when dense tiles are split) the ordered sum of their parts
+    # per step: the gather, (for points in random order) the sort of its
+    # results, the point-major value transpose, the gridding and (when dense
+    # blocks are split) the ordered sum of their parts
     blocks = plan.info.n_blk_items > 0  # 3D gridding on block lists
     n_split = plan.info.n_blk_split if blocks else plan.info.n_split_tiles
-    launches_per_step = 3 + (1 if n_split > 0 else 0)
+    launches_per_step = 3 + (1 if plan.call(True, N_COIL)[1] > 0 else 0) + (1 if n_split > 0 else 0)
 
     stream = torch.cuda.current_stream(dev)
     for _ in range(args.warmup):
@@ -754,7 +755,7 @@ def bench_one_coil(locs, dev, peak):
     Toeplitz kernel's single image): ungrid a 256^3 complex image at the 2^21
     points and grid the points back, each the mean of 10 CUDA-event timings
     with a 512 MB write between timings to flush L2 (the image alone is about
-    the size of L2). The 8-entry kernels run with the other 7 entries empty;
+    the size of L2). Both directions run on their one-entry kernels;
     the algorithmic bytes are one entry's grid and values plus the
     coordinates."""
     import torchlinops_gb300 as T

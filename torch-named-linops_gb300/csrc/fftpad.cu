@@ -77,12 +77,19 @@ __device__ __forceinline__ void split_index(long long v, long long vol, int n1, 
 // batch is cut into blockIdx.y runs (batch_runs) and kBatchAhead loads are
 // issued before the first store: 56 and 42 us, 6.1 and 6.4 TB/s.
 constexpr int kBatchAhead = 8;
+// With coil maps a pad reads its map and writes 1.95 times as much for each
+// entry, and more resident threads serve it better than more loads each: 8
+// coils on 160^3 take 83, 86, 87 and 97 us (with the call) at 1, 2, 4 and 8
+// ahead. The crop, whose coils are a sum, keeps 8: 32 coils on 320^2 take 22, 31,
+// 19 and 16 us, 8 coils on 160^3 63-68.
+constexpr int kMapsPadAhead = 1;
 
 // out[e][j] = maps[e % C][i] * apod[i] * x[e / C][i] for the source i of j, else 0
 template <bool MAPS>
 __global__ void __launch_bounds__(256) pad_shift_kernel(PadGeo G, const float2* __restrict__ x, long long nent, long long run,
                                                         const float* __restrict__ apod, const float2* __restrict__ maps,
                                                         int nmaps, float2* __restrict__ out) {
+  constexpr int AH = MAPS ? kMapsPadAhead : kBatchAhead;
   const long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= G.npvol) return;
   int j0, j1, j2;
@@ -98,10 +105,10 @@ __global__ void __launch_bounds__(256) pad_shift_kernel(PadGeo G, const float2* 
   const long long e0 = blockIdx.y * run, e1 = min(nent, e0 + run);
   long long b = MAPS ? e0 / nmaps : e0;
   int c = MAPS ? (int)(e0 - b * nmaps) : 0;
-  for (long long e = e0; e < e1; e += kBatchAhead) {
-    float2 v[kBatchAhead];
+  for (long long e = e0; e < e1; e += AH) {
+    float2 v[AH];
 #pragma unroll
-    for (int u = 0; u < kBatchAhead; ++u) {
+    for (int u = 0; u < AH; ++u) {
       v[u] = make_float2(0.f, 0.f);
       if (!in || e + u >= e1) continue;
       const float2 q = x[b * G.nvol + i];
@@ -113,7 +120,7 @@ __global__ void __launch_bounds__(256) pad_shift_kernel(PadGeo G, const float2* 
       }
     }
 #pragma unroll
-    for (int u = 0; u < kBatchAhead; ++u) {
+    for (int u = 0; u < AH; ++u) {
       if (e + u >= e1) break;
       out[(e + u) * G.npvol + j] = in && G.modulate ? cmul(v[u], md) : v[u];
     }
@@ -231,7 +238,7 @@ extern "C" int tlgb_pad_shift_c64(const void* x, int64_t nbatch, int32_t ndim, c
   if (!x || !out) TLGB_FAIL(TLGB_ERR_INVALID, "null pointer");
   const long long nent = (long long)nbatch * (maps ? nmaps : 1), ctas = cdiv(G.npvol, 256);
   dim3 grid((unsigned)ctas);
-  const long long run = batch_runs(ctas, nent, kBatchAhead, grid.y);
+  const long long run = batch_runs(ctas, nent, maps ? kMapsPadAhead : kBatchAhead, grid.y);
   (maps ? pad_shift_kernel<true> : pad_shift_kernel<false>)<<<grid, 256, 0, (cudaStream_t)stream>>>(
       G, (const float2*)x, nent, run, apod, (const float2*)maps, nmaps, (float2*)out);
   TLGB_CHECK_LAUNCH();

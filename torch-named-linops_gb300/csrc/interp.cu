@@ -850,12 +850,12 @@ __device__ __forceinline__ int axis_blocks(const Geo& g, int e, int st, int c, i
 // The plan is built on the device from start to end: the host reads the
 // lists' lengths back once, after the last launch. Pairs, items and splits
 // are counted per CTA, the CTAs' sums scanned, and emitted at their places,
-// so every list's order depends on the points alone. A build is 16 to 20
+// so every list's order depends on the points alone. A build is 16 to 30
 // short launches: bound by them up to about 10^5 points, by the pairs' bytes
 // (sorts, rows, records) above. Measured with the Python call around it:
-// 2^21 points of a dense-centre ball in 256^3 0.85 ms (about 5.5 ms with host-built
+// 2^21 points of a dense-centre ball in 256^3 1.0 ms (about 5.5 ms with host-built
 // item lists, read-backs between the stages and one-warp sort chunks of 2048
-// pairs), 2^18 in 160^3 0.28 ms (1.5 ms), 205,824 in 320^2 0.23 ms.
+// pairs), 2^18 in 160^3 0.32 ms (1.5 ms), 205,824 in 320^2 0.24 ms.
 constexpr int kPlanPts = 256;  // points (or work units) per CTA
 constexpr int kWinBits = 5;    // bits per tap count of a window
 
@@ -3130,7 +3130,7 @@ int make_geo(const tlgb_interp_desc* d, Geo& g) {
   if (d->norm != 1 && d->norm != 2) TLGB_FAIL(TLGB_ERR_INVALID, "norm must be 1 or 2");
   if (d->pad_mode != TLGB_PAD_CIRCULAR && d->pad_mode != TLGB_PAD_ZERO) TLGB_FAIL(TLGB_ERR_INVALID, "unknown pad mode");
   if (d->npts < 0 || d->nbatch < 0) TLGB_FAIL(TLGB_ERR_INVALID, "negative size");
-  // the 8-entry kernels launch one grid row per 8 batch entries (at most 65535)
+  // the value transpose and the sums of parts launch one grid row per 8 batch entries (at most 65535)
   if (d->nbatch > TLGB_INTERP_MAX_BATCH)
     TLGB_FAIL(TLGB_ERR_UNSUPPORTED, "batch above 524280 entries in one call: split the batch");
   memset(&g, 0, sizeof(g));
