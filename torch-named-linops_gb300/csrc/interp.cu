@@ -1358,7 +1358,7 @@ __device__ __forceinline__ float2 mul2_bcast(float s, float2 v) {
 // a warp per item); now the next chunk is copied during a chunk's products,
 // across items and groups, the splits and sums are packed two to an
 // instruction, whole blocks are stored without a check per cell, and values
-// are checked once per item: 610 and 671 us. Not faster: four lanes per entry
+// are checked once per item: 595 and 671 us. Not faster: four lanes per entry
 // (fewer lines per copy, 755 against 726 us at that stage), three or four
 // buffers, two or four row tiles' products interleaved.
 constexpr int kBC = 16;       // entries per chunk, two lanes per entry while staging
@@ -1533,7 +1533,13 @@ __device__ __forceinline__ void frag_store(const Geo& g, float* __restrict__ gri
 #pragma unroll
       for (int m = 0; m < 4; ++m)
 #pragma unroll
-        for (int h = 0; h < 2; ++h) q[m * sm + h * sh] = make_float2(D[m][nt][2 * h], D[m][nt][2 * h + 1]);
+        for (int h = 0; h < 2; ++h) {
+          // a grid larger than L2 leaves it early, before the rows and values
+          // that other blocks still need (256^3: 707 -> 688 us; 2D: no change)
+          const float2 v = make_float2(D[m][nt][2 * h], D[m][nt][2 * h + 1]);
+          if constexpr (NDIM == 3) __stcs(&q[m * sm + h * sh], v);
+          else q[m * sm + h * sh] = v;
+        }
     return;
   }
 #pragma unroll
