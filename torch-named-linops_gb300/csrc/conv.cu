@@ -51,8 +51,8 @@ __device__ __forceinline__ void cp_async16_zfill(uint32_t dst, const void* src, 
 // ---- the tcgen05 path of the forward / data gradient
 //
 // Persistent CTAs, two per SM: 4 epilogue warps, 4 loader warps and one warp
-// that issues the MMAs. A work unit is a column segment of up to kTcRows output
-// rows (fixed d, consecutive h) of 128 voxels along W (MMA M = 128). The input
+// that issues the MMAs. A work unit is a column segment of some output rows
+// (unit_rows) (fixed d, consecutive h) of 128 voxels along W (MMA M = 128). The input
 // rows (d + kd - 1, h'), kd = 0..2, contribute through their taps to the output
 // rows h' - 1, h', h' + 1: one MMA of N = 48 per (kd, kw), whose B operand holds
 // the weights of kh = 2, 1, 0 side by side, into the 128 x 48 FP32 accumulator
@@ -65,7 +65,7 @@ __device__ __forceinline__ void cp_async16_zfill(uint32_t dst, const void* src, 
 // layout is 16 bytes wide, 780 such rows per h'); tap kw is the A operand kw
 // rows into the slot. Accumulators sit in a ring of 5, so the epilogue of one
 // row overlaps the MMAs of the next. Weights stay in shared memory for the
-// CTA's lifetime. 128^3: 79 us (99 with 27 MMAs per row fed by TMA; 110 with one
+// CTA's lifetime. 128^3: 72 us (99 with 27 MMAs per row fed by TMA; 110 with one
 // CTA per SM, whose waits nothing covers; 54 without the copies, 33 with one
 // MMA per row and no copies or stores; HBM floor 20 us).
 // Every wait is bounded; a timeout sets the status word and a CTA flag, every
@@ -73,7 +73,6 @@ __device__ __forceinline__ void cp_async16_zfill(uint32_t dst, const void* src, 
 // freed.
 constexpr int kTcM = 128;
 constexpr int kTcHalo = kTcM + 2;
-constexpr int kTcRows = 16;                               // output rows per work unit
 constexpr int kTcHalfBytes = 2176;                        // >= 130 * 16, a multiple of 128
 constexpr int kTcRowBytes = 2 * kTcHalfBytes;
 constexpr int kTcSlotBytes = 3 * kTcRowBytes;             // the 3 kd rows of one h'
@@ -92,7 +91,7 @@ constexpr uint32_t kTcWait = 1u << 22;
 __device__ int g_conv_status;
 
 template <int MODE, bool OUTF32>
-__global__ void __launch_bounds__(kTcThreads, kTcCtas) conv3d_tc_kernel(int D, int H, int W, const uint4* __restrict__ x,
+__global__ void __launch_bounds__(kTcThreads, kTcCtas) conv3d_tc_kernel(int D, int H, int W, int rows, const uint4* __restrict__ x,
                                                                   const uint4* __restrict__ wts,
                                                                   const __nv_bfloat16* __restrict__ aux,
                                                                   void* __restrict__ y) {
@@ -107,7 +106,7 @@ __global__ void __launch_bounds__(kTcThreads, kTcCtas) conv3d_tc_kernel(int D, i
   uint32_t* slot = reinterpret_cast<uint32_t*>(drain + 1);  // [0] TMEM address, [1] failure flag
   volatile uint32_t* failed = slot + 1;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int ntw = (W + kTcM - 1) / kTcM, nseg = (H + kTcRows - 1) / kTcRows;
+  const int ntw = (W + kTcM - 1) / kTcM, nseg = (H + rows - 1) / rows;
   const long long nunits = (long long)D * ntw * nseg;
   if (warp == 0) {
     tmem_alloc(slot, kTcCols);
@@ -143,7 +142,7 @@ __global__ void __launch_bounds__(kTcThreads, kTcCtas) conv3d_tc_kernel(int D, i
   auto unit = [&](long long u, int& d, int& w0, int& h0, int& R) {
     const int hs = (int)(u % nseg);
     const long long dw = u / nseg;
-    w0 = (int)(dw % ntw) * kTcM, d = (int)(dw / ntw), h0 = hs * kTcRows, R = min(kTcRows, H - h0);
+    w0 = (int)(dw % ntw) * kTcM, d = (int)(dw / ntw), h0 = hs * rows, R = min(rows, H - h0);
   };
 
   if (warp >= 4 && warp < 8) {
@@ -284,8 +283,8 @@ __global__ void __launch_bounds__(kTcThreads, kTcCtas) conv3d_tc_kernel(int D, i
 }
 
 // Weight gradient: dW[t][co][ci] = sum over output voxels v of gy[v][co] *
-// x[v + offset(t)][ci]. A work unit is a column segment of up to kWgRows output
-// rows (fixed d, consecutive h) of 64 voxels along W; CTA b takes units b, b +
+// x[v + offset(t)][ci]. A work unit is a column segment of some output rows
+// (unit_rows) (fixed d, consecutive h) of 64 voxels along W; CTA b takes units b, b +
 // grid, ... (fixed), warp w the taps w, w + 4, ...; partial sums per CTA are
 // reduced in CTA order. The input rows (d + kd - 1, h') sit in a ring of 4
 // slots per kd: a new output row needs 3 new input rows and its gy row, copied
@@ -294,17 +293,17 @@ __global__ void __launch_bounds__(kTcThreads, kTcCtas) conv3d_tc_kernel(int D, i
 // bounds it now are the ldmatrix reads: 512 shared-memory wavefronts per row
 // of 64 voxels against 448 cycles of mma.sync.
 constexpr int kWgTapsPerWarp = 7;
-constexpr int kWgRows = 16;                                // output rows per unit
+constexpr int kWgCtas = 4 * 152;                           // 4 per SM
 constexpr int kWgRowBytes = kHaloW * kVoxBytes;            // one staged input row
 constexpr int kWgCopies = (3 * kHaloW * 2 + 127) / 128;    // 16-byte copies per thread for the 3 kd rows
 
-__global__ void __launch_bounds__(128, 4) conv3d_wgrad_kernel(int D, int H, int W, const uint4* __restrict__ x,
+__global__ void __launch_bounds__(128, 4) conv3d_wgrad_kernel(int D, int H, int W, int rows, const uint4* __restrict__ x,
                                                               const uint4* __restrict__ gy,
                                                               float* __restrict__ partial) {
   __shared__ __align__(128) unsigned char halo[3 * 4 * kWgRowBytes];  // [kd][slot][voxel][32 B]
   __shared__ __align__(128) unsigned char gsm[2 * kTileW * kVoxBytes];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int ntw = (W + kTileW - 1) / kTileW, nseg = (H + kWgRows - 1) / kWgRows;
+  const int ntw = (W + kTileW - 1) / kTileW, nseg = (H + rows - 1) / rows;
   const long long nunits = (long long)D * ntw * nseg;
   float acc[kWgTapsPerWarp][2][4];
 #pragma unroll
@@ -324,7 +323,7 @@ __global__ void __launch_bounds__(128, 4) conv3d_wgrad_kernel(int D, int H, int 
     const int hs = (int)(u % nseg);
     const long long dw = u / nseg;
     const int wt = (int)(dw % ntw), d = (int)(dw / ntw);
-    const int w0 = wt * kTileW, h0 = hs * kWgRows, h1 = min(H, h0 + kWgRows);
+    const int w0 = wt * kTileW, h0 = hs * rows, h1 = min(H, h0 + rows);
     // this thread's copies of an input row set: source (without the row) and slot offset
     long long xoff[kWgCopies];
     int soff[kWgCopies];
@@ -467,20 +466,38 @@ int check_conv(const tlgb_conv3d_desc* d) {
   return TLGB_OK;
 }
 
+// Output rows per work unit. A unit of R rows reads R + 2, and a persistent
+// grid takes cdiv(units, CTAs) units one after the other, so R is the one with
+// the least product: fixed units of 16 rows of 128^3 are 3.4 per CTA, whose last
+// round three CTAs in five sit out (72 row steps; 63 with 19 rows: 77 -> 72.5 us,
+// weight gradient 94 -> 91), and leave most SMs idle on small volumes.
+int unit_rows(long long planes, int H, long long ctas) {
+  int best = H;
+  long long least = cdiv(planes, ctas) * (H + 2);
+  for (int seg = 2; seg <= std::min(H, 256); ++seg) {
+    const int r = (int)cdiv(H, seg);
+    const long long steps = cdiv(planes * cdiv(H, r), ctas) * (r + 2);
+    if (steps < least) least = steps, best = r;
+  }
+  return best;
+}
+
 template <int MODE, bool OUTF32>
 int launch_conv_tc(const tlgb_conv3d_desc* d, const void* x, const void* w, const void* aux, void* y, cudaStream_t s) {
   auto* k = conv3d_tc_kernel<MODE, OUTF32>;
   TLGB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem));
-  const long long units = (long long)d->D * ((d->W + kTcM - 1) / kTcM) * ((d->H + kTcRows - 1) / kTcRows);
-  const unsigned grid = (unsigned)std::min<long long>(units, (long long)kTcCtas * sm_count());
-  k<<<grid, kTcThreads, kTcSmem, s>>>(d->D, d->H, d->W, (const uint4*)x, (const uint4*)w, (const __nv_bfloat16*)aux, y);
+  const long long planes = (long long)d->D * ((d->W + kTcM - 1) / kTcM), ctas = (long long)kTcCtas * sm_count();
+  const int rows = unit_rows(planes, d->H, ctas);
+  const unsigned grid = (unsigned)std::min<long long>(planes * cdiv(d->H, rows), ctas);
+  k<<<grid, kTcThreads, kTcSmem, s>>>(d->D, d->H, d->W, rows, (const uint4*)x, (const uint4*)w, (const __nv_bfloat16*)aux, y);
   TLGB_CHECK_LAUNCH();
   return TLGB_OK;
 }
 
-int wgrad_parts(const tlgb_conv3d_desc* d) {
-  const long long units = (long long)d->D * ((d->H + kWgRows - 1) / kWgRows) * ((d->W + kTileW - 1) / kTileW);
-  return (int)std::min<long long>(units, 4 * 152);  // 4 CTAs per SM
+int wgrad_parts(const tlgb_conv3d_desc* d, int* rows) {
+  const long long planes = (long long)d->D * ((d->W + kTileW - 1) / kTileW);
+  *rows = unit_rows(planes, d->H, kWgCtas);
+  return (int)std::min<long long>(planes * cdiv(d->H, *rows), kWgCtas);
 }
 
 }  // namespace
@@ -508,7 +525,8 @@ extern "C" int tlgb_conv3d_fwd(const tlgb_conv3d_desc* d, const void* x, const v
 extern "C" int tlgb_conv3d_wgrad_scratch_size(const tlgb_conv3d_desc* d, size_t* bytes) {
   TLGB_TRY(check_conv(d));
   if (!bytes) TLGB_FAIL(TLGB_ERR_INVALID, "null pointer");
-  *bytes = (size_t)wgrad_parts(d) * kTaps * 256 * sizeof(float);
+  int rows = 0;
+  *bytes = (size_t)wgrad_parts(d, &rows) * kTaps * 256 * sizeof(float);
   return TLGB_OK;
 }
 
@@ -522,8 +540,9 @@ extern "C" int tlgb_conv3d_wgrad(const tlgb_conv3d_desc* d, const void* x, const
   TLGB_TRY(tlgb_conv3d_wgrad_scratch_size(d, &need));
   if (scratch_bytes < need) TLGB_FAIL(TLGB_ERR_WORKSPACE, "conv3d wgrad scratch too small");
   cudaStream_t s = (cudaStream_t)stream;
-  const int parts = wgrad_parts(d);
-  conv3d_wgrad_kernel<<<parts, 128, 0, s>>>(d->D, d->H, d->W, (const uint4*)x, (const uint4*)gy, (float*)scratch);
+  int rows = 0;
+  const int parts = wgrad_parts(d, &rows);
+  conv3d_wgrad_kernel<<<parts, 128, 0, s>>>(d->D, d->H, d->W, rows, (const uint4*)x, (const uint4*)gy, (float*)scratch);
   TLGB_CHECK_LAUNCH();
   static_assert(kTaps * 256 % 32 == 0, "32 values per CTA");
   wgrad_reduce_kernel<<<kTaps * 256 / 32, 256, 0, s>>>((const float*)scratch, parts, dw);
