@@ -3734,7 +3734,11 @@ int launch_gather(const Geo& g, const tlgb_interp_plan_info* info, const char* P
   TLGB_TRY(set_smem(k, sm));
   const int64_t ncg = cdiv(g.nbatch, CG), items = info->n_fwd_items, ctas = (int64_t)CTAS * sm_count();
   int64_t run = ncg;
-  while (run > 1 && items * cdiv(ncg, run) < 6 * ctas) run = cdiv(run, 2);
+  // (item, run of groups) units go round the CTAs in turn, and items differ in
+  // points: 24 units per CTA even out what 6 do not (320^2 x 20 at width 6: 178
+  // -> 127 us; 320^2 x 256: 562 -> 526 us), at 48 the records' reloads show
+  // (ragged 3D x 12: 247 -> 326 us)
+  while (run > 1 && items * cdiv(ncg, run) < 24 * ctas) run = cdiv(run, 2);
   const int64_t nruns = cdiv(ncg, run), nunits = items * nruns;
   if (nunits >= (1ll << 31) - ctas) TLGB_FAIL(TLGB_ERR_UNSUPPORTED, "interp forward: too many points and batch entries in one call");
   k<<<(unsigned)std::min(nunits, ctas), NW * 32 + kGatherProd, sm, s>>>(
