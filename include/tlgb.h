@@ -117,7 +117,8 @@ typedef struct tlgb_interp_plan_info {
   int64_t n_home;         /* points with at least one valid tap (home pairs) */
   int64_t off_records;    /* byte offset of the per-point tap records, 0 = none */
   int64_t kernel_key;     /* kernel, norm and beta the records and rows were built for;
-                           * bit 52: the points are in no spatial order */
+                           * bit 52: the points are in no spatial order; bit 53: some
+                           * window has fewer taps than the gather's box of cells */
   /* Block lists of the 2D/3D gridding of complex batches (0 when the plan has
    * none): the (point, block) pairs of 4x4x4-cell (3D) or 8x8-cell (2D) output
    * blocks, sorted stably by block, and their work items (dense blocks are

@@ -33,6 +33,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <cfloat>
 #include <cmath>
 #include <cstring>
 #include <mutex>
@@ -2125,7 +2126,7 @@ constexpr int kGatherProd = 160;  // producer threads (a 12 x 12 plane of a 3D r
 template <int NDIM, int KT>
 struct __align__(16) GatherRec {
   float w[NDIM][KT];  // weights of the first KT valid taps per dim, zero beyond
-  unsigned view;      // region cell of the first tap | fast << 20 | ok << 21
+  unsigned view;      // region cell of the first tap | fast << 20 (at most KT taps per dim) | partial << 21 (fewer in some)
   int p;              // point index
   int pad[2];
 };
@@ -2165,7 +2166,8 @@ __device__ __forceinline__ void item_origin(const Geo& g, int tile, int (&o)[3])
 // plans also each point's place in that order (`rank`), and of every 16th
 // item's points (jumps[-1]) how many lie in another 32-byte sector of an output
 // row than the point before (jumps[0]: nearly all for points in random order,
-// a quarter in runs).
+// a quarter in runs). jumps[-2]: whether some window has fewer than KT taps in a
+// dim.
 template <int NDIM, int KT, bool FROM_ROWS>
 __global__ void __launch_bounds__(128) plan_records_kernel(Geo g, const uint32_t* __restrict__ cnt,
                                                            const int4* __restrict__ win,
@@ -2184,7 +2186,7 @@ __global__ void __launch_bounds__(128) plan_records_kernel(Geo g, const uint32_t
     const int p = entries[j];
     GatherRec<NDIM, KT> R;
     unsigned base = 0;
-    bool fast = true;
+    bool fast = true, partial = false;
     int4 w4;
     if constexpr (FROM_ROWS) w4 = win[p];
 #pragma unroll
@@ -2231,8 +2233,10 @@ __global__ void __launch_bounds__(128) plan_records_kernel(Geo g, const uint32_t
       // a home point's first tap lies in the tile
       base = base * S + (unsigned)(st - o[e]);
       fast = fast && c <= KT;
+      partial = partial || c < KT;
     }
-    R.view = (fast ? base : 0u) | ((fast ? 1u : 0u) << 20) | (1u << 21);
+    R.view = (fast ? base : 0u) | ((fast ? 1u : 0u) << 20) | ((partial ? 1u : 0u) << 21);
+    if (fast && partial) jumps[-2] = 1u;
     R.p = p;
     R.pad[0] = R.pad[1] = 0;
     const float4* src = reinterpret_cast<const float4*>(&R);
@@ -2296,7 +2300,12 @@ __device__ __forceinline__ void copy_region(const Geo& g, const float* __restric
   }
 }
 
-template <int NDIM, int KT, int CG, int NW, int NST, int CTAS>
+// PARTIAL: some window has fewer than KT taps in a dim. Its zero weights carry a
+// NaN or Inf of the box's cells past the window into the sum, so such results
+// are summed again over the valid taps. Plans without such windows (width 4 or 8
+// off the edges) leave the check out: it makes each step wait for its sums (256^3
+// x 8: 573 -> 580 us; 256 entries of 320^2: 50 us of a training step's 2.75 ms).
+template <int NDIM, int KT, int CG, int NW, int NST, int CTAS, bool PARTIAL>
 __global__ void __launch_bounds__(NW * 32 + kGatherProd, CTAS)
     gather_kernel(const __grid_constant__ CUtensorMap tmap, int use_tma, Geo g, const int4* __restrict__ items, int nruns,
                   int run, int nunits, const GatherRec<NDIM, KT>* __restrict__ recs, const float* __restrict__ locs,
@@ -2486,8 +2495,12 @@ __global__ void __launch_bounds__(NW * 32 + kGatherProd, CTAS)
           else
             out[((long long)(c0 + ent) * g.npts + p) * 2 + comp] = sum;
         }
-        // the step's points with more than KT taps in a dim, one at a time by the whole warp
-        unsigned rest = __ballot_sync(0xffffffffu, on && !fast);
+        // the step's points with more than KT taps in a dim (and those to sum
+        // again), one at a time by the whole warp
+        bool odd = !fast;
+        if constexpr (PARTIAL) odd = odd || (((view >> 21) & 1) && !(fabsf(sum) <= FLT_MAX));
+        const unsigned again = __ballot_sync(0xffffffffu, on && odd);
+        unsigned rest = again;
         while (rest) {
           const int hh = (__ffs(rest) - 1) / (4 * CL);
           rest &= ~(((1u << (4 * CL)) - 1u) << (4 * CL * hh));
@@ -2534,7 +2547,9 @@ __global__ void __launch_bounds__(NW * 32 + kGatherProd, CTAS)
             v2.x += __shfl_xor_sync(0xffffffffu, v2.x, m);
             v2.y += __shfl_xor_sync(0xffffffffu, v2.y, m);
           }
-          if (lane < CG && c0 + lane < g.nbatch && TLGB_IN_RANGE(Q.p, g.npts))
+          // only entries with a flagged component: in lanes 4 (e % CL) + 2 (e / CL) and one on from the point's first
+          const bool mine = !PARTIAL || ((again >> ((4 * CL * hh + 4 * (lane % CL) + 2 * (lane / CL)) & 31)) & 3);
+          if (lane < CG && mine && c0 + lane < g.nbatch && TLGB_IN_RANGE(Q.p, g.npts))
             *reinterpret_cast<float2*>(sorted ? sorted + (((long long)cg * g.npts + it.w + base + hh) * CG + lane) * 2
                                               : out + ((long long)(c0 + lane) * g.npts + Q.p) * 2) = v2;
           __syncwarp();
@@ -3211,6 +3226,8 @@ int64_t max_tiles_per_dim(const Geo& g, int e) {
 
 // in kernel_key: most points' outputs lie in another sector than the point's before
 constexpr int64_t kScattered = (int64_t)1 << 52;
+// in kernel_key: some window has fewer taps in a dim than its gather record holds
+constexpr int64_t kPartial = (int64_t)1 << 53;
 
 // The kernel, norm and beta a plan's records hold weights for
 int64_t kernel_key(const Geo& g) {
@@ -3398,7 +3415,7 @@ int check_plan(const Geo& g, const tlgb_interp_plan_info* info, const void* plan
   for (int e = 0; e < 3; ++e)
     if (info->tile[e] != g.T[e] || info->n_tile[e] != g.nt[e])
       TLGB_FAIL(TLGB_ERR_INVALID, "plan was built for another grid");
-  if (((info->off_records > 0 && records_ok(g)) || info->n_blk_items > 0) && (info->kernel_key & ~kScattered) != kernel_key(g))
+  if (((info->off_records > 0 && records_ok(g)) || info->n_blk_items > 0) && (info->kernel_key & ~(kScattered | kPartial)) != kernel_key(g))
     TLGB_FAIL(TLGB_ERR_INVALID, "plan was built for another kernel, norm or beta (its tap weights are stored)");
   return TLGB_OK;
 }
@@ -3605,6 +3622,7 @@ extern "C" int tlgb_interp_plan_build(const tlgb_interp_desc* d, const float* lo
   info->off_records = L.off_recs;
   info->kernel_key = L.off_recs > 0 || blocks ? kernel_key(g) : 0;
   if (2ll * c[15] > (int64_t)c[14]) info->kernel_key |= kScattered;
+  if (c[13]) info->kernel_key |= kPartial;
   info->n_home = c[2];
   if (blocks) {
     info->n_blk_entries = c[1];
@@ -3730,7 +3748,9 @@ int launch_gather(const Geo& g, const tlgb_interp_plan_info* info, const char* P
   CUtensorMap tmap;
   const int use_tma = region_map(g, grid, region_edge<NDIM, KT>(), CG, tmap);
   constexpr size_t sm = gather_smem<NDIM, KT, CG, NW, NST>();
-  auto* k = gather_kernel<NDIM, KT, CG, NW, NST, CTAS>;
+  auto* k = gather_kernel<NDIM, KT, CG, NW, NST, CTAS, true>;
+  if constexpr (KT == 4)  // the check costs nothing at KT = 8
+    if (!(info->kernel_key & kPartial)) k = gather_kernel<NDIM, KT, CG, NW, NST, CTAS, false>;
   TLGB_TRY(set_smem(k, sm));
   const int64_t ncg = cdiv(g.nbatch, CG), items = info->n_fwd_items, ctas = (int64_t)CTAS * sm_count();
   int64_t run = ncg;
