@@ -9,6 +9,7 @@ from conftest import rel_l2
 from oracle import interp as OI
 
 import torchlinops_gb300 as T
+from torchlinops_gb300 import interp
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -53,3 +54,22 @@ def test_ungrid(shape, width, pad, nb):
         finite = torch.isfinite(torch.view_as_real(got[-1])).all(-1)
         assert torch.equal(finite, ~hit)
         assert rel_l2(got[-1][~hit], good[-1][~hit]) < TOL
+
+
+@pytest.mark.parametrize("shape", SHAPES_2D)
+@pytest.mark.parametrize("width", [2.0, 3.0, 3.5, 4.0])
+@pytest.mark.parametrize("pad", ["circular", "zero"])
+@pytest.mark.parametrize("nb", [1, 3, 9, 40])
+def test_trajectory_gradient(shape, width, pad, nb):
+    for cell, value in zip(_cells(shape), (complex(float("nan"), 1.0), complex(2.0, float("-inf")))):
+        locs, img, kp, hit = _case(shape, width, pad, nb, cell)
+        gen = torch.Generator().manual_seed(nb)
+        a = torch.complex(torch.randn(nb, len(locs), generator=gen), torch.randn(nb, len(locs), generator=gen)).to(DEV)
+        img[(nb - 1, *cell)] = 0
+        args = (a, locs.to(DEV), width, "kaiser_bessel", 1, pad, kp)
+        good = interp._grad_locs(img.to(DEV), *args).cpu()
+        img[(nb - 1, *cell)] = value
+        got = interp._grad_locs(img.to(DEV), *args).cpu()
+        finite = torch.isfinite(got).all(-1)
+        assert torch.equal(finite, ~hit)
+        assert torch.equal(got[~hit], good[~hit])  # the same sums without the cell

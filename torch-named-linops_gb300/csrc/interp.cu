@@ -3024,6 +3024,7 @@ __global__ void __launch_bounds__(kGradWarps * 32 + kGatherProd, 1)
       const int d = (lane >> 3) & 1, kk = lane & 7, e = 1 + d;
       if (kk < 4) dw[4 * d + kk] = 0.f;
       __syncwarp();
+      int ny, nz;  // the window's taps per dim: sums of cells past it may be NaN or Inf and are left out
       {
         Tap t;
         t.valid = false;
@@ -3034,13 +3035,15 @@ __global__ void __launch_bounds__(kGradWarps * 32 + kGatherProd, 1)
         const unsigned m = (__ballot_sync(0xffffffffu, t.valid) >> (lane & 24)) & 255u;
         const int q = kk - (__ffs(m) - 1);
         if (t.valid && q < 4) dw[4 * d + q] = kern_deriv(g.kernel, t.d, g.beta) / g.r[e];
+        ny = __shfl_sync(0xffffffffu, __popc(m), lane & 16), nz = __shfl_sync(0xffffffffu, __popc(m), (lane & 16) | 8);
       }
       __syncwarp();
       float ry = 0.f, rz = 0.f;
 #pragma unroll
       for (int t = 0; t < 4; ++t) {
-        ry = fmaf(dw[kyo[t]], sum[st][t], ry);
-        rz = fmaf(R.w[0][kyo[t]], sum[st][t], rz);
+        const float v = kyo[t] < ny && kz < nz ? sum[st][t] : 0.f;
+        ry = fmaf(dw[kyo[t]], v, ry);
+        rz = fmaf(R.w[0][kyo[t]], v, rz);
       }
       ry *= R.w[1][kz];
       rz *= dw[4 + kz];
