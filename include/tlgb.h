@@ -64,8 +64,10 @@ int tlgb_device_status(int32_t* status, int32_t clear);
  * and the 2D trajectory gradient without their copies, and those
  * kernels poll the copy's mbarrier once: the wait runs out with nothing in
  * flight, the kernel sets status bit 1 and its CTAs return, leaving the
- * output incomplete. Returns the previous setting. For tests of
- * tlgb_device_status only; no counterpart in the reference. */
+ * output incomplete. With 2 the copies are made and the waits for them give
+ * up at once: the CTAs then end when their copies have landed. Returns the
+ * previous setting. For tests of tlgb_device_status only; no counterpart in
+ * the reference. */
 int tlgb_test_skip_region_copy(int32_t on);
 
 /* ------------------------------------------------------------------------ */

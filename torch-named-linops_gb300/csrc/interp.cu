@@ -69,7 +69,10 @@ struct Geo {
   long long npts, nbatch;
   int wrap_safe;  // every active N >= NT: a window never overlaps itself
   long long tv_off;  // gridding: byte offset in scratch of the point-major values, -1 = none
-  int skip_copy;     // test hook (tlgb_test_skip_region_copy): TMA kernels skip their region copy
+  // test hook of the gather and the 2D gradient (tlgb_test_skip_region_copy): 1 = nothing is copied and the
+  // consumers' waits run out, 2 = they run out while copies are under way
+  int skip_copy;
+  uint32_t wait;     // polls of the consumers' bounded waits, kWaitLimit without the hook
   int nrow;          // block lists: blocks a window can meet per dim (2 or 3), 0 = no block lists
 };
 
@@ -2119,8 +2122,10 @@ __global__ void __launch_bounds__(256) adj_reduce_bn_kernel(Geo g, const int4* _
 // apart (the same banks), so lane group l reads its y taps from row l & 3 on:
 // one load of a half-warp then spans all banks.
 // Every wait is bounded: on a timeout the warp sets the device status and a
-// CTA flag and returns, the producer waits (bounded) for its copies in flight.
+// CTA flag and returns; the producers always end with their copies landed.
 constexpr int kGatherPts = 256;
+constexpr uint32_t kWaitLimit = 1u << 22;   // polls of a bounded wait, each of some microseconds at most
+constexpr uint32_t kDrainLimit = 1u << 18;  // for copies in flight at a producer's end: about a second
 constexpr int kGatherProd = 160;  // producer threads (a 12 x 12 plane of a 3D region takes 144)
 
 template <int NDIM, int KT>
@@ -2257,6 +2262,18 @@ __global__ void __launch_bounds__(128) plan_records_kernel(Geo g, const uint32_t
   }
 }
 
+// The end of a producer thread, whether it has issued every copy or given up:
+// nothing that it started is in flight when the CTA ends. A consumer whose wait
+// ran out returns at once, and the CTA's shared memory may be another's next. In
+// a pass without a failure the copies have landed or are about to.
+__device__ __forceinline__ void producer_drain(uint64_t* full, uint32_t stages, uint32_t nst, uint64_t* rfull,
+                                               uint32_t recs_sent, int pt) {
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  if (pt != 0) return;
+  for (uint32_t i = stages > nst ? stages - nst : 0; i < stages; ++i) mbar_wait_bounded(&full[i % nst], (i / nst) & 1, kDrainLimit);
+  for (uint32_t i = recs_sent > 2 ? recs_sent - 2 : 0; i < recs_sent; ++i) mbar_wait_bounded(&rfull[i & 1], (i >> 1) & 1, kDrainLimit);
+}
+
 // A region by asynchronous 8-byte copies of the producer threads, wrapped or
 // zero-filled: a thread copies its (y, z) cells of every (entry, x) plane.
 template <int NDIM, int KT, int CG>
@@ -2336,14 +2353,14 @@ __global__ void __launch_bounds__(NW * 32 + kGatherProd, CTAS)
     failed = 0;
   }
   __syncthreads();
-  const uint32_t limit = g.skip_copy ? 1u : 1u << 22;  // test hook: nothing is copied, so the waits run out
+  const uint32_t limit = g.wait;
   const int ncg = (int)((g.nbatch + CG - 1) / CG);
   volatile int* vfailed = &failed;
   if (warp >= NW) {
     // ---- producers
-    if (g.skip_copy) return;
+    if (g.skip_copy == 1) return;
     const int pt = tid - NW * 32;
-    uint32_t k = 0, u_done = 0;
+    uint32_t k = 0, u_done = 0, recs_sent = 0;  // stages, units, record copies begun (thread 0)
     bool ok = true;
     int4 next = blockIdx.x < nunits ? items[blockIdx.x / nruns] : make_int4(0, 0, 0, 0);
     for (int u = blockIdx.x; u < nunits && ok; u += gridDim.x, ++u_done) {
@@ -2357,16 +2374,17 @@ __global__ void __launch_bounds__(NW * 32 + kGatherProd, CTAS)
       const bool tma = use_tma && !wraps;
       if (pt == 0) {
         const uint32_t b = u_done & 1;
-        ok = mbar_wait_bounded(&rempty[b], ((u_done >> 1) & 1) ^ 1, limit);
+        ok = mbar_wait_bounded(&rempty[b], ((u_done >> 1) & 1) ^ 1, kWaitLimit);
         if (ok) {
           const uint32_t bytes = (uint32_t)(it.z - it.y) * (uint32_t)sizeof(Rec);
           mbar_arrive_expect_tx(&rfull[b], bytes);
           sm100::bulk_load(recbuf + b * kGatherPts, recs + it.w, bytes, &rfull[b]);
+          ++recs_sent;
         }
       }
       for (int cg = g0; cg < g1 && ok; ++cg, ++k) {
         const uint32_t s = k % NST;
-        ok = mbar_wait_bounded(&empty[s], ((k / NST) & 1) ^ 1, limit) && !*vfailed;
+        ok = mbar_wait_bounded(&empty[s], ((k / NST) & 1) ^ 1, kWaitLimit) && !*vfailed;
         if (!ok) break;
         float2* reg = reinterpret_cast<float2*>(smem + s * RBYTES);
         if (tma) {
@@ -2384,15 +2402,11 @@ __global__ void __launch_bounds__(NW * 32 + kGatherProd, CTAS)
       }
       ok = ok && !*vfailed;
     }
-    if (!ok) {  // every copy lands before the CTA ends
-      asm volatile("cp.async.wait_all;" ::: "memory");
-      if (pt == 0) {
-        *vfailed = 1;
-        atomicExch(&g_tlgb_status, 1);
-        for (uint32_t i = k > NST ? k - NST : 0; i < k; ++i) mbar_wait_bounded(&full[i % NST], (i / NST) & 1, limit);
-        for (uint32_t i = u_done > 1 ? u_done - 1 : 0; i <= u_done; ++i) mbar_wait_bounded(&rfull[i & 1], (i >> 1) & 1, 1u << 12);
-      }
+    if (!ok && pt == 0) {
+      *vfailed = 1;
+      atomicExch(&g_tlgb_status, 1);
     }
+    producer_drain(full, k, NST, rfull, recs_sent, pt);
     return;
   }
   // ---- consumers
@@ -2830,14 +2844,14 @@ __global__ void __launch_bounds__(kGradWarps * 32 + kGatherProd, 1)
     failed = 0;
   }
   __syncthreads();
-  const uint32_t limit = g.skip_copy ? 1u : 1u << 22;  // test hook: nothing is copied, so the waits run out
+  const uint32_t limit = g.wait;
   const int ncg = (int)((g.nbatch + 7) / 8);
   volatile int* vfailed = &failed;
   if (warp >= NW) {
     // ---- producers
-    if (g.skip_copy) return;
+    if (g.skip_copy == 1) return;
     const int pt = tid - NW * 32;
-    uint32_t k = 0, ui = 0;
+    uint32_t k = 0, ui = 0, recs_sent = 0;  // stages, units, record copies begun (thread 0)
     bool ok = true;
     int4 next = items[blockIdx.x / nruns];
     for (int u = blockIdx.x; u < nunits && ok; u += gridDim.x, ++ui) {
@@ -2850,17 +2864,18 @@ __global__ void __launch_bounds__(kGradWarps * 32 + kGatherProd, 1)
       const bool tma = use_tma && !wraps;
       const Rec* rec = recbuf + (ui & 1) * kGatherPts;
       if (pt == 0) {
-        ok = mbar_wait_bounded(&rempty[ui & 1], ((ui >> 1) & 1) ^ 1, limit);
+        ok = mbar_wait_bounded(&rempty[ui & 1], ((ui >> 1) & 1) ^ 1, kWaitLimit);
         if (ok) {
           const uint32_t bytes = (uint32_t)npt * (uint32_t)sizeof(Rec);
           mbar_arrive_expect_tx(&rfull[ui & 1], bytes);
           sm100::bulk_load(recbuf + (ui & 1) * kGatherPts, recs + it.w, bytes, &rfull[ui & 1]);
+          ++recs_sent;
         }
       }
-      ok = ok && mbar_wait_bounded(&rfull[ui & 1], (ui >> 1) & 1, limit);
+      ok = ok && mbar_wait_bounded(&rfull[ui & 1], (ui >> 1) & 1, kWaitLimit);
       for (int cg = g0; cg < g1 && ok; ++cg, ++k) {
         const uint32_t s = k % NST;
-        ok = mbar_wait_bounded(&empty[s], ((k / NST) & 1) ^ 1, limit) && !*vfailed;
+        ok = mbar_wait_bounded(&empty[s], ((k / NST) & 1) ^ 1, kWaitLimit) && !*vfailed;
         if (!ok) break;
         float2* reg = reinterpret_cast<float2*>(smem + s * kGradStage);
         float2* av = reinterpret_cast<float2*>(smem + s * kGradStage + kGradRegion);
@@ -2885,15 +2900,11 @@ __global__ void __launch_bounds__(kGradWarps * 32 + kGatherProd, 1)
       }
       ok = ok && !*vfailed;
     }
-    if (!ok) {  // every copy lands before the CTA ends
-      asm volatile("cp.async.wait_all;" ::: "memory");
-      if (pt == 0) {
-        *vfailed = 1;
-        atomicExch(&g_tlgb_status, 1);
-        for (uint32_t i = k > NST ? k - NST : 0; i < k; ++i) mbar_wait_bounded(&full[i % NST], (i / NST) & 1, limit);
-        for (uint32_t i = ui > 1 ? ui - 1 : 0; i <= ui; ++i) mbar_wait_bounded(&rfull[i & 1], (i >> 1) & 1, 1u << 12);
-      }
+    if (!ok && pt == 0) {
+      *vfailed = 1;
+      atomicExch(&g_tlgb_status, 1);
     }
+    producer_drain(full, k, NST, rfull, recs_sent, pt);
     return;
   }
   // ---- consumers: lane = (point h of a step, entry c and c + 4, z tap kz)
@@ -3159,6 +3170,7 @@ int make_geo(const tlgb_interp_desc* d, Geo& g) {
     TLGB_FAIL(TLGB_ERR_UNSUPPORTED, "batch above 524280 entries in one call: split the batch");
   memset(&g, 0, sizeof(g));
   g.skip_copy = g_test_skip_copy.load();
+  g.wait = g.skip_copy ? 2u - g.skip_copy : kWaitLimit;
   g.ndim = d->ndim;
   const int off = 3 - d->ndim;
   int maxnt = 1;
@@ -4179,7 +4191,7 @@ extern "C" int tlgb_interp_adjoint_fixed(const tlgb_interp_desc* d, const tlgb_i
 }
 
 extern "C" int tlgb_test_skip_region_copy(int32_t on) {
-  return tlgb::g_test_skip_copy.exchange(on ? 1 : 0);
+  return tlgb::g_test_skip_copy.exchange(on == 2 ? 2 : (on ? 1 : 0));
 }
 
 extern "C" int tlgb_device_status(int32_t* status, int32_t clear) {
