@@ -3450,34 +3450,12 @@ CtxGetCurrentFn ctx_get_current() {
   return fn;
 }
 
-// A kernel's shared-memory limit and carveout, set once per CUDA context (the
-// attributes belong to the context's module; two calls of about 2 us each on
-// every launch otherwise) and again when a launch needs more.
+// A kernel's shared-memory limit and carveout, set before every launch: they
+// belong to the current context's module, so a remembered setting would have to
+// know of every context's end. A call takes 0.2 us; 48 KB need no limit set.
 int set_smem(const void* kernel, size_t bytes) {
-  struct Entry {
-    CUcontext ctx;
-    const void* kernel;
-    size_t bytes;
-  };
-  static std::mutex mu;
-  static std::vector<Entry> known;
-  CUcontext ctx = nullptr;
-  CtxGetCurrentFn get = ctx_get_current();
-  const bool keyed = get && get(&ctx) == CUDA_SUCCESS && ctx;
-  std::lock_guard<std::mutex> lock(mu);
-  if (keyed)
-    for (const Entry& e : known)
-      if (e.kernel == kernel && e.ctx == ctx && e.bytes >= bytes) return TLGB_OK;
-  TLGB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  if (bytes > 48 * 1024) TLGB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
   TLGB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-  if (!keyed) return TLGB_OK;
-  for (Entry& e : known)
-    if (e.kernel == kernel && e.ctx == ctx) {
-      e.bytes = bytes;
-      return TLGB_OK;
-    }
-  if (known.size() >= 1024) known.clear();  // contexts come and go in a long-lived host
-  known.push_back({ctx, kernel, bytes});
   return TLGB_OK;
 }
 template <typename F>
