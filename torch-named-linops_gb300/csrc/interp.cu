@@ -3452,9 +3452,9 @@ CtxGetCurrentFn ctx_get_current() {
 
 // A kernel's shared-memory limit and carveout, set before every launch: they
 // belong to the current context's module, so a remembered setting would have to
-// know of every context's end. A call takes 0.2 us; 48 KB need no limit set.
+// know of every context's end. A call takes 0.2 us.
 int set_smem(const void* kernel, size_t bytes) {
-  if (bytes > 48 * 1024) TLGB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  TLGB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
   TLGB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
   return TLGB_OK;
 }
