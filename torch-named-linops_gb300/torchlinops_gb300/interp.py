@@ -79,13 +79,19 @@ def _width_tuple(width, ndim: int) -> tuple[float, ...]:
     return width
 
 
+def _check_norm(norm) -> None:
+    if norm not in (1, 2):
+        raise ValueError(f"Unexpected norm: {norm}.")
+    if not isinstance(norm, int):
+        raise TypeError(f"norm must be an int, got {type(norm).__name__}")
+
+
 def _desc(ndim, grid_size, width, kernel, norm, pad_mode, beta, is_complex, nbatch, npts) -> _ext.InterpDesc:
     if kernel not in _ext.KERNELS:
         raise ValueError(f"Unrecognized kernel type: {kernel}")
     if pad_mode not in _ext.PAD_MODES:
         raise ValueError(f"Unrecognized padding mode: {pad_mode}")
-    if norm not in (1, 2):
-        raise ValueError(f"Unexpected norm: {norm}.")
+    _check_norm(norm)
     d = _ext.InterpDesc()
     d.ndim = ndim
     d.kernel = _ext.KERNELS[kernel]
@@ -295,6 +301,7 @@ def ungrid(
     npts = prod(locs_batch_shape)
     width = _width_tuple(width, ndim)
     is_complex = _check_values(vals)
+    _check_norm(norm)  # a plan is looked up by int(norm)
     beta = kernel_params["beta"] if kernel == "kaiser_bessel" else 1.0
     plan = get_plan(locs, grid_size, width, kernel, pad_mode, beta, norm)
     out = torch.empty((*batch_shape, *locs_batch_shape), dtype=vals.dtype, device=dev)
@@ -354,6 +361,7 @@ def grid(
     nbatch = prod(batch_shape)
     width = _width_tuple(width, ndim)
     is_complex = _check_values(vals)
+    _check_norm(norm)  # a plan is looked up by int(norm)
     beta = kernel_params["beta"] if kernel == "kaiser_bessel" else 1.0
     plan = get_plan(locs, grid_size, width, kernel, pad_mode, beta, norm)
     L = _ext.lib()
