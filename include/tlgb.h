@@ -193,7 +193,9 @@ int tlgb_interp_adjoint(const tlgb_interp_desc* d, const tlgb_interp_plan_info* 
  * it is loaded on until the process exits. The caller still provides the
  * plan, the inputs and the output.
  *  - A plan whose partial tiles alone need more than the buffer is rejected
- *    with TLGB_ERR_WORKSPACE before anything is launched. The point-major
+ *    with TLGB_ERR_WORKSPACE before anything is launched. A plan whose partial
+ *    blocks do not fit, but whose partial tiles do, is gridded tile by tile
+ *    (slower, and equal up to the order of the sums). The point-major
  *    copy of the values is made only when it fits beside them; otherwise
  *    the values are read in place (same result, bit for bit).
  *  - The first call in each CUDA context (the primary context of a device,
