@@ -3980,7 +3980,8 @@ template <typename V, int NORM>
 int launch_grad(const Geo& g, const tlgb_interp_plan_info* info, const char* P, const float* locs, const void* grid,
                 const void* a, float* grad, void* scratch, size_t scratch_bytes, cudaStream_t s) {
   if constexpr (std::is_same<V, float2>::value && NORM == 1)
-    if (grad_on_ring(g, info)) return launch_grad2(g, info, P, locs, grid, a, grad, scratch, scratch_bytes, s);
+    if (grad_on_ring(g, info) && ((uintptr_t)grad & 7) == 0)  // it stores a point's two components together
+      return launch_grad2(g, info, P, locs, grid, a, grad, scratch, scratch_bytes, s);
   const int cg = grad_cg(g, sizeof(PTaps<true>));
   const size_t sm = grad_smem(g, cg, sizeof(PTaps<true>)) + kFwdChunk * 3 * sizeof(float);
   auto* k = interp_grad_kernel<V, NORM>;
