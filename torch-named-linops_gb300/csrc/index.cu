@@ -135,15 +135,127 @@ struct Acc<double2> {
 // single loads, 143 with eight entries per chain, 104 us now.
 constexpr int kAdjChunk = 256;  // samples in shared memory
 // Resident CTAs, by registers: 104 us with 4, 124 and 143 with 5 and 6, which spill
-constexpr int adj_ctas(size_t bytes, int entries) { return (entries == 1 ? 8 : 4) / (bytes > 8 ? 2 : 1); }
+constexpr int adj_ctas(size_t bytes, int entries) { return entries == 1 ? (bytes > 8 ? 4 : 8) : (bytes > 8 ? 3 : 4); }
+
+// One cell's samples, a run of perm, in order; K values are read ahead of adding
+// them. Whole groups of K go without checks, which kept the loads from overlapping
+// (2^22 samples in 512 cells of 160^3: 2.3 ms, 1.4 without).
+template <typename T, int K>
+__device__ __forceinline__ T cell_sum(const T* __restrict__ vb, const int32_t* __restrict__ perm, uint32_t k0, uint32_t k1) {
+  Acc<T> a;
+  T v[K];
+  uint32_t k = k0;
+  for (; k1 - k >= K; k += K) {  // whole groups: nothing to check between the loads
+#pragma unroll
+    for (int i = 0; i < K; ++i) v[i] = vb[perm[k + i]];
+#pragma unroll
+    for (int i = 0; i < K; ++i) a.add(v[i]);
+  }
+  if (k < k1) {
+#pragma unroll
+    for (int i = 0; i < K - 1; ++i)
+      if (k + i < k1) v[i] = vb[perm[k + i]];
+#pragma unroll
+    for (int i = 0; i < K - 1; ++i)
+      if (k + i < k1) a.add(v[i]);
+  }
+  return a.v;
+}
+
+// The cells [first, last) of a CTA where samples crowd into few of
+// them, as around a trajectory's centre: light cells by their own threads, and the
+// crowded ones, when they are at most kCrowdPerWarp for each warp, by a warp each.
+// Its lanes fetch 64 samples' values of U entries ahead, and lane u adds entry u's
+// from shared memory, 32 at a time, in order: 15 cycles a sample against 200 of a
+// thread's chain, which is why more crowded cells than that are left to their
+// threads. 2^21 samples in 512 cells of 160^3, 2 entries: 0.94 ms (12.3 ms when the
+// staged chunks of such a run were added by one lane after the other, 3.1 ms as
+// chains of single loads).
+constexpr uint32_t kCrowded = 256;  // samples
+constexpr int kCrowdPerWarp = 12;
+template <typename T, int U>
+struct CrowdShared {
+  T v[8][U][33];
+  int list[kCrowdPerWarp * 8];
+  int n;
+};
+
+template <typename T, int U>
+__device__ __noinline__ void crowded_cells(const T* __restrict__ vals, const int32_t* __restrict__ perm,
+                                           const uint32_t* __restrict__ off, T* __restrict__ out, int64_t npts, int64_t ncells,
+                                           int64_t nbatch, int64_t first, int64_t last, CrowdShared<T, U>& sm) {
+  constexpr int NT = 256, W = 8;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (tid == 0) sm.n = 0;
+  __syncthreads();
+  for (int64_t c = first + tid; c < last; c += NT)
+    if (off[c + 1] - off[c] > kCrowded) {  // in any order: a cell's sum is its own
+      const int i = atomicAdd(&sm.n, 1);
+      if (i < kCrowdPerWarp * W) sm.list[i] = (int)(c - first);
+    }
+  __syncthreads();
+  const int n = sm.n <= kCrowdPerWarp * W ? sm.n : 0;
+  const uint32_t light = n > 0 ? kCrowded : 0xffffffffu;
+  for (int64_t b = (int64_t)blockIdx.y * U; b < nbatch; b += (int64_t)gridDim.y * U) {
+    for (int64_t e = b; e < min(nbatch, b + U); ++e)
+#pragma unroll 1
+      for (int64_t c = first + tid; c < last; c += NT)
+        if (off[c + 1] - off[c] <= light) __stcs(&out[e * ncells + c], cell_sum<T, 8>(vals + e * npts, perm, off[c], off[c + 1]));
+    for (int i = warp; i < n; i += W) {
+      const int64_t c = first + sm.list[i];
+      const uint32_t k0 = off[c], k1 = off[c + 1];
+      T v[2][U];
+      auto fetch = [&](T (&d)[U], uint32_t k) {
+        if (k + lane >= k1) return;
+        const int64_t m = perm[k + lane];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          if (b + u < nbatch) d[u] = vals[(b + u) * npts + m];
+      };
+      Acc<T> a;  // of entry b + lane
+      fetch(v[0], k0);
+      fetch(v[1], k0 + 32);
+      for (uint32_t k = k0; k < k1; k += 64)
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          if (k + 32 * q >= k1) break;
+          __syncwarp();  // the 32 before have been added
+#pragma unroll
+          for (int u = 0; u < U; ++u) sm.v[warp][u][lane] = v[q][u];
+          __syncwarp();
+          if (k1 - k > 64 + 32 * q) fetch(v[q], k + 64 + 32 * q);
+          if (lane < U) {
+            const T* r = sm.v[warp][lane];
+            const uint32_t len = k1 - k - 32 * q;
+            if (len >= 32) {
+#pragma unroll
+              for (int j = 0; j < 32; ++j) a.add(r[j]);
+            } else {
+              for (uint32_t j = 0; j < len; ++j) a.add(r[j]);
+            }
+          }
+        }
+      if (lane < U && b + lane < nbatch) __stcs(&out[(b + lane) * ncells + c], a.v);
+    }
+  }
+}
 
 template <typename T, int U, int C>
 __global__ void __launch_bounds__(256, adj_ctas(sizeof(T), U)) index_adj_kernel(const T* __restrict__ vals, const int32_t* __restrict__ perm,
                                                         const uint32_t* __restrict__ off, T* __restrict__ out, int64_t npts,
                                                         int64_t ncells, int64_t nbatch) {
-  __shared__ T sm[U][kAdjChunk];
+  __shared__ union Shared {
+    T chunk[U][kAdjChunk];
+    CrowdShared<T, U> crowd;
+    __device__ Shared() {}
+  } shared;
+  T(&sm)[U][kAdjChunk] = shared.chunk;
   const int64_t first = (int64_t)blockIdx.x * (256 * C), c0 = first + threadIdx.x;
   const uint32_t ka = off[first], kb = off[min(first + 256 * C, ncells)];
+  if (kb - ka > 2 * 256 * C) {
+    crowded_cells<T, U>(vals, perm, off, out, npts, ncells, nbatch, first, min(first + 256 * C, ncells), shared.crowd);
+    return;
+  }
   uint32_t k0[C], k1[C];
 #pragma unroll
   for (int j = 0; j < C; ++j) {
@@ -183,13 +295,15 @@ __global__ void __launch_bounds__(256, adj_ctas(sizeof(T), U)) index_adj_kernel(
   }
 }
 
-// The same on grids whose cells hold several samples: a cell's samples are
-// contiguous in perm, and K of its values are read ahead of adding them. 8
-// entries of 64^2 at 2^20 samples: 2150 us one value at a time, 292 and 254 us
-// with K = 4 and 8, 807 us through shared memory, where a chunk holds one cell
-// and its CTA waits for that one lane; 12 entries of 320^2 (10 samples per
-// cell): 187, 79 and 78, 129 us; at a quarter sample per cell 160^3 prefers
-// shared memory, 104 against 160 us. The line is at two samples per cell.
+// The same on grids whose cells hold several samples, a cell per thread with K
+// values read ahead. The line is at one sample per cell, with K = 4 up to four:
+// 2^22 samples on 160^3 take 71 us for 2 entries and 262 for 8 (through shared
+// memory 91 and 384), 2^23 of 8 entries 398 (463 with K = 8, but 1.45 ms against
+// 2.65 where they crowd into few cells). 20 entries of 320^2 at 2^20 samples: 89 us.
+// 16-byte values, which fill the shared memory and the registers, cross over at a
+// quarter sample and prefer K = 2: 2 entries of 160^3 at 2^20, 2^21 and 2^22 samples
+// 82, 110 and 165 us, 4 entries a CTA through shared memory 149, 233 and 432, one
+// value at a time 97, 129 and 197.
 template <typename T, int K>
 __global__ void __launch_bounds__(256) index_adj_dense_kernel(const T* __restrict__ vals, const int32_t* __restrict__ perm,
                                                               const uint32_t* __restrict__ off, T* __restrict__ out,
@@ -198,18 +312,7 @@ __global__ void __launch_bounds__(256) index_adj_dense_kernel(const T* __restric
   if (c >= ncells) return;
   const uint32_t k0 = off[c], k1 = off[c + 1];
   for (int64_t b = blockIdx.y; b < nbatch; b += gridDim.y) {
-    const T* vb = vals + b * npts;
-    Acc<T> a;
-    for (uint32_t k = k0; k < k1; k += K) {
-      T v[K];
-#pragma unroll
-      for (int i = 0; i < K; ++i)
-        if (k + i < k1) v[i] = vb[perm[k + i]];
-#pragma unroll
-      for (int i = 0; i < K; ++i)
-        if (k + i < k1) a.add(v[i]);
-    }
-    out[b * ncells + c] = a.v;
+    out[b * ncells + c] = cell_sum<T, K>(vals + b * npts, perm, k0, k1);
   }
 }
 
@@ -219,20 +322,31 @@ void launch_index_adj_at(const IdxGeo& g, const void* vals, const int32_t* perm,
   const dim3 grd((unsigned)cdiv(g.ncells, 256 * C), (unsigned)std::min<int64_t>(cdiv(g.nbatch, U), 65535));
   index_adj_kernel<T, U, C><<<grd, 256, 0, s>>>((const T*)vals, perm, off, (T*)out, g.npts, g.ncells, g.nbatch);
 }
-// As many cells and entries per CTA as leave four CTAs per SM; small grids
-// take one cell per thread, and one entry where that is still too few.
+template <typename T, int K>
+void launch_index_adj_dense(const IdxGeo& g, const void* vals, const int32_t* perm, const uint32_t* off, void* out,
+                            cudaStream_t s) {
+  const dim3 grd((unsigned)cdiv(g.ncells, 128), (unsigned)std::min<int64_t>(g.nbatch, 65535));
+  index_adj_dense_kernel<T, K><<<grd, 128, 0, s>>>((const T*)vals, perm, off, (T*)out, g.npts, g.ncells, g.nbatch);
+}
+// Through shared memory, as many cells and entries per CTA as leave four CTAs
+// per SM; small grids take one cell per thread, and one entry where that is still
+// too few. 16-byte values take at most two entries (four need 119 registers).
 template <typename T>
 void launch_index_adj(const IdxGeo& g, const void* vals, const int32_t* perm, const uint32_t* off, void* out, cudaStream_t s) {
-  if (g.npts >= 2 * g.ncells) {
-    const dim3 grd((unsigned)cdiv(g.ncells, 128), (unsigned)std::min<int64_t>(g.nbatch, 65535));
-    index_adj_dense_kernel<T, 8><<<grd, 128, 0, s>>>((const T*)vals, perm, off, (T*)out, g.npts, g.ncells, g.nbatch);
-    return;
+  if constexpr (sizeof(T) > 8) {
+    if (g.npts >= 16 * g.ncells) launch_index_adj_dense<T, 4>(g, vals, perm, off, out, s);
+    else if (4 * g.npts >= g.ncells) launch_index_adj_dense<T, 2>(g, vals, perm, off, out, s);
+    else if (g.nbatch == 1) launch_index_adj_at<T, 1, 4>(g, vals, perm, off, out, s);
+    else launch_index_adj_at<T, 2, 4>(g, vals, perm, off, out, s);
+  } else {
+    const int64_t want = 4ll * sm_count(), groups = cdiv(g.nbatch, 4);
+    if (g.npts >= 4 * g.ncells) launch_index_adj_dense<T, 8>(g, vals, perm, off, out, s);
+    else if (g.npts >= g.ncells) launch_index_adj_dense<T, 4>(g, vals, perm, off, out, s);
+    else if (g.nbatch > 1 && cdiv(g.ncells, 1024) * groups >= want) launch_index_adj_at<T, 4, 4>(g, vals, perm, off, out, s);
+    else if (g.nbatch == 1 && cdiv(g.ncells, 1024) >= want) launch_index_adj_at<T, 1, 4>(g, vals, perm, off, out, s);
+    else if (g.nbatch > 1 && cdiv(g.ncells, 256) * groups >= want) launch_index_adj_at<T, 4, 1>(g, vals, perm, off, out, s);
+    else launch_index_adj_at<T, 1, 1>(g, vals, perm, off, out, s);
   }
-  const int64_t want = 4ll * sm_count(), groups = cdiv(g.nbatch, 4);
-  if (g.nbatch > 1 && cdiv(g.ncells, 1024) * groups >= want) launch_index_adj_at<T, 4, 4>(g, vals, perm, off, out, s);
-  else if (g.nbatch == 1 && cdiv(g.ncells, 1024) >= want) launch_index_adj_at<T, 1, 4>(g, vals, perm, off, out, s);
-  else if (g.nbatch > 1 && cdiv(g.ncells, 256) * groups >= want) launch_index_adj_at<T, 4, 1>(g, vals, perm, off, out, s);
-  else launch_index_adj_at<T, 1, 1>(g, vals, perm, off, out, s);
 }
 
 int make_idx_geo(const tlgb_index_desc* d, IdxGeo& g) {
