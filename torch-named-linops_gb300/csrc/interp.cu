@@ -2168,7 +2168,7 @@ __device__ __forceinline__ void item_origin(const Geo& g, int tile, int (&o)[3])
 
 // One record per home point, in the order of the gather items' points
 // (item.w is the first one's index), so an item's records are one run. For 3D
-// plans also each point's place in that order (`rank`), and of every 16th
+// plans also each point's place in that order (`rank`). And of every 16th
 // item's points (jumps[-1]) how many lie in another 32-byte sector of an output
 // row than the point before (jumps[0]: nearly all for points in random order,
 // a quarter in runs). jumps[-2]: whether some window has fewer than KT taps in a
@@ -2248,15 +2248,13 @@ __global__ void __launch_bounds__(128) plan_records_kernel(Geo g, const uint32_t
     float4* dst = reinterpret_cast<float4*>(recs + it.w + (j - it.y));
 #pragma unroll
     for (int q = 0; q < (int)(sizeof(R) / 16); ++q) dst[q] = src[q];
-    if (rank) {
-      rank[p] = it.w + (j - it.y);
-      if (blockIdx.x % 16 == 0) {
-        const unsigned on = __activemask();
-        const unsigned m = __ballot_sync(on, j == it.y || entries[j - 1] >> 2 != p >> 2);
-        if ((threadIdx.x & 31) == 0) {
-          atomicAdd(jumps, (uint32_t)__popc(m));
-          atomicAdd(jumps - 1, (uint32_t)__popc(on));
-        }
+    if (rank) rank[p] = it.w + (j - it.y);
+    if (blockIdx.x % 16 == 0) {
+      const unsigned on = __activemask();
+      const unsigned m = __ballot_sync(on, j == it.y || entries[j - 1] >> 2 != p >> 2);
+      if ((threadIdx.x & 31) == 0) {
+        atomicAdd(jumps, (uint32_t)__popc(m));
+        atomicAdd(jumps - 1, (uint32_t)__popc(on));
       }
     }
   }
@@ -2545,10 +2543,13 @@ __global__ void __launch_bounds__(NW * 32 + kGatherProd, CTAS)
             }
           }
           __syncwarp();
-          const int e8 = lane % CG, n2 = T.n[NDIM - 1], n1 = T.n[NDIM - 2], tot = n1 * n2 * (NDIM == 3 ? T.n[0] : 1);
+          const int e8 = lane % CG, n2 = T.n[NDIM - 1], n1 = T.n[NDIM - 2], n0 = NDIM == 3 ? T.n[0] : 1;
           float2 v2 = make_float2(0.f, 0.f);
-          for (int t = lane / CG; t < tot; t += 32 / CG) {
-            const int z = t % n2, yx = t / n2, y = yx % n1, x = yx / n1;
+          // all KT + 1 taps per dim, for divisions by a constant: with the window's own counts 8 x 262,144 spline
+          // points on 128 x 120 x 96 (5 taps each) took 1057 us, 934 so
+          for (int t = lane / CG; t < (NDIM == 3 ? (KT + 1) * (KT + 1) : KT + 1) * (KT + 1); t += 32 / CG) {
+            const int z = t % (KT + 1), yx = t / (KT + 1), y = yx % (KT + 1), x = yx / (KT + 1);
+            if (z >= n2 || y >= n1 || x >= n0) continue;
             float w = T.w[NDIM - 2][y] * T.w[NDIM - 1][z];
             int cell = (T.f[NDIM - 2] + y) * S + T.f[NDIM - 1] + z;
             if (NDIM == 3) {
@@ -2813,6 +2814,11 @@ constexpr size_t grad2_smem() {
          kGradWarps * (sizeof(GradTaps) + 16 * sizeof(float)) + 8 * (2 * kGradStages + 4) + 16;
 }
 
+// AT: a is point-major ([group][point][8], transpose_vals_kernel's layout), for
+// points in random order: gathered entry by entry there, every 8-byte value is a
+// sector of its own (205,824 random points x 256 entries on 320^2: 1952 us, 765
+// with the transposition; 8 entries 287 and 265 at 524,288 points on 512^2).
+template <bool AT>
 __global__ void __launch_bounds__(kGradWarps * 32 + kGatherProd, 1)
     grad2_kernel(const __grid_constant__ CUtensorMap tmap, int use_tma, Geo g, const int4* __restrict__ items, int nruns,
                  int run, int nunits, const GatherRec<2, 4>* __restrict__ recs, const float* __restrict__ locs,
@@ -2888,12 +2894,19 @@ __global__ void __launch_bounds__(kGradWarps * 32 + kGatherProd, 1)
         } else {
           copy_region<2, 4, 8>(g, gridv, reg, o, cg, pt);
         }
-        for (int i = pt; i < npt; i += kGatherProd) {
-          const int p = rec[i].p;
+        if constexpr (AT) {  // 4 threads a point; the values of missing entries are zeros already
+          for (int i = pt; i < npt * 4; i += kGatherProd) {
+            const int p = rec[i >> 2].p;
+            if (TLGB_IN_RANGE(p, g.npts)) cp_async16(av + 2 * i, a + ((long long)cg * g.npts + p) * 8 + 2 * (i & 3));
+          }
+        } else {
+          for (int i = pt; i < npt; i += kGatherProd) {
+            const int p = rec[i].p;
 #pragma unroll
-          for (int c = 0; c < 8; ++c) {
-            const bool in = cg * 8 + c < g.nbatch && TLGB_IN_RANGE(p, g.npts);
-            sm100::cp_async8_zfill(av + c * kGatherPts + i, in ? a + (long long)(cg * 8 + c) * g.npts + p : a, in);
+            for (int c = 0; c < 8; ++c) {
+              const bool in = cg * 8 + c < g.nbatch && TLGB_IN_RANGE(p, g.npts);
+              sm100::cp_async8_zfill(av + c * kGatherPts + i, in ? a + (long long)(cg * 8 + c) * g.npts + p : a, in);
+            }
           }
         }
         sm100::cp_async_mbar_arrive(&full[s]);
@@ -2951,7 +2964,7 @@ __global__ void __launch_bounds__(kGradWarps * 32 + kGatherProd, 1)
         const int i = on ? base + h : base;
         const unsigned view = rec[i].view;
         const float2* v = reg + c * VOL + (view & 0xfffff) + kz;
-        const float2 a0 = av[c * kGatherPts + i], a1 = av[(c + 4) * kGatherPts + i];
+        const float2 a0 = av[AT ? i * 8 + c : c * kGatherPts + i], a1 = av[AT ? i * 8 + c + 4 : (c + 4) * kGatherPts + i];
         if (TLGB_IN_RANGE((view & 0xfffff) + 3 * S + 3, VOL)) {
 #pragma unroll
           for (int t = 0; t < 4; ++t) {
@@ -2997,16 +3010,23 @@ __global__ void __launch_bounds__(kGradWarps * 32 + kGatherProd, 1)
           }
           __syncwarp();
           const int c8 = lane & 7, n2 = T.n[1], tot = T.n[0] * n2;
-          const float2 ac = av[c8 * kGatherPts + base + hh];
+          const float2 ac = av[AT ? (base + hh) * 8 + c8 : c8 * kGatherPts + base + hh];
           float ry = 0.f, rz = 0.f;
-          for (int t = lane >> 3; t < tot; t += 4) {
-            const int z = t % n2, y = t / n2, cell = (T.f[0] + y) * S + T.f[1] + z;
-            if (!TLGB_IN_RANGE(cell, VOL)) continue;
+          auto tap = [&](int y, int z) {
+            const int cell = (T.f[0] + y) * S + T.f[1] + z;
+            if (!TLGB_IN_RANGE(cell, VOL)) return;
             const float2 vv = reg[c8 * VOL + cell];
             const float dot = fmaf(ac.x, vv.x, ac.y * vv.y);
             ry = fmaf(T.dw[0][y] * T.w[1][z], dot, ry);
             rz = fmaf(T.w[0][y] * T.dw[1][z], dot, rz);
-          }
+          };
+          // the loop that lets ptxas keep more of `sum` in registers, by variant: 810 against 860 us on radial
+          // points, 755 against 850 on random ones (256 entries of 320^2)
+          if constexpr (AT)
+            for (int y = 0; y < T.n[0]; ++y)
+              for (int z = lane >> 3; z < n2; z += 4) tap(y, z);
+          else
+            for (int t = lane >> 3; t < tot; t += 4) tap(t / n2, t % n2);
 #pragma unroll
           for (int m = 1; m < 32; m <<= 1) {
             ry += __shfl_xor_sync(0xffffffffu, ry, m);
@@ -3410,19 +3430,30 @@ size_t grad_scratch_bytes(const Geo& g, int nsplit) {
 
 // The 2D gradient on the gather's ring (grad2_kernel). A unit is an item and a
 // run of groups of 8 entries; with several runs each adds its own partial slot.
-// One run (no partial results) unless that leaves fewer than 4 units per SM.
+// One run (no partial results) unless that leaves fewer units than SMs: each
+// unit ends with some microseconds for its points' weights, so more are slower
+// (20 entries of 256 x 240 at 65,536 points: 109 us with 4 units per SM, 77 so).
+// Windows of the spline with width 4 always have 5 taps, which the ring takes one
+// point at a time: the generic kernel is faster (512^2 at 524,288 points: one entry
+// 383 us against 921, 8 entries 496 against 1119).
 bool grad_on_ring(const Geo& g, const tlgb_interp_plan_info* info) {
+  if (g.kernel != TLGB_KERNEL_KAISER_BESSEL && std::max(g.NT[1], g.NT[2]) > 4) return false;
   return g.cplx && g.ndim == 2 && rec_taps(g) == 4 && info->off_records > 0;
 }
 int64_t grad2_runs(const Geo& g, const tlgb_interp_plan_info* info) {
   const int64_t ncg = cdiv(std::max<long long>(g.nbatch, 1), 8), items = std::max<int64_t>(info->n_fwd_items, 1);
   int64_t run = ncg;
-  while (run > 1 && items * cdiv(ncg, run) < 4 * sm_count()) run = cdiv(run, 2);
+  while (run > 1 && items * cdiv(ncg, run) < sm_count()) run = cdiv(run, 2);
   return cdiv(ncg, run);
 }
-size_t grad2_scratch_bytes(const Geo& g, const tlgb_interp_plan_info* info) {
+// the runs' partial results, then (points in random order) the point-major values
+size_t grad2_partial_bytes(const Geo& g, const tlgb_interp_plan_info* info) {
   const int64_t n = grad2_runs(g, info);
-  return n > 1 ? (size_t)n * g.npts * 2 * sizeof(float) : 0;
+  return n > 1 ? align_up((size_t)n * g.npts * 2 * sizeof(float), 256) : 0;
+}
+size_t grad2_scratch_bytes(const Geo& g, const tlgb_interp_plan_info* info) {
+  const size_t at = (info->kernel_key & kScattered) && g.nbatch >= 4 ? (size_t)cdiv(g.nbatch, 8) * g.npts * 64 : 0;
+  return grad2_partial_bytes(g, info) + at;
 }
 
 int check_plan(const Geo& g, const tlgb_interp_plan_info* info, const void* plan) {
@@ -3996,7 +4027,16 @@ int launch_grad2(const Geo& g, const tlgb_interp_plan_info* info, const char* P,
   if ((uintptr_t)P & 15) TLGB_FAIL(TLGB_ERR_INVALID, "trajectory gradient: the plan must be 16-byte aligned");
   const int64_t ncg = cdiv(g.nbatch, 8);
   int64_t nruns = grad2_runs(g, info);
-  if (nruns > 1 && (!scratch || scratch_bytes < grad2_scratch_bytes(g, info) || ((uintptr_t)scratch & 7))) nruns = 1;
+  const size_t part = grad2_partial_bytes(g, info);
+  if (nruns > 1 && (!scratch || scratch_bytes < part || ((uintptr_t)scratch & 7))) nruns = 1;
+  const float2* at = nullptr;
+  if (scratch && ((uintptr_t)scratch & 15) == 0 && grad2_scratch_bytes(g, info) > part && scratch_bytes >= grad2_scratch_bytes(g, info)) {
+    float2* t = reinterpret_cast<float2*>(static_cast<char*>(scratch) + part);
+    transpose_vals_kernel<<<dim3((unsigned)cdiv(g.npts, kTrPts), (unsigned)ncg), 256, 0, s>>>((const float2*)a, g.npts,
+                                                                                              g.nbatch, t, nullptr);
+    TLGB_CHECK_LAUNCH();
+    at = t;
+  }
   const int64_t run = cdiv(ncg, nruns), nunits = info->n_fwd_items * nruns;
   if (nunits >= (1ll << 31) - sm_count()) TLGB_FAIL(TLGB_ERR_UNSUPPORTED, "trajectory gradient: too many points and batch entries in one call");
   const long long n = (long long)g.npts * 2;
@@ -4005,10 +4045,11 @@ int launch_grad2(const Geo& g, const tlgb_interp_plan_info* info, const char* P,
     TLGB_CUDA(cudaMemsetAsync(partial, 0, (size_t)nruns * n * sizeof(float), s));
   CUtensorMap tmap;
   const int use_tma = region_map(g, grid, 20, 8, tmap);
-  TLGB_TRY(set_smem(grad2_kernel, grad2_smem()));
-  grad2_kernel<<<(unsigned)std::min<int64_t>(nunits, sm_count()), kGradWarps * 32 + kGatherProd, grad2_smem(), s>>>(
+  auto* k = at ? grad2_kernel<true> : grad2_kernel<false>;
+  TLGB_TRY(set_smem(k, grad2_smem()));
+  k<<<(unsigned)std::min<int64_t>(nunits, sm_count()), kGradWarps * 32 + kGatherProd, grad2_smem(), s>>>(
       tmap, use_tma, g, (const int4*)(P + info->off_fwd_items), (int)nruns, (int)run, (int)nunits,
-      (const GatherRec<2, 4>*)(P + info->off_records), locs, (const float*)grid, (const float2*)a, grad, partial);
+      (const GatherRec<2, 4>*)(P + info->off_records), locs, (const float*)grid, at ? at : (const float2*)a, grad, partial);
   TLGB_CHECK_LAUNCH();
   if (nruns > 1) {
     grad_reduce_kernel<<<(unsigned)cdiv(n, 256), 256, 0, s>>>(partial, (int)nruns, n, grad);
