@@ -463,33 +463,25 @@ __device__ __forceinline__ void for_lane_taps(const Geo& g, const Rec<NTB>& R, c
 
 // ------------------------------------------------------------------ forward
 
+// Resident CTAs of the 8-warp kernel: three (80 registers) where the region
+// leaves room for them, for one entry of 320^2 at 524,288 points 122 against 155
+// us; with eight entries in 3D two, 449 against 474 (128 x 120 x 96).
+constexpr int fwd_ctas(int n, int ndim, int ntb, int nw) { return nw == 8 && ntb == 5 && (ndim == 2 || n == 1) ? 3 : 1; }
+
 // CTA = NW warps sharing one staged region (tile + halo, [x][y][z][batch]);
-// each warp interpolates 32 home points per batch.
+// each warp interpolates 32 home points per batch. A CTA takes `per` items one
+// after the other and stages a region once for those of one tile.
 template <int N, int NDIM, int NTB, int NW>
-__global__ void __launch_bounds__(NW * 32, 1) interp_fwd_kernel(Geo g, const int4* __restrict__ items,
-                                                                const int32_t* __restrict__ entries,
-                                                                const float* __restrict__ locs,
-                                                                const float* __restrict__ gridv,
-                                                                float* __restrict__ out, int CG) {
+__global__ void __launch_bounds__(NW * 32, fwd_ctas(N, NDIM, NTB, NW))
+    interp_fwd_kernel(Geo g, const int4* __restrict__ items, int nitems, int per, const int32_t* __restrict__ entries,
+                      const float* __restrict__ locs, const float* __restrict__ gridv, float* __restrict__ out, int CG) {
   extern __shared__ __align__(128) unsigned char smem[];
   const int es = g.cplx ? 2 : 1;
-  const int4 it = items[blockIdx.x];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int c0 = blockIdx.y * CG;
   const int ncoil = (int)min((long long)CG, g.nbatch - c0);
-  int tc[3];
-  {
-    int t = it.x;
-    tc[2] = t % g.nt[2];
-    t /= g.nt[2];
-    tc[1] = t % g.nt[1];
-    tc[0] = t / g.nt[1];
-  }
-  int o[3], S[3];
-  for (int e = 0; e < 3; ++e) {
-    o[e] = tc[e] * g.T[e];
-    S[e] = g.T[e] + g.NT[e] - 1;
-  }
+  int o[3] = {0, 0, 0}, S[3];
+  for (int e = 0; e < 3; ++e) S[e] = g.T[e] + g.NT[e] - 1;
   const int vstride = CG * es;  // floats per staged voxel
   float* reg = reinterpret_cast<float*>(smem);
   const size_t reg_bytes = (((size_t)S[0] * S[1] * S[2] * vstride * sizeof(float)) + 15) & ~(size_t)15;
@@ -500,112 +492,126 @@ __global__ void __launch_bounds__(NW * 32, 1) interp_fwd_kernel(Geo g, const int
   const int cgp = CG <= 1 ? 1 : (CG <= 2 ? 2 : (CG <= 4 ? 4 : 8));
   const int lgc = lg2i(cgp);
   const int rowlen = S[2] * cgp;
-  for (int row = warp; row < S[0] * S[1]; row += NW) {
-    const int x = row / S[1], y = row - x * S[1];
-    int gx = o[0] + x, gy = o[1] + y;
-    bool rin = true;
-    if (g.pad == TLGB_PAD_CIRCULAR) {
-      gx = wrapi(gx, g.N[0]);
-      gy = wrapi(gy, g.N[1]);
-    } else {
-      rin = gx < g.N[0] && gy < g.N[1];
-    }
-    const long long rbase = ((long long)gx * g.N[1] + gy) * g.N[2];
-    float* rdst = reg + (size_t)(x * S[1] + y) * S[2] * vstride;
-    // all loads of the row first (independent), then the stores
-    constexpr int MAXI = 8;
-    float2 vv[MAXI];
-#pragma unroll
-    for (int i = 0; i < MAXI; ++i) {
-      vv[i] = make_float2(0.f, 0.f);
-      const int idx = lane + 32 * i;
-      if (idx < rowlen) {
-        const int c = idx & (cgp - 1), z = idx >> lgc;
-        int gz = o[2] + z;
-        bool in = rin && c < ncoil;
-        if (g.pad == TLGB_PAD_CIRCULAR) gz = wrapi(gz, g.N[2]);
-        else in = in && gz < g.N[2];
-        if (in) {
-          const long long gi = (long long)(c0 + c) * gvol + rbase + gz;
-          if (es == 2) vv[i] = __ldg(reinterpret_cast<const float2*>(gridv) + gi);
-          else vv[i].x = __ldg(gridv + gi);
+  int staged = -1;
+  const int last = min(nitems, ((int)blockIdx.x + 1) * per);
+  for (int item = blockIdx.x * per; item < last; ++item) {
+    const int4 it = items[item];
+    if (it.x != staged) {
+      int t = it.x;
+      o[2] = t % g.nt[2] * g.T[2];
+      t /= g.nt[2];
+      o[1] = t % g.nt[1] * g.T[1];
+      o[0] = t / g.nt[1] * g.T[0];
+      if (staged >= 0) __syncthreads();  // the tile before has been read
+      for (int row = warp; row < S[0] * S[1]; row += NW) {
+        const int x = row / S[1], y = row - x * S[1];
+        int gx = o[0] + x, gy = o[1] + y;
+        bool rin = true;
+        if (g.pad == TLGB_PAD_CIRCULAR) {
+          gx = wrapi(gx, g.N[0]);
+          gy = wrapi(gy, g.N[1]);
+        } else {
+          rin = gx < g.N[0] && gy < g.N[1];
         }
-      }
-    }
+        const long long rbase = ((long long)gx * g.N[1] + gy) * g.N[2];
+        float* rdst = reg + (size_t)(x * S[1] + y) * S[2] * vstride;
+        // all loads of the row first (independent), then the stores
+        constexpr int MAXI = 8;
+        float2 vv[MAXI];
 #pragma unroll
-    for (int i = 0; i < MAXI; ++i) {
-      const int idx = lane + 32 * i;
-      if (idx < rowlen) {
-        const int c = idx & (cgp - 1), z = idx >> lgc;
-        if (c < CG) {
+        for (int i = 0; i < MAXI; ++i) {
+          vv[i] = make_float2(0.f, 0.f);
+          const int idx = lane + 32 * i;
+          if (idx < rowlen) {
+            const int c = idx & (cgp - 1), z = idx >> lgc;
+            int gz = o[2] + z;
+            bool in = rin && c < ncoil;
+            if (g.pad == TLGB_PAD_CIRCULAR) gz = wrapi(gz, g.N[2]);
+            else in = in && gz < g.N[2];
+            if (in) {
+              const long long gi = (long long)(c0 + c) * gvol + rbase + gz;
+              if (es == 2) vv[i] = __ldg(reinterpret_cast<const float2*>(gridv) + gi);
+              else vv[i].x = __ldg(gridv + gi);
+            }
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < MAXI; ++i) {
+          const int idx = lane + 32 * i;
+          if (idx < rowlen) {
+            const int c = idx & (cgp - 1), z = idx >> lgc;
+            if (c < CG) {
+              float* d = rdst + z * vstride + c * es;
+              if (es == 2) *reinterpret_cast<float2*>(d) = vv[i];
+              else d[0] = vv[i].x;
+            }
+          }
+        }
+        for (int idx = lane + 32 * MAXI; idx < rowlen; idx += 32) {  // long rows (1D tiles)
+          const int c = idx & (cgp - 1), z = idx >> lgc;
+          if (c >= CG) continue;
+          int gz = o[2] + z;
+          bool in = rin && c < ncoil;
+          if (g.pad == TLGB_PAD_CIRCULAR) gz = wrapi(gz, g.N[2]);
+          else in = in && gz < g.N[2];
           float* d = rdst + z * vstride + c * es;
-          if (es == 2) *reinterpret_cast<float2*>(d) = vv[i];
-          else d[0] = vv[i].x;
+          const long long gi = (long long)(c0 + c) * gvol + rbase + gz;
+          if (es == 2) *reinterpret_cast<float2*>(d) = in ? __ldg(reinterpret_cast<const float2*>(gridv) + gi) : make_float2(0.f, 0.f);
+          else d[0] = in ? __ldg(gridv + gi) : 0.f;
         }
       }
+      __syncthreads();
+      staged = it.x;
     }
-    for (int idx = lane + 32 * MAXI; idx < rowlen; idx += 32) {  // long rows (1D tiles)
-      const int c = idx & (cgp - 1), z = idx >> lgc;
-      if (c >= CG) continue;
-      int gz = o[2] + z;
-      bool in = rin && c < ncoil;
-      if (g.pad == TLGB_PAD_CIRCULAR) gz = wrapi(gz, g.N[2]);
-      else in = in && gz < g.N[2];
-      float* d = rdst + z * vstride + c * es;
-      const long long gi = (long long)(c0 + c) * gvol + rbase + gz;
-      if (es == 2) *reinterpret_cast<float2*>(d) = in ? __ldg(reinterpret_cast<const float2*>(gridv) + gi) : make_float2(0.f, 0.f);
-      else d[0] = in ? __ldg(gridv + gi) : 0.f;
-    }
-  }
-  __syncthreads();
 
-  const int U = N / es;  // batch entries per unit
-  const int nunits = (CG + U - 1) / U;
-  const Lanes L = lane_roles(lane, nunits);
-  for (int b = it.y + warp * 32; b < it.z; b += NW * 32) {
-    const int j = b + lane;
-    const int nb = min(32, it.z - b);
-    long long p = -1;
-    if (j < it.z) {
-      p = entries[j];
-      float x3[3];
-      for (int e = 0; e < 3; ++e) x3[e] = g.act[e] ? load_coord(g, locs, p, e) : 0.f;
-      lane_rec<NTB>(g, x3, o, true, rbuf[lane]);
-    }
-    __syncwarp();
-    for (int jj = 0; jj < nb; ++jj) {
-      const Rec<NTB>& R = rbuf[jj];
-      const long long pj = __shfl_sync(0xffffffffu, p, jj);
-      if (R.m[0] == 0) continue;  // warp-uniform
-      VecF<N> acc;
-#pragma unroll
-      for (int i = 0; i < N; ++i) acc.v[i] = 0.f;
-      if (L.cu < nunits) {
-        const float* base = reg + L.cu * N;
-        for_lane_taps<NDIM, NTB>(g, R, L, [&](int lx, int ly, int lz, float w) {
-          const VecF<N> v = ldv<N>(base + ((size_t)(lx * S[1] + ly) * S[2] + lz) * vstride);
-#pragma unroll
-          for (int i = 0; i < N; ++i) acc.v[i] = fmaf(w, v.v[i], acc.v[i]);
-        });
+    const int U = N / es;  // batch entries per unit
+    const int nunits = (CG + U - 1) / U;
+    const Lanes L = lane_roles(lane, nunits);
+    for (int b = it.y + warp * 32; b < it.z; b += NW * 32) {
+      const int j = b + lane;
+      const int nb = min(32, it.z - b);
+      long long p = -1;
+      if (j < it.z) {
+        p = entries[j];
+        float x3[3];
+        for (int e = 0; e < 3; ++e) x3[e] = g.act[e] ? load_coord(g, locs, p, e) : 0.f;
+        lane_rec<NTB>(g, x3, o, true, rbuf[lane]);
       }
-      for (int m = L.NUP; m < 32; m <<= 1)
+      __syncwarp();
+      for (int jj = 0; jj < nb; ++jj) {
+        const Rec<NTB>& R = rbuf[jj];
+        const long long pj = __shfl_sync(0xffffffffu, p, jj);
+        if (R.m[0] == 0) continue;  // warp-uniform
+        VecF<N> acc;
 #pragma unroll
-        for (int i = 0; i < N; ++i) acc.v[i] += __shfl_xor_sync(0xffffffffu, acc.v[i], m);
-      if (lane < L.NUP && L.cu < nunits) {
+        for (int i = 0; i < N; ++i) acc.v[i] = 0.f;
+        if (L.cu < nunits) {
+          const float* base = reg + L.cu * N;
+          for_lane_taps<NDIM, NTB>(g, R, L, [&](int lx, int ly, int lz, float w) {
+            const VecF<N> v = ldv<N>(base + ((size_t)(lx * S[1] + ly) * S[2] + lz) * vstride);
 #pragma unroll
-        for (int u = 0; u < N; u += (N >= 2 && es == 2) ? 2 : 1) {
-          const int c = L.cu * U + u / es;
-          if (c < ncoil) {
-            float* dst = out + ((long long)(c0 + c) * g.npts + pj) * es;
-            if (es == 2)
-              *reinterpret_cast<float2*>(dst) = make_float2(acc.v[u], acc.v[u + 1]);
-            else
-              dst[0] = acc.v[u];
+            for (int i = 0; i < N; ++i) acc.v[i] = fmaf(w, v.v[i], acc.v[i]);
+          });
+        }
+        for (int m = L.NUP; m < 32; m <<= 1)
+#pragma unroll
+          for (int i = 0; i < N; ++i) acc.v[i] += __shfl_xor_sync(0xffffffffu, acc.v[i], m);
+        if (lane < L.NUP && L.cu < nunits) {
+#pragma unroll
+          for (int u = 0; u < N; u += (N >= 2 && es == 2) ? 2 : 1) {
+            const int c = L.cu * U + u / es;
+            if (c < ncoil) {
+              float* dst = out + ((long long)(c0 + c) * g.npts + pj) * es;
+              if (es == 2)
+                *reinterpret_cast<float2*>(dst) = make_float2(acc.v[u], acc.v[u + 1]);
+              else
+                dst[0] = acc.v[u];
+            }
           }
         }
       }
+      __syncwarp();
     }
-    __syncwarp();
   }
 }
 
@@ -3379,8 +3385,8 @@ int fwd_cg(const Geo& g) {
   return cg;
 }
 
-size_t fwd_smem(const Geo& g, int cg) {
-  return align_up((size_t)region_vol(g) * cg * value_size(g), 16) + NWF * 32 * pt_bytes(ntb_for(g));
+size_t fwd_smem(const Geo& g, int cg, int warps) {
+  return align_up((size_t)region_vol(g) * cg * value_size(g), 16) + warps * 32 * pt_bytes(ntb_for(g));
 }
 
 int adj_cg(const Geo& g) { return (int)std::min<long long>(std::max<long long>(g.nbatch, 1), CGMAX); }
@@ -3755,12 +3761,24 @@ template <int N, int NDIM, int NTB>
 int launch_fwd_t2(const Geo& g, int cg, const tlgb_interp_plan_info* info, const char* P, const float* locs,
                   const void* grid, void* out, cudaStream_t s) {
   const int64_t ncg = cdiv(g.nbatch, cg);
-  const size_t sm = fwd_smem(g, cg);
+  // Real values on a plan with gather records: its items hold at most 256 points, a
+  // batch of 32 for 8 warps. 16 would leave half of them idle and one CTA per SM
+  // (2D, 131,072 points on 321 x 203: 82 -> 48 us for one entry, 99 -> 63 for 8).
+  int nw = NWF;
   auto* k = interp_fwd_kernel<N, NDIM, NTB, NWF>;
+  if constexpr (N <= 2 && NDIM >= 2)
+    if (records_ok(g)) nw = 8, k = interp_fwd_kernel<N, NDIM, NTB, 8>;
+  const size_t sm = fwd_smem(g, cg, nw);
   TLGB_TRY(set_smem(k, sm));
-  dim3 grd((unsigned)info->n_fwd_items, (unsigned)ncg);
-  k<<<grd, NWF * 32, sm, s>>>(g, (const int4*)(P + info->off_fwd_items), (const int32_t*)(P + info->off_entries),
-                             locs, (const float*)grid, (float*)out, cg);
+  // Tiles of many points are several such items: up to 4 in a CTA, unless that
+  // leaves fewer than 8 CTAs per SM (2D) or 2 (3D, whose regions cost more to
+  // stage). 8 entries of 64^3 at 524,288 points: 578 us staged for each item, 346
+  // so, 397 with 8 CTAs per SM; of 320^2 at 524,288: 159, 212 with 2.
+  int64_t per = nw == 8 ? std::min<int64_t>(4, info->n_fwd_items / std::max<int64_t>(info->n_tiles, 1)) : 1;
+  per = std::max<int64_t>(1, std::min<int64_t>(per, info->n_fwd_items * ncg / ((g.ndim == 3 ? 2 : 8) * sm_count())));
+  dim3 grd((unsigned)cdiv(info->n_fwd_items, per), (unsigned)ncg);
+  k<<<grd, nw * 32, sm, s>>>(g, (const int4*)(P + info->off_fwd_items), (int)info->n_fwd_items, (int)per,
+                             (const int32_t*)(P + info->off_entries), locs, (const float*)grid, (float*)out, cg);
   TLGB_CHECK_LAUNCH();
   return TLGB_OK;
 }
