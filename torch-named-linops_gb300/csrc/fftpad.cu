@@ -51,8 +51,10 @@ __device__ __forceinline__ float2 modulation(const PadGeo& G, int j0, int j1, in
   return sign ? make_float2(-c, -s) : make_float2(c, s);
 }
 
+// Rounded as written, so that an entry's result does not depend on the kernel
+// that its batch's size takes.
 __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
-  return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+  return make_float2(fmaf(a.x, b.x, -__fmul_rn(a.y, b.y)), fmaf(a.x, b.y, __fmul_rn(a.y, b.x)));
 }
 
 // row and column indices of voxel v of a volume with last extents n1, n2
@@ -83,13 +85,17 @@ constexpr int kBatchAhead = 8;
 // ahead. The crop, whose coils are a sum, keeps 8: 32 coils on 320^2 take 22, 31,
 // 19 and 16 us, 8 coils on 160^3 63-68.
 constexpr int kMapsPadAhead = 1;
+// Fewer entries (or coils of a crop) than 8 are not worth the registers of the
+// loads that never come. 205^3 in 256^3: one entry 165 us to pad and 161 to crop
+// with 8 ahead, 104 and 65 with one; three entries 180 and 184, 137 and 89 with 4.
+// 3 coils of 128^3, two entries: 67, 48 and 45 us with 8, 4 and one.
+int ahead(long long n, int four_from) { return n >= kBatchAhead ? kBatchAhead : (n >= four_from ? 4 : 1); }
 
 // out[e][j] = maps[e % C][i] * apod[i] * x[e / C][i] for the source i of j, else 0
-template <bool MAPS>
+template <bool MAPS, int AH>
 __global__ void __launch_bounds__(256) pad_shift_kernel(PadGeo G, const float2* __restrict__ x, long long nent, long long run,
                                                         const float* __restrict__ apod, const float2* __restrict__ maps,
                                                         int nmaps, float2* __restrict__ out) {
-  constexpr int AH = MAPS ? kMapsPadAhead : kBatchAhead;
   const long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= G.npvol) return;
   int j0, j1, j2;
@@ -112,7 +118,7 @@ __global__ void __launch_bounds__(256) pad_shift_kernel(PadGeo G, const float2* 
       v[u] = make_float2(0.f, 0.f);
       if (!in || e + u >= e1) continue;
       const float2 q = x[b * G.nvol + i];
-      v[u] = make_float2(q.x * a, q.y * a);
+      v[u] = make_float2(__fmul_rn(q.x, a), __fmul_rn(q.y, a));
       if (MAPS) v[u] = cmul(maps[c * G.nvol + i], v[u]);
       if (!MAPS || ++c == nmaps) {
         c = 0;
@@ -128,7 +134,7 @@ __global__ void __launch_bounds__(256) pad_shift_kernel(PadGeo G, const float2* 
 }
 
 // out[b][i] = alpha * apod[i] * sum_c conj(maps[c][i]) z[(b*C + c)][src(i)] + beta * add[b][i]
-template <bool MAPS>
+template <bool MAPS, int AH>
 __global__ void __launch_bounds__(256) crop_shift_kernel(PadGeo G, const float2* __restrict__ z, long long nbatch,
                                                          long long run, const float* __restrict__ apod,
                                                          const float2* __restrict__ maps, int nmaps, float alpha,
@@ -150,7 +156,7 @@ __global__ void __launch_bounds__(256) crop_shift_kernel(PadGeo G, const float2*
     md.y = -md.y;  // conj(m[j])
   }
   const long long b0 = blockIdx.y * run, b1 = min(nbatch, b0 + run);
-  constexpr int UB = MAPS ? 1 : kBatchAhead, UC = MAPS ? kBatchAhead : 1;  // coils ahead, or entries ahead
+  constexpr int UB = MAPS ? 1 : AH, UC = MAPS ? AH : 1;  // coils ahead, or entries ahead
   const int C = MAPS ? nmaps : 1;
   for (long long b = b0; b < b1; b += UB) {
     float2 s[UB];
@@ -169,8 +175,8 @@ __global__ void __launch_bounds__(256) crop_shift_kernel(PadGeo G, const float2*
         if (MAPS && c + u >= C) break;
         if (G.modulate) v[u] = cmul(v[u], md);
         if (MAPS) {  // conj(m) * v
-          s[0].x += m[u].x * v[u].x + m[u].y * v[u].y;
-          s[0].y += m[u].x * v[u].y - m[u].y * v[u].x;
+          s[0].x = __fadd_rn(s[0].x, fmaf(m[u].x, v[u].x, __fmul_rn(m[u].y, v[u].y)));
+          s[0].y = __fadd_rn(s[0].y, fmaf(m[u].x, v[u].y, -__fmul_rn(m[u].y, v[u].x)));
         } else {
           s[u] = v[u];
         }
@@ -179,7 +185,7 @@ __global__ void __launch_bounds__(256) crop_shift_kernel(PadGeo G, const float2*
 #pragma unroll
     for (int u = 0; u < UB; ++u) {
       if (b + u >= b1) break;
-      float2 o = make_float2(a * s[u].x, a * s[u].y);
+      float2 o = make_float2(__fmul_rn(a, s[u].x), __fmul_rn(a, s[u].y));
       if (add) {
         const float2 q = add[(b + u) * G.nvol + i];
         o.x = fmaf(beta, q.x, o.x);
@@ -238,8 +244,11 @@ extern "C" int tlgb_pad_shift_c64(const void* x, int64_t nbatch, int32_t ndim, c
   if (!x || !out) TLGB_FAIL(TLGB_ERR_INVALID, "null pointer");
   const long long nent = (long long)nbatch * (maps ? nmaps : 1), ctas = cdiv(G.npvol, 256);
   dim3 grid((unsigned)ctas);
-  const long long run = batch_runs(ctas, nent, maps ? kMapsPadAhead : kBatchAhead, grid.y);
-  (maps ? pad_shift_kernel<true> : pad_shift_kernel<false>)<<<grid, 256, 0, (cudaStream_t)stream>>>(
+  const int ah = maps ? kMapsPadAhead : ahead(nent, 3);
+  const long long run = batch_runs(ctas, nent, ah, grid.y);
+  auto* k = maps ? pad_shift_kernel<true, kMapsPadAhead>
+                 : (ah == 1 ? pad_shift_kernel<false, 1> : (ah == 4 ? pad_shift_kernel<false, 4> : pad_shift_kernel<false, kBatchAhead>));
+  k<<<grid, 256, 0, (cudaStream_t)stream>>>(
       G, (const float2*)x, nent, run, apod, (const float2*)maps, nmaps, (float2*)out);
   TLGB_CHECK_LAUNCH();
   return TLGB_OK;
@@ -256,8 +265,11 @@ extern "C" int tlgb_crop_shift_c64(const void* z, int64_t nbatch, int32_t ndim, 
   if (!z || !out) TLGB_FAIL(TLGB_ERR_INVALID, "null pointer");
   const long long ctas = cdiv(G.nvol, 256);
   dim3 grid((unsigned)ctas);
-  const long long run = batch_runs(ctas, nbatch, maps ? 1 : kBatchAhead, grid.y);
-  (maps ? crop_shift_kernel<true> : crop_shift_kernel<false>)<<<grid, 256, 0, (cudaStream_t)stream>>>(
+  const int ah = maps ? ahead(nmaps, 4) : ahead(nbatch, 3);
+  const long long run = batch_runs(ctas, nbatch, maps ? 1 : ah, grid.y);
+  auto* k = maps ? (ah == 1 ? crop_shift_kernel<true, 1> : (ah == 4 ? crop_shift_kernel<true, 4> : crop_shift_kernel<true, kBatchAhead>))
+                 : (ah == 1 ? crop_shift_kernel<false, 1> : (ah == 4 ? crop_shift_kernel<false, 4> : crop_shift_kernel<false, kBatchAhead>));
+  k<<<grid, 256, 0, (cudaStream_t)stream>>>(
       G, (const float2*)z, nbatch, run, apod, (const float2*)maps, nmaps, alpha, (const float2*)add, beta, (float2*)out);
   TLGB_CHECK_LAUNCH();
   return TLGB_OK;
