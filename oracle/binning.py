@@ -99,12 +99,13 @@ def plan_pairs(locs: torch.Tensor, grid_size, width, kernel: str = "kaiser_besse
     return keys[order], pts[order]
 
 
-def block_pairs(locs: torch.Tensor, grid_size, width, kernel: str = "kaiser_bessel", pad_mode: str = "circular"):
+def block_pairs(locs: torch.Tensor, grid_size, width, kernel: str = "kaiser_bessel", pad_mode: str = "circular", rows: int = 2):
     """(keys, entries) of the block lists: every (point, block) pair for
     blocks of 4 x 4 x 4 cells (3D) or 8 x 8 cells (2D), sorted by block key
     and, within a block, by point index; entries as stored by the plan (point
-    index and the block's index per internal dim; a 2D grid's leading
-    internal dim has one block)."""
+    index and the block's index per internal dim, a bit each above bit 29, or
+    with 3 ``rows`` per dim its three base-3 digits above bit 27; a 2D grid's
+    leading internal dim has one block)."""
     nd = len(grid_size)
     assert nd in (2, 3)
     N = (1,) * (3 - nd) + tuple(int(n) for n in grid_size)
@@ -146,9 +147,10 @@ def block_pairs(locs: torch.Tensor, grid_size, width, kernel: str = "kaiser_bess
                 m = ok & (b0 >= 0) & (b1 >= 0) & (b2 >= 0)
                 keys.append(((b0 * nb[1] + b1) * nb[2] + b2)[m])
                 pts.append(pidx[m])
-                sels.append(torch.full((int(m.sum()),), i0 | i1 << 1 | i2 << 2, dtype=torch.int64))
+                sel = 9 * i0 + 3 * i1 + i2 if rows == 3 else i0 | i1 << 1 | i2 << 2
+                sels.append(torch.full((int(m.sum()),), sel, dtype=torch.int64))
     keys = torch.cat(keys).numpy()
     pts = torch.cat(pts).numpy()
     sels = torch.cat(sels).numpy()
     order = np.lexsort((pts, keys))  # by block, then by point
-    return keys[order], pts[order] | (sels[order] << 29)
+    return keys[order], pts[order] | (sels[order] << (27 if rows == 3 else 29))
