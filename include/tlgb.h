@@ -140,6 +140,21 @@ typedef struct tlgb_interp_plan_info {
  * scratch buffers are 16-byte aligned (cudaMalloc gives 256). */
 int tlgb_interp_plan_size(const tlgb_interp_desc* d, size_t* plan_bytes, size_t* tmp_bytes);
 
+/* The same for points whose (point, block) pairs were counted: a circular grid
+ * whose extents are no multiples of the block edge, or a wide 3D kernel, can have
+ * 27 of them per point, and tlgb_interp_plan_size leaves room for so many, where
+ * points spread over the grid have about 5 (or 12). tlgb_interp_plan_count counts
+ * them (one pass over locs, 8 bytes of 8-byte aligned device memory in `counter`;
+ * synchronises `stream`); *blk_entries = -1 where a plan has at most 8 per point
+ * and counting saves nothing. Sizes and build take that count, -1 for none, and
+ * the build fails with TLGB_ERR_INVALID when its points have more. */
+int tlgb_interp_plan_count(const tlgb_interp_desc* d, const float* locs, void* counter, int64_t* blk_entries,
+                           tlgb_stream_t stream);
+int tlgb_interp_plan_size_counted(const tlgb_interp_desc* d, int64_t blk_entries, size_t* plan_bytes, size_t* tmp_bytes);
+int tlgb_interp_plan_build_counted(const tlgb_interp_desc* d, int64_t blk_entries, const float* locs, void* plan,
+                                   size_t plan_bytes, void* tmp, size_t tmp_bytes, tlgb_interp_plan_info* info,
+                                   tlgb_stream_t stream);
+
 /* Bin the points: sort (point, tile) pairs by output tile (stable, so points
  * keep their original order inside a tile) and cut the work into items of at
  * most `chunk` pairs. Everything is built on the device; `stream` is

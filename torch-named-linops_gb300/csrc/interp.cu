@@ -894,11 +894,13 @@ __device__ __forceinline__ uint4 cta_scan4(uint4 v, uint4& tot) {
   return make_uint4(base.x + x.x - v.x, base.y + x.y - v.y, base.z + x.z - v.z, base.w + x.w - v.w);
 }
 
-// CTA j scans job j's n CTA sums in place (exclusive); totals to tot[0..3].
+// CTA j scans job j's n CTA sums in place (exclusive); totals to tot[0..3]. With
+// `most_y` > 0, totals of y above it are cut to it and tot[3] is set.
 struct ScanJob {
   uint4* sums;
   long long n;
   uint32_t* tot;
+  uint32_t most_y;
 };
 __global__ void __launch_bounds__(1024) plan_scan_kernel(ScanJob j0, ScanJob j1, ScanJob j2) {
   const ScanJob j = blockIdx.x == 2 ? j2 : (blockIdx.x ? j1 : j0);
@@ -916,6 +918,7 @@ __global__ void __launch_bounds__(1024) plan_scan_kernel(ScanJob j0, ScanJob j1,
     j.sums[i] = run;
     run.x += v.x, run.y += v.y, run.z += v.z, run.w += v.w;
   }
+  if (j.most_y > 0 && tot.y > j.most_y) tot.y = j.most_y, tot.w = 1;
   if (threadIdx.x == 0) j.tot[0] = tot.x, j.tot[1] = tot.y, j.tot[2] = tot.z, j.tot[3] = tot.w;
 }
 
@@ -943,11 +946,13 @@ __device__ __forceinline__ uint4 win_pairs(const Geo& g, const int4& w) {
 // evaluated once and the rows are put together in shared memory, stored as
 // one contiguous run per CTA (evaluating every cell of every row in place
 // and storing them one by one took 47 us for 2^18 points in 3D).
-// NTM: taps evaluated per dim, at least the geometry's.
+// NTM: taps evaluated per dim, at least the geometry's. With `total` (and no
+// windows or sums) the block pairs are only counted.
 template <int NTM>
 __global__ void __launch_bounds__(kPlanPts) plan_points_kernel(Geo g, const float* __restrict__ locs,
                                                                int4* __restrict__ win, float* __restrict__ rows,
-                                                               uint4* __restrict__ sums) {
+                                                               uint4* __restrict__ sums,
+                                                               unsigned long long* __restrict__ total) {
   extern __shared__ __align__(16) float prow[];  // [points][row_floats], when rows are wanted
   const long long p0 = (long long)blockIdx.x * kPlanPts, p = p0 + threadIdx.x;
   const bool on = p < g.npts;
@@ -996,10 +1001,11 @@ __global__ void __launch_bounds__(kPlanPts) plan_points_kernel(Geo g, const floa
     if (e == 2) w4.z = st;
   }
   w4.w = ok ? cnts : 0;
-  if (on) win[p] = w4;
+  if (on && win) win[p] = w4;
   uint4 tot;
   cta_scan4<kPlanPts>(on ? win_pairs(g, w4) : make_uint4(0, 0, 0, 0), tot);  // its barriers also publish the rows
-  if (threadIdx.x == 0) sums[blockIdx.x] = tot;
+  if (threadIdx.x == 0 && sums) sums[blockIdx.x] = tot;
+  if (threadIdx.x == 0 && total) atomicAdd(total, (unsigned long long)tot.y);
   if (rows) {
     const long long n4 = min((long long)kPlanPts, g.npts - p0) * RF / 4;
     float4* dst = reinterpret_cast<float4*>(rows + p0 * RF);
@@ -1012,7 +1018,7 @@ __global__ void __launch_bounds__(kPlanPts) plan_emit_kernel(Geo g, const int4* 
                                                              const uint4* __restrict__ sums,
                                                              uint32_t* __restrict__ tkeys, int32_t* __restrict__ tvals,
                                                              uint32_t* __restrict__ bkeys,
-                                                             int32_t* __restrict__ bvals) {
+                                                             int32_t* __restrict__ bvals, uint32_t most_blk) {
   const long long p = (long long)blockIdx.x * kPlanPts + threadIdx.x;
   const int4 w = p < g.npts ? win[p] : make_int4(0, 0, 0, 0);
   uint4 tot;
@@ -1037,6 +1043,7 @@ __global__ void __launch_bounds__(kPlanPts) plan_emit_kernel(Geo g, const int4* 
   for (int i = 0; i < nc[0]; ++i)
     for (int j = 0; j < nc[1]; ++j)
       for (int k = 0; k < nc[2]; ++k) {
+        if (o >= most_blk) return;  // more pairs than the caller counted: refused at the end
         const uint32_t sel = g.nrow == 3 ? (uint32_t)(9 * i + 3 * j + k) : (uint32_t)(i | j << 1 | k << 2);
         bkeys[o] = ((uint32_t)l[0][i] * nb1 + (uint32_t)l[1][j]) * nb2 + (uint32_t)l[2][k];
         bvals[o] = (int32_t)((uint32_t)p | sel << sel_shift(g.nrow));
@@ -3190,17 +3197,15 @@ int max_blocks_per_dim(const Geo& g, int e) {
 int block_rows(const Geo& g) {
   if (g.ndim < 2 || g.norm != 1) return 0;
   int rows = 2;
-  int64_t per_point = 1;
   for (int e = 3 - g.ndim; e < 3; ++e) {
     if (g.NT[e] > 9) return 0;
     if (g.pad == TLGB_PAD_CIRCULAR && g.N[e] < g.NT[e] + block_edge(g.ndim, e) - 1) return 0;
     const int m = max_blocks_per_dim(g, e);
     if (m > 3) return 0;
     rows = std::max(rows, m);
-    per_point *= m;
   }
   const int64_t nb = (int64_t)blocks_along(g, 0) * blocks_along(g, 1) * blocks_along(g, 2);
-  if (nb >= (1ll << 31) || g.npts >= (1ll << sel_shift(rows)) || g.npts * per_point >= (1ll << 31)) return 0;
+  if (nb >= (1ll << 31) || g.npts >= (1ll << sel_shift(rows))) return 0;
   return rows;
 }
 
@@ -3314,7 +3319,9 @@ PlanUnits plan_units(const Geo& g, int64_t ntiles, bool blocks) {
   return U;
 }
 
-PlanLayout layout(const Geo& g) {
+// `pairs`: the (point, block) pairs of the plan's points, -1 = not counted (room
+// for as many as points can have). Without block lists when there are too many.
+PlanLayout layout(const Geo& g, int64_t pairs) {
   PlanLayout L;
   L.e_max = g.npts * max_tiles_per_dim(g, 0) * max_tiles_per_dim(g, 1) * max_tiles_per_dim(g, 2);
   L.ntiles = (int64_t)g.nt[0] * g.nt[1] * g.nt[2];
@@ -3337,9 +3344,10 @@ PlanLayout layout(const Geo& g) {
   }
   L.nblocks = L.eb_max = L.max_blk_items = L.max_blk_split = 0;
   L.off_blk_entries = L.off_blk_items = L.off_blk_split = L.off_blk_rows = 0;
-  if (g.nrow && g.npts > 0) {
+  const int64_t most = g.npts * max_blocks_per_dim(g, 0) * max_blocks_per_dim(g, 1) * max_blocks_per_dim(g, 2);
+  if (g.nrow && g.npts > 0 && (pairs >= 0 ? pairs : most) < (1ll << 31)) {
     L.nblocks = (int64_t)blocks_along(g, 0) * blocks_along(g, 1) * blocks_along(g, 2);
-    L.eb_max = g.npts * (int64_t)max_blocks_per_dim(g, 0) * max_blocks_per_dim(g, 1) * max_blocks_per_dim(g, 2);
+    L.eb_max = std::max<int64_t>(pairs >= 0 ? std::min(pairs, most) : most, 1);
     L.max_blk_items = L.nblocks + cdiv(L.eb_max, kBlkPart) + 1;
     L.max_blk_split = std::min(L.nblocks, L.eb_max / (kBlkPart + 1)) + 1;
     L.off_blk_entries = o;
@@ -3567,23 +3575,57 @@ int set_smem(F* kernel, size_t bytes) {
 
 using namespace tlgb;
 
-extern "C" int tlgb_interp_plan_size(const tlgb_interp_desc* d, size_t* plan_bytes, size_t* tmp_bytes) {
+extern "C" int tlgb_interp_plan_count(const tlgb_interp_desc* d, const float* locs, void* counter, int64_t* blk_entries,
+                                      tlgb_stream_t stream) {
   Geo g;
   TLGB_TRY(make_geo(d, g));
-  const PlanLayout L = layout(g);
-  if (std::max(L.e_max, L.eb_max) >= (1ll << 31)) TLGB_FAIL(TLGB_ERR_UNSUPPORTED, "too many points for one plan");
+  if (!blk_entries || !counter || (g.npts > 0 && !locs)) TLGB_FAIL(TLGB_ERR_INVALID, "null pointer");
+  if ((uintptr_t)counter & 7) TLGB_FAIL(TLGB_ERR_INVALID, "plan count: the counter must be 8-byte aligned");
+  *blk_entries = -1;
+  if (g.nrow != 3 || g.npts == 0) return TLGB_OK;
+  cudaStream_t s = (cudaStream_t)stream;
+  auto* total = static_cast<unsigned long long*>(counter);
+  TLGB_CUDA(cudaMemsetAsync(total, 0, 8, s));
+  const unsigned nb = (unsigned)cdiv(g.npts, kPlanPts);
+  (std::max(g.NT[0], std::max(g.NT[1], g.NT[2])) <= 5 ? plan_points_kernel<5> : plan_points_kernel<9>)<<<nb, kPlanPts, 0, s>>>(
+      g, locs, nullptr, nullptr, nullptr, total);
+  TLGB_CHECK_LAUNCH();
+  unsigned long long n = 0;
+  TLGB_CUDA(cudaMemcpyAsync(&n, total, 8, cudaMemcpyDeviceToHost, s));
+  TLGB_CUDA(cudaStreamSynchronize(s));
+  *blk_entries = (int64_t)n;
+  return TLGB_OK;
+}
+
+extern "C" int tlgb_interp_plan_size_counted(const tlgb_interp_desc* d, int64_t blk_entries, size_t* plan_bytes,
+                                             size_t* tmp_bytes) {
+  Geo g;
+  TLGB_TRY(make_geo(d, g));
+  const PlanLayout L = layout(g, blk_entries);
+  if (L.e_max >= (1ll << 31)) TLGB_FAIL(TLGB_ERR_UNSUPPORTED, "too many points for one plan");
   if (plan_bytes) *plan_bytes = (size_t)L.bytes;
   if (tmp_bytes) *tmp_bytes = (size_t)L.t_bytes;
   return TLGB_OK;
 }
 
+extern "C" int tlgb_interp_plan_size(const tlgb_interp_desc* d, size_t* plan_bytes, size_t* tmp_bytes) {
+  return tlgb_interp_plan_size_counted(d, -1, plan_bytes, tmp_bytes);
+}
+
 extern "C" int tlgb_interp_plan_build(const tlgb_interp_desc* d, const float* locs, void* plan, size_t plan_bytes,
                                       void* tmp, size_t tmp_bytes, tlgb_interp_plan_info* info,
                                       tlgb_stream_t stream) {
+  return tlgb_interp_plan_build_counted(d, -1, locs, plan, plan_bytes, tmp, tmp_bytes, info, stream);
+}
+
+extern "C" int tlgb_interp_plan_build_counted(const tlgb_interp_desc* d, int64_t blk_entries, const float* locs, void* plan,
+                                              size_t plan_bytes, void* tmp, size_t tmp_bytes, tlgb_interp_plan_info* info,
+                                              tlgb_stream_t stream) {
   Geo g;
   TLGB_TRY(make_geo(d, g));
-  const PlanLayout L = layout(g);
-  if (std::max(L.e_max, L.eb_max) >= (1ll << 31)) TLGB_FAIL(TLGB_ERR_UNSUPPORTED, "too many points for one plan");
+  const PlanLayout L = layout(g, blk_entries);
+  if (L.e_max >= (1ll << 31)) TLGB_FAIL(TLGB_ERR_UNSUPPORTED, "too many points for one plan");
+  if (L.nblocks == 0) g.nrow = 0;
   if (!info || !plan || !tmp || (g.npts > 0 && !locs)) TLGB_FAIL(TLGB_ERR_INVALID, "null pointer");
   if (plan_bytes < (size_t)L.bytes || tmp_bytes < (size_t)L.t_bytes) TLGB_FAIL(TLGB_ERR_WORKSPACE, "plan workspace too small");
   cudaStream_t s = (cudaStream_t)stream;
@@ -3623,15 +3665,16 @@ extern "C" int tlgb_interp_plan_build(const tlgb_interp_desc* d, const float* lo
     const int maxnt = std::max(g.NT[0], std::max(g.NT[1], g.NT[2]));
     auto points = [&](auto* k) -> int {
       TLGB_TRY(set_smem(k, sm));
-      k<<<nb, kPlanPts, sm, s>>>(g, locs, win, rows, sums);
+      k<<<nb, kPlanPts, sm, s>>>(g, locs, win, rows, sums, nullptr);
       TLGB_CHECK_LAUNCH();
       return TLGB_OK;
     };
     TLGB_TRY(maxnt <= 5 ? points(plan_points_kernel<5>) : (maxnt <= 9 ? points(plan_points_kernel<9>) : points(plan_points_kernel<NTMAX>)));
-    plan_scan_kernel<<<1, 1024, 0, s>>>({sums, (long long)nb, cnt}, {}, {});
+    plan_scan_kernel<<<1, 1024, 0, s>>>({sums, (long long)nb, cnt, blocks ? (uint32_t)L.eb_max : 0u}, {}, {});
     TLGB_CHECK_LAUNCH();
     plan_emit_kernel<<<nb, kPlanPts, 0, s>>>(g, win, sums, jobs[0].keys[0], jobs[0].vals[0],
-                                             blocks ? jobs[1].keys[0] : nullptr, blocks ? jobs[1].vals[0] : nullptr);
+                                             blocks ? jobs[1].keys[0] : nullptr, blocks ? jobs[1].vals[0] : nullptr,
+                                             (uint32_t)L.eb_max);
     TLGB_CHECK_LAUNCH();
     TLGB_TRY(radix_sort_jobs(jobs, njobs, s));
   }
@@ -3698,6 +3741,7 @@ extern "C" int tlgb_interp_plan_build(const tlgb_interp_desc* d, const float* lo
   uint32_t c[16];
   TLGB_CUDA(cudaMemcpyAsync(c, cnt, sizeof(c), cudaMemcpyDeviceToHost, s));
   TLGB_CUDA(cudaStreamSynchronize(s));
+  if (c[3]) TLGB_FAIL(TLGB_ERR_INVALID, "interp plan: the points have more (point, block) pairs than were counted");
   if ((int64_t)c[4] > L.max_fwd || (int64_t)c[5] > L.max_adj || (blocks && ((int64_t)c[8] > L.max_blk_items || (int64_t)c[10] > L.max_blk_split)))
     TLGB_FAIL(TLGB_ERR_DEVICE, "work list larger than its bound");
 

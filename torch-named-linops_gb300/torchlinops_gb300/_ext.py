@@ -150,6 +150,9 @@ _SIGNATURES = {
     "tlgb_test_skip_region_copy": ([ctypes.c_int32], ctypes.c_int),
     "tlgb_interp_plan_size": ([_P, _P, _P], ctypes.c_int),
     "tlgb_interp_plan_build": ([_P, _P, _P, ctypes.c_size_t, _P, ctypes.c_size_t, _P, _P], ctypes.c_int),
+    "tlgb_interp_plan_count": ([_P, _P, _P, ctypes.POINTER(ctypes.c_int64), _P], ctypes.c_int),
+    "tlgb_interp_plan_size_counted": ([_P, ctypes.c_int64, _P, _P], ctypes.c_int),
+    "tlgb_interp_plan_build_counted": ([_P, ctypes.c_int64, _P, _P, ctypes.c_size_t, _P, ctypes.c_size_t, _P, _P], ctypes.c_int),
     "tlgb_interp_adjoint_scratch_size": ([_P, _P, _P], ctypes.c_int),
     "tlgb_interp_forward": ([_P, _P, _P, _P, _P, _P, _P], ctypes.c_int),
     "tlgb_interp_forward_scratch_size": ([_P, _P, _P], ctypes.c_int),

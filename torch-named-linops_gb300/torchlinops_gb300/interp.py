@@ -45,6 +45,11 @@ __all__ = [
 
 _F32, _F32_BITS = struct.Struct("f"), struct.Struct("i")
 
+# Plans of more points have their (point, block) pairs counted before their memory
+# is allocated, where the bound is far from the count: one more pass and
+# synchronisation (about 40 us) against up to 500 MB at this many points
+COUNT_POINTS = 1 << 19
+
 # Maximum kernel width per dimension handled by the CUDA kernels
 MAX_WIDTH_1D_2D = 15.0
 MAX_WIDTH_3D = 8.0
@@ -126,21 +131,25 @@ class InterpolatePlan:
         # 2D and 3D plans also hold each point's tap weights, so they are built for one (kernel, norm, beta)
         d = _desc(ndim, self.grid_size, self.width, kernel, self.norm, pad_mode, self.beta, False, 1, self.npts)
         L = _ext.lib()
-        pb, tb = ctypes.c_size_t(0), ctypes.c_size_t(0)
-        _ext.check(L.tlgb_interp_plan_size(ctypes.byref(d), ctypes.byref(pb), ctypes.byref(tb)), "plan size")
-        self.buffer = torch.empty(max(pb.value, 1), dtype=torch.uint8, device=dev)
-        tmp = torch.empty(max(tb.value, 1), dtype=torch.uint8, device=dev)
-        self.info = _ext.PlanInfo()
+        pb, tb, pairs = ctypes.c_size_t(0), ctypes.c_size_t(0), ctypes.c_int64(-1)
         with torch.cuda.device(dev):
             st = _ext.stream_ptr(dev)
+            if self.npts > COUNT_POINTS:
+                counter = torch.empty(1, dtype=torch.int64, device=dev)
+                _ext.check(L.tlgb_interp_plan_count(ctypes.byref(d), _ext.ptr(locs_c), _ext.ptr(counter), ctypes.byref(pairs), st),
+                           "plan count")
+            _ext.check(L.tlgb_interp_plan_size_counted(ctypes.byref(d), pairs, ctypes.byref(pb), ctypes.byref(tb)), "plan size")
+            self.buffer = torch.empty(max(pb.value, 1), dtype=torch.uint8, device=dev)
+            tmp = torch.empty(max(tb.value, 1), dtype=torch.uint8, device=dev)
+            self.info = _ext.PlanInfo()
             _ext.check(
-                L.tlgb_interp_plan_build(
-                    ctypes.byref(d), _ext.ptr(locs_c), _ext.ptr(self.buffer), pb.value, _ext.ptr(tmp), tb.value,
+                L.tlgb_interp_plan_build_counted(
+                    ctypes.byref(d), pairs, _ext.ptr(locs_c), _ext.ptr(self.buffer), pb.value, _ext.ptr(tmp), tb.value,
                     ctypes.byref(self.info), st,
                 ),
                 "interpolation plan",
             )
-            # the build's last kernels are still in flight on this stream
+            # the build has ended: it reads its lists' lengths back
             self.stream = torch.cuda.current_stream(dev)
             self._raw_stream = self.stream.cuda_stream
             self.ready = torch.cuda.Event()
