@@ -492,17 +492,19 @@ __global__ void __launch_bounds__(NW * 32, fwd_ctas(N, NDIM, NTB, NW))
   const int cgp = CG <= 1 ? 1 : (CG <= 2 ? 2 : (CG <= 4 ? 4 : 8));
   const int lgc = lg2i(cgp);
   const int rowlen = S[2] * cgp;
+  constexpr bool MANY = NW == 8;  // a loop over items costs the 16-warp kernel half its speed (registers)
   int staged = -1;
-  const int last = min(nitems, ((int)blockIdx.x + 1) * per);
-  for (int item = blockIdx.x * per; item < last; ++item) {
+  int item = MANY ? blockIdx.x * per : blockIdx.x;
+  const int last = min(nitems, item + per);
+  do {
     const int4 it = items[item];
-    if (it.x != staged) {
+    if (!MANY || it.x != staged) {
       int t = it.x;
       o[2] = t % g.nt[2] * g.T[2];
       t /= g.nt[2];
       o[1] = t % g.nt[1] * g.T[1];
       o[0] = t / g.nt[1] * g.T[0];
-      if (staged >= 0) __syncthreads();  // the tile before has been read
+      if (MANY && staged >= 0) __syncthreads();  // the tile before has been read
       for (int row = warp; row < S[0] * S[1]; row += NW) {
         const int x = row / S[1], y = row - x * S[1];
         int gx = o[0] + x, gy = o[1] + y;
@@ -612,7 +614,7 @@ __global__ void __launch_bounds__(NW * 32, fwd_ctas(N, NDIM, NTB, NW))
       }
       __syncwarp();
     }
-  }
+  } while (MANY && ++item < last);
 }
 
 // ------------------------------------------------------------------ adjoint
