@@ -14,6 +14,7 @@
 
 #include <algorithm>
 #include <string>
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -296,10 +297,11 @@ __global__ void __launch_bounds__(256, adj_ctas(sizeof(T), U)) index_adj_kernel(
 }
 
 // The same on grids whose cells hold several samples, a cell per thread with K
-// values read ahead. The line is at one sample per cell, with K = 4 up to four:
-// 2^22 samples on 160^3 take 71 us for 2 entries and 262 for 8 (through shared
-// memory 91 and 384), 2^23 of 8 entries 398 (463 with K = 8, but 1.45 ms against
-// 2.65 where they crowd into few cells). 20 entries of 320^2 at 2^20 samples: 89 us.
+// values read ahead. The line is at one sample per cell: 2^22 complex64 samples on
+// 160^3 take 71 us for 2 entries and 262 for 8 (through shared memory 91 and 384).
+// K is 4, and 8 from two samples per cell on (complex64: from four): 8 entries at
+// 2^23 samples 308 us with 8 and 316 with 4 (float32), 369 and 399 (int64), 463 and
+// 398 (complex64). 20 entries of 320^2 at 2^20 samples: 89 us.
 // 16-byte values, which fill the shared memory and the registers, cross over at a
 // quarter sample and prefer K = 2: 2 entries of 160^3 at 2^20, 2^21 and 2^22 samples
 // 82, 110 and 165 us, 4 entries a CTA through shared memory 149, 233 and 432, one
@@ -340,7 +342,7 @@ void launch_index_adj(const IdxGeo& g, const void* vals, const int32_t* perm, co
     else launch_index_adj_at<T, 2, 4>(g, vals, perm, off, out, s);
   } else {
     const int64_t want = 4ll * sm_count(), groups = cdiv(g.nbatch, 4);
-    if (g.npts >= 4 * g.ncells) launch_index_adj_dense<T, 8>(g, vals, perm, off, out, s);
+    if (g.npts >= (std::is_same<T, float2>::value ? 4 : 2) * g.ncells) launch_index_adj_dense<T, 8>(g, vals, perm, off, out, s);
     else if (g.npts >= g.ncells) launch_index_adj_dense<T, 4>(g, vals, perm, off, out, s);
     else if (g.nbatch > 1 && cdiv(g.ncells, 1024) * groups >= want) launch_index_adj_at<T, 4, 4>(g, vals, perm, off, out, s);
     else if (g.nbatch == 1 && cdiv(g.ncells, 1024) >= want) launch_index_adj_at<T, 1, 4>(g, vals, perm, off, out, s);
