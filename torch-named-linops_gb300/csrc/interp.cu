@@ -4290,37 +4290,30 @@ namespace {
 // The buffer's device address differs per CUDA context: the primary context
 // of each device, and any context a caller made itself with the driver API
 // (FFI hosts often do). The address is looked up once per context, with that
-// context current, and remembered; the first lookup in a context may load the
-// module there, which is when the buffer is allocated on that GPU.
+// context current, and remembered by the context's id (its handle may be given
+// again, to a context in which the buffer lies elsewhere); the first lookup in a
+// context may load the module there, which is when the buffer is allocated on
+// that GPU.
 std::mutex g_fixed_mu;
-std::vector<std::pair<CUcontext, void*>> g_fixed_addr;
+std::vector<std::pair<unsigned long long, void*>> g_fixed_addr;
 
 // Device address of the fixed buffer in the current context.
 int fixed_scratch_address(void** out) {
-  CtxGetCurrentFn get = ctx_get_current();
-  if (!get) TLGB_FAIL(TLGB_ERR_CUDA, "cuCtxGetCurrent is not available from the driver");
-  CUcontext ctx = nullptr;
-  if (get(&ctx) != CUDA_SUCCESS) TLGB_FAIL(TLGB_ERR_CUDA, "cuCtxGetCurrent failed");
+  unsigned long long ctx = context_id();
   std::lock_guard<std::mutex> lock(g_fixed_mu);
-  if (ctx != nullptr)
-    for (const auto& e : g_fixed_addr)
-      if (e.first == ctx) {
-        *out = e.second;
-        return TLGB_OK;
-      }
-  // with no context current, this first runtime call makes the current
-  // device's primary context current on this thread
-  void* p = nullptr;
-  TLGB_CUDA(cudaGetSymbolAddress(&p, g_adjoint_fixed_scratch));
-  if (ctx == nullptr && (get(&ctx) != CUDA_SUCCESS || ctx == nullptr))
-    TLGB_FAIL(TLGB_ERR_CUDA, "no current CUDA context");
   for (const auto& e : g_fixed_addr)
-    if (e.first == ctx) {
+    if (ctx != 0 && e.first == ctx) {
       *out = e.second;
       return TLGB_OK;
     }
-  g_fixed_addr.emplace_back(ctx, p);
-  *out = p;
+  // with no context current, this first runtime call makes the current
+  // device's primary context current on this thread
+  TLGB_CUDA(cudaGetSymbolAddress(out, g_adjoint_fixed_scratch));
+  if (ctx == 0) ctx = context_id();
+  if (ctx == 0) return TLGB_OK;  // looked up again on the next call
+  for (const auto& e : g_fixed_addr)
+    if (e.first == ctx) return TLGB_OK;
+  g_fixed_addr.emplace_back(ctx, *out);
   return TLGB_OK;
 }
 
