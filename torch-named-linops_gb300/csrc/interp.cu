@@ -1042,10 +1042,13 @@ __global__ void __launch_bounds__(kPlanPts) plan_emit_kernel(Geo g, const int4* 
   for (int e = 0; e < 3; ++e) nc[e] = axis_blocks(g, e, win_st(w, e), win_cnt(w, e), l[e]);
   const uint32_t nb1 = (uint32_t)blocks_along(g, 1), nb2 = (uint32_t)blocks_along(g, 2);
   o = base.y + x.y;
+  if (o + nc[0] * nc[1] * nc[2] > most_blk) {  // more pairs than the caller counted: refused at the end
+    for (; o < most_blk; ++o) bkeys[o] = 0u, bvals[o] = (int32_t)p;
+    return;
+  }
   for (int i = 0; i < nc[0]; ++i)
     for (int j = 0; j < nc[1]; ++j)
       for (int k = 0; k < nc[2]; ++k) {
-        if (o >= most_blk) return;  // more pairs than the caller counted: refused at the end
         const uint32_t sel = g.nrow == 3 ? (uint32_t)(9 * i + 3 * j + k) : (uint32_t)(i | j << 1 | k << 2);
         bkeys[o] = ((uint32_t)l[0][i] * nb1 + (uint32_t)l[1][j]) * nb2 + (uint32_t)l[2][k];
         bvals[o] = (int32_t)((uint32_t)p | sel << sel_shift(g.nrow));
