@@ -897,7 +897,7 @@ __device__ __forceinline__ uint4 cta_scan4(uint4 v, uint4& tot) {
 }
 
 // CTA j scans job j's n CTA sums in place (exclusive); totals to tot[0..3]. With
-// `most_y` > 0, totals of y above it are cut to it and tot[3] is set.
+// `most_y` > 0, a total of y above it becomes 0 and tot[3] is set.
 struct ScanJob {
   uint4* sums;
   long long n;
@@ -920,7 +920,7 @@ __global__ void __launch_bounds__(1024) plan_scan_kernel(ScanJob j0, ScanJob j1,
     j.sums[i] = run;
     run.x += v.x, run.y += v.y, run.z += v.z, run.w += v.w;
   }
-  if (j.most_y > 0 && tot.y > j.most_y) tot.y = j.most_y, tot.w = 1;
+  if (j.most_y > 0 && tot.y > j.most_y) tot.y = 0, tot.w = 1;
   if (threadIdx.x == 0) j.tot[0] = tot.x, j.tot[1] = tot.y, j.tot[2] = tot.z, j.tot[3] = tot.w;
 }
 
@@ -1042,10 +1042,7 @@ __global__ void __launch_bounds__(kPlanPts) plan_emit_kernel(Geo g, const int4* 
   for (int e = 0; e < 3; ++e) nc[e] = axis_blocks(g, e, win_st(w, e), win_cnt(w, e), l[e]);
   const uint32_t nb1 = (uint32_t)blocks_along(g, 1), nb2 = (uint32_t)blocks_along(g, 2);
   o = base.y + x.y;
-  if (o + nc[0] * nc[1] * nc[2] > most_blk) {  // more pairs than the caller counted: refused at the end
-    for (; o < most_blk; ++o) bkeys[o] = 0u, bvals[o] = (int32_t)p;
-    return;
-  }
+  if (o + nc[0] * nc[1] * nc[2] > most_blk) return;  // more pairs than the caller counted: refused, the list is left empty
   for (int i = 0; i < nc[0]; ++i)
     for (int j = 0; j < nc[1]; ++j)
       for (int k = 0; k < nc[2]; ++k) {

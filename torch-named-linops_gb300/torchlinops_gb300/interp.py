@@ -49,6 +49,7 @@ _F32, _F32_BITS = struct.Struct("f"), struct.Struct("i")
 # is allocated, where the bound is far from the count: one more pass and
 # synchronisation (about 40 us) against up to 500 MB at this many points
 COUNT_POINTS = 1 << 19
+COUNT_TMP = {1: 0, 2: 130, 3: 230}  # bytes of temporary space per point: 116 and 218 with 4 and 8 pairs per point, 166 to 454 with 9 and 27
 
 # Maximum kernel width per dimension handled by the CUDA kernels
 MAX_WIDTH_1D_2D = 15.0
@@ -134,11 +135,12 @@ class InterpolatePlan:
         pb, tb, pairs = ctypes.c_size_t(0), ctypes.c_size_t(0), ctypes.c_int64(-1)
         with torch.cuda.device(dev):
             st = _ext.stream_ptr(dev)
-            if self.npts > COUNT_POINTS:
+            _ext.check(L.tlgb_interp_plan_size(ctypes.byref(d), ctypes.byref(pb), ctypes.byref(tb)), "plan size")
+            if self.npts > COUNT_POINTS and tb.value > COUNT_TMP[ndim] * self.npts:
                 counter = torch.empty(1, dtype=torch.int64, device=dev)
                 _ext.check(L.tlgb_interp_plan_count(ctypes.byref(d), _ext.ptr(locs_c), _ext.ptr(counter), ctypes.byref(pairs), st),
                            "plan count")
-            _ext.check(L.tlgb_interp_plan_size_counted(ctypes.byref(d), pairs, ctypes.byref(pb), ctypes.byref(tb)), "plan size")
+                _ext.check(L.tlgb_interp_plan_size_counted(ctypes.byref(d), pairs, ctypes.byref(pb), ctypes.byref(tb)), "plan size")
             self.buffer = torch.empty(max(pb.value, 1), dtype=torch.uint8, device=dev)
             tmp = torch.empty(max(tb.value, 1), dtype=torch.uint8, device=dev)
             self.info = _ext.PlanInfo()
