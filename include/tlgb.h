@@ -231,7 +231,8 @@ int tlgb_interp_adjoint_fixed(const tlgb_interp_desc* d, const tlgb_interp_plan_
                               const float* locs, const void* vals, void* grid, tlgb_stream_t stream);
 
 /* Scratch bytes tlgb_interp_grad_locs can use to split a batch of many
- * coil groups over several CTAs per tile (0 when it would not split). */
+ * coil groups over several CTAs per tile and, for 2D points in random order, to
+ * hold their values point by point (0 when it would do neither). */
 int tlgb_interp_grad_scratch_size(const tlgb_interp_desc* d, const tlgb_interp_plan_info* info, size_t* bytes);
 
 /* grad_locs[p, e] = sum_b Re( conj(a[b, p]) * sum_taps dw(p, tap)/dx_e * grid[b, tap] )

@@ -8,28 +8,24 @@
 // kaiser_bessel_torch kernels.py:28-89) operation for operation in float32.
 //
 // Design (GB300 first, not a translation of the Triton programs):
-//  * Plan (once per trajectory): every point is paired with each output tile
-//    its valid taps touch; the pairs are sorted by tile with a stable LSD
-//    radix sort, "home" pairs (the tile holding the point's first valid tap)
-//    first. Work items are chunks of at most `chunk` pairs of one tile, so
-//    dense k-space centres are spread over many CTAs.
-//  * Forward (gather): a CTA stages its tile plus the kernel halo for a group
-//    of up to 8 batch entries in shared memory ([x][y][z][batch] order, batch
-//    fastest) and each warp interpolates one home point at a time; lanes are
-//    (tap along the last dim, batch entry) so one warp load reads 4 taps x 8
-//    entries = 256 contiguous bytes, conflict-free.
-//  * Adjoint (scatter, deterministic, no global atomics): output-stationary.
-//    A CTA owns one output tile in shared memory and visits every point whose
-//    window touches it, in plan order. Warp w owns the tile planes with
-//    (outer index) % 8 == w, so every shared-memory cell is updated by one
-//    fixed warp in one fixed order: results are bit-identical run to run.
-//    Each tile is written to HBM exactly once. Tiles denser than `chunk`
-//    pairs are split: each part writes a partial tile to scratch and a second
-//    kernel sums the parts in order.
-//  * Kernel values are evaluated directly with the reference's A&S formula
-//    (expf/sqrtf, IEEE division), not from a lookup table: a table would add
-//    an interpolation error on top of the 1e-5 budget, and the 3 x (W+1)
-//    evaluations per point visit are shared by every batch entry of the visit.
+//  * Plan (once per trajectory, built on the device): every point is paired with
+//    each output tile that its valid taps touch, "home" pairs (the tile holding
+//    the first of them) first, and, for separable complex 2D and 3D geometries,
+//    with each output block; both lists are sorted by a stable radix sort and cut
+//    into work items. Such a plan also holds the points' tap weights: records in
+//    the gather's order and rows over the blocks.
+//  * Ungridding of complex values (gather_kernel): persistent CTAs whose producer
+//    warps fill a ring of tile regions, a group of batch entries each, while the
+//    consumer warps interpolate the tile's home points from the records.
+//  * Gridding of complex values (adj_b3_kernel, adj_bn_kernel): a warp owns an
+//    output block in registers and adds the entries of the block's list in order
+//    as rank-8 updates on the tensor cores. Deterministic, no global atomics: every
+//    cell is summed by one warp in plan order and written once; dense blocks are
+//    split, their parts added in order by a second kernel.
+//  * Real values, the radial norm, 1D and the widest kernels run on one-tile CTAs
+//    (interp_fwd_kernel, interp_adj_kernel) that evaluate the weights themselves,
+//    by the reference's A&S formula; nothing reads the kernel from a lookup table,
+//    which would add an interpolation error on top of the 1e-5 budget.
 
 #include <algorithm>
 #include <atomic>
@@ -764,12 +760,7 @@ __global__ void __launch_bounds__(32) interp_adj_kernel(Geo g, const int4* __res
   }
 }
 
-// ----------------------------------------- unrolled kernels of the 3D default
-//
-// 3D grids, 8^3 tiles, widths in (3, 4] (5 tap slots, <= 4 kept for
-// non-integer coordinates), 8 complex batch entries per CTA: the benchmark
-// configuration and the NUFFT default. Each point's taps are packed into a
-// 64-byte record read with vector loads; tap offsets are compile-time.
+// ------------------------------------------------ weights held by the plan
 
 // The weight of a tap at normalised offset d = diff / r for the plan's
 // records and rows, close to the float32 rounding of the A&S value in 64
@@ -1479,8 +1470,9 @@ struct ChunkStream {
 };
 
 // x = hi + lo: hi the nearest tf32 value, lo the rest (exact; the tensor
-// cores read its upper 11 bits). With cvt.rna (ties away) and a rounded lo the
-// gridding issued 45 warp instructions per (point, block) entry, 32 so; hi
+// cores cut it to its upper 11 bits: an operand is up to 2^-21 off, 2^-22 with a
+// rounded lo). With cvt.rna (ties away) and a rounded lo the gridding issued 45 warp
+// instructions per (point, block) entry, 32 so (before the chunk stream); hi
 // cut instead of rounded would bias every sum by 1.5e-7 (lo would have the
 // sign of x, and the bits dropped from it would add up).
 __device__ __forceinline__ void split_tf32(float x, unsigned& hi, unsigned& lo) {
@@ -3904,7 +3896,7 @@ int region_map(const Geo& g, const void* grid, int edge, int cg, CUtensorMap& tm
 }
 
 // A unit is an item and `run` groups: all of them (an item's records are
-// fetched once) unless that leaves fewer than 6 units per CTA.
+// fetched once) unless that leaves fewer than 24 units per CTA.
 template <int NDIM, int KT, int CG, int NW, int NST, int CTAS>
 int launch_gather(const Geo& g, const tlgb_interp_plan_info* info, const char* P, const float* locs, const void* grid,
                   void* out, cudaStream_t s, float* sorted = nullptr) {
